@@ -466,354 +466,359 @@ __global__ void k_ref_drag(int n, const __grid_constant__ RefBind b) {
 // ---------------------------------------------------------------------------
 // particle operators (explicit schedule)
 // ---------------------------------------------------------------------------
-// 27-cell traversal in the reference order: k outer, j, i inner; particles of a
-// cell in sorted order; neighbours whose out_id (indexed by sorted position, as in
-// the reference) is negative are skipped.
-// LE: neighbours at distance <= re (the temperature operator), else < re.
+// Neighbours of a target: the particles of its 27 cells, k outer, j, i inner, a cell's
+// in sorted order, closer than re (the temperature operator: at most re); particles whose
+// out_id (indexed by sorted position, as in the reference) is negative are skipped.
 // Screen: ref_sqrt never returns less than sqrt(x) (1 - 3e-7) (its Newton step from
 // below gives y <= 1/sqrt(x), the float roundings cost a few ulps), so a finite squared
 // distance >= re^2 (1 + 1e-5) is rejected by the reference's own test and is skipped
 // before the square root; the others take the reference's arithmetic unchanged
 // (+inf is not screened: the reference's sqrt of it is -0, which it accepts).
 __device__ __forceinline__ float ref_screen2(float re) { return re * re * 1.00001f; }
-template <bool LE, class F>
-__device__ __forceinline__ void ref_candidate(int x, const Scalar3& tp, const Scalar3& q, float re, float re2x, float mind,
-                                              F& f) {
-    const float dx = tp.x - q.x, dy = tp.y - q.y, dz = tp.z - q.z;
-    const float d2 = dx * dx + dy * dy + dz * dz;   // ref_dist's sum (no contraction in this file)
-    if (d2 >= re2x && d2 <= 3.402823466e38f) return;
-    float d = ref_sqrt(d2);
-    if (!(LE ? d <= re : d < re)) return;
-    if (d < mind) d = mind;
-    f(x, d, q);
-}
-template <bool LE = false, class F>
-__device__ __forceinline__ void ref_neighbours(const RefBind& b, int id, const Scalar3& tp, int cx, int cy, int cz,
-                                               float re, F&& f) {
-    const float mind = (float)(re * 1e-3);
-    const float re2x = ref_screen2(re);
-    for (int k = -1; k <= 1; ++k)
-        for (int j = -1; j <= 1; ++j)
-            for (int i = -1; i <= 1; ++i) {
-                const int m = cell_key(b.box.m_GridSize, cx + i, cy + j, cz + k);
-                if (m < 0 || m >= b.cell_num) continue;
-                const int s = b.cell_start[m];
-                if (s == -1) continue;
-                const int e = b.cell_end[m];
-                for (int x = s; x < e; ++x) {
-                    if (b.out_id[x] < 0) continue;
-                    if (x == id) continue;
-                    ref_candidate<LE>(x, tp, b.pos[x], re, re2x, mind, f);
-                }
-            }
-}
 
-// CalcExplicitly_Kernel (DeviceProcess_Kernel.h:390-582) for target id; nb(tp, cx, cy,
-// cz, re, f) runs the neighbour traversal
-template <class Nb>
-__device__ __forceinline__ void ref_explicitly_body(const RefBind& b, int id, Nb&& nb) {
-    const CParameter& P = b.param;
-    const int orig = b.id[id];
-    const Scalar3 tp = b.pos[id];
-    if (!in_zone<float>(b.box, tp.x, tp.y, tp.z, P.Tolerance)) {
-        b.out_id[orig] = -1;
-        b.out_solid_rate[orig] = 9999;
-        return;
+}  // namespace mps
+#include "ref_pairs.cuh"
+namespace mps {
+
+// Before and after the pair sums of one operator, run by the target's own lane.
+// begin: false if the target is done (outside the compute zone, or without a cell where
+// the operator needs one); `walk` says whether it has neighbours to sum.
+template <class Op>
+struct RefOp;
+
+// CalcExplicitly_Kernel (DeviceProcess_Kernel.h:390-582)
+template <>
+struct RefOp<RpExplicitly> {
+    static __device__ __forceinline__ float radius(const CParameter& P) {
+        return P.LaplacianInfluenceRadiusCoefficient * P.InitialParticleDistance;
     }
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, tp, cx, cy, cz);
-    Scalar3 lap = s3(0, 0, 0), art = s3(0, 0, 0), col = s3(0, 0, 0);
-    Scalar3 v0 = b.vel[id];
-    Scalar3 tke = s3(0, 0, 0);
-    const float re = P.LaplacianInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    const float rc = P.r_coeff * P.InitialParticleDistance;
-    const float reg = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    const bool ep = P.bExplicitPressure;
-    const bool turb = P.bTurbulance;
-    if (cid >= 0 && cid < b.cell_num) {
-        nb(tp, cx, cy, cz, re, [&](int x, float d, const Scalar3& q) {
-            const float w = weight(re, d);
-            const Scalar3 v1 = b.vel[x];
-            lap.x += (v1.x - v0.x) * w;
-            lap.y += (v1.y - v0.y) * w;
-            lap.z += (v1.z - v0.z) * w;
-            // turbulent kinetic energy gradient (:477-485)
-            if (turb && d < reg) {
-                const float w1 = weight(reg, d);
-                const float sc = (b.strain[x] - b.strain[id]) * w1 / (d * d);
-                tke = s3add(tke, s3mul(s3sub(q, tp), sc));
-            }
-            if (ep && d < rc) {
-                const float a = P.ArtificialPressure * w / (d * d);
-                art = s3add(art, s3mul(s3sub(q, tp), a));
-                const float c = (rc - d) / d;
-                col = s3add(col, s3mul(s3sub(q, tp), c));
-            }
-        });
+    static __device__ __forceinline__ bool begin(const RefBind& b, int id, RpTarget& t, int& cx, int& cy, int& cz,
+                                                 bool& walk) {
+        if (!in_zone<float>(b.box, t.pos.x, t.pos.y, t.pos.z, b.param.Tolerance)) {
+            const int orig = b.id[id];
+            b.out_id[orig] = -1;
+            b.out_solid_rate[orig] = 9999;
+            return false;
+        }
+        t.vel = b.vel[id];
+        t.s = b.param.bTurbulance ? b.strain[id] : 0.0f;
+        const int cid = ref_cell(b.box, t.pos, cx, cy, cz);
+        walk = cid >= 0 && cid < b.cell_num;
+        return true;
     }
-    const float wd = b.stl_distance[id].Magnitude;
-    const int tri = b.stl_id[id];
-    if (tri >= 0 && tri < b.triangle_num && wd > 0 && wd < re) {
-        const float ww = ref_zlap(P.Dimension, wd, P.InitialParticleDistance);
-        const Scalar3 v1 = b.tri_params[b.triangles[tri].ModelIDNumber].Velocity;
-        lap.x += P.WallFrictionCoeffieicnt * (v1.x - v0.x) * ww;
-        lap.y += P.WallFrictionCoeffieicnt * (v1.y - v0.y) * ww;
-        lap.z += P.WallFrictionCoeffieicnt * (v1.z - v0.z) * ww;
+    // coef = (float)(2 Dimension / (double)(lambda n0)), from the host
+    static __device__ __forceinline__ void finish(const RefBind& b, int id, const RpTarget& t, const float (&sum)[3],
+                                                  const float (&rare)[9], float coef) {
+        const CParameter& P = b.param;
+        const int orig = b.id[id];
+        const Scalar3 tp = t.pos;
+        Scalar3 v0 = t.vel;
+        Scalar3 lap = s3(sum[0], sum[1], sum[2]);
+        const Scalar3 art = s3(rare[0], rare[1], rare[2]), col = s3(rare[3], rare[4], rare[5]);
+        const float re = radius(P);
+        const float wd = b.stl_distance[id].Magnitude;
+        const int tri = b.stl_id[id];
+        if (tri >= 0 && tri < b.triangle_num && wd > 0 && wd < re) {
+            const float ww = ref_zlap(P.Dimension, wd, P.InitialParticleDistance);
+            const Scalar3 v1 = b.tri_params[b.triangles[tri].ModelIDNumber].Velocity;
+            lap.x += P.WallFrictionCoeffieicnt * (v1.x - v0.x) * ww;
+            lap.y += P.WallFrictionCoeffieicnt * (v1.y - v0.y) * ww;
+            lap.z += P.WallFrictionCoeffieicnt * (v1.z - v0.z) * ww;
+        }
+        lap.x *= coef; lap.y *= coef; lap.z *= coef;
+        Scalar3 dragv = s3(0, 0, 0);
+        Scalar3 acc = s3add(s3(0, 0, 0), P.GravityConstant);
+        if (b.drag_num > 0) dragv = b.drag_acc[id];
+        // laminar + turbulent viscosity (:545-552)
+        lap = s3mul(lap, P.bTurbulance ? b.kin_visc[id] + b.turb_visc[id] : b.kin_visc[id]);
+        acc = s3add(acc, lap);
+        v0 = s3sub(s3add(v0, s3mul(acc, P.Dt)), dragv);
+        if (P.bTurbulance) {
+            // (2/3) is the integer quotient 0 in the reference (:560): the term vanishes
+            const Scalar3 tke = s3mul(s3(rare[6], rare[7], rare[8]), (float)(2 / 3));
+            v0 = s3sub(v0, s3mul(tke, P.Dt));
+        }
+        if (P.bExplicitPressure) {
+            const float c = (float)(-P.Dimension) / (P.ConstantParticleDensity * P.Density);
+            acc = s3add(s3mul(art, c), s3mul(col, (float)0.01));
+            v0 = s3add(v0, s3mul(acc, P.Dt));
+        }
+        if (isfinite(v0.x) && isfinite(v0.y) && isfinite(v0.z)) {
+            b.out_pos[orig] = s3(tp.x + P.Dt * v0.x, tp.y + P.Dt * v0.y, tp.z + P.Dt * v0.z);
+            b.out_vel[orig] = v0;
+        }
     }
-    const float coef = (float)((2.0 * P.Dimension) / (double)(P.LambdaValue * P.ConstantParticleDensity));
-    lap.x *= coef; lap.y *= coef; lap.z *= coef;
-    Scalar3 dragv = s3(0, 0, 0);
-    Scalar3 acc = s3add(s3(0, 0, 0), P.GravityConstant);
-    if (b.drag_num > 0) dragv = b.drag_acc[id];
-    // laminar + turbulent viscosity (:545-552)
-    lap = s3mul(lap, turb ? b.kin_visc[id] + b.turb_visc[id] : b.kin_visc[id]);
-    acc = s3add(acc, lap);
-    v0 = s3sub(s3add(v0, s3mul(acc, P.Dt)), dragv);
-    if (turb) {
-        // (2/3) is the integer quotient 0 in the reference (:560): the term vanishes
-        tke = s3mul(tke, (float)(2 / 3));
-        v0 = s3sub(v0, s3mul(tke, P.Dt));
-    }
-    if (ep) {
-        const float c = (float)(-P.Dimension) / (P.ConstantParticleDensity * P.Density);
-        acc = s3add(s3mul(art, c), s3mul(col, (float)0.01));
-        v0 = s3add(v0, s3mul(acc, P.Dt));
-    }
-    if (isfinite(v0.x) && isfinite(v0.y) && isfinite(v0.z)) {
-        b.out_pos[orig] = s3(tp.x + P.Dt * v0.x, tp.y + P.Dt * v0.y, tp.z + P.Dt * v0.z);
-        b.out_vel[orig] = v0;
-    }
-}
+};
 
 // CalcTemperatureFactor_Kernel (DeviceProcess_Kernel.h:705-852): conduction over the
 // neighbours within the temperature radius (distance <= re), the nearest wall through
 // its gradient Z function, the drag heating; each sum counted only above FLT_EPSILON
 // in magnitude; clamped; viscosity linear in the temperature (original index)
-__global__ void k_ref_temperature(int n, const __grid_constant__ RefBind b) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const CParameter& P = b.param;
-    const float rho = P.Density;
-    const float ecoef = P.Dt * 2 * P.Dimension / (P.ConstantParticleDensity * rho * P.FruidSpecificHeat);
-    float hf = 0.0f, hw = 0.0f;
-    const float ret = P.TemperatureInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    const Scalar3 tp = b.pos[id];
-    float tt = b.temperature[id];
-    const int orig = b.id[id];
-    if (!in_zone<float>(b.box, tp.x, tp.y, tp.z, P.Tolerance)) {
-        b.out_id[orig] = -1;
-        return;
+template <>
+struct RefOp<RpTemperature> {
+    static __device__ __forceinline__ float radius(const CParameter& P) {
+        return P.TemperatureInfluenceRadiusCoefficient * P.InitialParticleDistance;
     }
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, tp, cx, cy, cz);
-    if (cid < 0 || cid >= b.cell_num) return;
-    ref_neighbours<true>(b, id, tp, cx, cy, cz, ret, [&](int x, float d, const Scalar3&) {
-        const float num = (b.temperature[x] - tt) * weight(ret, d);
-        const float den = d * d * (1 / P.FruidThermalConductivity + P.FruidThermalResistance / d);
-        hf += num / den;
-    });
-    const float wd = b.stl_distance[id].Magnitude;
-    const int tri = b.stl_id[id];
-    if (tri >= 0 && tri < b.triangle_num && wd > 0 && wd < ret) {
-        const CTriangleParameters& tq = b.tri_params[b.triangles[tri].ModelIDNumber];
-        const float res = tq.WallThermalResistivity;
-        const float cond = (2 * P.FruidThermalConductivity * tq.WallThermalConductivity) /
-                           (P.FruidThermalConductivity + tq.WallThermalConductivity);
-        const float ww = ref_zgrad(P.Dimension, wd, P.InitialParticleDistance);
-        const float num = (tq.Temperature - tt) * ww;
-        const float den = wd * wd * (1 / cond + res / wd);
-        hw = num / den;
+    static __device__ __forceinline__ bool begin(const RefBind& b, int id, RpTarget& t, int& cx, int& cy, int& cz,
+                                                 bool& walk) {
+        if (!in_zone<float>(b.box, t.pos.x, t.pos.y, t.pos.z, b.param.Tolerance)) {
+            b.out_id[b.id[id]] = -1;
+            return false;
+        }
+        t.s = b.temperature[id];
+        const int cid = ref_cell(b.box, t.pos, cx, cy, cz);
+        return walk = cid >= 0 && cid < b.cell_num;
     }
-    if (b.drag_num > 0) tt += b.drag_temperature[id];
-    float comb = 0.0f;
-    if (fabsf(hf) > FLT_EPSILON) comb += hf;
-    if (fabsf(hw) > FLT_EPSILON) comb += hw;
-    tt += (ecoef * (comb));
-    if (tt > P.MaxWallTemperature) tt = P.MaxWallTemperature;
-    if (tt < P.MinWallTemperature) tt = P.MinWallTemperature;
-    b.out_temperature[orig] = tt;
-    b.out_kin_visc[orig] = P.ViscosityUpdateParameterA * tt + P.ViscosityUpdateParameterB;
-}
+    static __device__ __forceinline__ void finish(const RefBind& b, int id, const RpTarget& t, const float (&sum)[1],
+                                                  const float (&)[1], float) {
+        const CParameter& P = b.param;
+        const int orig = b.id[id];
+        const float ecoef = P.Dt * 2 * P.Dimension / (P.ConstantParticleDensity * P.Density * P.FruidSpecificHeat);
+        const float ret = radius(P), hf = sum[0];
+        float tt = t.s, hw = 0.0f;
+        const float wd = b.stl_distance[id].Magnitude;
+        const int tri = b.stl_id[id];
+        if (tri >= 0 && tri < b.triangle_num && wd > 0 && wd < ret) {
+            const CTriangleParameters& tq = b.tri_params[b.triangles[tri].ModelIDNumber];
+            const float res = tq.WallThermalResistivity;
+            const float cond = (2 * P.FruidThermalConductivity * tq.WallThermalConductivity) /
+                               (P.FruidThermalConductivity + tq.WallThermalConductivity);
+            const float ww = ref_zgrad(P.Dimension, wd, P.InitialParticleDistance);
+            const float num = (tq.Temperature - tt) * ww;
+            const float den = wd * wd * (1 / cond + res / wd);
+            hw = num / den;
+        }
+        if (b.drag_num > 0) tt += b.drag_temperature[id];
+        float comb = 0.0f;
+        if (fabsf(hf) > FLT_EPSILON) comb += hf;
+        if (fabsf(hw) > FLT_EPSILON) comb += hw;
+        tt += (ecoef * (comb));
+        if (tt > P.MaxWallTemperature) tt = P.MaxWallTemperature;
+        if (tt < P.MinWallTemperature) tt = P.MinWallTemperature;
+        b.out_temperature[orig] = tt;
+        b.out_kin_visc[orig] = P.ViscosityUpdateParameterA * tt + P.ViscosityUpdateParameterB;
+    }
+};
 
 // CalcTurbulenceViscosity_Kernel (DeviceProcess_Kernel.h:1273-1476): velocity gradient
 // tensor within the gradient radius, strain-rate product, wall-damped Smagorinsky
 // viscosity (capped) and turbulent kinetic energy (capped), sorted order.  The
 // kernel's vorticity and PND are never read and are left out.
-__global__ void k_ref_turbulence(int n, const __grid_constant__ RefBind b) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const CParameter& P = b.param;
-    const int orig = b.id[id];
-    const Scalar3 tp = b.pos[id];
-    const Scalar3 v0 = b.vel[id];
-    if (!in_zone<float>(b.box, tp.x, tp.y, tp.z, P.Tolerance)) {
-        b.turb_visc[id] = 0.0f;
-        b.out_id[orig] = -1;
-        return;
+template <>
+struct RefOp<RpTurbulence> {
+    static __device__ __forceinline__ float radius(const CParameter& P) {
+        return P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
     }
-    Scalar3 X = s3(0, 0, 0), Y = s3(0, 0, 0), Z = s3(0, 0, 0), D = s3(0, 0, 0);
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, tp, cx, cy, cz);
-    if (cid < 0 || cid >= b.cell_num) {
-        b.pressure[id] = 0.0f;
-        return;
+    static __device__ __forceinline__ bool begin(const RefBind& b, int id, RpTarget& t, int& cx, int& cy, int& cz,
+                                                 bool& walk) {
+        if (!in_zone<float>(b.box, t.pos.x, t.pos.y, t.pos.z, b.param.Tolerance)) {
+            b.turb_visc[id] = 0.0f;
+            b.out_id[b.id[id]] = -1;
+            return false;
+        }
+        t.vel = b.vel[id];
+        const int cid = ref_cell(b.box, t.pos, cx, cy, cz);
+        if (cid < 0 || cid >= b.cell_num) {
+            b.pressure[id] = 0.0f;
+            return false;
+        }
+        return walk = true;
     }
-    const float re = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    ref_neighbours(b, id, tp, cx, cy, cz, re, [&](int x, float d, const Scalar3& q) {
-        const float w = weight(re, d);
-        const Scalar3 v1 = b.vel[x];
-        X.x += ((v1.x - v0.x) * (q.x - tp.x) * w) / (d * d);
-        X.y += ((v1.x - v0.x) * (q.y - tp.y) * w) / (d * d);
-        X.z += ((v1.x - v0.x) * (q.z - tp.z) * w) / (d * d);
-        Y.x += ((v1.y - v0.y) * (q.x - tp.x) * w) / (d * d);
-        Y.y += ((v1.y - v0.y) * (q.y - tp.y) * w) / (d * d);
-        Y.z += ((v1.y - v0.y) * (q.z - tp.z) * w) / (d * d);
-        Z.x += ((v1.z - v0.z) * (q.x - tp.x) * w) / (d * d);
-        Z.y += ((v1.z - v0.z) * (q.y - tp.y) * w) / (d * d);
-        Z.z += ((v1.z - v0.z) * (q.z - tp.z) * w) / (d * d);
-    });
-    const float g = P.Dimension / P.ConstantParticleDensity;
-    X.x = g * X.x; X.y = g * X.y; X.z = g * X.z;
-    Y.x = g * Y.x; Y.y = g * Y.y; Y.z = g * Y.z;
-    Z.x = g * Z.x; Z.y = g * Z.y; Z.z = g * Z.z;
-    D.x = (float)(0.5 * (X.y + Y.x));
-    D.y = (float)(0.5 * (X.z + Z.x));
-    D.z = (float)(0.5 * (Y.z + Z.y));
-    const float strain = X.x * X.x + Y.y * Y.y + Z.z * Z.z + 2 * D.x * D.x + 2 * D.y * D.y + 2 * D.z * D.z;
-    const float riw = b.stl_distance[id].Magnitude;
-    const float ratio = -(riw / re);
-    const float damp = 1 - expf(ratio);
-    const float smag = P.SmagorinskyConstant * damp;
-    const float coef = (smag * P.FilterWidth) * (smag * P.FilterWidth);
-    float tv = 0;
-    if (strain > 0) tv = coef * sqrtf(2 * strain);
-    if (tv > P.TurbulanViscosityRatio) tv = P.TurbulanViscosityRatio;
-    b.turb_visc[id] = tv;
-    const float tkc = 2 * P.Cnue * P.InitialParticleDistance * P.InitialParticleDistance / P.Cepsilon;
-    float tke = strain * tkc;
-    if (tke > P.TurbulanceIntensity) tke = P.TurbulanceIntensity;
-    b.strain[id] = tke;
-}
+    static __device__ __forceinline__ void finish(const RefBind& b, int id, const RpTarget&, const float (&sum)[9],
+                                                  const float (&)[1], float) {
+        const CParameter& P = b.param;
+        Scalar3 X = s3(sum[0], sum[1], sum[2]), Y = s3(sum[3], sum[4], sum[5]), Z = s3(sum[6], sum[7], sum[8]), D;
+        const float re = radius(P);
+        const float g = P.Dimension / P.ConstantParticleDensity;
+        X.x = g * X.x; X.y = g * X.y; X.z = g * X.z;
+        Y.x = g * Y.x; Y.y = g * Y.y; Y.z = g * Y.z;
+        Z.x = g * Z.x; Z.y = g * Z.y; Z.z = g * Z.z;
+        D.x = (float)(0.5 * (X.y + Y.x));
+        D.y = (float)(0.5 * (X.z + Z.x));
+        D.z = (float)(0.5 * (Y.z + Z.y));
+        const float strain = X.x * X.x + Y.y * Y.y + Z.z * Z.z + 2 * D.x * D.x + 2 * D.y * D.y + 2 * D.z * D.z;
+        const float riw = b.stl_distance[id].Magnitude;
+        const float ratio = -(riw / re);
+        const float damp = 1 - expf(ratio);
+        const float smag = P.SmagorinskyConstant * damp;
+        const float coef = (smag * P.FilterWidth) * (smag * P.FilterWidth);
+        float tv = 0;
+        if (strain > 0) tv = coef * sqrtf(2 * strain);
+        if (tv > P.TurbulanViscosityRatio) tv = P.TurbulanViscosityRatio;
+        b.turb_visc[id] = tv;
+        const float tkc = 2 * P.Cnue * P.InitialParticleDistance * P.InitialParticleDistance / P.Cepsilon;
+        float tke = strain * tkc;
+        if (tke > P.TurbulanceIntensity) tke = P.TurbulanceIntensity;
+        b.strain[id] = tke;
+    }
+};
 
 // CalcExplicitPressure_Kernel (DeviceProcess_Kernel.h:921-1054)
-template <class Nb>
-__device__ __forceinline__ void ref_pressure_body(const RefBind& b, int id, Nb&& nb) {
-    const CParameter& P = b.param;
-    const int orig = b.id[id];
-    const Scalar3 tp = b.pos[id];
-    if (!in_zone<float>(b.box, tp.x, tp.y, tp.z, P.Tolerance)) {
-        b.out_id[orig] = -1;
-        b.pressure[id] = 0.0f;
-        return;
+template <>
+struct RefOp<RpPressure> {
+    static __device__ __forceinline__ float radius(const CParameter& P) {
+        return P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
     }
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, tp, cx, cy, cz);
-    if (cid < 0 || cid >= b.cell_num) {
-        b.pressure[id] = 0.0f;
-        return;
+    static __device__ __forceinline__ bool begin(const RefBind& b, int id, RpTarget& t, int& cx, int& cy, int& cz,
+                                                 bool& walk) {
+        if (!in_zone<float>(b.box, t.pos.x, t.pos.y, t.pos.z, b.param.Tolerance)) {
+            b.out_id[b.id[id]] = -1;
+            b.pressure[id] = 0.0f;
+            return false;
+        }
+        const int cid = ref_cell(b.box, t.pos, cx, cy, cz);
+        if (cid < 0 || cid >= b.cell_num) {
+            b.pressure[id] = 0.0f;
+            return false;
+        }
+        return walk = true;
     }
-    const float re = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    const float coef = P.SonicVelocity * P.SonicVelocity * P.Density / P.ConstantParticleDensity;
-    float dens = 0.0f;
-    nb(tp, cx, cy, cz, re, [&](int, float d, const Scalar3&) { dens += weight(re, d); });
-    const float riw = b.stl_distance[id].Magnitude;
-    float ww = 0.0f;
-    if (b.stl_id[id] >= 0 && b.stl_id[id] < b.triangle_num && riw >= 0 && riw <= re)
-        ww = ref_zgrad(P.Dimension, riw, P.InitialParticleDistance);
-    dens += ww;
-    if (isfinite(dens)) b.out_density[orig] = dens;
-    float pr = 0.0f;
-    if (dens > P.ConstantParticleDensity * P.FreeSurfaceThreshold) pr = coef * (dens - P.ConstantParticleDensity);
-    if (isfinite(pr)) {
-        b.out_pressure[orig] = pr;
-        b.pressure[id] = pr;
+    static __device__ __forceinline__ void finish(const RefBind& b, int id, const RpTarget&, const float (&sum)[1],
+                                                  const float (&)[1], float) {
+        const CParameter& P = b.param;
+        const int orig = b.id[id];
+        const float re = radius(P);
+        const float coef = P.SonicVelocity * P.SonicVelocity * P.Density / P.ConstantParticleDensity;
+        float dens = sum[0];
+        const float riw = b.stl_distance[id].Magnitude;
+        float ww = 0.0f;
+        if (b.stl_id[id] >= 0 && b.stl_id[id] < b.triangle_num && riw >= 0 && riw <= re)
+            ww = ref_zgrad(P.Dimension, riw, P.InitialParticleDistance);
+        dens += ww;
+        if (isfinite(dens)) b.out_density[orig] = dens;
+        float pr = 0.0f;
+        if (dens > P.ConstantParticleDensity * P.FreeSurfaceThreshold) pr = coef * (dens - P.ConstantParticleDensity);
+        if (isfinite(pr)) {
+            b.out_pressure[orig] = pr;
+            b.pressure[id] = pr;
+        }
     }
-}
+};
 
 // CalcExplicitPressureGradient_Kernel (DeviceProcess_Kernel.h:1056-1271), without
 // the negative-pressure branch.
-template <class Nb>
-__device__ __forceinline__ void ref_gradient_body(const RefBind& b, int id, Nb&& nb) {
-    const CParameter& P = b.param;
-    const int orig = b.id[id];
-    const Scalar3 tp = b.pos[id];
-    if (!in_zone<float>(b.box, tp.x, tp.y, tp.z, P.Tolerance)) {
-        b.out_id[orig] = -1;
-        return;
+template <>
+struct RefOp<RpGradient> {
+    static __device__ __forceinline__ float radius(const CParameter& P) {
+        return P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
     }
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, tp, cx, cy, cz);
-    if (cid < 0 || cid >= b.cell_num) return;
-    const float re = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
-    Scalar3 gf = s3(0, 0, 0), gw = s3(0, 0, 0);
-    const float tpress = b.pressure[id];
-    nb(tp, cx, cy, cz, re, [&](int x, float d, const Scalar3& q) {
-        const float pc = (float)(0.5 * (double)(b.pressure[x] + tpress) * (double)weight(re, d));
-        gf.x += pc * (q.x - tp.x) / (d * d);
-        gf.y += pc * (q.y - tp.y) / (d * d);
-        gf.z += pc * (q.z - tp.z) / (d * d);
-    });
-    const float c1 = 2 * P.Dimension / (P.ConstantParticleDensity);
-    const float c2 = P.Density / (P.Dt * P.Dt);
-    const float c3 = -P.Dt / P.Density;
-    gf.x *= c1; gf.y *= c1; gf.z *= c1;
-    const CDistance riw = b.stl_distance[id];
-    if (b.stl_id[id] >= 0 && b.stl_id[id] < b.triangle_num) {
-        if (riw.Magnitude > 0 && riw.Magnitude <= re) {
-            const float ww = ref_z(c_zgrad3, 21, riw.Magnitude, P.InitialParticleDistance);
-            const float wc = (float)((((0.5 * (double)c1) * (double)ww) * (double)tpress) /
-                                     (double)(riw.Magnitude * riw.Magnitude));
-            gw = s3(wc * (-riw.Direction.x), wc * (-riw.Direction.y), wc * (-riw.Direction.z));
+    static __device__ __forceinline__ bool begin(const RefBind& b, int id, RpTarget& t, int& cx, int& cy, int& cz,
+                                                 bool& walk) {
+        if (!in_zone<float>(b.box, t.pos.x, t.pos.y, t.pos.z, b.param.Tolerance)) {
+            b.out_id[b.id[id]] = -1;
+            return false;
         }
-        if (riw.Magnitude > 0 && riw.Magnitude <= P.InitialParticleDistance * P.OffSet) {
-            const float dr = (P.InitialParticleDistance * P.OffSet - riw.Magnitude);
-            const float mc = c2 * dr / riw.Magnitude;
-            gw.x += mc * (-riw.Direction.x);
-            gw.y += mc * (-riw.Direction.y);
-            gw.z += mc * (-riw.Direction.z);
+        t.s = b.pressure[id];
+        const int cid = ref_cell(b.box, t.pos, cx, cy, cz);
+        return walk = cid >= 0 && cid < b.cell_num;
+    }
+    static __device__ __forceinline__ void finish(const RefBind& b, int id, const RpTarget& t, const float (&sum)[3],
+                                                  const float (&)[1], float) {
+        const CParameter& P = b.param;
+        const int orig = b.id[id];
+        const Scalar3 tp = t.pos;
+        const float re = radius(P), tpress = t.s;
+        Scalar3 gf = s3(sum[0], sum[1], sum[2]), gw = s3(0, 0, 0);
+        const float c1 = 2 * P.Dimension / (P.ConstantParticleDensity);
+        const float c2 = P.Density / (P.Dt * P.Dt);
+        const float c3 = -P.Dt / P.Density;
+        gf.x *= c1; gf.y *= c1; gf.z *= c1;
+        const CDistance riw = b.stl_distance[id];
+        if (b.stl_id[id] >= 0 && b.stl_id[id] < b.triangle_num) {
+            if (riw.Magnitude > 0 && riw.Magnitude <= re) {
+                const float ww = ref_z(c_zgrad3, 21, riw.Magnitude, P.InitialParticleDistance);
+                const float wc = (float)((((0.5 * (double)c1) * (double)ww) * (double)tpress) /
+                                         (double)(riw.Magnitude * riw.Magnitude));
+                gw = s3(wc * (-riw.Direction.x), wc * (-riw.Direction.y), wc * (-riw.Direction.z));
+            }
+            if (riw.Magnitude > 0 && riw.Magnitude <= P.InitialParticleDistance * P.OffSet) {
+                const float dr = (P.InitialParticleDistance * P.OffSet - riw.Magnitude);
+                const float mc = c2 * dr / riw.Magnitude;
+                gw.x += mc * (-riw.Direction.x);
+                gw.y += mc * (-riw.Direction.y);
+                gw.z += mc * (-riw.Direction.z);
+            }
+        }
+        const Scalar3 g = s3add(s3add(gf, gw), s3(0, 0, 0));
+        Scalar3 iv = s3(c3 * g.x, c3 * g.y, c3 * g.z);
+        if (isfinite(iv.x) && isfinite(iv.y) && isfinite(iv.z)) {
+            const Scalar3 v = b.vel[id];
+            Scalar3 ov = s3(v.x + iv.x, v.y + iv.y, v.z + iv.z);
+            // CorrectVelocity (Utility_Inline.h:2369-2396)
+            const float cmax = P.InitialParticleDistance * P.CourantNumber / P.Dt;
+            const float a = ref_sqrt(ov.x * ov.x + ov.y * ov.y + ov.z * ov.z);
+            if (a > cmax) ov = s3(cmax * ov.x / a, cmax * ov.y / a, cmax * ov.z / a);
+            b.out_vel[orig] = ov;
+            iv = s3(ov.x - v.x, ov.y - v.y, ov.z - v.z);
+            b.out_pos[orig] = s3(tp.x + iv.x * P.Dt, tp.y + iv.y * P.Dt, tp.z + iv.z * P.Dt);
         }
     }
-    const Scalar3 g = s3add(s3add(gf, gw), s3(0, 0, 0));
-    Scalar3 iv = s3(c3 * g.x, c3 * g.y, c3 * g.z);
-    if (isfinite(iv.x) && isfinite(iv.y) && isfinite(iv.z)) {
-        const Scalar3 v = b.vel[id];
-        Scalar3 ov = s3(v.x + iv.x, v.y + iv.y, v.z + iv.z);
-        // CorrectVelocity (Utility_Inline.h:2369-2396)
-        const float cmax = P.InitialParticleDistance * P.CourantNumber / P.Dt;
-        const float a = ref_sqrt(ov.x * ov.x + ov.y * ov.y + ov.z * ov.z);
-        if (a > cmax) ov = s3(cmax * ov.x / a, cmax * ov.y / a, cmax * ov.z / a);
-        b.out_vel[orig] = ov;
-        iv = s3(ov.x - v.x, ov.y - v.y, ov.z - v.z);
-        b.out_pos[orig] = s3(tp.x + iv.x * P.Dt, tp.y + iv.y * P.Dt, tp.z + iv.z * P.Dt);
+};
+
+// one operator over targets 0 .. n-1, T per warp
+template <class Op, int T>
+__global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::NS > 3 ? 5 : 7) k_ref_pairs(int n, float coef, float minus_zero, const __grid_constant__ RefBind b) {
+    using W = RpWarp<Op, T>;
+    __shared__ __align__(16) float sm[kRpWarps * W::kFloats];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = (blockIdx.x * kRpWarps + warp) * T;
+    if (first >= n) return;
+    const int id = first + lane;
+    RpTarget t{};
+    int cx = 0, cy = 0, cz = 0;
+    bool walk = false, fin = false;
+    if (lane < T && id < n) {
+        t.pos = b.pos[id];
+        fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
     }
+    W w(b, sm + warp * W::kFloats, RefOp<Op>::radius(b.param), minus_zero, first, t);
+    w.run(b, walk && fin, cx, cy, cz);
+    float sum[Op::NS], rare[W::NXR];
+#pragma unroll
+    for (int c = 0; c < Op::NS; ++c) sum[c] = w.sum(c);
+    if constexpr (Op::NX > 0) {
+#pragma unroll
+        for (int c = 0; c < Op::NX; ++c) rare[c] = w.rare_sum(c);
+    }
+    if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
-enum { REF_EXPLICITLY = 0, REF_PRESSURE = 1, REF_GRADIENT = 2 };
-template <int KIND, class Nb>
-__device__ __forceinline__ void ref_op_body(const RefBind& b, int id, Nb&& nb) {
-    if constexpr (KIND == REF_EXPLICITLY) ref_explicitly_body(b, id, nb);
-    else if constexpr (KIND == REF_PRESSURE) ref_pressure_body(b, id, nb);
-    else ref_gradient_body(b, id, nb);
-}
-// one thread per target, the traversal over global memory (the targets of a warp are
-// consecutive in the sorted order: mostly one cell, whose candidates they load together)
-template <int KIND>
-__global__ void k_ref_op(int n, const __grid_constant__ RefBind b) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    ref_op_body<KIND>(b, id, [&](const Scalar3& tp, int cx, int cy, int cz, float re, auto&& f) {
-        ref_neighbours(b, id, tp, cx, cy, cz, re, f);
-    });
+// the same, a lane per target
+template <class Op>
+__global__ void __launch_bounds__(128) k_ref_lanes(int n, float coef, float minus_zero, const __grid_constant__ RefBind b) {
+    const int id = blockIdx.x * 128 + threadIdx.x;
+    RpTarget t{};
+    int cx = 0, cy = 0, cz = 0;
+    bool walk = false, fin = false;
+    if (id < n) {
+        t.pos = b.pos[id];
+        fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
+    }
+    float sum[Op::NS], rare[RpShape<Op>::NXR];
+    rl_sums<Op>(b, t, n, id, walk && fin, cx, cy, cz, RefOp<Op>::radius(b.param), minus_zero, sum, rare);
+    if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
 inline int grid_of(int n) { return div_up(n, kBlock); }
 
-// the operator over targets 0 .. n-1
-template <int KIND>
-cudaError_t ref_op_launch(cudaStream_t st, int n) {
-    MPS_COUNT_LAUNCH k_ref_op<KIND><<<grid_of(n), kBlock, 0, st>>>(n, g_bind);
+// Targets per warp of an operator: kMany share each round's candidates; below `few` of
+// them that leaves too few warps per SM and two per warp finish sooner.  Measured in us,
+// two against kMany, on a jittered block: pressure 50 / 54 at 15,625 particles, 72 / 54
+// at 32,768; turbulence (9 sums, 4 per warp) 90 / 107 at 32,768, 297 / 296 at 103,823.
+template <class Op, int kMany>
+cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
+    if (n < few)
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, g_bind);
+    else
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f,
+                                                                                                        g_bind);
     return cudaGetLastError();
 }
+constexpr int kRefFew = 20000, kRefFewTurbulence = 100000;
+// From here on the predictor, whose radius is the cell size (250 of 1,728 candidates
+// accepted), runs a lane per target: 2.83 against 2.99 ms at 884,736 particles, 772
+// against 759 us at 216,000.  Its 16-byte loads need aligned arrays.
+constexpr int kRefLanes = 300000;
 
 CCTStatusType launch_status() { return cuda_status(cudaGetLastError()); }
 
@@ -1039,34 +1044,40 @@ CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
 CCTStatusType CalcExplicitly(cudaStream_t& Stream, Integer ParticleNum) {
     if (ParticleNum <= 0) return CCT_NOERR;
     if (g_bind.param.bTurbulance && (!g_bind.turb_visc || !g_bind.strain)) return CCT_PARAMERR;
-    MPS_CUDA_TRY(ref_op_launch<REF_EXPLICITLY>(Stream, ParticleNum));
+    const CParameter& P = g_bind.param;
+    const float coef = (float)((2.0 * P.Dimension) / (double)(P.LambdaValue * P.ConstantParticleDensity));
+    if (ParticleNum >= kRefLanes && (((uintptr_t)g_bind.pos | (uintptr_t)g_bind.out_id) & 15) == 0)
+        MPS_COUNT_LAUNCH k_ref_lanes<RpExplicitly><<<div_up(ParticleNum, 128), 128, 0, Stream>>>(ParticleNum, coef, -0.0f,
+                                                                                                  g_bind);
+    else
+        MPS_CUDA_TRY((ref_op_launch<RpExplicitly, 8>(Stream, ParticleNum, kRefFew, coef)));
     return launch_status();
 }
 
 CCTStatusType CalcExplicitPressure(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
-    MPS_CUDA_TRY(ref_op_launch<REF_PRESSURE>(Stream, ComputeParticleNum));
+    MPS_CUDA_TRY((ref_op_launch<RpPressure, 8>(Stream, ComputeParticleNum, kRefFew)));
     return launch_status();
 }
 
 CCTStatusType CalcExplicitPressureGradient(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (g_bind.param.bNegativePressure) return CCT_PARAMERR;
-    MPS_CUDA_TRY(ref_op_launch<REF_GRADIENT>(Stream, ComputeParticleNum));
+    MPS_CUDA_TRY((ref_op_launch<RpGradient, 8>(Stream, ComputeParticleNum, kRefFew)));
     return launch_status();
 }
 
 CCTStatusType CalcTemperatureFactor(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (!g_bind.temperature || !g_bind.out_temperature || !g_bind.out_kin_visc) return CCT_PARAMERR;
-    MPS_COUNT_LAUNCH k_ref_temperature<<<grid_of(ComputeParticleNum), kBlock, 0, Stream>>>(ComputeParticleNum, g_bind);
+    MPS_CUDA_TRY((ref_op_launch<RpTemperature, 8>(Stream, ComputeParticleNum, kRefFew)));
     return launch_status();
 }
 
 CCTStatusType CalcTurbulenceViscosity(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (!g_bind.turb_visc || !g_bind.strain) return CCT_PARAMERR;
-    MPS_COUNT_LAUNCH k_ref_turbulence<<<grid_of(ComputeParticleNum), kBlock, 0, Stream>>>(ComputeParticleNum, g_bind);
+    MPS_CUDA_TRY((ref_op_launch<RpTurbulence, 4>(Stream, ComputeParticleNum, kRefFewTurbulence)));
     return launch_status();
 }
 

@@ -1,0 +1,603 @@
+// ref_pairs.cuh - the pair sums of the reference-named particle operators.
+//
+// Include only from ref_kernels.cu (compiled without multiply-add contraction): the
+// sums below are the reference's, term by term and in its order (cells k outer, j, i
+// inner; a cell's particles in sorted order), so they round as its serial loops do.
+//
+// A warp owns T consecutive targets of the sorted order (mostly one cell's) and walks
+// the candidates of their 27 cells once for all of them:
+//   screen  32 candidates a round, a lane each; per target one squared distance, one
+//           ballot, and the accepted candidates appended to the target's queue in
+//           shared memory (rank within the ballot = traversal order);
+//   terms   when a queue could overflow: a lane per queued pair, so the square root,
+//           divisions and gathers run with full warps instead of under the union of 32
+//           targets' accepts;
+//   sums    a lane per (component, target) adds the queued terms one after another.
+// Adding +0 for a pair that the exact test then rejects leaves a sum's bits alone: a
+// sum that starts at +0 never becomes -0.
+//
+// What bounds it: instruction issue (per target about 560 warp instructions to walk the
+// cells, 17 per round of 32 candidates screened, 64 to 90 per 32 accepted pairs), the
+// screen's votes and population counts first.  A thread per target over global memory,
+// which this replaces, ran the terms of every candidate that any of its warp's 32 targets
+// accepted and left most of the chip idle below 100k particles.  Measured in us, before
+// and after: 15,625 particles pressure 312 / 50, heat 324 / 53, turbulence 414 / 62,
+// predictor 531 / 94; 103,823 pressure 334 / 137, gradient 462 / 177; 884,736 pressure
+// 1,520 / 1,040, gradient 2,450 / 1,370.
+#pragma once
+
+namespace mps {
+
+constexpr int kRpWarps = 4;        // warps per CTA
+constexpr int kRpCap = 64;         // queue entries per target: a round adds at most 32 to at most 32
+constexpr int kRpStride = 68;      // floats per queue row: 16-byte aligned, 17 16-byte units (odd: no bank conflicts)
+constexpr float kRpHuge = 1e18f;   // coordinates above it can overflow a squared distance
+
+// what a target brings to its pair terms
+struct RpTarget {
+    Scalar3 pos;
+    Scalar3 vel;
+    float s;      // scalar of the operator (pressure, temperature, strain)
+};
+
+// ---- operators: NS sums per target, NX sums over rarer pairs, terms and scalars ----
+struct RpExplicitly {
+    static constexpr int NS = 3, NX = 9;
+    static constexpr bool kLe = false, kPos = false, kVel = true, kScalar = false;
+    static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
+                                                 float (&v)[NS]) {
+        const float w = weight(re, d);
+        const Scalar3 v1 = b.vel[x];
+        v[0] = (v1.x - t.vel.x) * w;
+        v[1] = (v1.y - t.vel.y) * w;
+        v[2] = (v1.z - t.vel.z) * w;
+    }
+    // largest distance of a pair with a part in the other sums
+    static __device__ __forceinline__ float rare_radius(const CParameter& P) {
+        const float rc = P.r_coeff * P.InitialParticleDistance;
+        const float reg = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
+        return fmaxf(P.bExplicitPressure ? rc : 0.0f, P.bTurbulance ? reg : 0.0f);
+    }
+    static __device__ __forceinline__ void rare_terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
+                                                      float (&ex)[NX]) {
+        const CParameter& P = b.param;
+        const float rc = P.r_coeff * P.InitialParticleDistance;
+        const float reg = P.GradientInfluenceRadiusCoefficient * P.InitialParticleDistance;
+        const Scalar3 dq = s3sub(b.pos[x], t.pos);
+#pragma unroll
+        for (int c = 0; c < NX; ++c) ex[c] = 0.0f;
+        if (P.bExplicitPressure && d < rc) {
+            const Scalar3 a = s3mul(dq, P.ArtificialPressure * weight(re, d) / (d * d)), c = s3mul(dq, (rc - d) / d);
+            ex[0] = a.x; ex[1] = a.y; ex[2] = a.z;
+            ex[3] = c.x; ex[4] = c.y; ex[5] = c.z;
+        }
+        if (P.bTurbulance && d < reg) {   // turbulent kinetic energy gradient (:477-485)
+            const Scalar3 k = s3mul(dq, (b.strain[x] - t.s) * weight(reg, d) / (d * d));
+            ex[6] = k.x; ex[7] = k.y; ex[8] = k.z;
+        }
+    }
+};
+struct RpPressure {
+    static constexpr int NS = 1, NX = 0;
+    static constexpr bool kLe = false, kPos = false, kVel = false, kScalar = false;
+    static __device__ __forceinline__ void terms(const RefBind&, float re, const RpTarget&, int, float d,
+                                                 float (&v)[NS]) {
+        v[0] = weight(re, d);
+    }
+};
+struct RpGradient {
+    static constexpr int NS = 3, NX = 0;
+    static constexpr bool kLe = false, kPos = true, kVel = false, kScalar = true;
+    static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
+                                                 float (&v)[NS]) {
+        const Scalar3 q = b.pos[x];
+        const float s = b.pressure[x] + t.s, w = weight(re, d);
+        // the reference's (float)(0.5 * (double)s * (double)w): the double product is
+        // exact, so one float multiplication rounds alike wherever 0.5 s is exact
+        const float pc = (fabsf(s) < 1e-30f && s != 0.0f) ? (float)(0.5 * (double)s * (double)w) : (0.5f * s) * w;
+        v[0] = pc * (q.x - t.pos.x) / (d * d);
+        v[1] = pc * (q.y - t.pos.y) / (d * d);
+        v[2] = pc * (q.z - t.pos.z) / (d * d);
+    }
+};
+struct RpTemperature {
+    static constexpr int NS = 1, NX = 0;
+    static constexpr bool kLe = true, kPos = false, kVel = false, kScalar = true;
+    static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
+                                                 float (&v)[NS]) {
+        const CParameter& P = b.param;
+        const float num = (b.temperature[x] - t.s) * weight(re, d);
+        const float den = d * d * (1 / P.FruidThermalConductivity + P.FruidThermalResistance / d);
+        v[0] = num / den;
+    }
+};
+struct RpTurbulence {
+    static constexpr int NS = 9, NX = 0;
+    static constexpr bool kLe = false, kPos = true, kVel = true, kScalar = false;
+    static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
+                                                 float (&v)[NS]) {
+        const Scalar3 q = b.pos[x], v1 = b.vel[x];
+        const float w = weight(re, d), d2 = d * d;
+        const float du[3] = {v1.x - t.vel.x, v1.y - t.vel.y, v1.z - t.vel.z};
+        const float dx[3] = {q.x - t.pos.x, q.y - t.pos.y, q.z - t.pos.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[3 * a + c] = (du[a] * dx[c] * w) / d2;
+    }
+};
+
+// two single-precision lanes per instruction, each rounded as the scalar operation
+__device__ __forceinline__ unsigned long long rp_pack(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void rp_unpack(unsigned long long v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long rp_add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a * b as a * b + (-0), which rounds alike (and keeps the product's sign of zero).  ptxas
+// fuses a packed multiplication into a packed addition that follows it, whatever the
+// rounding modifiers and -fmad say, so nz = (-0, -0) has to come from the kernel's
+// arguments: a constant is folded away and the sum is fused all the same.
+__device__ __forceinline__ unsigned long long rp_mul2(unsigned long long a, unsigned long long b, unsigned long long nz) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+    return r;
+}
+
+template <class Op>
+struct RpShape {
+    static constexpr int NP = Op::NS > 2 ? Op::NS : 2;   // queue planes: squared distance and index, then terms
+    static constexpr int NXR = Op::NX > 0 ? Op::NX : 1;
+};
+
+// Pair sums of one warp's T targets.  Lane t < T holds target t (id = first + t): `live`,
+// its position and cell, its RpTarget.  Returns in lane t the NS sums and NX sums.
+template <class Op, int T>
+struct RpWarp {
+    static constexpr int NS = Op::NS, NX = Op::NX, NP = RpShape<Op>::NP, NXR = RpShape<Op>::NXR;
+    static constexpr int kQueue = NP * T * kRpStride;
+    // rarer pairs: sums of every target, then a queue of 64 (distance, index, target),
+    // whose first rows take the terms of 32 pairs
+    static constexpr int kRare = NX > 0 ? NX * T + 3 * 64 + NX * 32 : 0;
+    static constexpr int kFloats = kQueue + ((kRare + T + 3) & ~3);   // shared memory of a warp
+    static constexpr int NA = (NS * T + 31) / 32;                 // sums held per lane
+
+    float* sm;
+    float re, re2x, mind;
+    unsigned long long nz2;   // (-0, -0), see rp_mul2
+    int lane, first;
+    RpTarget me;        // lane t: target t
+    unsigned long long tx[T / 2], ty[T / 2], tz[T / 2];   // the group's targets, two a register pair
+    int cnt[T];
+    int rcnt;            // pairs in the queue of rarer pairs
+    float rare_re;
+    float acc[NA];
+
+    __device__ __forceinline__ RpWarp(const RefBind& b, float* smem, float radius, float minus_zero, int first_id, const RpTarget& t)
+        : sm(smem), re(radius), re2x(ref_screen2(radius)), mind((float)(radius * 1e-3)),
+          nz2(rp_pack(minus_zero, minus_zero)),
+          lane(threadIdx.x & 31), first(first_id), me(t) {
+#pragma unroll
+        for (int t_ = 0; t_ < T; ++t_) cnt[t_] = 0;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) acc[a] = 0.0f;
+        if constexpr (NX > 0) {
+            for (int i = lane; i < NX * T; i += 32) sm[kQueue + i] = 0.0f;
+        }
+        rcnt = 0;
+        rare_re = 0.0f;
+        if constexpr (NX > 0) rare_re = Op::rare_radius(b.param);
+        __syncwarp();
+    }
+
+    // candidate x of each lane against the targets of `um` (two at a time), the accepted
+    // ones queued; the target itself is dropped with the exact test
+    __device__ __forceinline__ void screen(int x, const Scalar3& q, unsigned um) {
+        const unsigned lt = (1u << lane) - 1u;
+        const unsigned long long nx = rp_pack(-q.x, -q.x), ny = rp_pack(-q.y, -q.y), nz = rp_pack(-q.z, -q.z);
+        constexpr int Q = 2;
+#pragma unroll
+        for (int t0 = 0; t0 < T; t0 += Q) {
+            if (!(um >> t0 & ((1u << Q) - 1u))) continue;
+            float d2[Q];
+#pragma unroll
+            for (int h = 0; h < Q; h += 2) {
+                const int p = (t0 + h) / 2;
+                const unsigned long long dx = rp_add2(tx[p], nx), dy = rp_add2(ty[p], ny), dz = rp_add2(tz[p], nz);
+                rp_unpack(rp_add2(rp_add2(rp_mul2(dx, dx, nz2), rp_mul2(dy, dy, nz2)), rp_mul2(dz, dz, nz2)), d2[h],
+                          d2[h + 1]);
+            }
+            unsigned m[Q];
+#pragma unroll
+            for (int h = 0; h < Q; ++h) m[h] = __ballot_sync(~0u, d2[h] < re2x);
+#pragma unroll
+            for (int h = 0; h < Q; ++h) {
+                const int t = t0 + h;
+                if (d2[h] < re2x) {
+                    float* const row = sm + t * kRpStride + cnt[t] + __popc(m[h] & lt);
+                    row[0] = d2[h];
+                    row[T * kRpStride] = __int_as_float(x);
+                }
+                cnt[t] += __popc(m[h]);
+            }
+        }
+    }
+    // the same against all of the group where a squared distance may overflow (the
+    // reference accepts an infinite one)
+    __device__ __forceinline__ void screen_all(int x, const Scalar3& q, unsigned grp) {
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const float dx = __shfl_sync(~0u, me.pos.x, t) - q.x, dy = __shfl_sync(~0u, me.pos.y, t) - q.y,
+                        dz = __shfl_sync(~0u, me.pos.z, t) - q.z;
+            const float d2 = dx * dx + dy * dy + dz * dz;
+            const bool hit = (grp >> t & 1u) && !(d2 >= re2x && d2 <= 3.402823466e38f);
+            const unsigned m = __ballot_sync(~0u, hit);
+            if (hit) {
+                float* const row = sm + t * kRpStride + cnt[t] + __popc(m & ((1u << lane) - 1u));
+                row[0] = d2;
+                row[T * kRpStride] = __int_as_float(x);
+            }
+            cnt[t] += __popc(m);
+        }
+    }
+
+    // Rarer pairs: a lane per pair computes the terms, then a lane per sum adds them in
+    // the order the pairs were queued.  Empties the queue (at most 64 pairs).
+    __device__ __forceinline__ void flush_rare(const RefBind& b) {
+        if constexpr (NX > 0) {
+            float* const xsum = sm + kQueue;
+            float* const q = xsum + NX * T;
+            float* const rows = q + 3 * 64;
+            __syncwarp();
+#pragma unroll 1
+            for (int e0 = 0; e0 < rcnt; e0 += 32) {
+                const int e = e0 + lane, k = min(rcnt - e0, 32);
+                const int t = lane < k ? __float_as_int(q[128 + e]) : 0;
+                RpTarget g;
+                g.pos.x = __shfl_sync(~0u, me.pos.x, t);
+                g.pos.y = __shfl_sync(~0u, me.pos.y, t);
+                g.pos.z = __shfl_sync(~0u, me.pos.z, t);
+                g.s = __shfl_sync(~0u, me.s, t);
+                if (lane < k) {
+                    float ex[NXR];
+                    Op::rare_terms(b, re, g, __float_as_int(q[64 + e]), q[e], ex);
+#pragma unroll
+                    for (int c = 0; c < NX; ++c) rows[lane * NX + c] = ex[c];
+                }
+                __syncwarp();
+                if (lane < NX)
+                    for (int r = 0; r < k; ++r) {
+                        float* const s = xsum + __float_as_int(q[128 + e0 + r]) * NX + lane;
+                        *s = *s + rows[r * NX + lane];
+                    }
+                __syncwarp();
+            }
+            rcnt = 0;
+        }
+    }
+
+    // queued pairs -> terms -> sums; empties the queues
+    __device__ __forceinline__ void flush(const RefBind& b) {
+        // entries of target t to lane t (through shared memory: selecting them by lane
+        // would put the counts into local memory)
+        int* const scnt = reinterpret_cast<int*>(sm + kQueue + kRare);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            if (lane == 0) scnt[t] = cnt[t];
+            cnt[t] = 0;
+        }
+        __syncwarp();
+        const int mine = lane < T ? scnt[lane] : 0;
+        // the queues as one sequence, target by target, 32 pairs a round
+        int end = mine;
+#pragma unroll
+        for (int o = 1; o < T; o <<= 1) {
+            const int v = __shfl_up_sync(~0u, end, o);
+            if (lane >= o) end += v;
+        }
+        const int total = __shfl_sync(~0u, end, T - 1), start = lane < T ? end - mine : 0x7fffffff;
+#pragma unroll 1
+        for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = e0 + lane;
+            int t = 0;   // the last target whose pairs start at or before e
+#pragma unroll
+            for (int o = T / 2; o > 0; o >>= 1) {
+                const int v = __shfl_sync(~0u, start, t + o);
+                if (v <= e) t += o;
+            }
+            float* const row = sm + t * kRpStride + (e - __shfl_sync(~0u, start, t));
+            RpTarget g;
+            if constexpr (Op::kPos) {
+                g.pos.x = __shfl_sync(~0u, me.pos.x, t);
+                g.pos.y = __shfl_sync(~0u, me.pos.y, t);
+                g.pos.z = __shfl_sync(~0u, me.pos.z, t);
+            }
+            if constexpr (Op::kVel) {
+                g.vel.x = __shfl_sync(~0u, me.vel.x, t);
+                g.vel.y = __shfl_sync(~0u, me.vel.y, t);
+                g.vel.z = __shfl_sync(~0u, me.vel.z, t);
+            }
+            if constexpr (Op::kScalar) g.s = __shfl_sync(~0u, me.s, t);
+            bool rare = false;
+            float d = 0.0f;
+            int x = 0;
+            if (e < total) {
+                float v[NS];
+#pragma unroll
+                for (int c = 0; c < NS; ++c) v[c] = 0.0f;
+                x = __float_as_int(row[T * kRpStride]);
+                d = ref_sqrt(row[0]);
+                const bool ok = (Op::kLe ? d <= re : d < re) && x != first + t;
+                if (d < mind) d = mind;
+                if (ok) Op::terms(b, re, g, x, d, v);
+                if constexpr (NX > 0) rare = ok && d < rare_re;
+#pragma unroll
+                for (int c = 0; c < NS; ++c) row[c * T * kRpStride] = v[c];
+            }
+            if constexpr (NX > 0) {
+                const unsigned m = __ballot_sync(~0u, rare);
+                if (m) {
+                    float* const q = sm + kQueue + NX * T + rcnt + __popc(m & ((1u << lane) - 1u));
+                    if (rare) {
+                        q[0] = d;
+                        q[64] = __int_as_float(x);
+                        q[128] = __int_as_float(t);
+                    }
+                    rcnt += __popc(m);
+                    if (rcnt > 32) flush_rare(b);
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const int l = a * 32 + lane, t = l % T;
+            const int n = __shfl_sync(~0u, mine, t);
+            if (l < NS * T) {
+                const float* const row = sm + ((l / T) * T + t) * kRpStride;
+                float s = acc[a];
+                int e = 0;
+                for (; e + 4 <= n; e += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(row + e);
+                    s += v.x;
+                    s += v.y;
+                    s += v.z;
+                    s += v.w;
+                }
+                for (; e < n; ++e) s += row[e];
+                acc[a] = s;
+            }
+        }
+        __syncwarp();
+    }
+
+    // bounds of the coordinates that truncate toward zero to cell index c
+    static __device__ __forceinline__ float low(int c, float cs) { return (float)(c <= 0 ? c - 1 : c) * cs; }
+    static __device__ __forceinline__ float high(int c, float cs) { return (float)(c >= 0 ? c + 1 : c) * cs; }
+
+    // position of candidate x < e (NaN, which no test accepts, where there is none)
+    static __device__ __forceinline__ Scalar3 fetch(const RefBind& b, int x, int e) {
+        const float nan = __int_as_float(0x7fffffff);
+        Scalar3 q = s3(nan, nan, nan);
+        if (x < e && b.out_id[x] >= 0) q = b.pos[x];
+        return q;
+    }
+
+    // Candidates of the targets `grp`, all in cell (cx, cy, cz).
+    __device__ __forceinline__ void walk(const RefBind& b, unsigned grp, int cx, int cy, int cz) {
+        const Integer3 G = b.box.m_GridSize;
+        const float cs = b.box.m_CellSize;
+        // lane m < 27: cell m of the traversal (k outer, j, i inner)
+        int s = 0, len = 0;
+        unsigned mask = 0;
+        const int i = lane % 3 - 1, j = (lane / 3) % 3 - 1, k = lane / 9 - 1;
+        if (grp && lane < 27) {
+            const int m = cell_key(G, (int)((unsigned)cx + (unsigned)i), (int)((unsigned)cy + (unsigned)j),
+                                   (int)((unsigned)cz + (unsigned)k));
+            if (m >= 0 && m < b.cell_num) {
+                s = b.cell_start[m];
+                if (s != -1) len = max(b.cell_end[m] - s, 0);
+            }
+            mask = grp;
+        }
+        // Targets that can have a neighbour in the cell: those within re of its box.  A
+        // particle within re <= cell size of a target lies in the box of the cell that its
+        // own indices give (ref_cell truncates toward zero, the box is widened by the
+        // rounding of that), and with at least 4 cells along y and z no other of the 27
+        // offsets shares that cell's key; elsewhere every target is tested.
+        const bool cull = G.y >= 4 && G.z >= 4 && re <= cs * 1.0001f && max(abs(cx), max(abs(cy), abs(cz))) < (1 << 20);
+        if (cull) {
+            const Scalar3 lo = b.box.m_BufferedZone.m_MinBound;
+            const float pad = cs * (1e-3f + 1e-6f * (float)(max(cx, max(cy, cz)) + 2));
+            const float x0 = low(cx + i, cs) - pad, x1 = high(cx + i, cs) + pad, y0 = low(cy + j, cs) - pad;
+            const float y1 = high(cy + j, cs) + pad, z0 = low(cz + k, cs) - pad, z1 = high(cz + k, cs) + pad;
+            unsigned near = 0;
+#pragma unroll 1
+            for (int t = 0; t < T; ++t) {
+                const float px = __shfl_sync(~0u, me.pos.x, t) - lo.x, py = __shfl_sync(~0u, me.pos.y, t) - lo.y,
+                            pz = __shfl_sync(~0u, me.pos.z, t) - lo.z;
+                const float ax = fmaxf(0.0f, fmaxf(x0 - px, px - x1)), ay = fmaxf(0.0f, fmaxf(y0 - py, py - y1)),
+                            az = fmaxf(0.0f, fmaxf(z0 - pz, pz - z1));
+                if (!(ax * ax + ay * ay + az * az > re2x)) near |= 1u << t;
+            }
+            mask &= near;
+        }
+        const bool far_target = __any_sync(~0u, lane < T && (grp >> lane & 1u) &&
+                                                    fmaxf(fabsf(me.pos.x), fmaxf(fabsf(me.pos.y), fabsf(me.pos.z))) > kRpHuge);
+        // targets of other cells: NaN, which no screen accepts
+        const float nan = __int_as_float(0x7fffffff);
+        const bool mine = lane < T && (grp >> lane & 1u);
+        const Scalar3 tp = mine ? me.pos : s3(nan, nan, nan);
+#pragma unroll
+        for (int p = 0; p < T / 2; ++p) {
+            tx[p] = rp_pack(__shfl_sync(~0u, tp.x, 2 * p), __shfl_sync(~0u, tp.x, 2 * p + 1));
+            ty[p] = rp_pack(__shfl_sync(~0u, tp.y, 2 * p), __shfl_sync(~0u, tp.y, 2 * p + 1));
+            tz[p] = rp_pack(__shfl_sync(~0u, tp.z, 2 * p), __shfl_sync(~0u, tp.z, 2 * p + 1));
+        }
+        // non-empty cells in order; after the last group one empty round, which flushes
+        // what is queued
+        unsigned cells = grp ? __ballot_sync(~0u, len > 0) : 1u;
+        const int limit = grp ? kRpCap - 32 : 0;
+        while (cells) {
+            const int m = __ffs(cells) - 1;
+            cells &= cells - 1u;
+            const int s0 = __shfl_sync(~0u, s, m), e = s0 + __shfl_sync(~0u, len, m);
+            const unsigned um = __shfl_sync(~0u, mask, m);
+            int x = s0 + lane;
+            Scalar3 q = fetch(b, x, e), qn;
+#pragma unroll 1
+            for (int r = s0;;) {
+                r += 32;
+                const bool more = r < e;
+                if (more) qn = fetch(b, x + 32, e);   // the next round's, before this one is screened
+                const bool huge = fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))) > kRpHuge;
+                if (far_target || __any_sync(~0u, huge)) screen_all(x, q, grp);
+                else if (um) screen(x, q, um);
+                int most = 0;
+#pragma unroll
+                for (int t = 0; t < T; ++t) most = max(most, cnt[t]);
+                if (most > limit) flush(b);
+                if (!more) break;
+                q = qn;
+                x += 32;
+            }
+        }
+    }
+
+    // all targets of the warp: `live` in lane t, its cell in (cx, cy, cz)
+    __device__ __forceinline__ void run(const RefBind& b, bool live, int cx, int cy, int cz) {
+        unsigned todo = __ballot_sync(~0u, live), grp = todo;
+        while (grp) {
+            const int l = todo ? __ffs(todo) - 1 : 0;
+            const int gx = __shfl_sync(~0u, cx, l), gy = __shfl_sync(~0u, cy, l), gz = __shfl_sync(~0u, cz, l);
+            grp = __ballot_sync(~0u, live && cx == gx && cy == gy && cz == gz) & todo;
+            walk(b, grp, gx, gy, gz);
+            todo &= ~grp;
+        }
+        flush_rare(b);
+    }
+    // sum c of this lane's target (lanes t < T; every lane calls it)
+    __device__ __forceinline__ float sum(int c) const {
+        const int l = c * T + (lane < T ? lane : 0);
+        float r = 0.0f;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const float v = __shfl_sync(~0u, acc[a], l & 31);
+            r = (l >> 5) == a ? v : r;
+        }
+        return r;
+    }
+    __device__ __forceinline__ float rare_sum(int c) const { return sm[kQueue + NX * (lane < T ? lane : 0) + c]; }
+};
+
+// A lane per target, each walking its own 27 cells: the candidates four at a time from
+// 16-byte loads (the lanes of a warp mostly share a cell, so one address), the next four
+// loaded before these are tested, an accepted pair's terms added at once.  It needs no
+// votes, ranks and second pass per pair, but runs the terms of every candidate that any
+// of 32 targets accepts, and has 1/32 warp per target: only for many accepted pairs per
+// candidate and many targets.
+template <class Op>
+__device__ __forceinline__ void rl_sums(const RefBind& b, const RpTarget& t, int n, int id, bool walk, int cx, int cy,
+                                        int cz, float re, float minus_zero, float (&acc)[Op::NS],
+                                        float (&xacc)[RpShape<Op>::NXR]) {
+    const float mind = (float)(re * 1e-3), re2x = ref_screen2(re);
+    float rare_re = 0.0f;
+    if constexpr (Op::NX > 0) rare_re = Op::rare_radius(b.param);
+    const unsigned long long nz2 = rp_pack(minus_zero, minus_zero);
+    // differences in the order that the components lie in memory (a square has no sign)
+    const unsigned long long txy = rp_pack(-t.pos.x, -t.pos.y), tzx = rp_pack(-t.pos.z, -t.pos.x),
+                             tyz = rp_pack(-t.pos.y, -t.pos.z);
+#pragma unroll
+    for (int c = 0; c < Op::NS; ++c) acc[c] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < RpShape<Op>::NXR; ++c) xacc[c] = 0.0f;
+    const Integer3 G = b.box.m_GridSize;
+    const ulonglong2* const pos16 = reinterpret_cast<const ulonglong2*>(b.pos);
+    const int4* const oid4 = reinterpret_cast<const int4*>(b.out_id);
+#pragma unroll 1
+    for (int m = 0; m < 27; ++m) {
+        const int i = m % 3 - 1, j = (m / 3) % 3 - 1, k = m / 9 - 1;
+        const int cell = cell_key(G, (int)((unsigned)cx + (unsigned)i), (int)((unsigned)cy + (unsigned)j),
+                                  (int)((unsigned)cz + (unsigned)k));
+        int s = 0, e = 0;
+        if (walk && cell >= 0 && cell < b.cell_num) {
+            s = b.cell_start[cell];
+            e = s == -1 ? s : b.cell_end[cell];
+        }
+        if (s >= e) continue;
+        const int g1 = (e + 3) >> 2;
+        int g = s >> 2;
+        int4 on = make_int4(0, 0, 0, 0);
+        ulonglong2 n0{}, n1{}, n2{};
+        if (4 * g + 4 <= n) {   // 16-byte loads stay inside the arrays
+            on = oid4[g];
+            n0 = pos16[3 * (size_t)g];
+            n1 = pos16[3 * (size_t)g + 1];
+            n2 = pos16[3 * (size_t)g + 2];
+        }
+#pragma unroll 1
+        for (; g < g1; ++g) {
+            const int4 o = on;
+            const ulonglong2 p0 = n0, p1 = n1, p2 = n2;
+            const bool safe = 4 * g + 4 <= n;
+            if (g + 1 < g1 && 4 * g + 8 <= n) {
+                on = oid4[g + 1];
+                n0 = pos16[3 * (size_t)g + 3];
+                n1 = pos16[3 * (size_t)g + 4];
+                n2 = pos16[3 * (size_t)g + 5];
+            }
+            const unsigned long long c[6] = {rp_add2(p0.x, txy), rp_add2(p0.y, tzx), rp_add2(p1.x, tyz),
+                                             rp_add2(p1.y, txy), rp_add2(p2.x, tzx), rp_add2(p2.y, tyz)};
+            float f[12], d2[4];
+#pragma unroll
+            for (int h = 0; h < 6; ++h) rp_unpack(rp_mul2(c[h], c[h], nz2), f[2 * h], f[2 * h + 1]);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) d2[h] = f[3 * h] + f[3 * h + 1] + f[3 * h + 2];
+            if (!safe || 4 * g < s || 4 * g + 4 > e || ((o.x | o.y) | (o.z | o.w)) < 0) {
+                // a cell's first or last group, or particles to be skipped
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const int x = 4 * g + h;
+                    const bool valid = x >= s && x < e;
+                    int oid = h == 0 ? o.x : h == 1 ? o.y : h == 2 ? o.z : o.w;
+                    if (!safe && valid) {
+                        oid = b.out_id[x];
+                        const Scalar3 p = b.pos[x];
+                        const float dx = t.pos.x - p.x, dy = t.pos.y - p.y, dz = t.pos.z - p.z;
+                        d2[h] = dx * dx + dy * dy + dz * dz;
+                    }
+                    if (!valid || oid < 0) d2[h] = 3.402823466e38f;   // screened out
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (d2[h] >= re2x && d2[h] <= 3.402823466e38f) continue;
+                const int x = 4 * g + h;
+                float d = ref_sqrt(d2[h]);
+                if (!(Op::kLe ? d <= re : d < re) || x == id) continue;
+                if (d < mind) d = mind;
+                float v[Op::NS];
+                Op::terms(b, re, t, x, d, v);
+#pragma unroll
+                for (int q = 0; q < Op::NS; ++q) acc[q] += v[q];
+                if constexpr (Op::NX > 0) {
+                    if (d < rare_re) {
+                        float ex[Op::NX];
+                        Op::rare_terms(b, re, t, x, d, ex);
+#pragma unroll
+                        for (int q = 0; q < Op::NX; ++q) xacc[q] += ex[q];
+                    }
+                }
+            }
+        }
+    }
+}
+
+}  // namespace mps
