@@ -34,6 +34,22 @@ size_t scan_tile_sums_capacity();
 // library-owned scratch for the reference-named entry points, which take no scratch
 // argument (runtime.cu).  Grows on demand; one buffer per slot.
 void* scratch_get(int slot, size_t bytes);
+// A call's turn with that scratch: one host thread at a time, and on the GPU after the
+// work that the turn before queued on its own stream, so calls on several streams do not
+// overwrite each other's buffers.  Without a stream only the host threads take turns (the
+// call has waited for its own work by then).
+class ScratchTurn {
+public:
+    ScratchTurn();
+    explicit ScratchTurn(cudaStream_t st);
+    ~ScratchTurn();
+    ScratchTurn(const ScratchTurn&) = delete;
+    ScratchTurn& operator=(const ScratchTurn&) = delete;
+
+private:
+    cudaStream_t st_ = nullptr;
+    bool on_stream_ = false;
+};
 // records "where: CUDA error string" for mps_last_error()
 void note_error(const char* where, cudaError_t e);
 // records a message of the library's own for mps_last_error()

@@ -938,6 +938,7 @@ static unsigned* scan_sums() { return (unsigned*)scratch_get(8, sizeof(unsigned)
 CCTStatusType SortUsingThrust(Integer MaxParticleNum, Integer* daNumberHash, Integer* daNumberIndex) {
     const int n = MaxParticleNum;
     if (n <= 1) return CCT_NOERR;
+    const ScratchTurn turn;
     cudaStream_t st = 0;
     int* mm = (int*)scratch_get(0, 2 * sizeof(int));
     if (!mm) return CCT_MEMERR;
@@ -959,6 +960,7 @@ CCTStatusType StableSortUsingThrust(Integer MaxParticleNum, Integer* daNumberHas
 CCTStatusType CheckParticleOutsideComputeZone(cudaStream_t& Stream, Integer* ParticleNum) {
     const int n = *ParticleNum;
     if (n <= 0) return CCT_NOERR;
+    const ScratchTurn turn(Stream);
     unsigned* flag = (unsigned*)scratch_get(2, sizeof(unsigned) * ((size_t)n + 4));
     unsigned* rank = (unsigned*)scratch_get(3, sizeof(unsigned) * ((size_t)n + 4));
     if (!flag || !rank) return CCT_MEMERR;
@@ -986,6 +988,7 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
                                        Integer CellNum) {
     const int t = TriangleNum;
     if (t <= 0 || CellNum <= 0) return CCT_NOERR;
+    const ScratchTurn turn(Stream);
     unsigned* off = (unsigned*)scratch_get(4, sizeof(unsigned) * ((size_t)t + 4));
     if (!off) return CCT_MEMERR;
     unsigned* total_dev = off + t;

@@ -3,6 +3,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <mutex>
+
 #include "mps_internal.h"
 #include "../../include/mps_runtime.h"
 
@@ -15,6 +17,8 @@ struct Slot {
 };
 constexpr int kSlots = 16;
 Slot g_slots[kSlots];
+std::mutex g_turn;
+cudaEvent_t g_turn_done = nullptr;   // end of the last turn's work on its stream
 thread_local char g_err[256] = "no error";
 
 CCTStatusType rec(cudaError_t e) {
@@ -50,6 +54,18 @@ void* scratch_get(int slot, size_t bytes) {
     }
     s.bytes = want;
     return s.ptr;
+}
+
+ScratchTurn::ScratchTurn() { g_turn.lock(); }
+ScratchTurn::ScratchTurn(cudaStream_t st) : st_(st), on_stream_(true) {
+    g_turn.lock();
+    if (g_turn_done) cudaStreamWaitEvent(st, g_turn_done, 0);
+    else if (cudaEventCreateWithFlags(&g_turn_done, cudaEventDisableTiming) != cudaSuccess) g_turn_done = nullptr;
+}
+ScratchTurn::~ScratchTurn() {
+    // without an event (none could be created) the turn ends when its work does
+    if (on_stream_ && (!g_turn_done || cudaEventRecord(g_turn_done, st_) != cudaSuccess)) cudaStreamSynchronize(st_);
+    g_turn.unlock();
 }
 
 void scratch_release_all() {
