@@ -163,51 +163,81 @@ __device__ __forceinline__ Scalar3 ref_line(const Scalar3& l0, const Scalar3& l1
     if (u > 1) dv = s3sub(l0, p);
     return dv;
 }
-__device__ __forceinline__ float ref_tri_distance(const CTriangle& T, const Scalar3& p, Scalar3& dir) {
-    const Scalar3 n = T.Normal;
-    Scalar3 c;
-    c.x = (float)((double)(T.Vertex[0].x + T.Vertex[1].x + T.Vertex[2].x) / 3.0);
-    c.y = (float)((double)(T.Vertex[0].y + T.Vertex[1].y + T.Vertex[2].y) / 3.0);
-    c.z = (float)((double)(T.Vertex[0].z + T.Vertex[1].z + T.Vertex[2].z) / 3.0);
-    const float sd = ref_sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
+// CalcDistance(triangle): what depends on the triangle alone, then a point's distance.
+// The reference's centroid divides in double, (float)((double)s / 3.0); s / 3.0f is the
+// same float: the quotient of a float by 3 lies at least 2^-26 of itself away from every
+// midpoint of two floats, so rounding to double first never decides (GB300 has few FP64
+// units).
+struct RefTri {
+    Scalar3 a, b, c, n, e0, e1;   // vertices, normal, edges a-c and a-b
+    float nc, sd, d00, d01, d11, inv;
+};
+__device__ __forceinline__ RefTri ref_tri(const CTriangle& T) {
+    RefTri r;
+    r.a = T.Vertex[0];
+    r.b = T.Vertex[1];
+    r.c = T.Vertex[2];
+    r.n = T.Normal;
+    Scalar3 m;
+    m.x = (r.a.x + r.b.x + r.c.x) / 3.0f;
+    m.y = (r.a.y + r.b.y + r.c.y) / 3.0f;
+    m.z = (r.a.z + r.b.z + r.c.z) / 3.0f;
+    r.nc = r.n.x * m.x + r.n.y * m.y + r.n.z * m.z;
+    r.sd = ref_sqrt(r.n.x * r.n.x + r.n.y * r.n.y + r.n.z * r.n.z);
+    r.e0 = s3sub(r.c, r.a);
+    r.e1 = s3sub(r.b, r.a);
+    r.d00 = ref_dot(r.e0, r.e0);
+    r.d01 = ref_dot(r.e0, r.e1);
+    r.d11 = ref_dot(r.e1, r.e1);
+    r.inv = 1.0f / (r.d00 * r.d11 - r.d01 * r.d01);
+    return r;
+}
+__device__ __forceinline__ float ref_tri_distance(const RefTri& T, const Scalar3& p, Scalar3& dir) {
+    const Scalar3 n = T.n;
     Scalar3 dv = s3(0, 0, 0);
-    if (sd != 0.0f) {
-        const float coef = ((n.x * p.x + n.y * p.y + n.z * p.z) - (n.x * c.x + n.y * c.y + n.z * c.z)) / sd;
-        dv = s3(coef / sd * n.x, coef / sd * n.y, coef / sd * n.z);
+    if (T.sd != 0.0f) {
+        const float coef = ((n.x * p.x + n.y * p.y + n.z * p.z) - T.nc) / T.sd;
+        dv = s3(coef / T.sd * n.x, coef / T.sd * n.y, coef / T.sd * n.z);
     }
     const Scalar3 P = s3(p.x - dv.x, p.y - dv.y, p.z - dv.z);
-    const Scalar3 v0 = s3sub(T.Vertex[2], T.Vertex[0]);
-    const Scalar3 v1 = s3sub(T.Vertex[1], T.Vertex[0]);
-    const Scalar3 v2 = s3sub(P, T.Vertex[0]);
-    const float d00 = ref_dot(v0, v0), d01 = ref_dot(v0, v1), d02 = ref_dot(v0, v2);
-    const float d11 = ref_dot(v1, v1), d12 = ref_dot(v1, v2);
-    const float inv = 1.0f / (d00 * d11 - d01 * d01);
-    const float u = (d11 * d02 - d01 * d12) * inv;
-    const float v = (d00 * d12 - d01 * d02) * inv;
-    if (u >= 0 && v >= 0 && u + v > 1) dv = ref_line(T.Vertex[1], T.Vertex[2], p);
-    if (u < 0) dv = ref_line(T.Vertex[0], T.Vertex[1], p);
-    if (v < 0) dv = ref_line(T.Vertex[0], T.Vertex[2], p);
+    const Scalar3 v2 = s3sub(P, T.a);
+    const float d02 = ref_dot(T.e0, v2), d12 = ref_dot(T.e1, v2);
+    const float u = (T.d11 * d02 - T.d01 * d12) * T.inv;
+    const float v = (T.d00 * d12 - T.d01 * d02) * T.inv;
+    // the reference's three edge tests, of which the last one that holds decides
+    const bool bc = u >= 0 && v >= 0 && u + v > 1, ab = u < 0, ac = v < 0;
+    if (bc || ab || ac) dv = ref_line(ab || ac ? T.a : T.b, ac ? T.c : ab ? T.b : T.c, p);
     dir = dv;
     return ref_mag(dv);
 }
 
 // RegisterLine / RegisterTriangle (Utility_Inline.h:1745-1855): walk the three edges
 // in cell-size steps, shrink the triangle toward its interior by one cell, repeat.
-// Visit(cell) is called for every sample point inside the grid.
-template <class Visit>
-__device__ void ref_walk_line(const CGridBox& B, Scalar3 v, Scalar3 d, float m, int cells, Visit& visit) {
+// visit(cell, ok) is called for every sample point, ok where it lies inside the grid, by
+// the G lanes of `group` together: lane l takes steps l, l + G, ... of a line, each step's
+// offset summed from cell sizes as the reference's loop sums it.
+template <int G, class Visit>
+__device__ __forceinline__ void ref_walk_line(const CGridBox& B, Scalar3 v, Scalar3 d, float m, int cells, unsigned group,
+                                              int lane, Visit& visit) {
+    constexpr int kMost = 100000;   // steps of a line
     float tab = 0.0f;
-    int guard = 0;
-    do {
-        const Scalar3 t = s3(v.x + tab * d.x, v.y + tab * d.y, v.z + tab * d.z);
-        int i, j, k;
-        const int cid = ref_cell(B, t, i, j, k);
-        if (cid >= 0 && cid < cells) visit(cid);
-        tab += B.m_CellSize;
-    } while (tab <= m && ++guard < 100000);
+    for (int q = 0; q < lane && tab <= m; ++q) tab += B.m_CellSize;
+    for (int step = lane;; step += G) {
+        const bool in = (step == 0 || tab <= m) && step < kMost;
+        if (!__any_sync(group, in)) break;
+        int cid = -1;
+        if (in) {
+            const Scalar3 t = s3(v.x + tab * d.x, v.y + tab * d.y, v.z + tab * d.z);
+            int i, j, k;
+            cid = ref_cell(B, t, i, j, k);
+        }
+        visit(cid, cid >= 0 && cid < cells);
+#pragma unroll
+        for (int q = 0; q < G; ++q) tab += B.m_CellSize;
+    }
 }
-template <class Visit>
-__device__ void ref_walk_triangle(const CGridBox& B, const CTriangle& T, int cells, Visit& visit) {
+template <int G, class Visit>
+__device__ void ref_walk_triangle(const CGridBox& B, const CTriangle& T, int cells, unsigned group, int lane, Visit& visit) {
     Scalar3 A = T.Vertex[0], Bv = T.Vertex[1], C = T.Vertex[2];
     const float cs = B.m_CellSize;
     float mbc, mab, mca;
@@ -218,9 +248,13 @@ __device__ void ref_walk_triangle(const CGridBox& B, const CTriangle& T, int cel
         mbc = ref_mag(bc);
         mab = ref_mag(ab);
         mca = ref_mag(ca);
-        if (mab > 0.0f) ref_walk_line(B, A, s3(ab.x / mab, ab.y / mab, ab.z / mab), mab, cells, visit);
-        if (mbc > 0.0f) ref_walk_line(B, Bv, s3(bc.x / mbc, bc.y / mbc, bc.z / mbc), mbc, cells, visit);
-        if (mca > 0.0f) ref_walk_line(B, C, s3(ca.x / mca, ca.y / mca, ca.z / mca), mca, cells, visit);
+#pragma unroll 1
+        for (int e = 0; e < 3; ++e) {
+            const Scalar3 from = e == 0 ? A : e == 1 ? Bv : C, along = e == 0 ? ab : e == 1 ? bc : ca;
+            const float m = e == 0 ? mab : e == 1 ? mbc : mca;
+            if (m > 0.0f)
+                ref_walk_line<G>(B, from, s3(along.x / m, along.y / m, along.z / m), m, cells, group, lane, visit);
+        }
         Scalar3 am = s3add(ab, ac), bm = s3add(ba, bc), cm = s3add(ca, cb);
         const float mam = ref_mag(am), mbm = ref_mag(bm), mcm = ref_mag(cm);
         if (mam > 0.0f) {
@@ -240,35 +274,56 @@ __device__ void ref_walk_triangle(const CGridBox& B, const CTriangle& T, int cel
 
 struct CountVisit {
     int n = 0;
-    __device__ void operator()(int) { ++n; }
+    __device__ __forceinline__ void operator()(int, bool ok) { n += ok; }
 };
+// the visits of a triangle in any order: they are sorted by cell, and a cell takes each
+// triangle once
 struct StoreVisit {
     int* cell;
     int* tri;
     int t;
+    unsigned group, below;
     int k = 0;
-    __device__ void operator()(int c) { cell[k] = c; tri[k] = t; ++k; }
+    __device__ __forceinline__ void operator()(int c, bool ok) {
+        const unsigned m = __ballot_sync(group, ok) & group;
+        if (ok) {
+            const int at = k + __popc(m & below);
+            cell[at] = c;
+            tri[at] = t;
+        }
+        k += __popc(m);
+    }
 };
 
-__global__ void k_tri_count(int t, const CTriangle* __restrict__ tri, const __grid_constant__ CGridBox box, int cells,
-                            unsigned* __restrict__ count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= t) return;
+// G lanes per triangle
+template <int G>
+__global__ void __launch_bounds__(kBlock) k_tri_count(int t, const CTriangle* __restrict__ tri,
+                                                      const __grid_constant__ CGridBox box, int cells,
+                                                      unsigned* __restrict__ count) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G;
+    if (i >= t) return;   // the G lanes of a triangle leave together
+    const unsigned group = G == 32 ? ~0u : ((1u << (G % 32)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
     CountVisit v;
     const CTriangle T = tri[i];
-    ref_walk_triangle(box, T, cells, v);
-    count[i] = (unsigned)v.n;
+    ref_walk_triangle<G>(box, T, cells, group, lane, v);
+    for (int o = G / 2; o > 0; o >>= 1) v.n += __shfl_xor_sync(group, v.n, o);
+    if (lane == 0) count[i] = (unsigned)v.n;
 }
-__global__ void k_tri_fill(int t, const CTriangle* __restrict__ tri, const __grid_constant__ CGridBox box, int cells,
-                           const unsigned* __restrict__ off, int* __restrict__ vcell, int* __restrict__ vtri) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+template <int G>
+__global__ void __launch_bounds__(kBlock) k_tri_fill(int t, const CTriangle* __restrict__ tri,
+                                                     const __grid_constant__ CGridBox box, int cells,
+                                                     const unsigned* __restrict__ off, int* __restrict__ vcell,
+                                                     int* __restrict__ vtri) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G;
     if (i >= t) return;
     StoreVisit v;
+    v.group = G == 32 ? ~0u : ((1u << (G % 32)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+    v.below = (1u << (threadIdx.x & 31)) - 1u;
     v.cell = vcell + off[i];
     v.tri = vtri + off[i];
     v.t = i;
     const CTriangle T = tri[i];
-    ref_walk_triangle(box, T, cells, v);
+    ref_walk_triangle<G>(box, T, cells, v.group, lane, v);
 }
 // visits sorted (stably) by cell: unique triangle ids per cell, ascending, first 100
 __global__ void k_tri_bounds(int nv, const int* __restrict__ vcell, int* __restrict__ vs, int* __restrict__ ve) {
@@ -281,25 +336,28 @@ __global__ void k_tri_bounds(int nv, const int* __restrict__ vcell, int* __restr
     }
     if (i == nv - 1) ve[c] = i + 1;
 }
-__global__ void k_tri_cells(int cells, const int* __restrict__ vs, const int* __restrict__ ve,
-                            const int* __restrict__ vtri, CCell* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per cell: 32 visits a round, a triangle taken where its run of visits begins
+// (they ascend) unless the cell held it before.
+__global__ void __launch_bounds__(kBlock) k_tri_cells(int cells, const int* __restrict__ vs, const int* __restrict__ ve,
+                                                      const int* __restrict__ vtri, CCell* __restrict__ out) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (c >= cells) return;
     const int s = vs[c];
     if (s < 0) return;
     const int e = ve[c];
-    unsigned cnt = out[c].m_TriangleNum;
-    int last = -1;
-    for (int i = s; i < e; ++i) {
-        const int t = vtri[i];
-        if (t == last) continue;
-        last = t;
-        bool have = false;
-        for (unsigned l = 0; l < cnt; ++l)
-            if (out[c].m_TriangleID[l] == t) { have = true; break; }
-        if (!have && cnt < CELLMAXTRIANGLENUM) out[c].m_TriangleID[cnt++] = t;
+    const unsigned held = out[c].m_TriangleNum;
+    unsigned cnt = held;
+    for (int i0 = s; i0 < e && cnt < CELLMAXTRIANGLENUM; i0 += 32) {
+        const int i = i0 + lane;
+        const int t = i < e ? vtri[i] : -1;
+        bool take = i < e && t != (i > s ? vtri[i - 1] : -1);
+        for (unsigned l = 0; take && l < held && l < CELLMAXTRIANGLENUM; ++l) take = out[c].m_TriangleID[l] != t;
+        const unsigned m = __ballot_sync(~0u, take);
+        const unsigned at = cnt + __popc(m & ((1u << lane) - 1u));
+        if (take && at < CELLMAXTRIANGLENUM) out[c].m_TriangleID[at] = t;
+        cnt += __popc(m);
     }
-    out[c].m_TriangleNum = cnt;
+    if (lane == 0) out[c].m_TriangleNum = cnt > CELLMAXTRIANGLENUM && held <= CELLMAXTRIANGLENUM ? CELLMAXTRIANGLENUM : cnt;
 }
 
 // ResetTriangleTopology_Kernel (DeviceProcess_Kernel.h:594-602)
@@ -365,63 +423,138 @@ __global__ void k_tri_reset_wall(int t, int step, const CTriangle* __restrict__ 
         b.triangles[id] = orig[id];
 }
 
-// Nearest triangle over the 27 cells, (k, j, i) order, first minimum wins.
-__device__ void ref_nearest(const RefBind& b, const Scalar3& p, bool drag_only, CDistance& nd, int& nid) {
-    int cx, cy, cz;
-    const int cid = ref_cell(b.box, p, cx, cy, cz);
-    if (!(cid >= 0 && cid < b.cell_num)) return;
-    for (int k = -1; k <= 1; ++k)
-        for (int j = -1; j <= 1; ++j)
-            for (int i = -1; i <= 1; ++i) {
-                const int m = cell_key(b.box.m_GridSize, cx + i, cy + j, cz + k);
-                if (m < 0 || m >= b.cell_num) continue;
-                const unsigned tn = b.cells[m].m_TriangleNum;
-                for (unsigned l = 0; l < tn && l < CELLMAXTRIANGLENUM; ++l) {
-                    const int t = b.cells[m].m_TriangleID[l];
-                    if (t < 0 || t >= b.triangle_num) continue;
-                    if (drag_only && !b.tri_params[b.triangles[t].ModelIDNumber].isDrag) continue;
-                    if (t != nid) {
-                        CDistance d;
-                        d.Magnitude = ref_tri_distance(b.triangles[t], p, d.Direction);
-                        if (d.Magnitude < nd.Magnitude) {
-                            nd = d;
-                            nid = t;
+// Nearest triangle over the 27 cells, (k, j, i) order, first minimum wins: a warp for T
+// consecutive particles, lane t holding particle t (`live`: it has a cell).  The cells'
+// triangle lists as one sequence, a lane per entry: what depends on the triangle alone is
+// computed once for all particles of a cell, each lane keeps its first minimum per
+// particle, and the earliest of the warp's minima is the serial loop's (a triangle met
+// again changes nothing).  Returns in lane t the triangle (-1: none) and its distance.
+//
+// Bound by the latency of long lists: particles beside drag spheres meet hundreds of
+// entries while most meet none, and a thread per particle ran them one after another, each
+// with three FP64 divisions: 535 us for 108,186 particles and 9,216 triangles, DRAM idle.
+// A warp for four: 184 us (drag 548 -> 179); 882,080 particles 478 -> 367 (376 -> 314).
+constexpr int kNearT = 4;
+template <bool DRAG>
+__device__ __forceinline__ void ref_nearest(const RefBind& b, const Scalar3& p, bool live, CDistance& nd, int& nid) {
+    constexpr int T = kNearT;
+    const int lane = threadIdx.x & 31;
+    int cx = 0, cy = 0, cz = 0;
+    if (live) {
+        const int cid = ref_cell(b.box, p, cx, cy, cz);
+        live = cid >= 0 && cid < b.cell_num;
+    }
+    Scalar3 q[T];
+    float best[T];
+    int at[T], id[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        q[t] = s3(__shfl_sync(~0u, p.x, t), __shfl_sync(~0u, p.y, t), __shfl_sync(~0u, p.z, t));
+        best[t] = 1e8f;
+        at[t] = 0x7fffffff;
+        id[t] = -1;
+    }
+    unsigned todo = __ballot_sync(~0u, live);
+#pragma unroll 1
+    while (todo) {
+        const int l = __ffs(todo) - 1;
+        const int gx = __shfl_sync(~0u, cx, l), gy = __shfl_sync(~0u, cy, l), gz = __shfl_sync(~0u, cz, l);
+        const unsigned grp = __ballot_sync(~0u, live && cx == gx && cy == gy && cz == gz) & todo;
+        todo &= ~grp;
+        int m = -1, len = 0;
+        if (lane < 27) {
+            m = cell_key(b.box.m_GridSize, (int)((unsigned)gx + (unsigned)(lane % 3) - 1u),
+                         (int)((unsigned)gy + (unsigned)(lane / 3 % 3) - 1u), (int)((unsigned)gz + (unsigned)(lane / 9) - 1u));
+            if (m >= 0 && m < b.cell_num) len = (int)min(b.cells[m].m_TriangleNum, (unsigned)CELLMAXTRIANGLENUM);
+        }
+        int off = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(~0u, off, o);
+            if (lane >= o) off += v;
+        }
+        const int total = __shfl_sync(~0u, off, 31);
+        off -= len;
+#pragma unroll 1
+        for (int c0 = 0; c0 < total; c0 += 32) {
+            const int c = c0 + lane;
+            int k = 0;   // the last cell whose list starts at or before c
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int v = __shfl_sync(~0u, off, k + o);
+                if (v <= c) k += o;
+            }
+            const int cell = __shfl_sync(~0u, m, k), first = __shfl_sync(~0u, off, k);
+            if (c < total) {
+                const int t = b.cells[cell].m_TriangleID[c - first];
+                if (t >= 0 && t < b.triangle_num &&
+                    !(DRAG && !b.tri_params[b.triangles[t].ModelIDNumber].isDrag)) {
+                    const RefTri tri = ref_tri(b.triangles[t]);
+#pragma unroll
+                    for (int u = 0; u < T; ++u) {
+                        if (!(grp >> u & 1u)) continue;
+                        Scalar3 dir;
+                        const float d = ref_tri_distance(tri, q[u], dir);
+                        if (d < best[u]) {
+                            best[u] = d;
+                            at[u] = c;
+                            id[u] = t;
                         }
                     }
                 }
             }
+        }
+    }
+    nd.Magnitude = 1e8f;
+    nd.Direction = s3(0, 0, 0);
+    nid = -1;
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float d = __shfl_xor_sync(~0u, best[t], o);
+            const int c = __shfl_xor_sync(~0u, at[t], o), i = __shfl_xor_sync(~0u, id[t], o);
+            if (d < best[t] || (d == best[t] && c < at[t])) {
+                best[t] = d;
+                at[t] = c;
+                id[t] = i;
+            }
+        }
+        if (lane == t) nid = id[t];
+    }
+    if (nid != -1) nd.Magnitude = ref_tri_distance(ref_tri(b.triangles[nid]), p, nd.Direction);
 }
 
 // CalcSTLDistance_Kernel (DeviceProcess_Kernel.h:853-919)
-__global__ void k_ref_stl_distance(int n, const __grid_constant__ RefBind b) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
+__global__ void __launch_bounds__(128, 8) k_ref_stl_distance(int n, const __grid_constant__ RefBind b) {
+    const int lane = threadIdx.x & 31;
+    const int id = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kNearT + lane;
+    const bool mine = lane < kNearT && id < n;
     CDistance nd;
-    nd.Magnitude = 1e8f;
-    nd.Direction = s3(0, 0, 0);
-    int nid = -1;
-    ref_nearest(b, b.pos[id], false, nd, nid);
+    int nid;
+    ref_nearest<false>(b, mine ? b.pos[id] : s3(0, 0, 0), mine, nd, nid);
+    if (!mine) return;
     b.stl_distance[id] = nd;
     b.stl_id[id] = nid;
 }
 
 // CalcDragEffect_Kernel and mode helpers (DeviceProcess_Kernel.h:125-389), with the
 // reference's index use and brace placement (mode 'F' acts outside the region).
-__global__ void k_ref_drag(int n, const __grid_constant__ RefBind b) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
+__global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constant__ RefBind b) {
+    const int lane = threadIdx.x & 31;
+    const int id = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kNearT + lane;
+    const bool mine = lane < kNearT && id < n;
+    const bool gone = mine && b.out_id[id] < -1;
+    CDistance nd;
+    int nid;
+    ref_nearest<true>(b, mine ? b.pos[id] : s3(0, 0, 0), mine && !gone, nd, nid);
+    if (!mine) return;
     const CParameter& P = b.param;
     if (b.magnifier_count[id] > 0) b.magnifier_count[id]++;
     if (b.magnifier_count[id] == 10) b.magnifier_count[id] = 0;
-    CDistance nd;
-    nd.Magnitude = 1e8f;
-    nd.Direction = s3(0, 0, 0);
-    int nid = -1;
-    if (b.out_id[id] < -1) {
+    if (gone) {
         b.stl_distance[id] = nd;
         b.stl_id[id] = nid;
-    } else {
-        ref_nearest(b, b.pos[id], true, nd, nid);
     }
     b.drag_acc[id] = s3(0, 0, 0);
     b.drag_temperature[id] = 0;
@@ -814,6 +947,8 @@ cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
                                                                                                         g_bind);
     return cudaGetLastError();
 }
+// Below it a triangle is walked by 32 lanes (few triangles are large ones), else by 8.
+constexpr int kTriFew = 2048;
 constexpr int kRefFew = 20000, kRefFewTurbulence = 100000;
 // From here on the predictor, whose radius is the cell size (250 of 1,728 candidates
 // accepted), runs a lane per target: 2.83 against 2.99 ms at 884,736 particles, 772
@@ -992,7 +1127,11 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
     unsigned* off = (unsigned*)scratch_get(4, sizeof(unsigned) * ((size_t)t + 4));
     if (!off) return CCT_MEMERR;
     unsigned* total_dev = off + t;
-    MPS_COUNT_LAUNCH k_tri_count<<<grid_of(t), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off);
+    const bool few = t < kTriFew;
+    if (few)
+        MPS_COUNT_LAUNCH k_tri_count<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off);
+    else
+        MPS_COUNT_LAUNCH k_tri_count<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off);
     MPS_CUDA_TRY(scan_exclusive(off, t, total_dev, Stream, scan_sums()));
     unsigned nv = 0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&nv, total_dev, sizeof(unsigned), cudaMemcpyDeviceToHost, Stream));
@@ -1003,11 +1142,14 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
     void* sscr = scratch_get(7, radix_scratch_bytes((int)nv));
     if (!vcell || !vrange || !sscr) return CCT_MEMERR;
     int* vtri = vcell + nv;
-    MPS_COUNT_LAUNCH k_tri_fill<<<grid_of(t), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
+    if (few)
+        MPS_COUNT_LAUNCH k_tri_fill<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
+    else
+        MPS_COUNT_LAUNCH k_tri_fill<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
     MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, 0, radix_passes((unsigned)CellNum), sscr, Stream));
     MPS_CUDA_TRY(cudaMemsetAsync(vrange, 0xff, sizeof(int) * (size_t)CellNum * 2, Stream));
     MPS_COUNT_LAUNCH k_tri_bounds<<<grid_of((int)nv), kBlock, 0, Stream>>>((int)nv, vcell, vrange, vrange + CellNum);
-    MPS_COUNT_LAUNCH k_tri_cells<<<grid_of(CellNum), kBlock, 0, Stream>>>(CellNum, vrange, vrange + CellNum, vtri, daCell);
+    MPS_COUNT_LAUNCH k_tri_cells<<<div_up(32ll * CellNum, kBlock), kBlock, 0, Stream>>>(CellNum, vrange, vrange + CellNum, vtri, daCell);
     return launch_status();
 }
 
@@ -1033,14 +1175,13 @@ CCTStatusType ResetWallPosition(cudaStream_t& Stream, const Integer TriangleNum,
 
 CCTStatusType CalcSTLDistance(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
-    MPS_CUDA_TRY(cudaMemsetAsync(g_bind.stl_id, 0xff, sizeof(int) * (size_t)ComputeParticleNum, Stream));
-    MPS_COUNT_LAUNCH k_ref_stl_distance<<<grid_of(ComputeParticleNum), kBlock, 0, Stream>>>(ComputeParticleNum, g_bind);
+    MPS_COUNT_LAUNCH k_ref_stl_distance<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
     return launch_status();
 }
 
 CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
-    MPS_COUNT_LAUNCH k_ref_drag<<<grid_of(ComputeParticleNum), kBlock, 0, Stream>>>(ComputeParticleNum, g_bind);
+    MPS_COUNT_LAUNCH k_ref_drag<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
     return launch_status();
 }
 
