@@ -35,8 +35,7 @@ extern "C" {
  * may be NULL.  act: 0 none, 1 SiLU (Cz, if given, receives the pre-activation FP32).
  * split_k > 1 splits the K loop over CTAs and accumulates into C with atomics
  * (beta must be 1 and act 0 then).  Runs on the 5th-generation tensor cores
- * (tcgen05.mma into TMEM, 128 x 16..64 tiles, K in stages of 64); the MLP's forward
- * and backward passes of training use it. */
+ * (tcgen05.mma into TMEM, 128 x 16..64 tiles, K in stages of 64). */
 CCTStatusType mps_gemm_bf16(int M, int N, int K, const void* A, int lda, int transA, const void* B, int ldb,
                             int transB, float* C, int ldc, void* Cb, int ldcb, float* Cz, const float* bias, int act,
                             float beta, int split_k, void* stream);
@@ -69,7 +68,8 @@ CCTStatusType mps_mlp_tc_timeouts(unsigned* out);
  * device and clears the mps_mlp_tc_timeouts flag. */
 CCTStatusType mps_mlp_debug_wait_spins(long long spins);
 /* loss = mean over rows of (y0-t0)^2 + w1 (y1-t1)^2 and the gradient of every
- * parameter (device FP32, MPS_MLP_PARAMS floats) by the tensor-core backward pass */
+ * parameter (device FP32, MPS_MLP_PARAMS floats), forward and backward pass in one kernel
+ * on the tensor cores (an array that is not 16-byte aligned costs a copy) */
 CCTStatusType mps_mlp_loss_grad(MpsMlp* m, int M, const float* X, const float* T, float w1, float* grad,
                                 float* host_loss, void* stream);
 /* one Adam step (lr, beta1 0.9, beta2 0.999, eps 1e-8) on a mini-batch */

@@ -1,7 +1,8 @@
 // mlp.cu - BF16 tensor-core GEMM and the learned-preconditioner MLP (forward,
 // backward, Adam) of the GB300 MPS library (include/mps_learned.h).
 //
-// GEMM (training): k_gemm_tc on the 5th-generation tensor cores (tcgen05.mma into
+// Training: one kernel for loss and gradients (k_mlp_train, tcgen05), then Adam.
+// GEMM (mps_gemm_bf16): k_gemm_tc on the 5th-generation tensor cores (tcgen05.mma into
 // TMEM, see below).  Cross-check variant k_gemm_bf16: one CTA of 4 warps computes a
 // 64x64 FP32 tile of C with warp-level
 // mma.sync.m16n8k16 (BF16 in, FP32 accumulate); each warp owns a 32x32 sub-tile
@@ -158,12 +159,6 @@ cudaError_t gemm_mma_sync(int M, int N, int K, const bf16* A, int lda, int ta, c
 // ---------------------------------------------------------------------------
 // elementwise helpers of the MLP
 // ---------------------------------------------------------------------------
-__global__ void k_pack_input(int M, const float* __restrict__ X, bf16* __restrict__ Xb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * FINP) return;
-    const int r = i / FINP, c = i % FINP;
-    Xb[i] = __float2bfloat16(c < FIN ? X[(size_t)r * FIN + c] : 0.f);
-}
 // FP32 master parameters -> padded BF16 weights and FP32 biases
 struct Layers {
     bf16 *W1, *W2, *W3, *W4;      // [16][128], [128][128], [128][128], [128][16]
@@ -193,12 +188,6 @@ __global__ void k_params_to_layers(const float* __restrict__ p, Layers L) {
     }
     if (i < FOUTP) L.b4[i] = i < FOUT ? p[o7 + i] : 0.f;
 }
-__global__ void k_unpad_output(int M, const float* __restrict__ Yp, float* __restrict__ Y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * FOUT) return;
-    Y[i] = Yp[(size_t)(i / FOUT) * FOUTP + (i % FOUT)];
-}
-
 // ---------------------------------------------------------------------------
 // Fused inference: the whole 12 -> 128 -> 128 -> 128 -> 2 network in one
 // persistent kernel.  Each CTA stages the four weight matrices once in shared
@@ -483,7 +472,7 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, uint32_t (&v)[16]) {
 }
 
 // ---------------------------------------------------------------------------
-// BF16 GEMM on the 5th-generation tensor cores, the training path of the MLP:
+// BF16 GEMM on the 5th-generation tensor cores:
 // C[M x N] (+)= op(A)[M x K] op(B)[K x N], FP32 accumulate, with the epilogue of
 // k_gemm_bf16 (bias, FP32 pre-activation Cz, SiLU, FP32 C with beta, BF16 Cb;
 // split-K CTAs add into C with FP32 atomics).  A CTA of 4 warps owns a 128 x BN tile
@@ -499,8 +488,8 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, uint32_t (&v)[16]) {
 // tcgen05.ld.  Bounded waits that run out set g_mlp_tc_timeout, wait (bounded) for
 // the MMAs in flight and skip the epilogue.
 // ---------------------------------------------------------------------------
-// BN at most 64: twice the CTAs of 128-column tiles on the MLP's 128-wide layers (the
-// training GEMMs are small, so their time is latency, not tensor throughput)
+// BN at most 64: twice the CTAs of 128-column tiles on 128-wide outputs (small products
+// take latency, not tensor throughput)
 constexpr int kGtBM = 128, kGtBK = 64, kGtMaxBN = 64, kGtThreads = 128;
 constexpr int kGtStageA = kGtBM * kGtBK * 2;                 // 16 KB
 constexpr int kGtStageB = kGtMaxBN * kGtBK * 2;              // 8 KB
@@ -1015,60 +1004,295 @@ __global__ void __launch_bounds__(TcShape<NS>::Threads, 1) k_mlp_infer_tc(int M,
     }
 }
 
-// dY = d loss / d y for loss = mean((y0 - t0)^2 + w1 (y1 - t1)^2); loss partial sums
-__global__ void k_loss_grad(int M, const float* __restrict__ Yp, const float* __restrict__ T, float w1,
-                            bf16* __restrict__ dYb, float* __restrict__ dY, double* __restrict__ loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < M) {
-        const float e0 = Yp[(size_t)i * FOUTP] - T[2 * (size_t)i];
-        const float e1 = Yp[(size_t)i * FOUTP + 1] - T[2 * (size_t)i + 1];
-        l = (double)e0 * e0 + (double)w1 * e1 * e1;
-        const float s = 2.0f / (float)M;
-        for (int c = 0; c < FOUTP; ++c) {
-            const float gv = c == 0 ? s * e0 : (c == 1 ? s * w1 * e1 : 0.f);
-            dY[(size_t)i * FOUTP + c] = gv;
-            dYb[(size_t)i * FOUTP + c] = __float2bfloat16(gv);
+// ---------------------------------------------------------------------------
+// Training pass: loss and the gradient of every parameter in one kernel.
+//
+// A CTA of 16 warps takes a 128-row tile (a tile per CTA up to one CTA per SM, then in
+// turn) through the forward and backward passes with everything in shared memory and
+// TMEM: the layer inputs X, H1, H2, H3 and the gradients dY, dZ as BF16 operands, the
+// pre-activations Z1, Z2, Z3 as the FP32 accumulators they were computed in (128 TMEM
+// columns each).  Warp w holds rows 32 (w % 4) + lane and columns 32 (w / 4) ..; one
+// thread issues a stage's MMAs (M = 128, K = 16 each) and commits them to one mbarrier.
+// Stages, with the accumulator columns they write:
+//   Z1 = X W1 | Z2 = H1 W2 | Z3 = H2 W3 | W[0,16) = H3 W4 | W = dY W4^T
+//   W = dZ3 W3^T, Z3 = H2^T dZ3 (dW3) | W = dZ2 W2^T, Z2 = H1^T dZ2 (dW2)
+//   W[0,16) = dZ1^T X (dW1^T), W[16,32) = H3^T dY (dW4)
+// A tile is stored once, rows of 16-byte pieces in the canonical layout without swizzle:
+// read along a row it is a K-major operand, read down the rows the MN-major operand of the
+// transposed product (piece stride 128 bytes along the columns, 8-row stride along K), so
+// neither weights nor activations are kept twice.  The weight gradients leave TMEM as
+// FP32 reductions into the parameter vector (four columns each; they add in any order),
+// the bias gradients as column sums of the FP32 dZ.  Rounding points: BF16 weights,
+// activations, dY and dZ in the products, FP32 everywhere else.
+//
+// It replaces 24 launches per batch, of which the column sums of the bias gradients (one
+// CTA, 4 x 450 us at 8,192 rows) and the weight-gradient products on 32 CTAs (4 x 70 us)
+// took most: 1,297 -> 55 us a pass at 8,192 rows (kernel 35 us, then the loss copy and its
+// wait), 52 us from 512 to 16,384 rows, 57 us at 19,456.  Bound by the latency of its chain
+// of stages (eight MMA stages with SiLU or its derivative between them), 64 CTAs at 8,192
+// rows.
+// Every wait is bounded; when one runs out the CTA flags it, waits (bounded) for its MMAs
+// and leaves its gradients out.
+// ---------------------------------------------------------------------------
+constexpr int kTrRows = 128, kTrThreads = 512;
+constexpr int kTrWide = kTrRows * H * 2;       // bytes of a [128][128] BF16 tile
+constexpr int kTrNarrow = kTrRows * 16 * 2;    // of a [128][16] or [16][128] one
+constexpr int kTrH = 0;                        // H1, H2, H3
+constexpr int kTrDz = kTrH + 3 * kTrWide;
+constexpr int kTrW2 = kTrDz + kTrWide, kTrW3 = kTrW2 + kTrWide;
+constexpr int kTrX = kTrW3 + kTrWide, kTrDy = kTrX + kTrNarrow, kTrW1 = kTrDy + kTrNarrow, kTrW4 = kTrW1 + kTrNarrow;
+constexpr int kTrBias = kTrW4 + kTrNarrow;     // b1, b2, b3 [128], b4 [16]
+constexpr int kTrBar = kTrBias + (3 * H + 16) * 4;
+constexpr size_t kTrSmem = kTrBar + 32 + 1024;
+static_assert(kTrSmem <= 227 * 1024, "shared memory of one CTA");
+
+// operand of a tile with `cols` columns: K-major (K along a row) or MN-major (K down the rows)
+__device__ __forceinline__ unsigned long long tr_kmajor(unsigned a, int cols) { return tc_desc(a, 128, 16 * cols); }
+__device__ __forceinline__ unsigned long long tr_mnmajor(unsigned a, int cols) { return tc_desc(a, 16 * cols, 128); }
+constexpr unsigned kTrTransA = 1u << 15, kTrTransB = 1u << 16;   // operand is MN-major
+
+__device__ __forceinline__ void red_add4(float* p, const uint32_t* v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(__uint_as_float(v[0])),
+                 "f"(__uint_as_float(v[1])), "f"(__uint_as_float(v[2])), "f"(__uint_as_float(v[3]))
+                 : "memory");
+}
+// sums of v[0..32) over the warp's lanes: lane l returns the sum of v[l]
+__device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < o; ++q) {
+            const float give = up ? v[q] : v[q + o], keep = up ? v[q + o] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
     }
+    return v[0];
+}
+
+// g: MPS_MLP_PARAMS floats, 16-byte aligned, zero on entry, as is *loss
+__global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(int M, const float* __restrict__ X, const float* __restrict__ T,
+                                                             float w1, Layers L, float* __restrict__ g,
+                                                             double* __restrict__ loss) {
+    extern __shared__ unsigned char tr_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)tr_raw + 1023) & ~(uintptr_t)1023);
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(sm + kTrBar);
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(sm + kTrBar + 8);
+    float* bias = reinterpret_cast<float*>(sm + kTrBias);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(tmem_slot)), "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // weights [k][n] and biases
+    for (int e = tid; e < H * H / 8; e += kTrThreads) {
+        const int k = e >> 4, c = 8 * (e & 15);
+        *reinterpret_cast<uint4*>(sm + kTrW2 + tc_off(k, c, H)) = *reinterpret_cast<const uint4*>(L.W2 + k * H + c);
+        *reinterpret_cast<uint4*>(sm + kTrW3 + tc_off(k, c, H)) = *reinterpret_cast<const uint4*>(L.W3 + k * H + c);
+    }
+    if (tid < FINP * H / 8) {
+        const int k = tid >> 4, c = 8 * (tid & 15);
+        *reinterpret_cast<uint4*>(sm + kTrW1 + tc_off(k, c, H)) = *reinterpret_cast<const uint4*>(L.W1 + k * H + c);
+    } else if (tid < 2 * FINP * H / 8) {
+        const int e = tid - FINP * H / 8, k = e >> 1, c = 8 * (e & 1);
+        *reinterpret_cast<uint4*>(sm + kTrW4 + tc_off(k, c, FOUTP)) = *reinterpret_cast<const uint4*>(L.W4 + k * FOUTP + c);
+    }
+    if (tid < H) {
+        bias[tid] = L.b1[tid];
+        bias[H + tid] = L.b2[tid];
+        bias[2 * H + tid] = L.b3[tid];
+    }
+    if (tid < FOUTP) bias[3 * H + tid] = L.b4[tid];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+    const int r = 32 * (warp & 3) + lane, c0 = 32 * (warp >> 2);   // this thread's row and first column of a tile
+    const unsigned quad = (unsigned)(32 * (warp & 3)) << 16;
+    // TMEM columns
+    constexpr unsigned Z[3] = {0u, 128u, 256u}, W = 384u;
+    constexpr int o1 = FIN * H, o2 = o1 + H, o3 = o2 + H * H, o4 = o3 + H, o5 = o4 + H * H, o6 = o5 + H, o7 = o6 + H * FOUT;
+    const unsigned sa = tc_smem(sm);
+    const unsigned wide = tc_idesc(128, 128), narrow = tc_idesc(128, 16);
+    unsigned parity = 0u;
+    bool failed = false;
+    // what every thread wrote to shared memory and read from TMEM comes before the next
+    // stage's MMAs
+    auto ready = [&]() {
+        tc_fence_smem();
+        tc_fence_before();
+        __syncthreads();
+    };
+    // the stage's MMAs are done (false: the wait ran out, for all threads alike)
+    auto done = [&]() {
+        const bool ok = tc_bar_wait(bar, parity, 1ll << 22);
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) atomicOr(&g_mlp_tc_timeout, 1u);
+            tc_bar_wait(bar, parity, 1ll << 24);
+            failed = true;
+            return false;
+        }
+        parity ^= 1u;
+        tc_fence_after();
+        return true;
+    };
+    // D = A B over K = 128: A, B and their steps of 16 along K
+    auto mma8 = [&](unsigned d, unsigned long long a, int astep, unsigned long long b, int bstep, unsigned idesc) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
-}
-__global__ void k_silu_back(int n, const float* __restrict__ dH, const float* __restrict__ Z, float* __restrict__ dZ,
-                            bf16* __restrict__ dZb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = dH[i] * silu_grad(Z[i]);
-    dZ[i] = v;
-    dZb[i] = __float2bfloat16(v);
-}
-// column sums (bias gradients), FP32 -> out[c]
-__global__ void k_colsum(int M, int N, const float* __restrict__ A, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    float s = 0.f;
-    for (int r = 0; r < M; ++r) s += A[(size_t)r * N + c];
-    out[c] = s;
-}
-// gradient buffers (padded layer shapes) -> parameter-vector layout
-__global__ void k_grad_to_vec(const float* __restrict__ dW1, const float* __restrict__ db1, const float* __restrict__ dW2,
-                              const float* __restrict__ db2, const float* __restrict__ dW3, const float* __restrict__ db3,
-                              const float* __restrict__ dW4, const float* __restrict__ db4, float* __restrict__ g) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int o1 = FIN * H, o2 = o1 + H, o3 = o2 + H * H, o4 = o3 + H, o5 = o4 + H * H, o6 = o5 + H, o7 = o6 + H * FOUT;
-    if (i < FIN * H) g[i] = dW1[i];
-    if (i < H) {
-        g[o1 + i] = db1[i];
-        g[o3 + i] = db2[i];
-        g[o5 + i] = db3[i];
+        for (int k = 0; k < 8; ++k)
+            tc_mma(tmem + d, a + (unsigned long long)(k * astep >> 4), b + (unsigned long long)(k * bstep >> 4), idesc, k > 0);
+    };
+    // 32 columns of this thread's row -> BF16 operand
+    auto put = [&](int tile, const float (&v)[32]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<uint4*>(sm + tile + tc_off(r, c0 + 8 * q, H)) =
+                make_uint4(pack_bf16(v[8 * q], v[8 * q + 1]), pack_bf16(v[8 * q + 2], v[8 * q + 3]),
+                           pack_bf16(v[8 * q + 4], v[8 * q + 5]), pack_bf16(v[8 * q + 6], v[8 * q + 7]));
+    };
+    // a [128][128] gradient from TMEM into the parameter vector
+    auto flush = [&](unsigned d, float* out) {
+        uint32_t v[32];
+        tc_ld32(tmem + quad + d + c0, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) red_add4(out + r * H + c0 + 4 * q, v + 4 * q);
+    };
+    const int tiles = (M + kTrRows - 1) / kTrRows;
+    for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
+        const int row = t * kTrRows + r;
+        if (warp < 4) {   // X as [row][16]: 12 features, zeros
+            uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+            if (row < M) {
+                const float* x = X + (size_t)row * FIN;
+                lo = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+                hi.x = pack_bf16(x[8], x[9]);
+                hi.y = pack_bf16(x[10], x[11]);
+            }
+            *reinterpret_cast<uint4*>(sm + kTrX + tc_off(r, 0, FINP)) = lo;
+            *reinterpret_cast<uint4*>(sm + kTrX + tc_off(r, 8, FINP)) = hi;
+        }
+        ready();
+        // ---- forward ----
+#pragma unroll 1
+        for (int l = 0; l < 3; ++l) {
+            if (tid == 0) {
+                tc_fence_after();
+                if (l == 0)
+                    tc_mma(tmem + Z[0], tr_kmajor(sa + kTrX, FINP), tr_mnmajor(sa + kTrW1, H), wide | kTrTransB, 0);
+                else
+                    mma8(l == 1 ? Z[1] : Z[2], tr_kmajor(sa + kTrH + (l - 1) * kTrWide, H), 256,
+                         tr_mnmajor(sa + (l == 1 ? kTrW2 : kTrW3), H), 4096, wide | kTrTransB);
+                tc_commit(bar);
+            }
+            if (!done()) break;
+            uint32_t z[32];
+            float h[32];
+            tc_ld32(tmem + quad + 128u * l + c0, z);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) h[q] = silu(__uint_as_float(z[q]) + bias[l * H + c0 + q]);
+            put(kTrH + l * kTrWide, h);
+            ready();
+        }
+        if (failed) break;
+        if (tid == 0) {
+            tc_fence_after();
+            mma8(W, tr_kmajor(sa + kTrH + 2 * kTrWide, H), 256, tr_mnmajor(sa + kTrW4, FOUTP), 512, narrow | kTrTransB);
+            tc_commit(bar);
+        }
+        if (!done()) break;
+        // ---- loss and dY ----
+        if (warp < 4) {
+            uint32_t y0, y1;
+            tc_ld2(tmem + quad + W, y0, y1);
+            float e0 = 0.f, e1 = 0.f;
+            if (row < M) {
+                e0 = (__uint_as_float(y0) + bias[3 * H]) - T[2 * (size_t)row];
+                e1 = (__uint_as_float(y1) + bias[3 * H + 1]) - T[2 * (size_t)row + 1];
+            }
+            double ls = (double)e0 * e0 + (double)w1 * e1 * e1;
+            const float sc = 2.0f / (float)M;
+            float d0 = sc * e0, d1 = sc * w1 * e1;
+            *reinterpret_cast<uint4*>(sm + kTrDy + tc_off(r, 0, FOUTP)) = make_uint4(pack_bf16(d0, d1), 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(sm + kTrDy + tc_off(r, 8, FOUTP)) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                ls += __shfl_xor_sync(0xffffffffu, ls, o);
+                d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+                d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+            }
+            if (lane == 0) {
+                atomicAdd(loss, ls);
+                atomicAdd(g + o7, d0);
+                atomicAdd(g + o7 + 1, d1);
+            }
+        }
+        ready();
+        // ---- backward ----
+        if (tid == 0) {
+            tc_fence_after();
+            tc_mma(tmem + W, tr_kmajor(sa + kTrDy, FOUTP), tr_kmajor(sa + kTrW4, FOUTP), wide, 0);
+            tc_commit(bar);
+        }
+#pragma unroll 1
+        for (int l = 2; l >= 0; --l) {
+            if (!done()) break;
+            {
+                // dZ = dH silu'(Z); both accumulators are free afterwards
+                uint32_t dh[32], z[32];
+                float v[32];
+                tc_ld32(tmem + quad + W + c0, dh);
+                tc_ld32(tmem + quad + 128u * l + c0, z);
+#pragma unroll
+                for (int q = 0; q < 32; ++q)
+                    v[q] = __uint_as_float(dh[q]) * silu_grad(__uint_as_float(z[q]) + bias[l * H + c0 + q]);
+                put(kTrDz, v);
+                const float s = lane_sums(v, lane);
+                atomicAdd(g + (l == 2 ? o5 : l == 1 ? o3 : o1) + c0 + lane, s);
+            }
+            ready();
+            if (tid == 0) {
+                tc_fence_after();
+                if (l > 0) {
+                    mma8(W, tr_kmajor(sa + kTrDz, H), 256, tr_kmajor(sa + (l == 2 ? kTrW3 : kTrW2), H), 256, wide);
+                    mma8(l == 2 ? Z[2] : Z[1], tr_mnmajor(sa + kTrH + (l - 1) * kTrWide, H), 4096, tr_mnmajor(sa + kTrDz, H),
+                         4096, wide | kTrTransA | kTrTransB);
+                } else {
+                    mma8(W, tr_mnmajor(sa + kTrDz, H), 4096, tr_mnmajor(sa + kTrX, FINP), 512,
+                         narrow | kTrTransA | kTrTransB);
+                    mma8(W + 16, tr_mnmajor(sa + kTrH + 2 * kTrWide, H), 4096, tr_mnmajor(sa + kTrDy, FOUTP), 512,
+                         narrow | kTrTransA | kTrTransB);
+                }
+                tc_commit(bar);
+            }
+            if (l < 2) flush(l == 1 ? Z[2] : Z[1], g + (l == 1 ? o4 : o2));   // the stage before's weight gradient
+        }
+        if (failed || !done()) break;
+        if (warp < 4) {   // row r: n of dW1^T, k of dW4
+            uint32_t v[16], u0, u1;
+            tc_ld16(tmem + quad + W, v);
+            tc_ld2(tmem + quad + W + 16, u0, u1);
+#pragma unroll
+            for (int k = 0; k < FIN; ++k) atomicAdd(g + k * H + r, __uint_as_float(v[k]));
+            atomicAdd(g + o6 + FOUT * r, __uint_as_float(u0));
+            atomicAdd(g + o6 + FOUT * r + 1, __uint_as_float(u1));
+        }
+        tc_fence_before();
+        __syncthreads();   // the next tile overwrites X, dY and the accumulators
+        tc_fence_after();
     }
-    if (i < H * H) {
-        g[o2 + i] = dW2[i];
-        g[o4 + i] = dW3[i];
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
-    if (i < H * FOUT) g[o6 + i] = dW4[(i / FOUT) * FOUTP + (i % FOUT)];
-    if (i < FOUT) g[o7 + i] = db4[i];
 }
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, float lr, float b1t, float b2t) {
@@ -1092,9 +1316,6 @@ struct MpsMlp {
     int nparams = MPS_MLP_PARAMS;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     Layers L{};
-    bf16 *Xb = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dYb = nullptr, *dZb = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *Yp = nullptr, *dY = nullptr, *dH = nullptr, *dZ = nullptr;
-    float *dW1 = nullptr, *dW2 = nullptr, *dW3 = nullptr, *dW4 = nullptr, *db = nullptr;
     double* loss = nullptr;
     double* h_loss = nullptr;
     int t = 0;
@@ -1108,19 +1329,12 @@ struct MpsMlp {
     }
     cudaError_t init(int b) {
         maxb = (b + 63) / 64 * 64;
-        const size_t B = maxb;
         cudaError_t e = cudaSuccess;
         e = e ? e : mk(&p, nparams); e = e ? e : mk(&g, nparams); e = e ? e : mk(&m, nparams); e = e ? e : mk(&v, nparams);
         e = e ? e : mk(&L.W1, FINP * H); e = e ? e : mk(&L.W2, H * H); e = e ? e : mk(&L.W3, H * H);
         e = e ? e : mk(&L.W4, H * FOUTP);
         e = e ? e : mk(&L.b1, H); e = e ? e : mk(&L.b2, H); e = e ? e : mk(&L.b3, H); e = e ? e : mk(&L.b4, FOUTP);
         e = e ? e : mk(&L.tc, (size_t)kTcImage);
-        e = e ? e : mk(&Xb, B * FINP); e = e ? e : mk(&H1, B * H); e = e ? e : mk(&H2, B * H); e = e ? e : mk(&H3, B * H);
-        e = e ? e : mk(&Z1, B * H); e = e ? e : mk(&Z2, B * H); e = e ? e : mk(&Z3, B * H);
-        e = e ? e : mk(&Yp, B * FOUTP); e = e ? e : mk(&dY, B * FOUTP); e = e ? e : mk(&dYb, B * FOUTP);
-        e = e ? e : mk(&dH, B * H); e = e ? e : mk(&dZ, B * H); e = e ? e : mk(&dZb, B * H);
-        e = e ? e : mk(&dW1, FINP * H); e = e ? e : mk(&dW2, H * H); e = e ? e : mk(&dW3, H * H);
-        e = e ? e : mk(&dW4, H * FOUTP); e = e ? e : mk(&db, 4 * H);
         e = e ? e : mk(&loss, 1);
         if (e) return e;
         if ((e = cudaMallocHost((void**)&h_loss, sizeof(double)))) return e;
@@ -1140,60 +1354,23 @@ struct MpsMlp {
         MPS_COUNT_LAUNCH k_layers_to_tc<<<div_up(kTcK * H, 256), 256, 0, st>>>(p, L);
         return cudaGetLastError();
     }
-    // forward over M rows (M <= maxb); keep pre-activations when train
-    cudaError_t forward(int M, const float* X, cudaStream_t st, bool train) {
-        MPS_COUNT_LAUNCH k_pack_input<<<div_up(M * FINP, 256), 256, 0, st>>>(M, X, Xb);
-        cudaError_t e = gemm(M, H, FINP, Xb, FINP, 0, L.W1, H, 0, nullptr, H, H1, H, train ? Z1 : nullptr, L.b1, 1,
-                             0.f, 1, st);
-        if (!e) e = gemm(M, H, H, H1, H, 0, L.W2, H, 0, nullptr, H, H2, H, train ? Z2 : nullptr, L.b2, 1, 0.f, 1, st);
-        if (!e) e = gemm(M, H, H, H2, H, 0, L.W3, H, 0, nullptr, H, H3, H, train ? Z3 : nullptr, L.b3, 1, 0.f, 1, st);
-        if (!e) e = gemm(M, FOUTP, H, H3, H, 0, L.W4, FOUTP, 0, Yp, FOUTP, nullptr, 0, nullptr, L.b4, 0, 0.f, 1, st);
-        return e;
-    }
-    cudaError_t backward(int M, const float* T, float w1, cudaStream_t st) {
+    // loss (h_loss after a copy) and gradients (out: MPS_MLP_PARAMS floats, 16-byte aligned)
+    // of M rows
+    cudaError_t loss_grad(int M, const float* X, const float* T, float w1, float* out, cudaStream_t st) {
+        static bool set = false;   // the attribute is per function, set once
         cudaError_t e = cudaSuccess;
-#define MLP_STEP(label, call)                       \
-    do {                                             \
-        call;                                        \
-        if ((e = cudaGetLastError())) {              \
-            note_error(label, e);                    \
-            return e;                                \
-        }                                            \
-    } while (0)
-#define MLP_GEMM(label, ...)                         \
-    do {                                             \
-        if ((e = gemm(__VA_ARGS__))) {               \
-            note_error(label, e);                    \
-            return e;                                \
-        }                                            \
-    } while (0)
-        MLP_STEP("loss reset", cudaMemsetAsync(loss, 0, sizeof(double), st));
-        MLP_STEP("k_loss_grad", (MPS_COUNT_LAUNCH k_loss_grad<<<div_up(M, 256), 256, 0, st>>>(M, Yp, T, w1, dYb, dY, loss)));
-        const int split = max(1, min(64, M / 512));
-        MLP_STEP("grad reset", cudaMemsetAsync(dW4, 0, sizeof(float) * H * FOUTP, st));
-        MLP_STEP("grad reset", cudaMemsetAsync(dW3, 0, sizeof(float) * H * H, st));
-        MLP_STEP("grad reset", cudaMemsetAsync(dW2, 0, sizeof(float) * H * H, st));
-        MLP_STEP("grad reset", cudaMemsetAsync(dW1, 0, sizeof(float) * FINP * H, st));
-        const int Kb = M;   // batch as K; the tile loader zero-fills k >= K
-        MLP_GEMM("dW4", H, FOUTP, Kb, H3, H, 1, dYb, FOUTP, 0, dW4, FOUTP, nullptr, 0, nullptr, nullptr, 0, 1.f, split, st);
-        MLP_STEP("db4", (MPS_COUNT_LAUNCH k_colsum<<<1, 128, 0, st>>>(M, FOUTP, dY, db + 3 * H)));
-        MLP_GEMM("dH3", M, H, FOUTP, dYb, FOUTP, 0, L.W4, FOUTP, 1, dH, H, nullptr, 0, nullptr, nullptr, 0, 0.f, 1, st);
-        MLP_STEP("silu3", (MPS_COUNT_LAUNCH k_silu_back<<<div_up(M * H, 256), 256, 0, st>>>(M * H, dH, Z3, dZ, dZb)));
-        MLP_GEMM("dW3", H, H, Kb, H2, H, 1, dZb, H, 0, dW3, H, nullptr, 0, nullptr, nullptr, 0, 1.f, split, st);
-        MLP_STEP("db3", (MPS_COUNT_LAUNCH k_colsum<<<1, 128, 0, st>>>(M, H, dZ, db + 2 * H)));
-        MLP_GEMM("dH2", M, H, H, dZb, H, 0, L.W3, H, 1, dH, H, nullptr, 0, nullptr, nullptr, 0, 0.f, 1, st);
-        MLP_STEP("silu2", (MPS_COUNT_LAUNCH k_silu_back<<<div_up(M * H, 256), 256, 0, st>>>(M * H, dH, Z2, dZ, dZb)));
-        MLP_GEMM("dW2", H, H, Kb, H1, H, 1, dZb, H, 0, dW2, H, nullptr, 0, nullptr, nullptr, 0, 1.f, split, st);
-        MLP_STEP("db2", (MPS_COUNT_LAUNCH k_colsum<<<1, 128, 0, st>>>(M, H, dZ, db + 1 * H)));
-        MLP_GEMM("dH1", M, H, H, dZb, H, 0, L.W2, H, 1, dH, H, nullptr, 0, nullptr, nullptr, 0, 0.f, 1, st);
-        MLP_STEP("silu1", (MPS_COUNT_LAUNCH k_silu_back<<<div_up(M * H, 256), 256, 0, st>>>(M * H, dH, Z1, dZ, dZb)));
-        MLP_GEMM("dW1", FINP, H, Kb, Xb, FINP, 1, dZb, H, 0, dW1, H, nullptr, 0, nullptr, nullptr, 0, 1.f, split, st);
-        MLP_STEP("db1", (MPS_COUNT_LAUNCH k_colsum<<<1, 128, 0, st>>>(M, H, dZ, db)));
-        MLP_STEP("grad vec", (MPS_COUNT_LAUNCH k_grad_to_vec<<<div_up(H * H, 256), 256, 0, st>>>(dW1, db, dW2, db + H, dW3, db + 2 * H,
-                                                                                 dW4, db + 3 * H, g)));
-#undef MLP_STEP
-#undef MLP_GEMM
-        return cudaSuccess;
+        if (!set) {
+            if ((e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrSmem))) return e;
+            set = true;
+        }
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if ((e = cudaMemsetAsync(out, 0, sizeof(float) * MPS_MLP_PARAMS, st))) return e;
+        if ((e = cudaMemsetAsync(loss, 0, sizeof(double), st))) return e;
+        MPS_COUNT_LAUNCH k_mlp_train<<<std::max(1, std::min(div_up(M, kTrRows), sms)), kTrThreads, kTrSmem, st>>>(
+            M, X, T, w1, L, out, loss);
+        return cudaGetLastError();
     }
 };
 
@@ -1363,9 +1540,12 @@ CCTStatusType mps_mlp_loss_grad(MpsMlp* m, int M, const float* X, const float* T
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e = cudaGetLastError();
     if (e) { note_error("mps_mlp_loss_grad: pending error on entry", e); return CCT_CUDAERR; }
-    if ((e = m->forward(M, X, st, true))) { note_error("mlp forward", e); return CCT_CUDAERR; }
-    if ((e = m->backward(M, T, w1, st))) return CCT_CUDAERR;   // backward names the failing launch
-    if (grad && (e = cudaMemcpyAsync(grad, m->g, sizeof(float) * MPS_MLP_PARAMS, cudaMemcpyDeviceToDevice, st))) {
+    // the kernel adds four floats at a time: a gradient array that is not 16-byte aligned
+    // gets a copy
+    float* const out = grad && ((uintptr_t)grad & 15) == 0 ? grad : m->g;
+    if ((e = m->loss_grad(M, X, T, w1, out, st))) { note_error("mlp loss and gradient", e); return CCT_CUDAERR; }
+    if (grad && out != grad &&
+        (e = cudaMemcpyAsync(grad, m->g, sizeof(float) * MPS_MLP_PARAMS, cudaMemcpyDeviceToDevice, st))) {
         char what[96];
         snprintf(what, sizeof(what), "gradient copy %p <- %p", (void*)grad, (void*)m->g);
         note_error(what, e);
@@ -1384,8 +1564,7 @@ CCTStatusType mps_mlp_train_step(MpsMlp* m, int M, const float* X, const float* 
                                  float* host_loss, void* stream) {
     if (!m || M <= 0 || M > m->maxb) return CCT_PARAMERR;
     cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = m->forward(M, X, st, true);
-    if (!e) e = m->backward(M, T, w1, st);
+    cudaError_t e = m->loss_grad(M, X, T, w1, m->g, st);
     if (e) return cuda_status(e);
     m->t += 1;
     const float b1t = powf(0.9f, (float)m->t), b2t = powf(0.999f, (float)m->t);

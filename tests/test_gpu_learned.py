@@ -177,6 +177,35 @@ def test_mlp_gradient_matches_oracle():
     assert o == mo.NPARAMS
 
 
+@pytest.mark.parametrize("rows,shift", [(1, 0), (127, 0), (128, 4), (129, 0), (1000, 0), (19456, 0), (40003, 0)])
+def test_loss_and_gradients_in_one_kernel(rows, shift):
+    """k_mlp_train at ragged tiles, one tile per SM and several tiles per CTA, and with a
+    gradient array that is not 16-byte aligned.  The oracle rounds at the same points, so
+    the two differ by FP32 sums and by values near a BF16 midpoint that round the other way:
+    a product has three rounded factors (activation, weight, gradient), each off by at most
+    one BF16 step of 2^-8, and on average by far less."""
+    m = Mlp(max_batch=rows, seed=9)
+    p = m.params().astype(np.float64)
+    rng = np.random.default_rng(rows)
+    X = rng.normal(0, 1, (rows, 12)).astype(np.float32)
+    T = rng.normal(0, 1, (rows, 2)).astype(np.float32)
+    dX, dT = DeviceArray.from_host(X), DeviceArray.from_host(T)
+    g = DeviceArray((mo.NPARAMS + 1,), np.float32)
+    g.fill_bytes(0xFF)
+    for _ in range(2):   # the second pass starts from the first one's gradients
+        loss = m.loss_grad(dX.ptr, dT.ptr, rows, g.ptr + shift)
+    ref_loss, ref_g = mo.loss_grad(p, X, T)
+    got = g.download()[shift // 4:][:mo.NPARAMS].astype(np.float64)
+    assert abs(loss - ref_loss) <= 3 * 2.0 ** -8 * abs(ref_loss)
+    o = 0
+    for fi, fo in ((12, 128), (128, 128), (128, 128), (128, 2)):
+        for size in (fi * fo, fo):
+            a, b = got[o:o + size], ref_g[o:o + size]
+            assert np.linalg.norm(a - b) <= 3 * 2.0 ** -8 * np.linalg.norm(b), (o, size)
+            o += size
+    assert Mlp.tc_timeouts() == 0
+
+
 def test_training_reduces_loss_on_a_smooth_target():
     rng = np.random.default_rng(4)
     X = rng.normal(0, 1, (40000, 12)).astype(np.float32)
