@@ -129,11 +129,22 @@ template <class T> __device__ __forceinline__ V3<T> v3(T x, T y, T z) { V3<T> r;
 // TS: type of the in-warp shuffle stage (float for the FP32 inner solve, whose
 // per-thread partials are float anyway; the FP64 pipe is narrow on GB300); the
 // cross-warp and cross-block stages are always FP64.
+// FP64 additions are the cost of it (a warp instruction occupies GB300's FP64 units for
+// about 16 cycles however few lanes take part), so both FP64 stages are trees over lanes:
+// 3 additions per value and CTA of 8 warps instead of 8 in a row, and in the last CTA 5
+// plus 3 per value instead of 5 plus 8 in every warp.  out is valid in thread 0.
 template <int NV, class TS = double>
 __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* red, unsigned* counter, double (&out)[NV]) {
     __shared__ double sm[NV][32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // sum of sm[k][0 .. nw) in lane 0 of the calling warp
+    auto warp_total = [&](int k) {
+        double s = lane < nw ? sm[k][lane] : 0.0;
+        for (int o = nw > 16 ? 16 : nw > 8 ? 8 : nw > 4 ? 4 : nw > 2 ? 2 : 1; o > 0; o >>= 1)
+            s += __shfl_down_sync(0xffffffffu, s, o);
+        return s;
+    };
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         TS x = (TS)v[k];
@@ -142,16 +153,17 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* red, unsign
         if (lane == 0) sm[k][w] = (double)x;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (w == 0) {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
-            double s = 0.0;
-            for (int i = 0; i < nw; ++i) s += sm[k][i];
-            red[(size_t)k * gridDim.x + blockIdx.x] = s;
+            const double s = warp_total(k);
+            if (lane == 0) red[(size_t)k * gridDim.x + blockIdx.x] = s;
         }
-        __threadfence();
-        const unsigned t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
+        if (lane == 0) {
+            __threadfence();
+            const unsigned t = atomicAdd(counter, 1u);
+            last = (t == gridDim.x - 1);
+        }
     }
     __syncthreads();
     if (!last) return false;
@@ -160,16 +172,16 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* red, unsign
     for (int k = 0; k < NV; ++k) {
         double s = 0.0;
         for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) s += ((volatile double*)red)[(size_t)k * gridDim.x + i];
+        if (w * 32 < (int)gridDim.x) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        }
         if (lane == 0) sm[k][w] = s;
     }
     __syncthreads();
+    if (w == 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double s = 0.0;
-        for (int i = 0; i < nw; ++i) s += sm[k][i];
-        out[k] = s;
+        for (int k = 0; k < NV; ++k) out[k] = warp_total(k);
     }
     if (threadIdx.x == 0) *counter = 0;
     return true;
@@ -1437,7 +1449,8 @@ __device__ __forceinline__ int slice_kmax(int v) { return v >= 0 ? v : -1 - v; }
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
 
-template <int SC, int SS, class TW = float, bool WIDE = false>
+// SPLIT > 1: SPLIT warps share each slice, warp `sub` of them its share of the chunks
+template <int SC, int SS, class TW = float, bool WIDE = false, int SPLIT = 1>
 struct SliceRing {
     static constexpr int SB = stream_stage_bytes<SC, TW, WIDE>();
     static constexpr unsigned CB = WIDE ? 128u : 64u;            // column bytes per entry
@@ -1448,14 +1461,15 @@ struct SliceRing {
     const TW* w;
     const int* skmax;
     unsigned* err;
-    int nsl, nw, K, lane;
-    int ps, pc, pk, pn;          // producer: next chunk pc of slice ps (pk entries, pn chunks)
+    int nsl, nw, K, lane, sub;
+    int ps, pc, pk, pn;          // producer: next chunk pc of slice ps (pk entries, chunks to pn)
     unsigned q_issue, q_cons;
     bool streaming;
     unsigned long long pol;
 
     __device__ void init(const Dev& d, const TW* w_, unsigned char* ring_, unsigned long long* bar_, int gw,
-                         int nw_) {
+                         int nw_, int sub_ = 0) {
+        sub = sub_;
         ring = ring_;
         bar = bar_;
         cols = WIDE ? (const unsigned char*)d.nbr : (const unsigned char*)d.nbr16;
@@ -1475,14 +1489,19 @@ struct SliceRing {
         pol = l2_evict_first_policy();
         next_slice();
     }
+    // the warp's chunks of a slice with kmax entries
+    __device__ int first_chunk(int kmax) const { return SPLIT == 1 ? 0 : (kmax + SC - 1) / SC * sub / SPLIT; }
+    __device__ int end_chunk(int kmax) const {
+        return SPLIT == 1 ? (kmax + SC - 1) / SC : (kmax + SC - 1) / SC * (sub + 1) / SPLIT;
+    }
     __device__ void next_slice() {
         do {
             ps += nw;
             pk = ps < nsl ? skmax[ps] : 0;
             if (WIDE) pk = slice_kmax(pk);   // every slice; else 16-bit slices only
-        } while (ps < nsl && pk <= 0);
-        pc = 0;
-        pn = (pk + SC - 1) / SC;
+            pc = pk > 0 ? first_chunk(pk) : 0;
+            pn = pk > 0 ? end_chunk(pk) : 0;
+        } while (ps < nsl && pc >= pn);
     }
     // issue copies until SS stages are in flight or the warp's slices are exhausted
     __device__ void refill() {
@@ -1617,6 +1636,94 @@ __global__ void __launch_bounds__(W * 32, MINB) k_spmv_stream(const __grid_const
             d.scal[S_LS0] = out[0];
             d.scal[S_LS1] = out[1];
         }
+    }
+}
+
+// The inner CG's SpMV over the FP16 weights where whole slices do not fill the chip:
+// SPLIT warps share a 32-row slice, each streaming a contiguous share of its chunks as in
+// k_spmv_stream, and the first adds the shares in order.  A slice is a chain of 16 chunks,
+// each waiting for its copy and for two rounds of gathers of x, and 108,186 particles have
+// 3,381 slices for 4,864 warps: time is that chain's latency, which SPLIT divides.  Large
+// systems have several slices per warp and are bound by DRAM; there the shares only add
+// barriers.  Measured, whole slices / SPLIT 2 / 4 / 8, in us: Poisson solve of 103,823
+// particles (63 iterations) 4,168 / 3,671 / 3,621 / 3,690, of 343,000 (87) 11,447 / 10,490 /
+// 10,226 / 10,799; step of 108,186 3,476 / 3,428 / 3,370 / 3,366, of 453,356 7,718 / 7,791 /
+// 7,834 / 7,969.  Plain loads of the shares instead of bulk copies: 5,898 at 103,823.
+template <int SPLIT, int SC, int SS, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_spmv_ring_split(const __grid_constant__ Dev d, const __half* __restrict__ w,
+                                                         const float* __restrict__ x, float* __restrict__ y, int slot) {
+    constexpr int W = 8, G = W / SPLIT;
+    using Ring = SliceRing<SC, SS, __half, false, SPLIT>;
+    pdl_wait();
+    pdl_trigger();
+    if (d.scal[S_CONV] != 0.0) return;
+    extern __shared__ __align__(128) unsigned char stream_smem[];
+    __shared__ __align__(8) unsigned long long bars[W][SS];
+    __shared__ float part[2][W][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % SPLIT;
+    Ring R;
+    R.init(d, w, stream_smem + warp * SS * Ring::SB, bars[warp], blockIdx.x * G + warp / SPLIT, gridDim.x * G, sub);
+    float partw = 0.f;
+    int buf = 0;
+    for (int s0 = blockIdx.x * G; s0 < R.nsl; s0 += gridDim.x * G, buf ^= 1) {
+        const int sl = s0 + warp / SPLIT;
+        const int i = sl * 32 + lane;
+        const bool row = sl < R.nsl && i < d.n, in = row && d.inner[i];
+        const int cnt = in ? d.nbr_cnt[i] : 0;
+        const int km = sl < R.nsl ? d.skmax[sl] : 0;
+        float acc = 0.f;
+        if (km > 0) {
+            const int c0 = R.first_chunk(km), c1 = R.end_chunk(km), r0 = sl * 32;
+            bool done = R.streaming;
+            for (int c = c0; done && c < c1; ++c) {
+                const unsigned char* cs;
+                const __half* ws;
+                if (!R.acquire(cs, ws)) {
+                    done = false;
+                    break;
+                }
+                const int k0 = c * SC;
+#pragma unroll
+                for (int g = 0; g < SC; g += 8) {
+                    int j[8];
+                    float wv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        j[u] = r0 + (int)(short)((const unsigned short*)cs)[(g + u) * 32 + lane];
+                        wv[u] = __half2float(ws[(g + u) * 32 + lane]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (k0 + g + u < cnt) acc = __fmaf_rn(wv[u], __ldg(x + j[u]), acc);
+                }
+                R.release();
+            }
+            if (!done) {   // streaming given up: the register walk of the warp's share
+                const int k0 = c0 * SC;
+                acc = sell_row_dot<true, float>(d, w, x, ((size_t)sl * d.K + k0) * 32 + lane, cnt - k0,
+                                                min(km, c1 * SC) - k0, r0);
+            }
+        } else if (km < 0 && sub == 0) {
+            acc = sell_row_dot<false, float>(d, w, x, (size_t)sl * d.K * 32 + lane, cnt, __reduce_max_sync(0xffffffffu, cnt),
+                                             -1);
+        }
+        part[buf][warp][lane] = acc;
+        __syncthreads();
+        if (sub == 0 && row) {
+#pragma unroll
+            for (int q = 1; q < SPLIT; ++q) acc += part[buf][warp + q][lane];
+            float yi = 0.f;
+            if (in) {
+                yi = (float)(d.diag16[i] * (double)x[i] - d.c.coef_lap * (double)acc);
+                partw += x[i] * yi;
+            }
+            y[i] = yi;
+        }
+    }
+    double v[1] = {(double)partw}, out[1];
+    if (grid_reduce<1, float>(v, d.red, d.red_count + slot, out) && threadIdx.x == 0) {
+        d.scal[S_PQ] = out[0];
+        d.scal[S_ALPHA] = out[0] != 0.0 ? d.scal[S_RZ] / out[0] : 0.0;
     }
 }
 
@@ -1940,6 +2047,8 @@ template <class TV, class TXA>
 __global__ void __launch_bounds__(256) k_cg_update(const __grid_constant__ Dev d, TXA* x, TV* r, TV* z, const TV* p,
                                                    const TV* q, const double* m64, const float* m32, int slot,
                                                    int with_z, int flexible = 0) {
+    pdl_wait();
+    pdl_trigger();
     if (d.scal[S_CONV] != 0.0) return;
     const TV alpha = (TV)d.scal[S_ALPHA];
     TV prz = TV(0), prr = TV(0), pzq = TV(0);
@@ -1988,16 +2097,22 @@ __global__ void k_cg_p(const __grid_constant__ Dev d, TV* p, const TV* z) {
 
 // neighbour-entry counts of interior rows (PPE matrix) and all rows; interior rows
 __global__ void __launch_bounds__(256) k_count_nnz(const __grid_constant__ Dev d, int slot) {
-    double a = 0.0, b = 0.0, m = 0.0;
+    int a = 0, b = 0, m = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n; i += gridDim.x * blockDim.x) {
-        const double c = (double)d.nbr_cnt[i];
+        const int c = d.nbr_cnt[i];
         b += c;
         if (d.inner[i]) {
             a += c;
-            m += 1.0;
+            ++m;
         }
     }
-    double v[3] = {a, b, m}, out[3];
+    // a warp's counts stay below 2^31 (rows are at most n / 1216 CTAs / 8 warps), and the
+    // shuffles add whole numbers
+    a = __reduce_add_sync(0xffffffffu, a);
+    b = __reduce_add_sync(0xffffffffu, b);
+    m = __reduce_add_sync(0xffffffffu, m);
+    const bool first = (threadIdx.x & 31) == 0;
+    double v[3] = {first ? (double)a : 0.0, first ? (double)b : 0.0, first ? (double)m : 0.0}, out[3];
     if (grid_reduce<3>(v, d.red, d.red_count + slot, out) && threadIdx.x == 0) {
         d.scal[S_NNZ0] = out[0];
         d.scal[S_NNZ1] = out[1];

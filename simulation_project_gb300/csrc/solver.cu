@@ -48,6 +48,10 @@ struct DevBuf {
 };
 
 inline int blocks_for(int n, int threads = kBlock) { return std::max(1, div_up(n, threads)); }
+// CTAs of a kernel that ends in a grid reduction over n rows: no more than have rows, since
+// each one without costs a partial, an atomic and the last CTA's time (2,000 rows on 1,216
+// CTAs: 10-12 us, on 8: 4)
+inline int red_blocks(int n) { return std::min(blocks_for(n, 256), kRedBlocks); }
 
 enum Phase { PH_GRID = 0, PH_WALLS, PH_PRED, PH_LIST, PH_SETUP, PH_SPMV, PH_VEC, PH_CORRECT, PH_LEARNED, PH_PRECOND,
              PH_OTHER, PH_COUNT };
@@ -674,10 +678,10 @@ struct Solver {
             std::swap(L[1].e, L[1].e2);
         }
         if (post)
-            MPS_COUNT_LAUNCH k_mg_fine_post<float><<<kRedBlocks, 256, 0, st>>>(d, mg, r, z, p, d.m32, mode, 7, qf, sm_R,
+            MPS_COUNT_LAUNCH k_mg_fine_post<float><<<red_blocks(d.n), 256, 0, st>>>(d, mg, r, z, p, d.m32, mode, 7, qf, sm_R,
                                                                                 sm_mask, (float)opt.smoother_weight);
         else
-            MPS_COUNT_LAUNCH k_mg_fine_z<float><<<kRedBlocks, 256, 0, st>>>(d, mg, r, z, p, d.m32, mode, 7, qf);
+            MPS_COUNT_LAUNCH k_mg_fine_z<float><<<red_blocks(d.n), 256, 0, st>>>(d, mg, r, z, p, d.m32, mode, 7, qf);
     }
 
     // ---- phases ----
@@ -861,7 +865,7 @@ struct Solver {
             MPS_COUNT_LAUNCH k_eos<<<blocks_for(d.n), kBlock, 0, st>>>(d);
         } else {
             MPS_COUNT_LAUNCH k_ppe_setup<<<blocks_for(d.n), kBlock, 0, st>>>(d);
-            MPS_COUNT_LAUNCH k_count_nnz<<<kRedBlocks, 256, 0, st>>>(d, 4);
+            MPS_COUNT_LAUNCH k_count_nnz<<<red_blocks(d.n), 256, 0, st>>>(d, 4);
             // the multilevel setup runs on the second stream: its topology (grid and
             // interior flags only) beside the rows' transpose, its operators from the rows
             // on, beside the warm start, the first refinement residual and the learned guess
@@ -910,7 +914,7 @@ struct Solver {
                                                                                   d.r, d.rhs, 2);
                 else
                     residual_df((const float*)d.nbrw);
-                MPS_COUNT_LAUNCH k_pressure_scale<<<kRedBlocks, 256, 0, st>>>(d, 5);
+                MPS_COUNT_LAUNCH k_pressure_scale<<<red_blocks(d.n), 256, 0, st>>>(d, 5);
                 MPS_COUNT_LAUNCH k_to_float_p<<<blocks_for(d.n), kBlock, 0, st>>>(d.n, d.press, d.pf32);
                 MPS_COUNT_LAUNCH k_features<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
                 feat_valid = true;
@@ -926,7 +930,7 @@ struct Solver {
                     if (fp64()) {
                         MPS_COUNT_LAUNCH k_learned_finish<<<blocks_for(d.n), kBlock, 0, st>>>(d);
                     } else {
-                        MPS_COUNT_LAUNCH k_learned_finish_r<<<kRedBlocks, 256, 0, st>>>(d, 7);
+                        MPS_COUNT_LAUNCH k_learned_finish_r<<<red_blocks(d.n), 256, 0, st>>>(d, 7);
                         residual_ready = true;
                     }
                 }
@@ -1138,6 +1142,24 @@ struct Solver {
             MPS_COUNT_LAUNCH k<<<spmv16_grid, kSsWarps * 32, kS16Smem, st>>>(d, d.w16, x, y, nullptr, 0);
         }
     }
+    // the same for systems with few slices per warp (k_spmv_ring_split)
+    static constexpr int kSplitRows = 400000, kSplit = 4;
+    int spmv16_split_grid = 0;
+    void spmv_split16(const float* x, float* y) {
+        auto k = k_spmv_ring_split<kSplit, kS16Entries, kSsStages, kSsMinBlocks>;
+        const int resident = stream_grid_for(k, kS16Smem, spmv16_split_grid);
+        if (resident < 0) {
+            stream_failed = true;
+            return;
+        }
+        const int grid = std::max(1, std::min(div_up(div_up(d.n, 32), kSsWarps / kSplit), resident));
+        if (pdl) {
+            if (MPS_COUNT_LAUNCH launch_pdl(k, grid, kSsWarps * 32, kS16Smem, st, d, (const __half*)d.w16, x, y, 0))
+                stream_failed = true;
+        } else {
+            MPS_COUNT_LAUNCH k<<<grid, kSsWarps * 32, kS16Smem, st>>>(d, d.w16, x, y, 0);
+        }
+    }
     // the CG iteration's kernels (SpMV, update and restriction, fine level of the
     // V-cycle, direction update) are launched with programmatic dependent launch
     bool pdl = true;
@@ -1191,7 +1213,8 @@ struct Solver {
         }
         if constexpr (std::is_same<TW, float>::value && std::is_same<TV, float>::value) {
             if (opt.matrix_free == 0 && use_stream()) {
-                if (inner16()) spmv_stream16(p, q);
+                if (inner16() && !prefer_wide && d.n < kSplitRows) spmv_split16(p, q);
+                else if (inner16()) spmv_stream16(p, q);
                 else spmv_stream<0>(w, p, q, nullptr, 0);
                 return;
             }
@@ -1235,9 +1258,16 @@ struct Solver {
                 spmv_cg<TW, TV>(w, p, q);
                 timer.mark(PH_VEC, st);
                 const bool use_mg = std::is_same<TV, float>::value && mg_ready;
-                if (!use_mg)
-                    MPS_COUNT_LAUNCH k_cg_update<TV, TXA><<<kRedBlocks, 256, 0, st>>>(d, x, r, z, p, q, m64, m32, 1, 1,
-                                                                                    flex_step ? 1 : 0);
+                if (!use_mg) {
+                    if (pdl) {
+                        if (MPS_COUNT_LAUNCH launch_pdl(k_cg_update<TV, TXA>, red_blocks(d.n), 256, 0, st, d, x, r, z,
+                                                        (const TV*)p, (const TV*)q, m64, m32, 1, 1, flex_step ? 1 : 0))
+                            stream_failed = true;
+                    } else {
+                        MPS_COUNT_LAUNCH k_cg_update<TV, TXA><<<red_blocks(d.n), 256, 0, st>>>(d, x, r, z, p, q, m64, m32, 1,
+                                                                                               1, flex_step ? 1 : 0);
+                    }
+                }
                 if constexpr (std::is_same<TV, float>::value) {
                     if (use_mg) {
                         // two level-1 aggregates per warp, within the reduction buffer's 2 x kRedBlocks CTAs
@@ -1255,11 +1285,11 @@ struct Solver {
                         timer.mark(PH_VEC, st);
                     }
                 }
-                if (pdl && use_mg) {
-                    if (MPS_COUNT_LAUNCH launch_pdl(k_cg_p<TV>, kRedBlocks, 256, 0, st, d, p, (const TV*)z))
+                if (pdl) {
+                    if (MPS_COUNT_LAUNCH launch_pdl(k_cg_p<TV>, red_blocks(d.n), 256, 0, st, d, p, (const TV*)z))
                         stream_failed = true;
                 } else {
-                    MPS_COUNT_LAUNCH k_cg_p<TV><<<kRedBlocks, 256, 0, st>>>(d, p, z);
+                    MPS_COUNT_LAUNCH k_cg_p<TV><<<red_blocks(d.n), 256, 0, st>>>(d, p, z);
                 }
                 ++spmv_launches;
             }
@@ -1282,7 +1312,7 @@ struct Solver {
         const double bnorm = h_scal[S_BNORM];
         S.r0_relres = bnorm > 0 ? h_scal[S_RNORM] / bnorm : 0.0;
         const double tol = opt.cg_rtol * bnorm;
-        MPS_COUNT_LAUNCH k_cg_start<double><<<kRedBlocks, 256, 0, st>>>(d, d.r, d.z, d.p, nullptr, 1.0, d.minv, nullptr, nullptr, 3, tol,
+        MPS_COUNT_LAUNCH k_cg_start<double><<<red_blocks(d.n), 256, 0, st>>>(d, d.r, d.z, d.p, nullptr, 1.0, d.minv, nullptr, nullptr, 3, tol,
                                                        opt.cg_max_iter);
         const int it = cg_loop<double, double, double>(d.press, d.r, d.z, d.p, d.q, w, d.minv, nullptr, opt.cg_max_iter);
         if (it < 0) return CCT_CUDAERR;
@@ -1395,7 +1425,7 @@ struct Solver {
             // 0.3 margin), but not below what FP32 CG reliably reaches (ir_inner_rtol)
             const double need = 0.3 * opt.cg_rtol * bnorm / rn;
             const double inner_tol = std::max(need, ir_inner_rtol());
-            MPS_COUNT_LAUNCH k_cg_start<float><<<kRedBlocks, 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,
+            MPS_COUNT_LAUNCH k_cg_start<float><<<red_blocks(d.n), 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,
                                                           inner_tol, opt.cg_max_iter);
             if (mg_ready) {
                 timer.mark(PH_PRECOND, st);
@@ -1414,7 +1444,7 @@ struct Solver {
                 if (stream_failed) return CCT_CUDAERR;
                 residual_ready = true;
             } else {
-                MPS_COUNT_LAUNCH k_axpy_ir<<<kRedBlocks, 256, 0, st>>>(d, d.press, d.d32, rn);
+                MPS_COUNT_LAUNCH k_axpy_ir<<<red_blocks(d.n), 256, 0, st>>>(d, d.press, d.d32, rn);
             }
             ++outer;
         }
