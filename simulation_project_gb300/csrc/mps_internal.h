@@ -8,23 +8,27 @@
 
 namespace mps {
 
-// radix sort (sort.cu).  Scratch: alternate key and value arrays, the digit counts
-// of every tile (digit-major), 8 spare words and per-pass digit totals.
-constexpr int kRadixSortTile = 2048;
-constexpr int kRadixBuckets = 256;
-constexpr int kRadixMaxPasses = 4;
-constexpr size_t radix_scratch_bytes_for(long long n) {
-    return sizeof(int) * 2 * (size_t)(n > 0 ? n : 0) +
-           sizeof(unsigned) * ((size_t)kRadixBuckets * (size_t)(((n > 0 ? n : 1) + kRadixSortTile - 1) / kRadixSortTile) +
-                               8 + (size_t)kRadixMaxPasses * kRadixBuckets) +
-           256;
+// radix sort (sort.cu).  Scratch: barrier words, key ranges, digit totals, digit counts of
+// every CTA, alternate key and value arrays.
+constexpr int kRadixDigitBits = 9;
+constexpr int kRadixMaxCtas = 152;
+// CTAs of a sort: up to 4,096 keys one (no grid barriers), then one per 1,024 keys
+constexpr int radix_ctas_for(long long n) {
+    return n <= 4096 ? 1 : (n + 1023) / 1024 < kRadixMaxCtas ? (int)((n + 1023) / 1024) : kRadixMaxCtas;
 }
-size_t radix_scratch_bytes(int n);
-int radix_passes(unsigned range);
-cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int kmin, int passes, void* scratch, cudaStream_t st);
-// the same with the key range (min, max) in device memory (key_minmax): no host wait
-cudaError_t radix_sort_pairs_range(int n, int* keys, int* vals, const int* mm_dev, void* scratch, cudaStream_t st);
-cudaError_t key_minmax(int n, const int* keys, int* mm_dev, cudaStream_t st);
+constexpr size_t radix_scratch_bytes_for(long long n, int max_ctas = kRadixMaxCtas) {
+    const size_t ctas = (size_t)(radix_ctas_for(n) < max_ctas ? radix_ctas_for(n) : max_ctas);
+    return sizeof(unsigned) * (8 + 2 * (size_t)kRadixMaxCtas + ((size_t)1 << kRadixDigitBits) * (ctas + 1)) +
+           sizeof(int) * 2 * (size_t)(n > 0 ? n : 0);
+}
+inline size_t radix_scratch_bytes(int n) { return radix_scratch_bytes_for(n); }
+// bits of the keys 0 .. range
+int radix_bits(unsigned range);
+// stable sort of (keys, vals) by key; bits: the keys lie in [0, 2^bits), < 0: any int range.
+// err (may be NULL) gets MPS_ERR_STAGE_TIMEOUT if a grid barrier runs out; the arrays then
+// hold the pairs in no particular order.
+cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, cudaStream_t st,
+                             int max_ctas = kRadixMaxCtas);
 // in-place exclusive scan of len unsigned values, total to *total_dev (if not NULL);
 // tile_sums (scan_tile_sums_capacity() values, or NULL: single-CTA scan) lets it
 // run on many CTAs

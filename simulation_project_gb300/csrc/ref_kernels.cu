@@ -1068,23 +1068,40 @@ CCTStatusType reorderDataAndFindCellStart(cudaStream_t& Stream, Integer numParti
 // tile sums of the multi-CTA scan (NULL when the slot cannot be had: one-CTA scan)
 static unsigned* scan_sums() { return (unsigned*)scratch_get(8, sizeof(unsigned) * scan_tile_sums_capacity()); }
 
+// Error word of the sorts in host memory that the GPU can write: read without a copy once
+// the stream has been waited for.  NULL when it cannot be had (errors then go unseen).
+static unsigned* sort_error() {
+    static unsigned* const word = [] {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return (unsigned*)nullptr;
+        }
+        *(unsigned*)p = 0u;
+        return (unsigned*)p;
+    }();
+    return word;
+}
+
 // thrust::sort_by_key replacement: stable LSD radix sort on the legacy default
-// stream, keys of any int range (one min/max pass picks the digits to sort).
+// stream, keys of any int range.
 CCTStatusType SortUsingThrust(Integer MaxParticleNum, Integer* daNumberHash, Integer* daNumberIndex) {
     const int n = MaxParticleNum;
     if (n <= 1) return CCT_NOERR;
     const ScratchTurn turn;
     cudaStream_t st = 0;
-    int* mm = (int*)scratch_get(0, 2 * sizeof(int));
-    if (!mm) return CCT_MEMERR;
     void* scr = scratch_get(1, radix_scratch_bytes(n));
     if (!scr) return CCT_MEMERR;
-    // the key range stays on the device: the passes it does not need return at once
-    MPS_CUDA_TRY(key_minmax(n, daNumberHash, mm, st));
-    MPS_CUDA_TRY(radix_sort_pairs_range(n, daNumberHash, daNumberIndex, mm, scr, st));
+    unsigned* const err = sort_error();
+    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, st));
     // thrust::sort_by_key with the default policy returns after the sort completed;
     // callers rely on that (they launch the reorder on their own stream next).
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (err && *(volatile unsigned*)err) {   // this sort's, or that of an earlier triangle binning
+        *(volatile unsigned*)err = 0u;
+        note_message("SortUsingThrust: a grid barrier of a sort ran out");
+        return CCT_CUDAERR;
+    }
     return launch_status();
 }
 
@@ -1146,7 +1163,7 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
         MPS_COUNT_LAUNCH k_tri_fill<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
     else
         MPS_COUNT_LAUNCH k_tri_fill<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
-    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, 0, radix_passes((unsigned)CellNum), sscr, Stream));
+    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, radix_bits((unsigned)CellNum), sscr, sort_error(), Stream));
     MPS_CUDA_TRY(cudaMemsetAsync(vrange, 0xff, sizeof(int) * (size_t)CellNum * 2, Stream));
     MPS_COUNT_LAUNCH k_tri_bounds<<<grid_of((int)nv), kBlock, 0, Stream>>>((int)nv, vcell, vrange, vrange + CellNum);
     MPS_COUNT_LAUNCH k_tri_cells<<<div_up(32ll * CellNum, kBlock), kBlock, 0, Stream>>>(CellNum, vrange, vrange + CellNum, vtri, daCell);

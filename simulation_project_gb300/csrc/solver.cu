@@ -715,7 +715,7 @@ struct Solver {
         }
         MPS_COUNT_LAUNCH k_hash<<<blocks_for(n), kBlock, 0, st>>>(d);
         const unsigned krange = ((unsigned)d.cells << d.zbits) - 1u;
-        if (radix_sort_pairs(n, d.skey, d.idx, 0, radix_passes(krange), sort_scratch, st)) return CCT_CUDAERR;
+        if (radix_sort_pairs(n, d.skey, d.idx, radix_bits(krange), sort_scratch, d.err, st)) return CCT_CUDAERR;
         cudaMemsetAsync(d.cstart, 0xff, sizeof(int) * d.cells, st);
         cudaMemsetAsync(d.cend, 0xff, sizeof(int) * d.cells, st);
         cudaMemsetAsync(d.cell_count, 0, sizeof(int), st);
@@ -773,7 +773,7 @@ struct Solver {
         int* vcell = bin_visit;
         d.tids = bin_visit + bin_visit_cap;
         MPS_COUNT_LAUNCH k_bin_fill<<<div_up(t * 32, 256), 256, 0, ss>>>(d, bin_off, vcell, d.tids);
-        if (radix_sort_pairs((int)nv, vcell, d.tids, 0, radix_passes((unsigned)(2 * d.cells - 1)), bin_sort, ss))
+        if (radix_sort_pairs((int)nv, vcell, d.tids, radix_bits((unsigned)(2 * d.cells - 1)), bin_sort, d.err, ss))
             return CCT_CUDAERR;
         cudaMemsetAsync(d.tcs, 0xff, sizeof(int) * 4 * d.cells, ss);
         MPS_COUNT_LAUNCH k_bin_bounds<<<blocks_for((int)nv), kBlock, 0, ss>>>((int)nv, vcell, d.tcs,

@@ -5,66 +5,39 @@
 // sort is a stable radix sort, so the result is uniquely the stable order; this sort
 // produces exactly that order.
 //
-// Per 8-bit digit pass:
-//   k_digit_hist : each 2048-key tile counts its digits (warp-aggregated with
-//                  __match_any_sync, then shared-memory adds); counts stored
-//                  digit-major: counts[d * tiles + tile]
-//                  and adds its per-digit totals to dtot[pass][d]
-//   k_scan_digits: CTA per digit d: base(d) = sum of the totals of the smaller
-//                  digits, then the exclusive scan of counts[d][0..tiles) from base(d)
-//   k_scatter    : each tile re-reads its keys in index order (warp w owns keys
-//                  [w*256, w*256+256) of the tile, 32 per round), ranks them stably
-//                  with __match_any_sync + per-warp running digit counters, and
-//                  writes key and value to offset[d][tile] + warp prefix + rank.
-// Keys are sorted as unsigned offsets (key - kmin), so negative keys sort correctly
-// and a pass runs only for the digits the key range actually spans.  With the range in
-// device memory (radix_sort_pairs_range) the host launches the largest number of passes
-// and each pass's kernels read the range and return at once past the passes it needs,
-// so the caller does not wait for the key range on the host.
+// One cooperative launch (k_sort) does the whole sort: the key range when the caller does
+// not know it, then passes of equal digits of at most 9 bits, least significant first.  CTA
+// c owns the c-th contiguous part of the keys.  Per pass, with a grid barrier after each
+// step:
+//   count    each CTA counts its keys' digits (warp-aggregated with __match_any_sync, then
+//            shared-memory adds): counts[c][d]
+//   prefix   a warp per digit turns counts[.][d] into the exclusive prefix over the CTAs
+//            and leaves the digit's total
+//   scatter  each CTA scans the totals, ranks its keys stably (warp w owns a contiguous
+//            share, 32 keys a round, ranked with __match_any_sync and per-warp running
+//            counters) and writes key and value to total prefix + CTA prefix + warp prefix
+//            + rank
+// Up to 4,096 keys run on one CTA, without barriers.  Keys are sorted as unsigned offsets
+// (key - kmin), so negative keys sort correctly and only the bits that the range spans are
+// sorted.
+//
+// What bounds it: latency, of the barriers and of each step's few dependent loads; the keys
+// and values stay in L2.  It replaces three launches per 8-bit pass, 13 to 16 per sort with
+// the range's and those of passes beyond the range, which returned at once; finding the
+// range alone took 27 us at 882,080 keys (19,456 atomics on one address).
+#include <limits.h>
+
 #include "mps_common.cuh"
 #include "mps_internal.h"
 
 namespace mps {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;
-constexpr int kRadix = kRadixBuckets;
-static_assert(kSortTile == kRadixSortTile, "tile size of the scratch formula");
-
-__device__ __forceinline__ unsigned digit_of(int key, int kmin, int shift) {
-    return (((unsigned)key - (unsigned)kmin) >> shift) & 255u;
-}
-// 8-bit passes a key range needs (radix_passes on the device)
-__device__ __forceinline__ int range_passes(unsigned range) { return range == 0u ? 0 : (39 - __clz((int)range)) / 8; }
-// with the key range (min, max) in device memory: the pass's kmin, false when the pass
-// is past the ones the range needs
-__device__ __forceinline__ bool pass_live(const int* __restrict__ mm, int shift, int& kmin) {
-    if (!mm) return true;
-    kmin = mm[0];
-    return shift / 8 < range_passes((unsigned)mm[1] - (unsigned)mm[0]);
-}
-
-__global__ void __launch_bounds__(kSortThreads) k_digit_hist(const int* __restrict__ keys, int n, int kmin, int shift,
-                                                            int tiles, unsigned* __restrict__ counts,
-                                                            unsigned* __restrict__ dtot, const int* __restrict__ mm) {
-    if (!pass_live(mm, shift, kmin)) return;
-    __shared__ unsigned h[kRadix];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int base = blockIdx.x * kSortTile;
-    for (int r = 0; r < kSortItems; ++r) {
-        const int idx = base + r * kSortThreads + threadIdx.x;
-        const bool ok = idx < n;
-        const unsigned d = ok ? digit_of(keys[idx], kmin, shift) : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        if (ok && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&h[d], (unsigned)__popc(peers));
-    }
-    __syncthreads();
-    counts[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
-    if (h[threadIdx.x]) atomicAdd(&dtot[threadIdx.x], h[threadIdx.x]);
-}
+constexpr int kSortThreads = 512;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortRounds = 12;                          // most rounds of 32 keys per warp and tile
+constexpr int kSortTile = kSortThreads * kSortRounds;    // most keys of a tile
+constexpr int kRadix = 1 << kRadixDigitBits;
+static_assert(kRadix == kSortThreads, "a thread per digit");
 
 // Exclusive scan of len unsigned values, in place, by one CTA of 1024 threads.
 __global__ void __launch_bounds__(1024) k_scan_excl(unsigned* __restrict__ a, int len, unsigned* __restrict__ total) {
@@ -135,37 +108,6 @@ __device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned* ws, un
     return ex;
 }
 
-// CTA per digit: offsets[d][t] = base(d) + sum of counts[d][t' < t], in place
-__global__ void __launch_bounds__(kScanThreads) k_scan_digits(unsigned* __restrict__ counts, int tiles,
-                                                              const unsigned* __restrict__ dtot,
-                                                              const int* __restrict__ mm, int shift) {
-    int kmin_unused = 0;
-    if (!pass_live(mm, shift, kmin_unused)) return;
-    __shared__ unsigned ws[32];
-    __shared__ unsigned carry;
-    const int d = blockIdx.x;
-    unsigned v = threadIdx.x < (unsigned)d ? dtot[threadIdx.x] : 0u;   // d < 256 <= blockDim
-    unsigned base;
-    (void)block_exclusive(v, ws, base);
-    if (threadIdx.x == 0) carry = base;
-    __syncthreads();
-    unsigned* row = counts + (size_t)d * tiles;
-    for (int c0 = 0; c0 < tiles; c0 += 4 * kScanThreads) {
-        const int o4 = c0 + 4 * threadIdx.x;
-        const unsigned v0 = o4 < tiles ? row[o4] : 0u, v1 = o4 + 1 < tiles ? row[o4 + 1] : 0u;
-        const unsigned v2 = o4 + 2 < tiles ? row[o4 + 2] : 0u, v3 = o4 + 3 < tiles ? row[o4 + 3] : 0u;
-        unsigned total;
-        const unsigned ex = block_exclusive(v0 + v1 + v2 + v3, ws, total) + carry;
-        if (o4 < tiles) row[o4] = ex;
-        if (o4 + 1 < tiles) row[o4 + 1] = ex + v0;
-        if (o4 + 2 < tiles) row[o4 + 2] = ex + v0 + v1;
-        if (o4 + 3 < tiles) row[o4 + 3] = ex + v0 + v1 + v2;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += total;
-        __syncthreads();
-    }
-}
-
 __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(const unsigned* __restrict__ a, int len,
                                                                  unsigned* __restrict__ sums) {
     __shared__ unsigned ws[32];
@@ -218,168 +160,257 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(unsigned* __restric
     if (total_dev && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *total_dev = off + total;
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_scatter(const int* __restrict__ kin, const int* __restrict__ vin,
-                                                         int* __restrict__ kout, int* __restrict__ vout, int n,
-                                                         int kmin, int shift, int tiles,
-                                                         const unsigned* __restrict__ offsets,
-                                                         const int* __restrict__ mm) {
-    if (!pass_live(mm, shift, kmin)) return;
-    __shared__ unsigned wcount[kSortThreads / 32][kRadix];
-    __shared__ unsigned toff[kRadix];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (kSortThreads / 32) * kRadix; i += kSortThreads) (&wcount[0][0])[i] = 0;
-    toff[threadIdx.x] = offsets[threadIdx.x * tiles + blockIdx.x];
+// Bounded barrier of the CTAs of a cooperative launch: arrive on bar[0] (zero at launch),
+// the last arrival resets it and advances the generation bar[1].  False when the wait ran
+// out (the CTA then returns, so the others run out too).
+__device__ __forceinline__ bool sort_barrier(unsigned* bar, unsigned* err) {
+    __shared__ int ok;
     __syncthreads();
-    const int base = blockIdx.x * kSortTile + w * (32 * kSortItems);
-    int key[kSortItems], val[kSortItems];
-    unsigned dig[kSortItems], rank[kSortItems];
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const int idx = base + r * 32 + lane;
-        const bool ok = idx < n;
-        key[r] = ok ? kin[idx] : 0;
-        val[r] = ok ? vin[idx] : 0;
-        const unsigned d = ok ? digit_of(key[r], kmin, shift) : 256u;
-        dig[r] = d;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const unsigned lt = peers & ((1u << lane) - 1u);
-        const unsigned before = ok ? wcount[w][d] : 0u;
-        __syncwarp();
-        if (ok && lt == 0) wcount[w][d] = before + (unsigned)__popc(peers);
-        __syncwarp();
-        rank[r] = before + (unsigned)__popc(lt);
-    }
-    __syncthreads();
-    {
-        unsigned run = 0;
-        for (int ww = 0; ww < kSortThreads / 32; ++ww) {
-            const unsigned c = wcount[ww][threadIdx.x];
-            wcount[ww][threadIdx.x] = run;
-            run += c;
+    if (gridDim.x == 1) return true;
+    if (threadIdx.x == 0) {
+        volatile unsigned* gen = bar + 1;
+        const unsigned g = *gen;
+        __threadfence();
+        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
+            bar[0] = 0u;
+            __threadfence();
+            atomicAdd(bar + 1, 1u);
+            ok = 1;
+        } else {
+            long long k = 0;
+            while (*gen == g && ++k < (1ll << 20)) {
+            }
+            ok = *gen != g;
+            if (!ok && err) atomicOr(err, MPS_ERR_STAGE_TIMEOUT);
         }
+        __threadfence();
     }
     __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const unsigned d = dig[r];
-        if (d < 256u) {
-            const unsigned dst = toff[d] + wcount[w][d] + rank[r];
-            kout[dst] = key[r];
-            vout[dst] = val[r];
+    return ok != 0;
+}
+
+// Scratch of a sort: barrier words, per-CTA key ranges, digit totals, digit counts
+// [CTA][digit], then the alternate key and value arrays.
+struct SortScratch {
+    unsigned* bar;      // [2]
+    int* range;         // [2][CTAs]
+    unsigned* total;    // [kRadix]
+    unsigned* counts;   // [CTAs][kRadix]
+    int *keys, *vals;   // [n]
+};
+
+// bits: the keys lie in [0, 2^bits); < 0: any int range (found first)
+__global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* keys, int* vals, int bits, SortScratch s,
+                                                       unsigned* err) {
+    __shared__ unsigned wcount[kSortWarps][kRadix];
+    __shared__ unsigned off[kRadix];
+    __shared__ unsigned wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int c = blockIdx.x, ctas = gridDim.x;
+    const int beg = min(n, c * part), end = min(n, beg + part);
+    int kmin = 0;
+    if (bits < 0) {
+        int lo = INT_MAX, hi = INT_MIN;
+        for (int i = beg + tid; i < end; i += kSortThreads) {
+            const int k = keys[i];
+            lo = min(lo, k);
+            hi = max(hi, k);
         }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        int* const r = reinterpret_cast<int*>(wsum);
+        if (lane == 0) {
+            r[w] = lo;
+            r[16 + w] = hi;
+        }
+        __syncthreads();
+        if (w == 0) {
+            const int v = r[lane];   // lanes 0..15 minima, 16..31 maxima
+            const int l2 = __reduce_min_sync(0xffffffffu, lane < 16 ? v : INT_MAX);
+            const int h2 = __reduce_max_sync(0xffffffffu, lane < 16 ? INT_MIN : v);
+            if (lane == 0) {
+                s.range[c] = l2;
+                s.range[ctas + c] = h2;
+            }
+        }
+        if (!sort_barrier(s.bar, err)) return;
+        lo = INT_MAX;
+        hi = INT_MIN;
+        for (int i = lane; i < ctas; i += 32) {
+            lo = min(lo, __ldcg(s.range + i));
+            hi = max(hi, __ldcg(s.range + ctas + i));
+        }
+        kmin = __reduce_min_sync(0xffffffffu, lo);
+        const unsigned range = (unsigned)__reduce_max_sync(0xffffffffu, hi) - (unsigned)kmin;
+        bits = range == 0u ? 0 : 32 - __clz((int)range);
+        __syncthreads();
     }
-}
-
-__global__ void k_minmax(const int* __restrict__ keys, int n, int* __restrict__ mm) {
-    int lo = INT_MAX, hi = INT_MIN;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int k = keys[i];
-        lo = min(lo, k);
-        hi = max(hi, k);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&mm[0], lo);
-        atomicMax(&mm[1], hi);
-    }
-}
-
-// after the passes of radix_sort_pairs_range: an odd number of passes left the pairs
-// in the scratch arrays; copy them back
-__global__ void k_copy_back_odd(const int* __restrict__ mm, int n, const int* __restrict__ ka,
-                                const int* __restrict__ va, int* __restrict__ keys, int* __restrict__ vals) {
-    if ((range_passes((unsigned)mm[1] - (unsigned)mm[0]) & 1) == 0) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        keys[i] = ka[i];
-        vals[i] = va[i];
-    }
-}
-
-__global__ void k_minmax_init(int* mm) {
-    mm[0] = INT_MAX;
-    mm[1] = INT_MIN;
-}
-
-size_t radix_scratch_bytes(int n) { return radix_scratch_bytes_for(n); }
-
-int radix_passes(unsigned range) {
-    int bits = 0;
-    while (bits < 32 && (range >> bits) != 0u) ++bits;
-    return (bits + 7) / 8;
-}
-
-cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int kmin, int passes, void* scratch, cudaStream_t st) {
-    if (n <= 1 || passes <= 0) return cudaSuccess;
-    const int tiles = div_up(n, kSortTile);
-    char* p = (char*)scratch;
-    int* kalt = (int*)p;
-    p += sizeof(int) * (size_t)n;
-    int* valt = (int*)p;
-    p += sizeof(int) * (size_t)n;
-    unsigned* counts = (unsigned*)p;
-    unsigned* dtot = counts + (size_t)kRadix * tiles + 8;   // [kRadixMaxPasses][kRadix]
-    if (passes > kRadixMaxPasses) return cudaErrorInvalidValue;
-    cudaMemsetAsync(dtot, 0, sizeof(unsigned) * kRadix * passes, st);
-    int* ka = keys;
-    int* va = vals;
-    int* kb = kalt;
-    int* vb = valt;
+    const int passes = (bits + kRadixDigitBits - 1) / kRadixDigitBits;
+    if (passes == 0) return;
+    const int dbits = (bits + passes - 1) / passes;
+    const unsigned dmask = (1u << dbits) - 1u;
+    int *ka = keys, *va = vals, *kb = s.keys, *vb = s.vals;
     for (int pass = 0; pass < passes; ++pass) {
-        const int shift = pass * 8;
-        unsigned* dt = dtot + (size_t)kRadix * pass;
-        MPS_COUNT_LAUNCH k_digit_hist<<<tiles, kSortThreads, 0, st>>>(ka, n, kmin, shift, tiles, counts, dt, nullptr);
-        MPS_COUNT_LAUNCH k_scan_digits<<<kRadix, kScanThreads, 0, st>>>(counts, tiles, dt, nullptr, shift);
-        MPS_COUNT_LAUNCH k_scatter<<<tiles, kSortThreads, 0, st>>>(ka, va, kb, vb, n, kmin, shift, tiles, counts,
-                                                                   nullptr);
+        const int shift = pass * dbits;
+        auto digit = [&](int key) { return (((unsigned)key - (unsigned)kmin) >> shift) & dmask; };
+        // ---- count (the other CTAs wrote these keys in this launch: through L2) ----
+        off[tid] = 0;
+        __syncthreads();
+        for (int i0 = beg; i0 < end; i0 += kSortThreads) {
+            const int i = i0 + tid;
+            const unsigned d = i < end ? digit(__ldcg(ka + i)) : (unsigned)kRadix;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            if (i < end && (peers & lt) == 0) atomicAdd(&off[d], (unsigned)__popc(peers));
+        }
+        __syncthreads();
+        const unsigned mine = off[tid];
+        if (ctas > 1) {
+            s.counts[(size_t)c * kRadix + tid] = mine;
+            if (!sort_barrier(s.bar, err)) return;
+            // ---- prefix over the CTAs, a warp per digit ----
+            for (int d = c * kSortWarps + w; d < kRadix; d += ctas * kSortWarps) {
+                unsigned run = 0;
+                for (int q0 = 0; q0 < ctas; q0 += 32) {
+                    const int q = q0 + lane;
+                    unsigned* const at = s.counts + (size_t)q * kRadix + d;
+                    const unsigned x = q < ctas ? __ldcg(at) : 0u;
+                    unsigned inc = x;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+                        if (lane >= o) inc += v;
+                    }
+                    if (q < ctas) *at = run + inc - x;
+                    run += __shfl_sync(0xffffffffu, inc, 31);
+                }
+                if (lane == 0) s.total[d] = run;
+            }
+            if (!sort_barrier(s.bar, err)) return;
+        }
+        // ---- first position of each digit's keys of this CTA ----
+        {
+            const unsigned total = ctas > 1 ? __ldcg(s.total + tid) : mine;
+            const unsigned before = ctas > 1 ? __ldcg(s.counts + (size_t)c * kRadix + tid) : 0u;
+            unsigned inc = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            if (lane == 31) wsum[w] = inc;
+            __syncthreads();
+            if (w == 0) {
+                const unsigned x = lane < kSortWarps ? wsum[lane] : 0u;
+                unsigned xi = x;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned v = __shfl_up_sync(0xffffffffu, xi, o);
+                    if (lane >= o) xi += v;
+                }
+                wsum[lane] = xi - x;
+            }
+            __syncthreads();
+            off[tid] = inc - total + wsum[w] + before;
+        }
+        // ---- scatter ----
+        for (int t0 = beg; t0 < end; t0 += kSortTile) {
+            const int tend = min(end, t0 + kSortTile);
+            const int rounds = (tend - t0 + kSortThreads - 1) / kSortThreads;   // of 32 keys per warp
+            for (int q = 0; q < kSortWarps; ++q) wcount[q][tid] = 0;
+            __syncthreads();
+            const int base = t0 + w * 32 * rounds + lane;
+            int key[kSortRounds], val[kSortRounds];
+            unsigned at[kSortRounds];   // digit | rank << 10
+#pragma unroll
+            for (int r = 0; r < kSortRounds; ++r) {
+                if (r < rounds) {
+                    const int i = base + 32 * r;
+                    key[r] = i < tend ? __ldcg(ka + i) : 0;
+                    val[r] = i < tend ? __ldcg(va + i) : 0;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kSortRounds; ++r) {
+                if (r < rounds) {
+                    const bool ok = base + 32 * r < tend;
+                    const unsigned d = ok ? digit(key[r]) : (unsigned)kRadix;
+                    const unsigned peers = __match_any_sync(0xffffffffu, d);
+                    const unsigned lower = peers & lt;
+                    const unsigned seen = ok ? wcount[w][d] : 0u;
+                    __syncwarp();
+                    if (ok && lower == 0) wcount[w][d] = seen + (unsigned)__popc(peers);
+                    __syncwarp();
+                    at[r] = d | (seen + (unsigned)__popc(lower)) << 10;
+                }
+            }
+            __syncthreads();
+            {
+                unsigned run = off[tid];
+#pragma unroll
+                for (int q = 0; q < kSortWarps; ++q) {
+                    const unsigned x = wcount[q][tid];
+                    wcount[q][tid] = run;
+                    run += x;
+                }
+                off[tid] = run;   // the next tile's first positions
+            }
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kSortRounds; ++r) {
+                if (r < rounds) {
+                    const unsigned d = at[r] & 1023u;
+                    if (d < (unsigned)kRadix) {
+                        const unsigned dst = wcount[w][d] + (at[r] >> 10);
+                        kb[dst] = key[r];
+                        vb[dst] = val[r];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (!sort_barrier(s.bar, err)) return;
         int* t = ka; ka = kb; kb = t;
         t = va; va = vb; vb = t;
     }
     if (ka != keys) {
-        cudaMemcpyAsync(keys, ka, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
-        cudaMemcpyAsync(vals, va, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
+        for (int i = beg + tid; i < end; i += kSortThreads) {
+            keys[i] = __ldcg(ka + i);
+            vals[i] = __ldcg(va + i);
+        }
     }
-    return cudaGetLastError();
 }
 
-cudaError_t radix_sort_pairs_range(int n, int* keys, int* vals, const int* mm_dev, void* scratch, cudaStream_t st) {
-    if (n <= 1) return cudaSuccess;
-    const int tiles = div_up(n, kSortTile);
-    char* p = (char*)scratch;
-    int* kalt = (int*)p;
-    p += sizeof(int) * (size_t)n;
-    int* valt = (int*)p;
-    p += sizeof(int) * (size_t)n;
-    unsigned* counts = (unsigned*)p;
-    unsigned* dtot = counts + (size_t)kRadix * tiles + 8;   // [kRadixMaxPasses][kRadix]
-    cudaMemsetAsync(dtot, 0, sizeof(unsigned) * kRadix * kRadixMaxPasses, st);
-    int* ka = keys;
-    int* va = vals;
-    int* kb = kalt;
-    int* vb = valt;
-    for (int pass = 0; pass < kRadixMaxPasses; ++pass) {
-        const int shift = pass * 8;
-        unsigned* dt = dtot + (size_t)kRadix * pass;
-        MPS_COUNT_LAUNCH k_digit_hist<<<tiles, kSortThreads, 0, st>>>(ka, n, 0, shift, tiles, counts, dt, mm_dev);
-        MPS_COUNT_LAUNCH k_scan_digits<<<kRadix, kScanThreads, 0, st>>>(counts, tiles, dt, mm_dev, shift);
-        MPS_COUNT_LAUNCH k_scatter<<<tiles, kSortThreads, 0, st>>>(ka, va, kb, vb, n, 0, shift, tiles, counts, mm_dev);
-        int* t = ka; ka = kb; kb = t;
-        t = va; va = vb; vb = t;
-    }
-    // passes 0, 2 read the caller's arrays and 1, 3 the scratch: after the passes the
-    // range needed, the pairs sit in the scratch arrays when that number is odd
-    MPS_COUNT_LAUNCH k_copy_back_odd<<<min(div_up(n, 256), 152 * 8), 256, 0, st>>>(mm_dev, n, kalt, valt, keys, vals);
-    return cudaGetLastError();
+int radix_bits(unsigned range) {
+    int bits = 0;
+    while (bits < 32 && (range >> bits) != 0u) ++bits;
+    return bits;
 }
 
-cudaError_t key_minmax(int n, const int* keys, int* mm_dev, cudaStream_t st) {
-    MPS_COUNT_LAUNCH k_minmax_init<<<1, 1, 0, st>>>(mm_dev);
-    const int blocks = min(div_up(n, 1024), 152 * 4);
-    if (n > 0) MPS_COUNT_LAUNCH k_minmax<<<blocks, 1024, 0, st>>>(keys, n, mm_dev);
-    return cudaGetLastError();
+cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, cudaStream_t st,
+                             int max_ctas) {
+    if (n <= 1 || bits == 0) return cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), sms));   // one CTA per SM at most: all resident
+    int part = div_up(n, most);
+    part = (part + kSortThreads - 1) / kSortThreads * kSortThreads;
+    const int ctas = div_up(n, part);
+    SortScratch s;
+    unsigned* p = (unsigned*)scratch;
+    s.bar = p;
+    s.range = (int*)(p + 8);
+    s.total = p + 8 + 2 * kRadixMaxCtas;
+    s.counts = s.total + kRadix;
+    s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
+    s.vals = s.keys + n;
+    if (ctas > 1) {
+        const cudaError_t e = cudaMemsetAsync(s.bar, 0, 2 * sizeof(unsigned), st);
+        if (e) return e;
+    }
+    void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err};
+    return MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_sort, dim3(ctas), dim3(kSortThreads), args, 0, st);
 }
 
 cudaError_t scan_exclusive(unsigned* a, int len, unsigned* total_dev, cudaStream_t st, unsigned* tile_sums) {

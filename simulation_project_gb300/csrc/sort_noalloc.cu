@@ -20,8 +20,8 @@
 //     on a device also makes the runtime load the library's module there, so make that
 //     first call before any stream capture;
 //   * every call shares the array, and it keeps the last call's contents: the sort
-//     writes each scratch word before it reads it (min/max re-initialised, histograms
-//     fully rewritten per pass), so nothing is stale -- but calls that overlap on the
+//     writes each scratch word before it reads it (barrier words re-initialised, digit
+//     counts fully rewritten per pass), so nothing is stale -- but calls that overlap on the
 //     GPU (from several host threads or streams) race on it and must be serialised;
 //   * like SortUsingThrust it runs on the legacy default stream and returns after the
 //     sort has finished.
@@ -35,8 +35,10 @@ namespace mps {
 namespace {
 
 constexpr int kNoAllocMaxKeys = 1 << 18;
-constexpr size_t kNoAllocHeader = 256;  // min/max words, padded to the array alignment
-constexpr size_t kNoAllocSortBytes = radix_scratch_bytes_for(kNoAllocMaxKeys);
+constexpr int kNoAllocCtas = 64;        // of a sort: what their digit counts fit
+constexpr size_t kNoAllocHeader = 256;  // error word, padded to the array alignment
+constexpr size_t kNoAllocSortBytes = 2232864 - kNoAllocHeader;
+static_assert(radix_scratch_bytes_for(kNoAllocMaxKeys, kNoAllocCtas) <= kNoAllocSortBytes, "scratch of the largest sort");
 constexpr size_t kNoAllocBytes = kNoAllocHeader + kNoAllocSortBytes;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -67,19 +69,17 @@ extern "C" CCTStatusType SortUsingThrustNoAlloc(Integer MaxParticleNum, Integer*
         return CCT_PARAMERR;
     }
     if (n <= 1) return CCT_NOERR;
-    if (radix_scratch_bytes(n) > kNoAllocSortBytes) return CCT_PARAMERR;
     void* base = nullptr;
     CCTStatusType rc = noalloc_scratch(&base);
     if (rc != CCT_NOERR) return rc;
-    int* mm = (int*)base;
+    unsigned* err = (unsigned*)base;
     void* scr = (char*)base + kNoAllocHeader;
     cudaStream_t st = 0;
-    MPS_CUDA_TRY(key_minmax(n, daNumberHash, mm, st));
-    int h[2];
-    MPS_CUDA_TRY(cudaMemcpyAsync(h, mm, sizeof(h), cudaMemcpyDeviceToHost, st));
+    unsigned failed = 0;
+    MPS_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
+    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, st, kNoAllocCtas));
+    MPS_CUDA_TRY(cudaMemcpyAsync(&failed, err, sizeof(failed), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
-    const int passes = radix_passes((unsigned)h[1] - (unsigned)h[0]);
-    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, h[0], passes, scr, st));
-    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (failed) return CCT_CUDAERR;
     return cuda_status(cudaGetLastError());
 }
