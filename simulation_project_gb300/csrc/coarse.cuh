@@ -574,35 +574,6 @@ __global__ void k_mg_up(const double* __restrict__ scal, MgLevel lo, MgLevel hi,
     if (lane == 0) lo.e2[I] = lo.e[I] + hi.e2[lo.par[I]] + omega * lo.dinv[I] * (lo.r[I] - t);
 }
 
-// Bounded barrier of all CTAs of a cooperative launch (every CTA resident): arrive on
-// bar[0], the last arrival resets it and advances the generation bar[1]; a wait that
-// runs out sets MPS_ERR_STAGE_TIMEOUT and returns false (the CTA then stops, so the
-// others run out too).
-__device__ __forceinline__ bool coop_barrier(unsigned* bar, unsigned* err, long long spins) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* gen = bar + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            bar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-            ok = 1;
-        } else {
-            long long k = 0;
-            while (*gen == g && ++k < spins) {
-            }
-            ok = *gen != g;
-            if (!ok) atomicOr(err, MPS_ERR_STAGE_TIMEOUT);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 // The coarse part of a V-cycle in one cooperative launch: the restrictions level 1 ->
 // 2 -> ... -> last with their first down sweeps (as k_mg_down, a warp per aggregate of
 // the coarser level), the dense solve of the last level (a warp per row),
@@ -617,7 +588,6 @@ __global__ void __launch_bounds__(256) k_mg_coarse_cycle(const double* __restric
     const int w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int lv = mg.levels;
     const float omega = mg.omega;
-    constexpr long long kSpins = 1ll << 20;
     for (int l = 1; l < lv; ++l) {
         const MgLevel& lo = mg.L[l];
         const MgLevel& hi = mg.L[l + 1];
@@ -629,7 +599,7 @@ __global__ void __launch_bounds__(256) k_mg_coarse_cycle(const double* __restric
                 hi.e[I2] = omega * hi.dinv[I2] * s;
             }
         }
-        if (!coop_barrier(bar, err, kSpins)) return;
+        if (!coop_barrier(bar, err)) return;
     }
     {   // the last level: e2 = A^-1 r with the explicit inverse, a warp per row
         const MgLevel& L = mg.L[lv];
@@ -642,7 +612,7 @@ __global__ void __launch_bounds__(256) k_mg_coarse_cycle(const double* __restric
         }
     }
     if (lv <= 2) return;
-    if (!coop_barrier(bar, err, kSpins)) return;
+    if (!coop_barrier(bar, err)) return;
     for (int l = lv - 1; l >= 2; --l) {
         const MgLevel& lo = mg.L[l];
         const MgLevel& hi = mg.L[l + 1];
@@ -658,7 +628,7 @@ __global__ void __launch_bounds__(256) k_mg_coarse_cycle(const double* __restric
             if (lane == 0)
                 lo.e2[I] = __ldcg(lo.e + I) + __ldcg(hi.e2 + lo.par[I]) + omega * lo.dinv[I] * (__ldcg(lo.r + I) - t);
         }
-        if (l > 2 && !coop_barrier(bar, err, kSpins)) return;
+        if (l > 2 && !coop_barrier(bar, err)) return;
     }
 }
 

@@ -22,7 +22,10 @@
 // sorted.
 //
 // What bounds it: latency, of the barriers and of each step's few dependent loads; the keys
-// and values stay in L2.  It replaces three launches per 8-bit pass, 13 to 16 per sort with
+// and values stay in L2.  882,080 nearly sorted keys of 17 bits, in us: range 6, then per
+// pass count 2.6, prefix 1, scan 0.6, scatter 4.4 and three barriers of 1.2 to 2.2; 34 in
+// all (random keys 68: their scatter takes 14, 16,000 keys 21 to 26).  Two CTAs per SM took
+// 40 and 72.  It replaces three launches per 8-bit pass, 13 to 16 per sort with
 // the range's and those of passes beyond the range, which returned at once; finding the
 // range alone took 27 us at 882,080 keys (19,456 atomics on one address).
 #include <limits.h>
@@ -160,39 +163,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(unsigned* __restric
     if (total_dev && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *total_dev = off + total;
 }
 
-// Bounded barrier of the CTAs of a cooperative launch: arrive on bar[0] (zero at launch),
-// the last arrival resets it and advances the generation bar[1].  False when the wait ran
-// out (the CTA then returns, so the others run out too).
-__device__ __forceinline__ bool sort_barrier(unsigned* bar, unsigned* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (gridDim.x == 1) return true;
-    if (threadIdx.x == 0) {
-        volatile unsigned* gen = bar + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            bar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-            ok = 1;
-        } else {
-            long long k = 0;
-            while (*gen == g && ++k < (1ll << 20)) {
-            }
-            ok = *gen != g;
-            if (!ok && err) atomicOr(err, MPS_ERR_STAGE_TIMEOUT);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-// Scratch of a sort: barrier words, per-CTA key ranges, digit totals, digit counts
+// Scratch of a sort: the barrier's word, per-CTA key ranges, digit totals, digit counts
 // [CTA][digit], then the alternate key and value arrays.
 struct SortScratch {
-    unsigned* bar;      // [2]
+    unsigned* bar;
     int* range;         // [2][CTAs]
     unsigned* total;    // [kRadix]
     unsigned* counts;   // [CTAs][kRadix]
@@ -200,7 +174,7 @@ struct SortScratch {
 };
 
 // bits: the keys lie in [0, 2^bits); < 0: any int range (found first)
-__global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* keys, int* vals, int bits, SortScratch s,
+__global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* keys, int* vals, int bits, SortScratch s,
                                                        unsigned* err) {
     __shared__ unsigned wcount[kSortWarps][kRadix];
     __shared__ unsigned off[kRadix];
@@ -212,6 +186,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* key
     int kmin = 0;
     if (bits < 0) {
         int lo = INT_MAX, hi = INT_MIN;
+#pragma unroll 6
         for (int i = beg + tid; i < end; i += kSortThreads) {
             const int k = keys[i];
             lo = min(lo, k);
@@ -234,7 +209,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* key
                 s.range[ctas + c] = h2;
             }
         }
-        if (!sort_barrier(s.bar, err)) return;
+        if (!coop_barrier(s.bar, err)) return;
         lo = INT_MAX;
         hi = INT_MIN;
         for (int i = lane; i < ctas; i += 32) {
@@ -254,39 +229,70 @@ __global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* key
     for (int pass = 0; pass < passes; ++pass) {
         const int shift = pass * dbits;
         auto digit = [&](int key) { return (((unsigned)key - (unsigned)kmin) >> shift) & dmask; };
-        // ---- count (the other CTAs wrote these keys in this launch: through L2) ----
+        // a part of one tile is loaded once per pass, values included (the other CTAs wrote
+        // these pairs in this launch: through L2)
+        const bool one = end - beg <= kSortTile;
+        int key[kSortRounds], val[kSortRounds];
+        auto load = [&](int t0, int tend, int rounds) {
+            const int base = t0 + w * 32 * rounds + lane;
+#pragma unroll
+            for (int r = 0; r < kSortRounds; ++r) {
+                if (r < rounds) {
+                    const int i = base + 32 * r;
+                    key[r] = i < tend ? __ldcg(ka + i) : 0;
+                    val[r] = i < tend ? __ldcg(va + i) : 0;
+                }
+            }
+        };
+        // ---- count ----
         off[tid] = 0;
         __syncthreads();
-        for (int i0 = beg; i0 < end; i0 += kSortThreads) {
-            const int i = i0 + tid;
-            const unsigned d = i < end ? digit(__ldcg(ka + i)) : (unsigned)kRadix;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
-            if (i < end && (peers & lt) == 0) atomicAdd(&off[d], (unsigned)__popc(peers));
+        for (int t0 = beg; t0 < end; t0 += kSortTile) {
+            const int tend = min(end, t0 + kSortTile);
+            const int rounds = (tend - t0 + kSortThreads - 1) / kSortThreads;   // of 32 keys per warp
+            load(t0, tend, rounds);
+#pragma unroll
+            for (int r = 0; r < kSortRounds; ++r) {
+                if (r < rounds) {
+                    const bool ok = t0 + w * 32 * rounds + lane + 32 * r < tend;
+                    const unsigned d = ok ? digit(key[r]) : (unsigned)kRadix;
+                    const unsigned peers = __match_any_sync(0xffffffffu, d);
+                    if (ok && (peers & lt) == 0) atomicAdd(&off[d], (unsigned)__popc(peers));
+                }
+            }
         }
         __syncthreads();
         const unsigned mine = off[tid];
         if (ctas > 1) {
             s.counts[(size_t)c * kRadix + tid] = mine;
-            if (!sort_barrier(s.bar, err)) return;
-            // ---- prefix over the CTAs, a warp per digit ----
-            for (int d = c * kSortWarps + w; d < kRadix; d += ctas * kSortWarps) {
-                unsigned run = 0;
-                for (int q0 = 0; q0 < ctas; q0 += 32) {
-                    const int q = q0 + lane;
-                    unsigned* const at = s.counts + (size_t)q * kRadix + d;
-                    const unsigned x = q < ctas ? __ldcg(at) : 0u;
-                    unsigned inc = x;
+            if (!coop_barrier(s.bar, err)) return;
+            // ---- prefix over the CTAs, a warp per digit, a run of CTAs per lane ----
+            constexpr int kRun = (kRadixMaxCtas + 31) / 32;
+            for (int d = w * ctas + c; d < kRadix; d += ctas * kSortWarps) {   // spread over the SMs
+                unsigned x[kRun], sum = 0;
 #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
-                        if (lane >= o) inc += v;
-                    }
-                    if (q < ctas) *at = run + inc - x;
-                    run += __shfl_sync(0xffffffffu, inc, 31);
+                for (int q = 0; q < kRun; ++q) {
+                    const int k = lane * kRun + q;
+                    x[q] = k < ctas ? __ldcg(s.counts + (size_t)k * kRadix + d) : 0u;
                 }
-                if (lane == 0) s.total[d] = run;
+#pragma unroll
+                for (int q = 0; q < kRun; ++q) sum += x[q];
+                unsigned inc = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                unsigned run = inc - sum;
+#pragma unroll
+                for (int q = 0; q < kRun; ++q) {
+                    const int k = lane * kRun + q;
+                    if (k < ctas) s.counts[(size_t)k * kRadix + d] = run;
+                    run += x[q];
+                }
+                if (lane == 31) s.total[d] = inc;
             }
-            if (!sort_barrier(s.bar, err)) return;
+            if (!coop_barrier(s.bar, err)) return;
         }
         // ---- first position of each digit's keys of this CTA ----
         {
@@ -320,16 +326,8 @@ __global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* key
             for (int q = 0; q < kSortWarps; ++q) wcount[q][tid] = 0;
             __syncthreads();
             const int base = t0 + w * 32 * rounds + lane;
-            int key[kSortRounds], val[kSortRounds];
+            if (!one) load(t0, tend, rounds);
             unsigned at[kSortRounds];   // digit | rank << 10
-#pragma unroll
-            for (int r = 0; r < kSortRounds; ++r) {
-                if (r < rounds) {
-                    const int i = base + 32 * r;
-                    key[r] = i < tend ? __ldcg(ka + i) : 0;
-                    val[r] = i < tend ? __ldcg(va + i) : 0;
-                }
-            }
 #pragma unroll
             for (int r = 0; r < kSortRounds; ++r) {
                 if (r < rounds) {
@@ -369,7 +367,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort(int n, int part, int* key
             }
             __syncthreads();
         }
-        if (!sort_barrier(s.bar, err)) return;
+        if (!coop_barrier(s.bar, err)) return;
         int* t = ka; ka = kb; kb = t;
         t = va; va = vb; vb = t;
     }
@@ -393,7 +391,7 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), sms));   // one CTA per SM at most: all resident
+    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), sms));   // one per SM at most: all resident
     int part = div_up(n, most);
     part = (part + kSortThreads - 1) / kSortThreads * kSortThreads;
     const int ctas = div_up(n, part);
@@ -406,7 +404,7 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
     s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
     s.vals = s.keys + n;
     if (ctas > 1) {
-        const cudaError_t e = cudaMemsetAsync(s.bar, 0, 2 * sizeof(unsigned), st);
+        const cudaError_t e = cudaMemsetAsync(s.bar, 0, sizeof(unsigned), st);
         if (e) return e;
     }
     void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err};
