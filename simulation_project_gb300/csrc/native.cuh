@@ -39,6 +39,41 @@ struct Consts {
     double g[3];
     int dim;
     int explicit_pressure;
+    // what the particle kernels would otherwise compute per thread on GB300's few FP64 units
+    // (a warp instruction takes about 16 cycles of an SM's, a division ten of them); set by
+    // derive(), each by the expression it stands for, so results keep their bits
+    double grid_lo[3], ics;          // buffered zone's minimum, 1 / cell size
+    long long zone_lo[3], zone_hi[3];   // compute zone -/+ tol as ordered integers (ordered_f64)
+    double src;                      // gamma rho / dt^2
+    double c3;                       // -dt / rho
+    double vmax2;                    // below it a squared speed is certainly not above vmax^2
+
+    // integers in the order of the doubles (NaN aside); the two zeros are neighbours
+    __host__ __device__ static long long ordered_f64(double x) {
+        long long b;
+#ifdef __CUDA_ARCH__
+        b = __double_as_longlong(x);
+#else
+        __builtin_memcpy(&b, &x, sizeof(b));
+#endif
+        return b < 0 ? b ^ 0x7fffffffffffffffll : b;
+    }
+    void derive(const CGridBox& box) {
+        const Scalar3 &g0 = box.m_BufferedZone.m_MinBound, &z0 = box.m_ComputeZone.m_MinBound,
+                      &z1 = box.m_ComputeZone.m_MaxBound;
+        const float lo0[3] = {g0.x, g0.y, g0.z}, lo1[3] = {z0.x, z0.y, z0.z}, hi1[3] = {z1.x, z1.y, z1.z};
+        for (int a = 0; a < 3; ++a) {
+            grid_lo[a] = (double)lo0[a];
+            const double lo = (double)lo1[a] - tol, hi = (double)hi1[a] + tol;
+            // x < 0 holds for neither zero, x > 0 neither: the bound is the outer one
+            zone_lo[a] = ordered_f64(lo == 0.0 ? -0.0 : lo);
+            zone_hi[a] = ordered_f64(hi == 0.0 ? 0.0 : hi);
+        }
+        ics = 1.0 / (double)box.m_CellSize;
+        src = gamma * rho / (dt * dt);
+        c3 = -dt / rho;
+        vmax2 = vmax * vmax * (1.0 - 1e-12);
+    }
 };
 
 struct Dev {

@@ -190,11 +190,29 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* red, unsign
 // ---------------------------------------------------------------------------
 // grid build
 // ---------------------------------------------------------------------------
-__global__ void k_zone_flags(const __grid_constant__ Dev d, unsigned* keep) {
+// in_zone<double> by comparisons of ordered integers (six FP64 comparisons and as many
+// additions took 33 us at 882,080 particles, 28 MB of positions); NaN is in the zone
+__device__ __forceinline__ bool in_zone_f64(const Consts& c, const dbl4& p) {
+    const double x[3] = {p.x, p.y, p.z};
+    bool in = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const long long v = Consts::ordered_f64(x[a]), b = __double_as_longlong(x[a]);
+        const bool nan = (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+        in = in && (nan || (v >= c.zone_lo[a] && v <= c.zone_hi[a]));
+    }
+    return in;
+}
+// flags of the particles that stay, and how many leave (*gone, zero on entry)
+__global__ void k_zone_flags(const __grid_constant__ Dev d, unsigned* keep, unsigned* gone) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
-    const dbl4 p = d.pos[i];
-    keep[i] = in_zone<double>(d.box, p.x, p.y, p.z, d.c.tol) ? 1u : 0u;
+    bool in = true;
+    if (i < d.n) {
+        in = in_zone_f64(d.c, d.pos[i]);
+        keep[i] = in ? 1u : 0u;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, !in);
+    if (m && (threadIdx.x & 31) == 0) atomicAdd(gone, (unsigned)__popc(m));
 }
 
 // stable compaction: survivors keep their relative order
@@ -218,10 +236,9 @@ __global__ void k_hash(const __grid_constant__ Dev d) {
     const dbl4 p = d.pos[i];
     // cell coordinates from one reciprocal (FP64 divisions are slow on GB300's narrow
     // FP64 pipe); only a coordinate within an ulp of a cell face can land otherwise
-    const double ics = 1.0 / (double)d.box.m_CellSize;
-    const double fz = (p.z - (double)d.box.m_BufferedZone.m_MinBound.z) * ics;
-    const int a = f2i((p.x - (double)d.box.m_BufferedZone.m_MinBound.x) * ics);
-    const int b = f2i((p.y - (double)d.box.m_BufferedZone.m_MinBound.y) * ics);
+    const double fz = (p.z - d.c.grid_lo[2]) * d.c.ics;
+    const int a = f2i((p.x - d.c.grid_lo[0]) * d.c.ics);
+    const int b = f2i((p.y - d.c.grid_lo[1]) * d.c.ics);
     const int c = f2i(fz);
     int k = cell_key(d.box.m_GridSize, a, b, c);
     if (k < 0 || k >= d.cells) {
@@ -902,7 +919,7 @@ __global__ void k_ppe_setup(const __grid_constant__ Dev d) {
     if (in) {
         const double dg = d.c.coef_lap * d.sumw[i] + d.c.kappa;
         d.diag[i] = dg;
-        d.rhs[i] = d.c.gamma * d.c.rho / (d.c.dt * d.c.dt) * (pnd - d.c.n0_pnd) / d.c.n0_pnd;
+        d.rhs[i] = d.c.src * (pnd - d.c.n0_pnd) / d.c.n0_pnd;
         d.minv[i] = 1.0 / dg;
     } else {
         d.diag[i] = 1.0;
@@ -1825,7 +1842,7 @@ __global__ void __launch_bounds__(W * 32, MINB) k_spmv_stream64(const __grid_con
 // same per-entry operations and accumulator order as k_residual_df (entries of even
 // index into the first (hi, lo) pair, odd into the second, merged at the end), so r
 // is bit-identical to it.  Norms -> S_RR / S_RNORM and ||b|| -> S_BNORM.
-template <int SC, int SS, int W, int MINB, bool WIDE = false>
+template <int SC, int SS, int W, int MINB, bool WIDE = false, int SPLIT = 1>
 __global__ void __launch_bounds__(W * 32, MINB) k_residual_stream(const __grid_constant__ Dev d,
                                                                  const float* __restrict__ w,
                                                                  const double* __restrict__ x,
@@ -1835,24 +1852,29 @@ __global__ void __launch_bounds__(W * 32, MINB) k_residual_stream(const __grid_c
     extern __shared__ __align__(128) unsigned char stream_smem[];
     __shared__ __align__(8) unsigned long long bars[W][SS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gw = blockIdx.x * W + warp, nw = gridDim.x * W;
-    SliceRing<SC, SS, float, WIDE> R;
-    R.init(d, w, stream_smem + warp * SS * SliceRing<SC, SS, float, WIDE>::SB, bars[warp], gw, nw);
+    constexpr int G = W / SPLIT;   // slices of a CTA
+    const int sub = warp % SPLIT;
+    __shared__ float2 share[SPLIT > 1 ? 2 : 1][SPLIT > 1 ? W : 1][32];
+    using Ring = SliceRing<SC, SS, float, WIDE, SPLIT>;
+    Ring R;
+    R.init(d, w, stream_smem + warp * SS * Ring::SB, bars[warp], blockIdx.x * G + warp / SPLIT, gridDim.x * G, sub);
     const float2* __restrict__ xs = d.xs;
 
     double part0 = 0.0, part1 = 0.0;
-    for (int sl = gw; sl < R.nsl; sl += nw) {
+    for (int s0 = blockIdx.x * G, buf = 0; s0 < R.nsl; s0 += gridDim.x * G, buf ^= 1) {
+        const int sl = s0 + warp / SPLIT;
+        if (SPLIT == 1 && sl >= R.nsl) break;
         const int i = sl * 32 + lane;
-        const bool row = i < d.n;
+        const bool row = sl < R.nsl && i < d.n;
         const bool in = row && d.inner[i];
         const int cnt = in ? d.nbr_cnt[i] : 0;
-        const int km = d.skmax[sl];
+        const int km = sl < R.nsl ? d.skmax[sl] : 0;
         float S0 = 0.f, C0 = 0.f, S1 = 0.f, C1 = 0.f;
         bool done = false;
         if ((WIDE || km >= 0) && R.streaming) {
-            const int nc = (slice_kmax(km) + SC - 1) / SC;
+            const int c1 = R.end_chunk(slice_kmax(km));
             const int r0 = sl * 32;
-            for (int c = 0; c < nc; ++c) {
+            for (int c = R.first_chunk(slice_kmax(km)); c < c1; ++c) {
                 const unsigned char* cs;
                 const float* ws;
                 if (!R.acquire(cs, ws)) break;
@@ -1892,10 +1914,24 @@ __global__ void __launch_bounds__(W * 32, MINB) k_residual_stream(const __grid_c
             }
         }
         if (!done) {
-            const int kmax = __reduce_max_sync(0xffffffffu, cnt);
-            const size_t base = (size_t)sl * d.K * 32 + lane;
-            if (km >= 0) df_row_sum<true>(d, w, xs, base, cnt, kmax, sl * 32, S0, C0);
-            else df_row_sum<false>(d, w, xs, base, cnt, kmax, -1, S0, C0);
+            // 32-bit slice (the first of its warps), or streaming given up (the warp's share)
+            const bool wide = km < 0;
+            const int k0 = wide ? 0 : R.first_chunk(km) * SC;
+            const int kmax = wide ? (sub == 0 ? __reduce_max_sync(0xffffffffu, cnt) : 0) : min(km, R.end_chunk(km) * SC) - k0;
+            const size_t base = ((size_t)sl * d.K + k0) * 32 + lane;
+            S0 = C0 = 0.f;
+            if (!wide) df_row_sum<true>(d, w, xs, base, cnt - k0, kmax, sl * 32, S0, C0);
+            else if (sub == 0) df_row_sum<false>(d, w, xs, base, cnt, kmax, -1, S0, C0);
+        }
+        if constexpr (SPLIT > 1) {
+            share[buf][warp][lane] = make_float2(S0, C0);
+            __syncthreads();
+            if (sub != 0) continue;
+#pragma unroll
+            for (int q = 1; q < SPLIT; ++q) {
+                const float2 v = share[buf][warp + q][lane];
+                df_add(S0, C0, v.x, v.y);
+            }
         }
         if (!row) continue;
         if (!in) {
@@ -1924,7 +1960,7 @@ __global__ void __launch_bounds__(W * 32, MINB) k_residual_stream(const __grid_c
 // b - A x recomputed, this adds the FP64 rounding of the x update, 2^-53 |x_i| per row,
 // well inside the double-float residual's own 2^-44 of sum |w x|.  Non-interior rows keep
 // r = 0 and x.
-template <int SC, int SS, int W, int MINB, bool WIDE = false>
+template <int SC, int SS, int W, int MINB, bool WIDE = false, int SPLIT = 1>
 __global__ void __launch_bounds__(W * 32, MINB) k_residual_update_stream(const __grid_constant__ Dev d,
                                                                         const float* __restrict__ w,
                                                                         const float* __restrict__ dv, double s,
@@ -1934,23 +1970,28 @@ __global__ void __launch_bounds__(W * 32, MINB) k_residual_update_stream(const _
     extern __shared__ __align__(128) unsigned char stream_smem[];
     __shared__ __align__(8) unsigned long long bars[W][SS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gw = blockIdx.x * W + warp, nw = gridDim.x * W;
-    SliceRing<SC, SS, float, WIDE> R;
-    R.init(d, w, stream_smem + warp * SS * SliceRing<SC, SS, float, WIDE>::SB, bars[warp], gw, nw);
+    constexpr int G = W / SPLIT;   // slices of a CTA
+    const int sub = warp % SPLIT;
+    __shared__ float2 share[SPLIT > 1 ? 2 : 1][SPLIT > 1 ? W : 1][32];
+    using Ring = SliceRing<SC, SS, float, WIDE, SPLIT>;
+    Ring R;
+    R.init(d, w, stream_smem + warp * SS * Ring::SB, bars[warp], blockIdx.x * G + warp / SPLIT, gridDim.x * G, sub);
 
     double part0 = 0.0;
-    for (int sl = gw; sl < R.nsl; sl += nw) {
+    for (int s0 = blockIdx.x * G, buf = 0; s0 < R.nsl; s0 += gridDim.x * G, buf ^= 1) {
+        const int sl = s0 + warp / SPLIT;
+        if (SPLIT == 1 && sl >= R.nsl) break;
         const int i = sl * 32 + lane;
-        const bool row = i < d.n;
+        const bool row = sl < R.nsl && i < d.n;
         const bool in = row && d.inner[i];
         const int cnt = in ? d.nbr_cnt[i] : 0;
-        const int km = d.skmax[sl];
+        const int km = sl < R.nsl ? d.skmax[sl] : 0;
         float S0 = 0.f, C0 = 0.f, S1 = 0.f, C1 = 0.f;
         bool done = false;
         if ((WIDE || km >= 0) && R.streaming) {
-            const int nc = (slice_kmax(km) + SC - 1) / SC;
+            const int c1 = R.end_chunk(slice_kmax(km));
             const int r0 = sl * 32;
-            for (int c = 0; c < nc; ++c) {
+            for (int c = R.first_chunk(slice_kmax(km)); c < c1; ++c) {
                 const unsigned char* cs;
                 const float* ws;
                 if (!R.acquire(cs, ws)) break;
@@ -1985,10 +2026,24 @@ __global__ void __launch_bounds__(W * 32, MINB) k_residual_update_stream(const _
             }
         }
         if (!done) {
-            const int kmax = __reduce_max_sync(0xffffffffu, cnt);
-            const size_t base = (size_t)sl * d.K * 32 + lane;
-            if (km >= 0) df_row_sum<true>(d, w, dv, base, cnt, kmax, sl * 32, S0, C0);
-            else df_row_sum<false>(d, w, dv, base, cnt, kmax, -1, S0, C0);
+            // 32-bit slice (the first of its warps), or streaming given up (the warp's share)
+            const bool wide = km < 0;
+            const int k0 = wide ? 0 : R.first_chunk(km) * SC;
+            const int kmax = wide ? (sub == 0 ? __reduce_max_sync(0xffffffffu, cnt) : 0) : min(km, R.end_chunk(km) * SC) - k0;
+            const size_t base = ((size_t)sl * d.K + k0) * 32 + lane;
+            S0 = C0 = 0.f;
+            if (!wide) df_row_sum<true>(d, w, dv, base, cnt - k0, kmax, sl * 32, S0, C0);
+            else if (sub == 0) df_row_sum<false>(d, w, dv, base, cnt, kmax, -1, S0, C0);
+        }
+        if constexpr (SPLIT > 1) {
+            share[buf][warp][lane] = make_float2(S0, C0);
+            __syncthreads();
+            if (sub != 0) continue;
+#pragma unroll
+            for (int q = 1; q < SPLIT; ++q) {
+                const float2 v = share[buf][warp + q][lane];
+                df_add(S0, C0, v.x, v.y);
+            }
         }
         if (!in) continue;
         const double acc = (double)S0 + (double)C0;
@@ -2482,12 +2537,14 @@ __global__ void k_correct(const __grid_constant__ Dev d) {
 // FP32 copy of the solved pressure (no FP64 arithmetic per pair: GB300's FP64 pipe is
 // narrow), the sums are shuffle-reduced and parked in the particle's lane, and every
 // lane then finishes its own particle (correct_finish, FP64 state update).
-__global__ void k_correct_warp(const __grid_constant__ Dev d) {
+// share: particles per warp.  32 keep the FP64 end lane-parallel; few particles leave the
+// chip idle at that, and a warp's rows run one after another (51 us up to 108,186 particles)
+__global__ void k_correct_warp(const __grid_constant__ Dev d, int share) {
     const int lane = threadIdx.x & 31;
-    const int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
+    const int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * share;
     const float reg = (float)d.c.re_grad, mindg = (float)d.c.mind_grad;
     float mx = 0.f, my = 0.f, mz = 0.f;
-    for (int q = 0; q < 32 && base + q < d.n; ++q) {   // warp-uniform
+    for (int q = 0; q < share && base + q < d.n; ++q) {   // warp-uniform
         const int iq = base + q;
         const float4 pi = d.opos[iq];
         const float Pi = d.pf32[iq];
@@ -2517,7 +2574,7 @@ __global__ void k_correct_warp(const __grid_constant__ Dev d) {
         }
     }
     const int i = base + lane;
-    if (i < d.n) correct_finish<float>(d, i, mx, my, mz);
+    if (lane < share && i < d.n) correct_finish<float>(d, i, mx, my, mz);
 }
 
 // the per-particle end of the correction: FP64 gradient with the wall terms, velocity
@@ -2541,12 +2598,15 @@ __device__ void correct_finish(const Dev& d, int i, T gx, T gy, T gz) {
     }
     const dbl4 v = d.vel[i];
     const dbl4 p = d.pos[i];
-    const double c3 = -d.c.dt / d.c.rho;
+    const double c3 = d.c.c3;
     dbl4 vn = make_dbl4(v.x + c3 * g[0], v.y + c3 * g[1], v.z + c3 * g[2], 0.0);
-    const double a = sqrt(vn.x * vn.x + vn.y * vn.y + vn.z * vn.z);
-    if (a > d.c.vmax) {
-        const double s = d.c.vmax / a;
-        vn.x *= s; vn.y *= s; vn.z *= s;
+    const double a2 = vn.x * vn.x + vn.y * vn.y + vn.z * vn.z;
+    if (a2 > d.c.vmax2) {   // the root only where it can exceed vmax
+        const double a = sqrt(a2);
+        if (a > d.c.vmax) {
+            const double s = d.c.vmax / a;
+            vn.x *= s; vn.y *= s; vn.z *= s;
+        }
     }
     if (!(isfinite(vn.x) && isfinite(vn.y) && isfinite(vn.z))) {
         atomicOr(d.err, MPS_ERR_NONFINITE);

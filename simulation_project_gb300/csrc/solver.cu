@@ -251,6 +251,7 @@ struct Solver {
         c.g[1] = P.GravityConstant.y;
         c.g[2] = P.GravityConstant.z;
         c.explicit_pressure = opt.pressure_mode == MPS_PRESSURE_EXPLICIT;
+        c.derive(d.box);
         timer.on = opt.profile != 0;
         if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return CCT_CUDAERR;
         for (auto& e : gate_ev)
@@ -690,22 +691,29 @@ struct Solver {
         return compact_finish();
     }
     // the compaction's launches (no host wait) and, after them, the wait for the new count
+    // Most steps lose no particle: the flags and their number first, and the scan and the
+    // copy of the state only where particles left (they took 45 us a time at 882,080).
     void compact_launch() {
         const int n = d.n;
         if (n <= 0) return;
-        MPS_COUNT_LAUNCH k_zone_flags<<<blocks_for(n), kBlock, 0, st>>>(d, keep);
-        cudaMemcpyAsync(rank, keep, sizeof(unsigned) * n, cudaMemcpyDeviceToDevice, st);
-        scan_exclusive(rank, n, rank + n, st, scan_sums);
-        MPS_COUNT_LAUNCH k_compact<<<blocks_for(n), kBlock, 0, st>>>(d, keep, rank);
+        cudaMemsetAsync(rank + n, 0, sizeof(unsigned), st);
+        MPS_COUNT_LAUNCH k_zone_flags<<<blocks_for(n), kBlock, 0, st>>>(d, keep, rank + n);
         cudaMemcpyAsync(h_int, rank + n, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
     }
     CCTStatusType compact_finish() {
-        if (d.n <= 0) return CCT_NOERR;
+        const int n = d.n;
+        if (n <= 0) return CCT_NOERR;
         if (cudaStreamSynchronize(st) != cudaSuccess) return CCT_CUDAERR;
+        if (h_int[0] == 0) return CCT_NOERR;
+        cudaMemcpyAsync(rank, keep, sizeof(unsigned) * n, cudaMemcpyDeviceToDevice, st);
+        scan_exclusive(rank, n, nullptr, st, scan_sums);
+        MPS_COUNT_LAUNCH k_compact<<<blocks_for(n), kBlock, 0, st>>>(d, keep, rank);
         swap_state();
-        d.n = h_int[0];
-        return CCT_NOERR;
+        d.n = n - h_int[0];
+        return cuda_status(cudaGetLastError());
     }
+
+    int correct_share() const { return d.n < 20000 ? 4 : d.n < 200000 ? 16 : 32; }
 
     CCTStatusType grid() {
         const int n = d.n;
@@ -913,7 +921,7 @@ struct Solver {
                     MPS_COUNT_LAUNCH k_spmv<double, double, double, 1><<<kRedBlocks, 256, 0, st>>>(d, (const double*)d.nbrw, d.press,
                                                                                   d.r, d.rhs, 2);
                 else
-                    residual_df((const float*)d.nbrw);
+                    residual_df((const float*)d.nbrw, true, residual_by_update());
                 MPS_COUNT_LAUNCH k_pressure_scale<<<red_blocks(d.n), 256, 0, st>>>(d, 5);
                 MPS_COUNT_LAUNCH k_to_float_p<<<blocks_for(d.n), kBlock, 0, st>>>(d.n, d.press, d.pf32);
                 MPS_COUNT_LAUNCH k_features<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
@@ -940,7 +948,7 @@ struct Solver {
                 // the first refinement residual of the warm start, here so that the
                 // multilevel setup runs beside it (and inside the span the gate compares)
                 timer.mark(PH_VEC, st);
-                residual_df((const float*)d.nbrw);
+                residual_df((const float*)d.nbrw, true, residual_by_update());
                 if (stream_failed) return CCT_CUDAERR;
                 residual_ready = true;
             }
@@ -976,7 +984,7 @@ struct Solver {
         timer.mark(PH_CORRECT, st);
         if (!pressure_only) {
             if constexpr (sizeof(T) == 4)
-                MPS_COUNT_LAUNCH k_correct_warp<<<blocks_for((d.n + 31) / 32, 8), 256, 0, st>>>(d);
+                MPS_COUNT_LAUNCH k_correct_warp<<<blocks_for(div_up(d.n, correct_share()), 8), 256, 0, st>>>(d, correct_share());
             else
                 MPS_COUNT_LAUNCH k_correct<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
             std::swap(d.pos, d.pos2);
@@ -1145,6 +1153,10 @@ struct Solver {
     // the same for systems with few slices per warp (k_spmv_ring_split)
     static constexpr int kSplitRows = 400000, kSplit = 4;
     int spmv16_split_grid = 0;
+    // CTAs of a kernel whose warps share slices
+    int split_blocks(int resident) const {
+        return std::max(1, std::min(div_up(div_up(d.n, 32), kSsWarps / kSplit), resident));
+    }
     void spmv_split16(const float* x, float* y) {
         auto k = k_spmv_ring_split<kSplit, kS16Entries, kSsStages, kSsMinBlocks>;
         const int resident = stream_grid_for(k, kS16Smem, spmv16_split_grid);
@@ -1152,7 +1164,7 @@ struct Solver {
             stream_failed = true;
             return;
         }
-        const int grid = std::max(1, std::min(div_up(div_up(d.n, 32), kSsWarps / kSplit), resident));
+        const int grid = split_blocks(resident);
         if (pdl) {
             if (MPS_COUNT_LAUNCH launch_pdl(k, grid, kSsWarps * 32, kS16Smem, st, d, (const __half*)d.w16, x, y, 0))
                 stream_failed = true;
@@ -1328,7 +1340,10 @@ struct Solver {
 
     // r = rhs - A press (FP32 weights) in double-float arithmetic; norms to the scalars
     // (rows streamed through shared memory over the 16-bit slices, else the register walk)
-    void residual_df(const float* w, bool stream = true) {
+    // split: as the solver runs it, four warps to a slice below kSplitRows (the sums then
+    // round otherwise than the register walk's)
+    int resid_split_grid = 0, upd_split_grid = 0;
+    void residual_df(const float* w, bool stream = true, bool split = false) {
         MPS_COUNT_LAUNCH k_split_x<<<blocks_for(d.n), kBlock, 0, st>>>(d.n, d.press, d.xs);
         if (stream && use_stream() && prefer_wide) {
             auto k = k_residual_stream<kSsEntries, kSsStages, kSsWarps, kSsMinBlocks, true>;
@@ -1339,6 +1354,14 @@ struct Solver {
                 return;
             }
             MPS_COUNT_LAUNCH k<<<g, kSsWarps * 32, smem, st>>>(d, w, d.press, d.r, d.rhs, 2);
+        } else if (stream && split && use_stream() && d.n < kSplitRows) {
+            auto k = k_residual_stream<kSsEntries, kSsStages, kSsWarps, kSsMinBlocks, false, kSplit>;
+            const int g = stream_grid_for(k, kSsSmem, resid_split_grid);
+            if (g < 0) {
+                stream_failed = true;
+                return;
+            }
+            MPS_COUNT_LAUNCH k<<<split_blocks(g), kSsWarps * 32, kSsSmem, st>>>(d, w, d.press, d.r, d.rhs, 2);
         } else if (stream && use_stream()) {
             const int g = resid_blocks();
             if (g < 0) {
@@ -1366,6 +1389,14 @@ struct Solver {
                 return;
             }
             MPS_COUNT_LAUNCH k<<<g, kSsWarps * 32, smem, st>>>(d, w, d.d32, s, d.press, d.r, 2);
+        } else if (d.n < kSplitRows) {
+            auto k = k_residual_update_stream<kSsEntries, kSsStages, kSsWarps, kSsMinBlocks, false, kSplit>;
+            const int g = stream_grid_for(k, kSsSmem, upd_split_grid);
+            if (g < 0) {
+                stream_failed = true;
+                return;
+            }
+            MPS_COUNT_LAUNCH k<<<split_blocks(g), kSsWarps * 32, kSsSmem, st>>>(d, w, d.d32, s, d.press, d.r, 2);
         } else {
             auto k = k_residual_update_stream<kSsEntries, kSsStages, kSsWarps, kSsMinBlocks>;
             const int g = stream_grid_for(k, kSsSmem, upd_grid);
@@ -1405,7 +1436,7 @@ struct Solver {
             // before the solve (or from the learned guess), and for the later passes when
             // the last pass updated it with its correction
             const bool have = residual_ready;
-            if (!have) residual_df(w);
+            if (!have) residual_df(w, true, residual_by_update());
             if (stream_failed || pull_scal()) return CCT_CUDAERR;
             if (outer == 0) {
                 h_nnz[0] = h_scal[S_NNZ0];
@@ -1484,6 +1515,7 @@ struct Solver {
         c.kappa = opt.compressibility * c.rho / (c.dt * c.dt);
         c.c2 = c.rho / (c.dt * c.dt);
         c.vmax = c.l0 * (double)param.CourantNumber / c.dt;
+        c.derive(d.box);
         hist = 0;   // the increments were taken over the old step
         return CCT_NOERR;
     }

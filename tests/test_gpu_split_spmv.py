@@ -49,3 +49,43 @@ def test_whole_slices_take_over():
         its.append(r["cg_iterations"])
         s.close()
     assert abs(its[0] - its[1]) <= 3
+
+
+def test_compaction_at_the_zone_bounds():
+    """k_zone_flags compares doubles as ordered integers: the bounds themselves, both zeros
+    against a zero bound, the nearest doubles outside, subnormals and infinities, and which
+    particles stay when some leave and when none do."""
+    p = scenes.default_param(0.01, 1e-4)
+    hi = float(np.float32(0.3))
+    box = scenes.grid_box(np.zeros(3), np.full(3, 0.3), p)
+    mid = np.random.default_rng(0).uniform(0.1, 0.2, (300, 3))
+    edge = [0.0, -0.0, hi, np.nextafter(hi, 1), np.nextafter(0.0, -1), 5e-324, -1e-300, np.inf, -np.inf, np.nextafter(hi, 0)]
+    stays = [v for v in edge if not (v < 0.0 or v > hi)]
+    for values in (edge, stays):
+        pos = mid.copy()
+        for k, v in enumerate(values):
+            pos[7 * k, k % 3] = v
+        want = np.flatnonzero(~((pos < 0.0) | (pos > hi)).any(1))
+        sc = scenes._finish("zone", p, mid, np.zeros((0, 3, 3)), np.zeros(0, np.int32), [scenes._tri_normal_params(dt=p.Dt)],
+                            [], 0, 0.01, np.zeros(3), np.full(3, 0.3))
+        assert sc.box.m_ComputeZone.m_MaxBound.x == np.float32(hi) and sc.box.cell_num == box.cell_num
+        sc.pos = pos
+        s = Solver(sc, precision="fp32_ir")
+        assert s.pressure()["particles"] == len(want)
+        assert np.array_equal(np.sort(s.state()["id"]), want)
+        s.close()
+
+
+@pytest.mark.parametrize("n_side", [3, 27, 28, 58, 59])
+def test_correction_shares(n_side):
+    """k_correct_warp with 4, 16 and 32 particles per warp gives every particle its own
+    update: the velocities of a step against the FP64 solver's, to the FP32 operators'
+    accuracy over one step."""
+    out = []
+    for precision in ("fp32_ir", "fp64"):
+        s = Solver(_block((n_side,) * 3), precision=precision)
+        assert s.step(0)["error_flags"] == 0
+        out.append(s.state()["vel"])
+        s.close()
+    scale = np.abs(out[1]).max()
+    assert np.abs(out[0] - out[1]).max() <= 2e-3 * scale
