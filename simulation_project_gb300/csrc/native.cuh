@@ -47,6 +47,9 @@ struct Consts {
     double src;                      // gamma rho / dt^2
     double c3;                       // -dt / rho
     double vmax2;                    // below it a squared speed is certainly not above vmax^2
+    float reach2;                    // re_lap^2 and a little: FP32 screen of a candidate against a box
+    float wmax_lap, wmax_grad;       // largest weights, re / mind - 1
+    int wide_cells;                  // cells are at least re_lap wide
 
     // integers in the order of the doubles (NaN aside); the two zeros are neighbours
     __host__ __device__ static long long ordered_f64(double x) {
@@ -73,6 +76,10 @@ struct Consts {
         src = gamma * rho / (dt * dt);
         c3 = -dt / rho;
         vmax2 = vmax * vmax * (1.0 - 1e-12);
+        reach2 = (float)(re_lap * re_lap) * 1.0002f;
+        wmax_lap = (float)(re_lap / mind_lap) - 1.f;
+        wmax_grad = (float)(re_grad / mind_grad) - 1.f;
+        wide_cells = (double)box.m_CellSize >= re_lap * (1.0 - 1e-6) ? 1 : 0;
     }
 };
 
@@ -108,8 +115,8 @@ struct Dev {
     double* wdir;
     int* wid;
     double* dragv;
-    // neighbour rows: the list pass writes each row contiguously (row i at i*K: rnbr, rw);
-    // k_rows_sell turns the interior rows into SELL-32 (nbr, nbrw, nbr16, w16)
+    // neighbour rows: the FP32 list pass writes SELL-32 (nbr, nbrw, nbr16, w16); the FP64 one
+    // writes each row contiguously (row i at i*K: rnbr, rw), k_rows_sell transposes the interior ones
     int* rnbr;
     void* rw;
     int* nbr;                  // SELL-32 32-bit columns: slices with sbase = -1, or every slice when rows_c32
@@ -118,6 +125,7 @@ struct Dev {
     int* sbase;                // [slices] smallest column index of the slice, -1: 32-bit slice
     int* skmax;                // [slices] longest interior row of a 16-bit slice, -1: 32-bit slice
     int rows16;                // nbr16 / sbase are valid for the current rows
+    int rows_major;            // the current rows came row by row (rnbr, rw)
     int rows_c32;              // nbr holds the 32-bit columns of every slice
     __half* w16;               // FP16 copies of the FP32 weights (interior rows; inner CG operator)
     double* diag16;            // diagonal of the FP16-weight operator: coef * sum of FP16 weights + kappa

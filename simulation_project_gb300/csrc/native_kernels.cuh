@@ -1,7 +1,7 @@
 // native_kernels.cuh - kernels of the GB300-native semi-implicit step.
 //
-// Every particle kernel works in the cell-sorted order.  Neighbour passes run one CTA
-// per non-empty cell: the CTA stages the nine z-runs of the 27 surrounding cells (each
+// Every particle kernel works in the cell-sorted order.  The FP64 neighbour passes (the FP32
+// ones are in neighbours.cuh) run one CTA per non-empty cell: the CTA stages the nine z-runs of the 27 surrounding cells (each
 // run is contiguous in sorted order) into shared memory as float4, then each warp takes
 // one target particle at a time and its 32 lanes test 32 staged candidates per step;
 // accepted neighbours are compacted with __ballot_sync/__popc so a warp writes each
@@ -537,7 +537,7 @@ __device__ __forceinline__ double exact_r(double dx, double dy, double dz) {
 // Epilogue of one target of k_neighbours (run lane-parallel: each lane finishes the
 // target it parked, so the FP64 state update uses every lane of the FP64 pipe).
 template <class T, int MODE>
-__device__ __forceinline__ void nb_epilogue(const Dev& d, int i, T a0, T a1, T a2, T a3, int cnt, int gcnt) {
+__device__ __forceinline__ double nb_epilogue(const Dev& d, int i, double a0, double a1, double a2, int cnt, int gcnt) {
     if constexpr (MODE == NB_PREDICT) {
         // wall friction term, viscosity, gravity, drag (CalcExplicitly_Kernel)
         const V3<T> vi = load_v<T>(d, i);
@@ -571,17 +571,19 @@ __device__ __forceinline__ void nb_epilogue(const Dev& d, int i, T a0, T a1, T a
         }
         d.vel2[i] = vn;
         d.pos2[i] = pn;
+        return 0.0;
     } else {
         if (cnt > d.K || gcnt > d.KG) atomicOr(d.err, MPS_ERR_NEIGHBOUR_CAP);
         atomicMax(d.istat, cnt);
         d.nbr_cnt[i] = cnt < d.K ? cnt : d.K;
         d.gcnt[i] = gcnt < d.KG ? gcnt : d.KG;
-        double pnd = (double)a2;
+        double pnd = a2;
         const double riw = d.wdist[i];
         if (d.wid[i] >= 0 && riw >= 0 && riw <= d.c.re_grad)
             pnd += exact_z<double>(d.c.dim == 2 ? c_zgrad2 : c_zgrad3, d.c.dim == 2 ? 23 : 21, riw, d.c.l0);
         d.pnd[i] = pnd;
-        d.sumw[i] = (double)a0;
+        d.sumw[i] = a0;
+        return pnd;
     }
 }
 
@@ -593,12 +595,13 @@ __device__ __forceinline__ float dist2_f32(float dx, float dy, float dz) {
 }
 // w = re / max(r, mind) - 1 from one reciprocal square root; rinv = 1 / r, rr = r
 __device__ __forceinline__ float lap_weight_f32(float d2, float re, float mind, float wmax, float& rinv, float& rr) {
-    rinv = rsqrtf(fmaxf(d2, 1e-30f));
+    // never a denormal argument: the flushing form gives the same bits without its scaling
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(fmaxf(d2, 1e-30f)));
     rr = __fmul_rn(d2, rinv);
     return rr > mind ? __fmaf_rn(re, rinv, -1.f) : wmax;
 }
 
-// Neighbour passes, CTA per non-empty cell.  The 9 (x, y) columns of the 27-cell
+// FP64 neighbour passes (the FP32 ones are in neighbours.cuh), CTA per non-empty cell.  The 9 (x, y) columns of the 27-cell
 // neighbourhood are contiguous z-runs in the sorted order; their positions are
 // staged in shared memory (float4), a warp takes one target particle at a time and
 // its lanes test 32 candidates per round, in a z window of each run found by binary
@@ -607,15 +610,12 @@ __device__ __forceinline__ float lap_weight_f32(float d2, float re, float mind, 
 //   NB_LIST       Laplacian rows (row-major staging), gradient rows, PND, sum of weights
 // The warp's butterfly sums are parked in lane k%32 for its k-th target and the
 // epilogues run lane-parallel.
-template <class T, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(kNbThreads) k_neighbours(const __grid_constant__ Dev d) {
+    using T = double;
     __shared__ __align__(16) float4 spos[kStageCap];
     __shared__ __align__(8) unsigned long long stage_bar;
     __shared__ int rs[9], rl[9], rp[10];
-    // per-warp queues of accepted candidates (FP32 path): index and squared distance;
-    // a round adds at most 32 to fewer than 32 waiting entries
-    __shared__ int nb_qj[kNbThreads / 32][64];
-    __shared__ float nb_qd[kNbThreads / 32][64];
     const int ci = blockIdx.x;
     if (ci >= *d.cell_count) return;
     const int cell = d.cell_list[ci];
@@ -671,18 +671,15 @@ __global__ void __launch_bounds__(kNbThreads) k_neighbours(const __grid_constant
     const unsigned lt = (1u << lane) - 1u;
     const T re = (T)d.c.re_lap, reg = (T)d.c.re_grad, mind = (T)d.c.mind_lap, mindg = (T)d.c.mind_grad;
     const float re2f = (float)(d.c.re_lap * d.c.re_lap) * 1.0001f;
-    // FP32 path: one reciprocal square root per accepted pair gives r and both weights
-    const float re2s = (float)d.c.re_lap * (float)d.c.re_lap;
-    const float wmax = (float)(d.c.re_lap / d.c.mind_lap) - 1.f, wgmax = (float)(d.c.re_grad / d.c.mind_grad) - 1.f;
     // target parked in this lane for the lane-parallel epilogue
     int my_i = -1, my_cnt = 0, my_gcnt = 0;
-    T m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+    T m0 = 0, m1 = 0, m2 = 0;
     int k = 0;
     for (int i = s0 + warp; i < e0; i += nwarp, ++k) {
         const float4 pf = d.opos[i];
         const V3<T> pi = load_p<T>(d, i);
         const V3<T> vi = load_v<T>(d, i);
-        T a0 = 0, a1 = 0, a2 = 0, a3 = 0;   // mode-specific accumulators
+        T a0 = 0, a1 = 0, a2 = 0;   // mode-specific accumulators
         int cnt = 0, gcnt = 0;
         // the row's entries are stored contiguously (row i at i*K; k_rows_sell turns the
         // interior rows into SELL-32), so a batch of 32 accepted entries is one line
@@ -728,154 +725,61 @@ __global__ void __launch_bounds__(kNbThreads) k_neighbours(const __grid_constant
                 }
             }
         }
-        if constexpr (sizeof(T) == 4) {
-            // FP32: the candidates a round accepts queue up in candidate order; the
-            // weight, the sums and the row stores run on full batches of 32 entries,
-            // so the expensive path executes ~accepted/32 times per target instead of
-            // once per 32-candidate round.  Entry order (hence every row) is unchanged.
-            int* const qj = nb_qj[warp];
-            float* const qd = nb_qd[warp];
-            int qn = 0;
-            auto flush = [&](int nq) {   // the first nq <= 32 entries (nq warp-uniform)
-                const bool on = lane < nq;
-                const int j = on ? qj[lane] : 0;
-                float rinv = 0.f, rrf = 0.f, w = 0.f;
-                if (on) w = lap_weight_f32(qd[lane], (float)re, (float)mind, wmax, rinv, rrf);
-                bool gacc = false;
-                if constexpr (MODE == NB_PREDICT) {
-                    if (on) {
-                        const float4 v = d.ovel[j];
+        // FP64: the FP32 distance screens, the exact FP64 distance decides
+        for (int r = 0; r < 9; ++r) {
+            const int kb = __shfl_sync(0xffffffffu, bound, r);
+            const int len = max(kb, __shfl_sync(0xffffffffu, bound, 16 + r));
+            const int rsr = rs[r], rpr = rp[r];   // run start (global) and stage offset
+            for (int b = kb; b < len; b += 32) {
+                const int o = b + lane;
+                const bool valid = o < len;
+                const int j = rsr + o;
+                bool acc = false, gacc = false;
+                T rr = T(0);
+                if (valid && j != i) {
+                    const float4 q = staged ? spos[rpr + o] : d.opos[j];
+                    const float d2f = dist2_f32(q.x - pf.x, q.y - pf.y, q.z - pf.z);
+                    if (d2f < re2f) {
+                        const dbl4 pj = d.pos[j];
+                        const double rd = exact_r(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z);
+                        if (rd < re) {
+                            acc = true;
+                            rr = rd;
+                        }
+                    }
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, acc);
+                if (acc) {
+                    const T w = wdiv<T>(re, rr > mind ? rr : mind) - T(1);
+                    if constexpr (MODE == NB_PREDICT) {
+                        const dbl4 v = d.vel[j];
                         a0 += (v.x - vi.x) * w;
                         a1 += (v.y - vi.y) * w;
                         a2 += (v.z - vi.z) * w;
-                    }
-                } else {
-                    if (on) {
-                        const int slot = cnt + lane;
+                    } else {
+                        const int slot = cnt + __popc(bal & lt);
                         if (slot < d.K) {
                             nrow[slot] = j;
                             wrow[slot] = w;
                         }
                         a0 += w;                                   // sum of Laplacian weights
-                        if (rrf < reg) {
+                        if (rr < reg) {
                             gacc = true;
-                            a2 += rrf > mindg ? __fmaf_rn(reg, rinv, -1.f) : wgmax;   // PND
+                            a2 += wdiv<T>(reg, rr > mindg ? rr : mindg) - T(1);   // PND
                         }
                     }
+                }
+                cnt += __popc(bal);
+                if constexpr (MODE != NB_PREDICT) {
                     const unsigned gb = __ballot_sync(0xffffffffu, gacc);
                     if (gb != 0u && gacc) {
                         const int slot = gcnt + __popc(gb & lt);
                         if (slot < d.KG) {
                             grow[slot] = j;
-                            grrow[slot] = rrf;
+                            grrow[slot] = rr;
                         }
                     }
                     gcnt += __popc(gb);
-                }
-                cnt += nq;
-            };
-            for (int r = 0; r < 9; ++r) {
-                const int kb = __shfl_sync(0xffffffffu, bound, r);
-                const int len = max(kb, __shfl_sync(0xffffffffu, bound, 16 + r));
-                const int rsr = rs[r], rpr = rp[r];   // run start (global) and stage offset
-                for (int b = kb; b < len; b += 32) {
-                    const int o = b + lane;
-                    const int j = rsr + o;
-                    bool acc = false;
-                    float d2f = 0.f;
-                    if (o < len && j != i) {
-                        const float4 q = staged ? spos[rpr + o] : d.opos[j];
-                        d2f = dist2_f32(q.x - pf.x, q.y - pf.y, q.z - pf.z);
-                        acc = d2f < re2s;
-                    }
-                    const unsigned bal = __ballot_sync(0xffffffffu, acc);
-                    if (acc) {
-                        const int pos = qn + __popc(bal & lt);
-                        qj[pos] = j;
-                        qd[pos] = d2f;
-                    }
-                    qn += __popc(bal);
-                    if (qn >= 32) {
-                        __syncwarp();
-                        flush(32);
-                        // the entries past the batch move to the front of the queue
-                        const int rest = qn - 32;
-                        int mj = 0;
-                        float md = 0.f;
-                        if (lane < rest) {
-                            mj = qj[32 + lane];
-                            md = qd[32 + lane];
-                        }
-                        __syncwarp();
-                        if (lane < rest) {
-                            qj[lane] = mj;
-                            qd[lane] = md;
-                        }
-                        __syncwarp();
-                        qn = rest;
-                    }
-                }
-            }
-            __syncwarp();
-            if (qn > 0) flush(qn);
-            __syncwarp();   // the queue is reused for the warp's next target
-        } else {
-            // FP64: the FP32 distance screens, the exact FP64 distance decides
-            for (int r = 0; r < 9; ++r) {
-                const int kb = __shfl_sync(0xffffffffu, bound, r);
-                const int len = max(kb, __shfl_sync(0xffffffffu, bound, 16 + r));
-                const int rsr = rs[r], rpr = rp[r];   // run start (global) and stage offset
-                for (int b = kb; b < len; b += 32) {
-                    const int o = b + lane;
-                    const bool valid = o < len;
-                    const int j = rsr + o;
-                    bool acc = false, gacc = false;
-                    T rr = T(0);
-                    if (valid && j != i) {
-                        const float4 q = staged ? spos[rpr + o] : d.opos[j];
-                        const float d2f = dist2_f32(q.x - pf.x, q.y - pf.y, q.z - pf.z);
-                        if (d2f < re2f) {
-                            const dbl4 pj = d.pos[j];
-                            const double rd = exact_r(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z);
-                            if (rd < re) {
-                                acc = true;
-                                rr = rd;
-                            }
-                        }
-                    }
-                    const unsigned bal = __ballot_sync(0xffffffffu, acc);
-                    if (acc) {
-                        const T w = wdiv<T>(re, rr > mind ? rr : mind) - T(1);
-                        if constexpr (MODE == NB_PREDICT) {
-                            const dbl4 v = d.vel[j];
-                            a0 += (v.x - vi.x) * w;
-                            a1 += (v.y - vi.y) * w;
-                            a2 += (v.z - vi.z) * w;
-                        } else {
-                            const int slot = cnt + __popc(bal & lt);
-                            if (slot < d.K) {
-                                nrow[slot] = j;
-                                wrow[slot] = w;
-                            }
-                            a0 += w;                                   // sum of Laplacian weights
-                            if (rr < reg) {
-                                gacc = true;
-                                a2 += wdiv<T>(reg, rr > mindg ? rr : mindg) - T(1);   // PND
-                            }
-                        }
-                    }
-                    cnt += __popc(bal);
-                    if constexpr (MODE != NB_PREDICT) {
-                        const unsigned gb = __ballot_sync(0xffffffffu, gacc);
-                        if (gb != 0u && gacc) {
-                            const int slot = gcnt + __popc(gb & lt);
-                            if (slot < d.KG) {
-                                grow[slot] = j;
-                                grrow[slot] = rr;
-                            }
-                        }
-                        gcnt += __popc(gb);
-                    }
                 }
             }
         }
@@ -884,17 +788,16 @@ __global__ void __launch_bounds__(kNbThreads) k_neighbours(const __grid_constant
             a0 += __shfl_xor_sync(0xffffffffu, a0, o);
             a1 += __shfl_xor_sync(0xffffffffu, a1, o);
             a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-            a3 += __shfl_xor_sync(0xffffffffu, a3, o);
         }
         if (lane == (k & 31)) {
-            my_i = i; m0 = a0; m1 = a1; m2 = a2; m3 = a3; my_cnt = cnt; my_gcnt = gcnt;
+            my_i = i; m0 = a0; m1 = a1; m2 = a2; my_cnt = cnt; my_gcnt = gcnt;
         }
         if ((k & 31) == 31) {
-            if (my_i >= 0) nb_epilogue<T, MODE>(d, my_i, m0, m1, m2, m3, my_cnt, my_gcnt);
+            if (my_i >= 0) nb_epilogue<T, MODE>(d, my_i, m0, m1, m2, my_cnt, my_gcnt);
             my_i = -1;
         }
     }
-    if (my_i >= 0) nb_epilogue<T, MODE>(d, my_i, m0, m1, m2, m3, my_cnt, my_gcnt);
+    if (my_i >= 0) nb_epilogue<T, MODE>(d, my_i, m0, m1, m2, my_cnt, my_gcnt);
 }
 
 // FP64 checksum of the neighbour ids of every row (neighbour-set comparison in tests)
@@ -902,8 +805,12 @@ __global__ void k_row_idsum(const __grid_constant__ Dev d, double* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
     double s = 0.0;
-    const int cnt = d.nbr_cnt[i];
-    for (int k = 0; k < cnt; ++k) s += (double)d.id[d.rnbr[(size_t)i * d.K + k]];
+    const int cnt = d.nbr_cnt[i], sb = d.rows16 ? d.sbase[i >> 5] : -1;
+    for (int k = 0; k < cnt; ++k) {
+        const size_t e = sell_index(i, k, d.K);
+        const int j = d.rows_major ? d.rnbr[(size_t)i * d.K + k] : sb >= 0 ? sb + (short)d.nbr16[e] : d.nbr[e];
+        s += (double)d.id[j];
+    }
     out[i] = s;
 }
 
@@ -951,37 +858,33 @@ __device__ __forceinline__ int sell_col(const Dev& d, size_t e, int sb) {
     return __ldcs(d.nbr + e);
 }
 
-// SELL-32 rows of the interior rows from the list pass's row-major rows, one read
+// FP64: SELL-32 rows of the interior rows from the list pass's row-major rows, one read
 // pass: warp per 32-row slice; each 32-entry chunk of the slice's rows is loaded one
 // 128-byte line per row into a [32][33] shared-memory tile and written back transposed,
 // so entry k of the slice's 32 rows is again one contiguous store per array.
 // flags bit 0: 16-bit column offsets j - 32*slice (sbase / skmax; a slice with an offset
-// outside [-32768, 32767] keeps 32-bit columns, sbase = -1); bit 1: the FP16 copy of each
-// FP32 weight (round to nearest) and the diagonal of that operator, coef * (sum of the
-// FP16 weights in entry order, in FP32) + kappa, so the FP16-weight operator is again a
+// outside [-32768, 32767] keeps 32-bit columns, sbase = -1); bit 1 (k_list only): the FP16
+// copy of each FP32 weight (round to nearest) and the diagonal of that operator, coef * (sum
+// of the FP16 weights in entry order, in FP32) + kappa, so the FP16-weight operator is again a
 // Laplacian plus kappa; bit 2: 32-bit columns for every slice (the wide streamed SpMV,
 // uncompressed rows); bit 3: leave the wide-entry count alone (a repeated transpose).
-// The weights (T) are always written.  A row's columns ascend (its candidates are
+// The weights are always written.  A row's columns ascend (its candidates are
 // visited run by run in cell-key order, each run in index order), so its first and last
 // entries decide whether the slice fits 16 bits; every offset is still checked as it is
 // written, and an offset that breaks that order sets MPS_ERR_NEIGHBOUR_CAP.
-template <class T>
-constexpr int rows_sell_warps() { return sizeof(T) == 4 ? 4 : 2; }
-
-template <class T>
-__global__ void __launch_bounds__(rows_sell_warps<T>() * 32) k_rows_sell(const __grid_constant__ Dev d, int flags) {
-    constexpr int WARPS = rows_sell_warps<T>();
-    __shared__ int tj[WARPS][32][33];
-    __shared__ T tw[WARPS][32][33];
+constexpr int kRsWarps = 2;
+__global__ void __launch_bounds__(kRsWarps * 32) k_rows_sell(const __grid_constant__ Dev d, int flags) {
+    __shared__ int tj[kRsWarps][32][33];
+    __shared__ double tw[kRsWarps][32][33];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int sl = blockIdx.x * WARPS + wl;
+    const int sl = blockIdx.x * kRsWarps + wl;
     if (sl >= (d.n + 31) >> 5) return;   // warp-uniform
-    const bool narrow = (flags & 1) != 0, w16 = sizeof(T) == 4 && (flags & 2) != 0, full32 = (flags & 4) != 0;
+    const bool narrow = (flags & 1) != 0, full32 = (flags & 4) != 0;
     const int r0 = sl * 32, i = r0 + lane;
     const int cnt = (i < d.n && d.inner[i]) ? min(d.nbr_cnt[i], d.K) : 0;
     const int kmax = __reduce_max_sync(0xffffffffu, cnt);
     const int* __restrict__ rj = d.rnbr + (size_t)r0 * d.K;
-    const T* __restrict__ rwt = (const T*)d.rw + (size_t)r0 * d.K;
+    const double* __restrict__ rwt = (const double*)d.rw + (size_t)r0 * d.K;
     bool fit = true;
     if (cnt > 0) {
         const int lo = __ldcs(rj + (size_t)lane * d.K) - r0, hi = __ldcs(rj + (size_t)lane * d.K + cnt - 1) - r0;
@@ -990,8 +893,7 @@ __global__ void __launch_bounds__(rows_sell_warps<T>() * 32) k_rows_sell(const _
     const bool n16 = narrow && __all_sync(0xffffffffu, fit);
     const bool c32 = full32 || !n16;
     const size_t e0 = (size_t)sl * d.K * 32 + lane;   // SELL position of this lane's entry 0
-    T* __restrict__ ws = (T*)d.nbrw;
-    float sw16 = 0.f;
+    double* __restrict__ ws = (double*)d.nbrw;
     bool bad = false;
     for (int c = 0; c < kmax; c += 32) {
 #pragma unroll 8
@@ -1007,25 +909,18 @@ __global__ void __launch_bounds__(rows_sell_warps<T>() * 32) k_rows_sell(const _
         for (int k = 0; k < m; ++k) {
             if (c + k < cnt) {
                 const int j = tj[wl][lane][k];
-                const T w = tw[wl][lane][k];
                 const size_t e = e0 + (size_t)(c + k) * 32;
-                ws[e] = w;
+                ws[e] = tw[wl][lane][k];
                 if (c32) d.nbr[e] = j;
                 if (n16) {
                     const int off = j - r0;
                     bad = bad || off < -32768 || off > 32767;
                     d.nbr16[e] = (unsigned short)(short)off;
                 }
-                if (w16) {
-                    const __half h = __float2half_rn((float)w);
-                    d.w16[e] = h;
-                    sw16 += __half2float(h);
-                }
             }
         }
         __syncwarp();   // the tile is refilled for the next chunk
     }
-    if (w16 && cnt > 0) d.diag16[i] = d.c.coef_lap * (double)sw16 + d.c.kappa;
     if (bad) atomicOr(d.err, MPS_ERR_NEIGHBOUR_CAP);
     if (lane == 0) {
         d.sbase[sl] = n16 ? r0 : -1;
@@ -1033,117 +928,6 @@ __global__ void __launch_bounds__(rows_sell_warps<T>() * 32) k_rows_sell(const _
     }
     if (narrow && !(flags & 8)) {
         // interior entries kept at 32 bits (counted for the bytes-per-launch figure)
-        int wide = n16 ? 0 : cnt;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) wide += __shfl_down_sync(0xffffffffu, wide, o);
-        if (lane == 0 && wide) atomicAdd(d.istat + 1, wide);
-    }
-}
-
-// FP32 rows (the step's default): the same transpose with the chunks moved global ->
-// shared by 16-byte cp.async pieces, double-buffered so that the next chunk's copies
-// are in flight while the current chunk is written out.  A warp per slice, 2 warps per
-// CTA (32 KB: 2 stages x columns and weights x 32 rows x 128 B).  Piece q (entries
-// 4q..4q+3) of row r sits at piece position q ^ (r & 7) of the row's 128 bytes, so the
-// 16-byte reads of lanes 0..7 (rows 0..7, one piece each) cover the 32 banks.  Pieces
-// of a chunk past a row's count copy stale staging entries inside the row's capacity
-// (K is a multiple of 128) and are never read.  Same outputs as k_rows_sell<float>.
-constexpr int kRsWarps = 2;
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__global__ void __launch_bounds__(kRsWarps * 32) k_rows_sell_async(const __grid_constant__ Dev d, int flags) {
-    __shared__ __align__(128) unsigned char tiles[kRsWarps][2][2][32 * 128];   // [warp][stage][cols, weights]
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int sl = blockIdx.x * kRsWarps + wl;
-    if (sl >= (d.n + 31) >> 5) return;   // warp-uniform
-    const bool narrow = (flags & 1) != 0, w16 = (flags & 2) != 0, full32 = (flags & 4) != 0;
-    const int r0 = sl * 32, i = r0 + lane;
-    const int cnt = (i < d.n && d.inner[i]) ? min(d.nbr_cnt[i], d.K) : 0;
-    const int kmax = __reduce_max_sync(0xffffffffu, cnt);
-    const int* __restrict__ rj = d.rnbr + (size_t)r0 * d.K;
-    const float* __restrict__ rwt = (const float*)d.rw + (size_t)r0 * d.K;
-    bool fit = true;
-    if (cnt > 0) {
-        const int lo = __ldcs(rj + (size_t)lane * d.K) - r0, hi = __ldcs(rj + (size_t)lane * d.K + cnt - 1) - r0;
-        fit = lo >= -32768 && hi <= 32767;
-    }
-    const bool n16 = narrow && __all_sync(0xffffffffu, fit);
-    const bool c32 = full32 || !n16;
-    const size_t e0 = (size_t)sl * d.K * 32 + lane;
-    float* __restrict__ ws = (float*)d.nbrw;
-    // lane t copies piece t & 7 of rows 4u + t / 8, u = 0..7
-    const int cq = lane & 7, crow = lane >> 3;
-    auto issue = [&](int c, int st) {
-        unsigned char* tj = tiles[wl][st][0];
-        unsigned char* tw = tiles[wl][st][1];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int r = 4 * u + crow;
-            const int cr = __shfl_sync(0xffffffffu, cnt, r);
-            if (c < cr) {
-                const size_t g = (size_t)r * d.K + c + 4 * cq;
-                const int pos = r * 128 + ((cq ^ (r & 7)) << 4);
-                cp_async16(tj + pos, rj + g);
-                cp_async16(tw + pos, rwt + g);
-            }
-        }
-        cp_async_commit();
-    };
-    const int nch = (kmax + 31) >> 5;
-    if (nch > 0) issue(0, 0);
-    float sw16 = 0.f;
-    bool bad = false;
-    for (int ci = 0; ci < nch; ++ci) {
-        if (ci + 1 < nch) {
-            issue((ci + 1) * 32, (ci + 1) & 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncwarp();   // every lane's pieces of chunk ci have landed
-        const unsigned char* tj = tiles[wl][ci & 1][0];
-        const unsigned char* tw = tiles[wl][ci & 1][1];
-        const int c = ci * 32;
-        for (int q = 0; q < 8 && c + 4 * q < kmax; ++q) {
-            const int pos = lane * 128 + ((q ^ (lane & 7)) << 4);
-            const int4 jv = *(const int4*)(tj + pos);
-            const float4 wv = *(const float4*)(tw + pos);
-            const int jj[4] = {jv.x, jv.y, jv.z, jv.w};
-            const float wf[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = c + 4 * q + u;
-                if (k < cnt) {
-                    const size_t e = e0 + (size_t)k * 32;
-                    ws[e] = wf[u];
-                    if (c32) d.nbr[e] = jj[u];
-                    if (n16) {
-                        const int off = jj[u] - r0;
-                        bad = bad || off < -32768 || off > 32767;
-                        d.nbr16[e] = (unsigned short)(short)off;
-                    }
-                    if (w16) {
-                        const __half h = __float2half_rn(wf[u]);
-                        d.w16[e] = h;
-                        sw16 += __half2float(h);
-                    }
-                }
-            }
-        }
-        __syncwarp();   // stage ci & 1 is refilled by the next iteration's copies
-    }
-    if (w16 && cnt > 0) d.diag16[i] = d.c.coef_lap * (double)sw16 + d.c.kappa;
-    if (bad) atomicOr(d.err, MPS_ERR_NEIGHBOUR_CAP);
-    if (lane == 0) {
-        d.sbase[sl] = n16 ? r0 : -1;
-        d.skmax[sl] = n16 ? kmax : -1 - kmax;
-    }
-    if (narrow && !(flags & 8)) {
         int wide = n16 ? 0 : cnt;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wide += __shfl_down_sync(0xffffffffu, wide, o);

@@ -25,6 +25,7 @@
 
 #include "../../include/mps_io.h"
 #include "native_kernels.cuh"
+#include "neighbours.cuh"
 #include "coarse.cuh"
 #include "../../include/mps_learned.h"
 
@@ -790,23 +791,61 @@ struct Solver {
         return cuda_status(cudaGetLastError());
     }
 
-    // SELL-32 transpose of the current rows (k_rows_sell flags)
+    // k_rows_sell flags of the rows: 16-bit column offsets for the streamed SpMVs (the FP64
+    // solver streams them with its FP64 weights), FP16 weight copies only for the FP32 inner
+    // CG, 32-bit columns where they are read
+    int row_flags() {
+        if (opt.pressure_mode == MPS_PRESSURE_EXPLICIT) return 4;
+        const int narrow = (opt.compress_rows && (!fp64() || opt.spmv_stream)) ? 1 : 0;
+        const int w16 = (narrow && !fp64() && want_inner16() && d.w16) ? 1 : 0;
+        // 32-bit columns: the wide streamed kernels, the register walks of uncompressed
+        // rows, the non-streamed refinement residual (k_residual_df) and every FP64
+        // register walk (the FP64 learned-guess SpMVs, the stream's timeout fallback)
+        const int full32 = (!narrow || prefer_wide || !opt.spmv_stream || fp64()) ? 1 : 0;
+        return narrow | (w16 << 1) | (full32 << 2);
+    }
+    // SELL-32 transpose of the FP64 list pass's rows (k_rows_sell flags)
     void rows_sell(int flags) {
         const int slices = (d.n + 31) / 32;
-        if (slices == 0) return;
-        if (fp64())
-            MPS_COUNT_LAUNCH k_rows_sell<double><<<div_up(slices, rows_sell_warps<double>()), rows_sell_warps<double>() * 32,
-                                                   0, st>>>(d, flags);
-        else if (opt.rows_sell == 1)
-            MPS_COUNT_LAUNCH k_rows_sell<float><<<div_up(slices, rows_sell_warps<float>()), rows_sell_warps<float>() * 32,
-                                                  0, st>>>(d, flags);
-        else
-            MPS_COUNT_LAUNCH k_rows_sell_async<<<div_up(slices, kRsWarps), kRsWarps * 32, 0, st>>>(d, flags);
+        if (slices > 0) MPS_COUNT_LAUNCH k_rows_sell<<<div_up(slices, kRsWarps), kRsWarps * 32, 0, st>>>(d, flags);
+    }
+    void predict() {
+        const int slices = (d.n + 31) / 32;
+        if (fp64()) {
+            const int grid = std::max(1, std::min(d.cells, d.n));
+            MPS_COUNT_LAUNCH k_neighbours<NB_PREDICT><<<grid, kNbThreads, 0, st>>>(d);
+        } else if (slices <= 0) {
+        } else if (d.n < kPredictSplit) {
+            MPS_COUNT_LAUNCH k_predict<3><<<slices, 96, 0, st>>>(d);
+        } else {
+            MPS_COUNT_LAUNCH k_predict<1><<<div_up(slices, kNpWarps), kNpWarps * 32, 0, st>>>(d);
+        }
+    }
+    // rows at the current positions: FP32 ones in SELL-32 at once, FP64 ones row by row
+    void list_rows() {
+        d.rows_major = fp64() ? 1 : 0;
+        if (fp64()) {
+            const int grid = std::max(1, std::min(d.cells, d.n));
+            MPS_COUNT_LAUNCH k_neighbours<NB_LIST><<<grid, kNbThreads, 0, st>>>(d);
+            return;
+        }
+        const int slices = (d.n + 31) / 32, flags = row_flags();
+        // room for an eighth more entries than the last step's longest row had: less shared memory
+        // per slice, eight CTAs on an SM instead of seven (1359 us instead of 1445 at 882,080
+        // particles); a slice with a longer row takes the direct walk, with the same rows
+        const int room = last.max_row > 0 ? (last.max_row + last.max_row / 8 + 15) / 8 * 8 : d.K;
+        const int L = std::min(room, d.K);
+        if (slices > 0)
+            MPS_COUNT_LAUNCH k_list<<<slices, 64, nb_list_smem(L), st>>>(d, flags | (opt.rows_sell == 1 ? 16 : 0), L);
+        d.rows16 = flags & 1;
+        d.rows_w16 = flags >> 1 & 1;
+        d.rows_c32 = flags >> 2 & 1;
     }
     // the 32-bit columns of every slice (debug entries that force the wide SpMV)
     void ensure_cols32() {
         if (d.rows_c32 || d.n <= 0) return;
-        rows_sell(d.rows16 | (d.rows_w16 << 1) | 4 | 8);
+        if (d.rows_major) rows_sell(d.rows16 | 4 | 8);
+        else MPS_COUNT_LAUNCH k_rows_widen<<<blocks_for(d.n), kBlock, 0, st>>>(d);
         d.rows_c32 = 1;
     }
 
@@ -854,8 +893,7 @@ struct Solver {
             if (d.drag_n > 0 && d.tri_n > 0) MPS_COUNT_LAUNCH k_drag<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
             else cudaMemsetAsync(d.dragv, 0, sizeof(double) * 3 * d.n, st);
             timer.mark(PH_PRED, st);
-            const int nb_grid = std::max(1, std::min(d.cells, d.n));
-            MPS_COUNT_LAUNCH k_neighbours<T, NB_PREDICT><<<nb_grid, kNbThreads, 0, st>>>(d);
+            predict();
             std::swap(d.pos, d.pos2);
             std::swap(d.vel, d.vel2);
             timer.mark(PH_GRID, st);
@@ -866,8 +904,7 @@ struct Solver {
         if (pressure_only && d.tri_n > 0 && bins_dirty && (rc = bin_walls(st, h_int, scan_sums))) return rc;
         walls_distance<T>();
         timer.mark(PH_LIST, st);
-        const int nb_cells = std::max(1, std::min(d.cells, d.n));
-        MPS_COUNT_LAUNCH k_neighbours<T, NB_LIST><<<nb_cells, kNbThreads, 0, st>>>(d);
+        list_rows();
         timer.mark(PH_SETUP, st);
         if (opt.pressure_mode == MPS_PRESSURE_EXPLICIT) {
             MPS_COUNT_LAUNCH k_eos<<<blocks_for(d.n), kBlock, 0, st>>>(d);
@@ -884,20 +921,11 @@ struct Solver {
                 cudaStreamWaitEvent(st2, ev_setup, 0);
                 if (mg_setup_topology(st2)) return CCT_CUDAERR;
             }
-            // SELL-32 rows from the list pass's row-major rows: 16-bit column offsets for
-            // the streamed SpMVs (the FP64 solver streams them with its FP64 weights), FP16
-            // weight copies only for the FP32 inner CG, 32-bit columns where they are read
-            {
-                const int narrow = (opt.compress_rows && (!fp64() || opt.spmv_stream)) ? 1 : 0;
-                const int w16 = (narrow && !fp64() && want_inner16() && d.w16) ? 1 : 0;
-                // 32-bit columns: the wide streamed kernels, the register walks of uncompressed
-                // rows, the non-streamed refinement residual (k_residual_df) and every FP64
-                // register walk (the FP64 learned-guess SpMVs, the stream's timeout fallback)
-                const int full32 = (!narrow || prefer_wide || !opt.spmv_stream || fp64()) ? 1 : 0;
-                rows_sell(narrow | (w16 << 1) | (full32 << 2));
-                d.rows16 = narrow;
-                d.rows_w16 = w16;
-                d.rows_c32 = full32;
+            if (fp64()) {
+                const int flags = row_flags();
+                rows_sell(flags);
+                d.rows16 = flags & 1;
+                d.rows_c32 = flags >> 2 & 1;
             }
             bool use_learned = learned_ready && opt.learned && d.n > 0;
             // the gate: a learned guess that cost more than it saved sits out a few steps
@@ -1152,6 +1180,9 @@ struct Solver {
     }
     // the same for systems with few slices per warp (k_spmv_ring_split)
     static constexpr int kSplitRows = 400000, kSplit = 4;
+    // below it three warps share a slice of the predictor (k_predict<3> / <1>, us: 22.8 / 34.6
+    // at 2,000 particles, 35 / 49 at 12,635, 53 / 55 at 29,500, 108 / 77 at 53,000)
+    static constexpr int kPredictSplit = 25000;
     int spmv16_split_grid = 0;
     // CTAs of a kernel whose warps share slices
     int split_blocks(int resident) const {
