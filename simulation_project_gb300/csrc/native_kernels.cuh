@@ -1309,7 +1309,7 @@ struct SliceRing {
         while (streaming && ps < nsl && q_issue - q_cons < (unsigned)SS) {
             const int st = (int)(q_issue % SS);
             const int k0 = pc * SC;
-            const int ne = min(SC, pk - k0);
+            const int ne = SPLIT > 1 ? SC : min(SC, pk - k0);   // shared slices: rows padded to whole chunks
             if (lane == 0) {
                 const size_t e0 = ((size_t)ps * K + k0) * 32;
                 fence_proxy_async_smem();
@@ -1450,6 +1450,10 @@ __global__ void __launch_bounds__(W * 32, MINB) k_spmv_stream(const __grid_const
 // particles (63 iterations) 4,168 / 3,671 / 3,621 / 3,690, of 343,000 (87) 11,447 / 10,490 /
 // 10,226 / 10,799; step of 108,186 3,476 / 3,428 / 3,370 / 3,366, of 453,356 7,718 / 7,791 /
 // 7,834 / 7,969.  Plain loads of the shares instead of bulk copies: 5,898 at 103,823.
+// A lane holds two rows and takes every other entry of them, so that a column and a weight of
+// two rows are one 32-bit read each and nothing is predicated (27.3 us instead of 29.7 at
+// 108,186 particles, Poisson solve 3,060 instead of 3,169); what is left is the gathers of x,
+// six L1 wavefronts each.
 template <int SPLIT, int SC, int SS, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_spmv_ring_split(const __grid_constant__ Dev d, const __half* __restrict__ w,
                                                          const float* __restrict__ x, float* __restrict__ y, int slot) {
@@ -1472,9 +1476,10 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_ring_split(const __grid_cons
         const bool row = sl < R.nsl && i < d.n, in = row && d.inner[i];
         const int cnt = in ? d.nbr_cnt[i] : 0;
         const int km = sl < R.nsl ? d.skmax[sl] : 0;
-        float acc = 0.f;
+        float acc = 0.f, acc1 = 0.f;   // rows 2 (lane mod 16) and the next one of the slice
         if (km > 0) {
             const int c0 = R.first_chunk(km), c1 = R.end_chunk(km), r0 = sl * 32;
+            const float* const xs = x + r0;
             bool done = R.streaming;
             for (int c = c0; done && c < c1; ++c) {
                 const unsigned char* cs;
@@ -1483,22 +1488,34 @@ __global__ void __launch_bounds__(256, MINB) k_spmv_ring_split(const __grid_cons
                     done = false;
                     break;
                 }
-                const int k0 = c * SC;
+                // two rows and every other entry a lane: 32-bit reads of two columns and two
+                // weights; entries past a row's end have weight 0 (k_list)
+                unsigned cw[SC / 2], ww[SC / 2];
 #pragma unroll
-                for (int g = 0; g < SC; g += 8) {
-                    int j[8];
-                    float wv[8];
+                for (int g = 0; g < SC / 2; ++g) {
+                    cw[g] = ((const unsigned*)cs)[g * 32 + lane];
+                    ww[g] = ((const unsigned*)ws)[g * 32 + lane];
+                }
+                float x0[SC / 2], x1[SC / 2];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        j[u] = r0 + (int)(short)((const unsigned short*)cs)[(g + u) * 32 + lane];
-                        wv[u] = __half2float(ws[(g + u) * 32 + lane]);
-                    }
+                for (int g = 0; g < SC / 2; ++g) {
+                    x0[g] = __ldg(xs + (int)(short)(cw[g] & 0xffffu));
+                    x1[g] = __ldg(xs + ((int)cw[g] >> 16));
+                }
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (k0 + g + u < cnt) acc = __fmaf_rn(wv[u], __ldg(x + j[u]), acc);
+                for (int g = 0; g < SC / 2; ++g) {
+                    const float2 wv = __half22float2(*(const __half2*)&ww[g]);
+                    acc = __fmaf_rn(wv.x, x0[g], acc);
+                    acc1 = __fmaf_rn(wv.y, x1[g], acc1);
                 }
                 R.release();
             }
+            // lane = row again: the even rows' sums are in lanes 0..15's acc, the odd ones' in acc1
+            acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+            acc1 += __shfl_xor_sync(0xffffffffu, acc1, 16);
+            acc = __shfl_sync(0xffffffffu, acc, lane >> 1);
+            acc1 = __shfl_sync(0xffffffffu, acc1, lane >> 1);
+            if (lane & 1) acc = acc1;
             if (!done) {   // streaming given up: the register walk of the warp's share
                 const int k0 = c0 * SC;
                 acc = sell_row_dot<true, float>(d, w, x, ((size_t)sl * d.K + k0) * 32 + lane, cnt - k0,

@@ -444,6 +444,9 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
         });
     }
     const int cap = min(cnt, d.K), kmax = __reduce_max_sync(~0u, cap);
+    // FP16 weights are padded with zeros (column offset 0) to whole chunks of 16 entries, so that
+    // k_spmv_ring_split needs no bounds
+    const int kpad = w16 ? (kmax + 15) & ~15 : kmax;
     const int khalf = (kmax + 63) / 64 * 32;   // entries of the first warp: [0, khalf)
     auto decode = [&](unsigned code) { return rtab[rt + (code >> 12)] + (int)code; };
     auto code_of = [&](int k) { return (unsigned)list[(k < low ? k : L + 15 + low - k) * 32 + lane]; };
@@ -476,6 +479,12 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
         b[0] += w;
         b[1] += grad_weight(rinv);
         b[2] += __half2float(hw);
+    };
+    auto pad = [&](int k) {
+        if (w16 && k < kpad) {
+            wh[k * 32] = __ushort_as_half((unsigned short)0);
+            if (n16) c16[k * 32] = 0;
+        }
     };
     auto fold = [&]() {
 #pragma unroll
@@ -510,6 +519,7 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
                     a[q] = al[q] = 0.f;
                 }
         });
+        for (int t = k; t < kpad; ++t) pad(t);
         fold();
         if (k < khalf) {   // the whole row lies in the first half
 #pragma unroll
@@ -520,7 +530,7 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
             }
         }
     } else {
-        const int idle = min(i, d.n - 1), kb = warp ? khalf : 0, ke = warp ? kmax : min(khalf, kmax);
+        const int idle = min(i, d.n - 1), kb = warp ? khalf : 0, ke = warp ? kpad : min(khalf, kpad);
         // the first warp's gradient entries from the bottom of the list, the second one's from its top
         unsigned ga = smem_u32(glist + lane * kGradStride + (warp ? d.KG - 1 : 0));
         const int gs = warp ? -2 : 2;
@@ -595,6 +605,7 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (k + u < cap) entry(k + u, cj[u], w[u], rinv[u]);
+                    else pad(k + u);
                     grad(k + u < cap, rr[u], cc[u]);
                 }
             }
