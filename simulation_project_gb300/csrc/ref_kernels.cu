@@ -932,7 +932,41 @@ __global__ void __launch_bounds__(128) k_ref_lanes(int n, float coef, float minu
     if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
+// 32 targets per warp, operators without rarer pairs
+template <class Op>
+constexpr int rs_warps() { return Op::NS == 1 ? 4 : 2; }
+template <class Op>
+__global__ void __launch_bounds__(rs_warps<Op>() * 32) k_ref_slices(int n, float minus_zero, const __grid_constant__ RefBind b) {
+    using W = RpSlice<Op>;
+    __shared__ __align__(16) float sm[rs_warps<Op>() * W::kFloats];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = (blockIdx.x * rs_warps<Op>() + warp) * 32;
+    if (first >= n) return;
+    const int id = first + lane;
+    RpTarget t{};
+    int cx = 0, cy = 0, cz = 0;
+    bool walk = false, fin = false;
+    if (id < n) {
+        t.pos = b.pos[id];
+        fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
+    }
+    W w(sm + warp * W::kFloats, RefOp<Op>::radius(b.param), minus_zero, first, t);
+    w.run(b, walk && fin, cx, cy, cz);
+    float sum[Op::NS];
+    const float none[1] = {0.0f};
+#pragma unroll
+    for (int c = 0; c < Op::NS; ++c) sum[c] = w.sum(c);
+    if (fin) RefOp<Op>::finish(b, id, t, sum, none, 0.0f);
+}
+
 inline int grid_of(int n) { return div_up(n, kBlock); }
+
+// From here on a warp takes 32 targets of the pressure, its gradient and the temperature (us,
+// k_ref_pairs / k_ref_slices): pressure 58 / 60 at 32,768 particles, 104 / 64 at 64,000,
+// 1,160 / 437 at 884,736; gradient 130 / 101 and 1,406 / 884; temperature 112 / 89 and
+// 1,248 / 642.  The predictor accepts seven times as many pairs and empties its lists too
+// often (3,120 / 3,514 at 884,736); the turbulence has nine sums.
+constexpr int kRefSlices = 40000;
 
 // Targets per warp of an operator: kMany share each round's candidates; below `few` of
 // them that leaves too few warps per SM and two per warp finish sooner.  Measured in us,
@@ -940,11 +974,20 @@ inline int grid_of(int n) { return div_up(n, kBlock); }
 // at 32,768; turbulence (9 sums, 4 per warp) 90 / 107 at 32,768, 297 / 296 at 103,823.
 template <class Op, int kMany>
 cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
-    if (n < few)
+    constexpr bool kSlices = std::is_same<Op, RpPressure>::value || std::is_same<Op, RpGradient>::value ||
+                             std::is_same<Op, RpTemperature>::value;
+    if (n < few) {
         MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, g_bind);
-    else
-        MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f,
-                                                                                                        g_bind);
+        return cudaGetLastError();
+    }
+    if constexpr (kSlices) {
+        if (n >= kRefSlices) {
+            constexpr int W = rs_warps<Op>();
+            MPS_COUNT_LAUNCH k_ref_slices<Op><<<div_up(n, W * 32), W * 32, 0, st>>>(n, -0.0f, g_bind);
+            return cudaGetLastError();
+        }
+    }
+    MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, g_bind);
     return cudaGetLastError();
 }
 // Below it a triangle is walked by 32 lanes (few triangles are large ones), else by 8.

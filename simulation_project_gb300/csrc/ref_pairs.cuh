@@ -23,7 +23,7 @@
 // accepted and left most of the chip idle below 100k particles.  Measured in us, before
 // and after: 15,625 particles pressure 312 / 50, heat 324 / 53, turbulence 414 / 62,
 // predictor 531 / 94; 103,823 pressure 334 / 137, gradient 462 / 177; 884,736 pressure
-// 1,520 / 1,040, gradient 2,450 / 1,370.
+// 1,520 / 1,160, gradient 2,450 / 1,406 (from 40,000 particles on RpSlice takes over these).
 #pragma once
 
 namespace mps {
@@ -43,6 +43,7 @@ struct RpTarget {
 // ---- operators: NS sums per target, NX sums over rarer pairs, terms and scalars ----
 struct RpExplicitly {
     static constexpr int NS = 3, NX = 9;
+    static constexpr bool kIndex = true;   // its terms read the candidate
     static constexpr bool kLe = false, kPos = false, kVel = true, kScalar = false;
     static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
                                                  float (&v)[NS]) {
@@ -79,6 +80,7 @@ struct RpExplicitly {
 };
 struct RpPressure {
     static constexpr int NS = 1, NX = 0;
+    static constexpr bool kIndex = false;
     static constexpr bool kLe = false, kPos = false, kVel = false, kScalar = false;
     static __device__ __forceinline__ void terms(const RefBind&, float re, const RpTarget&, int, float d,
                                                  float (&v)[NS]) {
@@ -87,6 +89,7 @@ struct RpPressure {
 };
 struct RpGradient {
     static constexpr int NS = 3, NX = 0;
+    static constexpr bool kIndex = true;
     static constexpr bool kLe = false, kPos = true, kVel = false, kScalar = true;
     static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
                                                  float (&v)[NS]) {
@@ -102,6 +105,7 @@ struct RpGradient {
 };
 struct RpTemperature {
     static constexpr int NS = 1, NX = 0;
+    static constexpr bool kIndex = true;
     static constexpr bool kLe = true, kPos = false, kVel = false, kScalar = true;
     static __device__ __forceinline__ void terms(const RefBind& b, float re, const RpTarget& t, int x, float d,
                                                  float (&v)[NS]) {
@@ -495,6 +499,343 @@ struct RpWarp {
         return r;
     }
     __device__ __forceinline__ float rare_sum(int c) const { return sm[kQueue + NX * (lane < T ? lane : 0) + c]; }
+};
+
+// Many targets: a warp owns 32 consecutive ones, a lane each.  Consecutive particles of the
+// sorted order follow a column of cells in z, so they lie in one cell or in two on top of each
+// other and share nearly all candidates:
+//   cull    32 candidates a round, a lane each, against the box around the targets; what is
+//           in reach goes to a ring in shared memory
+//   screen  every candidate of the ring against all 32 targets at once (its coordinates
+//           broadcast, two candidates per packed instruction); a lane appends what it accepts
+//           to its own list, without votes or ranks
+//   terms   when a list could overflow: the lists as one sequence, a lane per pair
+//   sums    a lane per (component, target) adds the terms in order
+// Per candidate that is about 8 instructions for 32 targets where RpWarp needs 17 for 8, at a
+// quarter of the warps.  A list entry is one word and its squared distance is computed
+// again with the terms: with both kept, 15.6 instead of 10.9 KB per warp, the gradient took 1,083
+// instead of 884 us at 884,736 particles and, beside the pressure on other streams, lost it all.
+template <class Op>
+struct RpSlice {
+    static constexpr int NS = Op::NS;
+    static_assert(Op::NX == 0, "no rarer pairs");
+    static constexpr int kCap = 48, kStride = 49;             // a list: at most 32 entries and 16 new ones
+    static constexpr int kPlane = 32 * kStride;               // a word per entry: the candidate or, if the
+                                                              // terms need no more, the squared distance
+    static constexpr int G = NS > 1 ? 8 : 32, NG = 32 / G;    // targets whose terms are held at a time
+    static constexpr int kMore = NS > 1 ? 9 + (NS - 1) * (G * kStride + 9) : 0;   // terms past the first, which takes its entry's place
+    static constexpr int kRing = (kPlane + kMore + 3) & ~3, kSum = kRing + 4 * 64;
+    static constexpr int kFloats = kSum + NS * 32;
+    static_assert(NS * G <= 32 || NS == 1, "a lane per sum");
+
+    float* sm;
+    float re, re2x, mind;
+    unsigned long long nz2;
+    int lane, first, cnt;
+    RpTarget me;
+
+    __device__ __forceinline__ RpSlice(float* smem, float radius, float minus_zero, int first_id,
+                                       const RpTarget& t)
+        : sm(smem), re(radius), re2x(ref_screen2(radius)), mind((float)(radius * 1e-3)),
+          nz2(rp_pack(minus_zero, minus_zero)), lane(threadIdx.x & 31), first(first_id), cnt(0), me(t) {
+#pragma unroll
+        for (int c = 0; c < NS; ++c) sm[kSum + c * 32 + lane] = 0.0f;
+        __syncwarp();
+    }
+
+    // row of component c of target t's terms
+    __device__ __forceinline__ float* row(int c, int t) const {
+        return c == 0 ? sm + t * kStride : sm + kPlane + 9 + (c - 1) * (G * kStride + 9) + (t % G) * kStride;
+    }
+
+    // Lists -> terms -> sums; empties the lists.  Terms of several components are called, not
+    // inlined, at the places that need them: their code would not fit the instruction cache
+    // (the gradient took twice as long).
+    __device__ __forceinline__ void flush(const RefBind& b) {
+        if constexpr (NS > 1) {
+            flush_call(b, sm, re, cnt, me);
+        } else {
+            flush_lists(b);
+        }
+        cnt = 0;
+    }
+    static __device__ __noinline__ void flush_call(const RefBind& b, float* sm, float re, int cnt, RpTarget me) {
+        RpSlice(sm, re, cnt, me).flush_lists(b);
+    }
+    __device__ __forceinline__ RpSlice(float* smem, float radius, int n, const RpTarget& t)
+        : sm(smem), re(radius), re2x(0.0f), mind((float)(radius * 1e-3)), nz2(0), lane(threadIdx.x & 31), first(0),
+          cnt(n), me(t) {}
+    __device__ __forceinline__ void flush_lists(const RefBind& b) {
+        __syncwarp();
+        int end = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(~0u, end, o);
+            if (lane >= o) end += v;
+        }
+        const int start = end - cnt;
+#pragma unroll 1
+        for (int g = 0; g < NG; ++g) {
+            const int e1 = __shfl_sync(~0u, end, g * G + G - 1);
+#pragma unroll 1
+            for (int e0 = __shfl_sync(~0u, start, g * G); e0 < e1; e0 += 32) {
+                const int e = e0 + lane;
+                int t = g * G;   // the last target whose pairs start at or before e
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) {
+                    const int v = __shfl_sync(~0u, start, t + o);
+                    if (v <= e) t += o;
+                }
+                const int at = e - __shfl_sync(~0u, start, t);
+                RpTarget q;
+                if constexpr (Op::kPos || Op::kIndex) {
+                    q.pos.x = __shfl_sync(~0u, me.pos.x, t);
+                    q.pos.y = __shfl_sync(~0u, me.pos.y, t);
+                    q.pos.z = __shfl_sync(~0u, me.pos.z, t);
+                }
+                if constexpr (Op::kVel) {
+                    q.vel.x = __shfl_sync(~0u, me.vel.x, t);
+                    q.vel.y = __shfl_sync(~0u, me.vel.y, t);
+                    q.vel.z = __shfl_sync(~0u, me.vel.z, t);
+                }
+                if constexpr (Op::kScalar) q.s = __shfl_sync(~0u, me.s, t);
+                if (e < e1) {
+                    float v[NS];
+#pragma unroll
+                    for (int c = 0; c < NS; ++c) v[c] = 0.0f;
+                    float d2 = row(0, t)[at];
+                    int x = 0;
+                    if constexpr (Op::kIndex) {
+                        x = __float_as_int(d2);
+                        const Scalar3 p = b.pos[x];
+                        const float dx = q.pos.x - p.x, dy = q.pos.y - p.y, dz = q.pos.z - p.z;
+                        d2 = dx * dx + dy * dy + dz * dz;
+                    }
+                    float d = ref_sqrt(d2);
+                    const bool ok = Op::kLe ? d <= re : d < re;
+                    if (d < mind) d = mind;
+                    if (ok) Op::terms(b, re, q, x, d, v);
+#pragma unroll
+                    for (int c = 0; c < NS; ++c) row(c, t)[at] = v[c];
+                }
+            }
+            __syncwarp();
+            const int t = g * G + lane % G, n = __shfl_sync(~0u, cnt, t), most = __reduce_max_sync(~0u, n);
+            const int c = lane < NS * G ? lane / G : 0;
+            const float* const r = row(c, t);
+            float s = sm[kSum + c * 32 + t];
+#pragma unroll 1
+            for (int e = 0; e < most; e += 4) {
+                float v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = e + u < n ? r[e + u] : 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s += v[u];   // + 0 leaves a sum that starts at + 0 alone
+            }
+            __syncwarp();
+            if (lane < NS * G) sm[kSum + c * 32 + t] = s;
+        }
+        cnt = 0;
+    }
+
+    // Candidates of the targets `grp`, all in cells (cx, cy, cz) and (cx, cy, cz + 1); this
+    // lane's target in cell layer tz
+    __device__ __forceinline__ void walk(const RefBind& b, unsigned grp, int cx, int cy, int cz, bool two, int tz) {
+        const Integer3 dims = b.box.m_GridSize;
+        const bool mine = grp >> lane & 1u;
+        float* const rx = sm + kRing;
+        float* const ry = rx + 64;
+        float* const rz = ry + 64;
+        int* const ri = reinterpret_cast<int*>(rz + 64);
+        const float nan = __int_as_float(0x7fffffff);
+        const bool far_target = __any_sync(
+            ~0u, mine && fmaxf(fabsf(me.pos.x), fmaxf(fabsf(me.pos.y), fabsf(me.pos.z))) > kRpHuge);
+        const int id = first + lane;
+        unsigned long long tx = 0, ty = 0, tz2 = 0;   // (-t, -t) per coordinate
+        float lo[3], hi[3];
+        bool in = false;
+        int wp = 0, rp = 0, own_until = 0;   // ring positions below own_until may hold targets
+        // 16 candidates of the ring against every target
+        auto screen = [&](int at, bool self) {
+            float* const list = sm + lane * kStride;
+            unsigned qa = (unsigned)__cvta_generic_to_shared(list + cnt);
+            const unsigned q0 = (unsigned)__cvta_generic_to_shared(list);
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                ulonglong2 X[2], Y[2], Z[2];
+                int4 I[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int o = at + 8 * part + 4 * c;
+                    X[c] = *reinterpret_cast<const ulonglong2*>(rx + o);
+                    Y[c] = *reinterpret_cast<const ulonglong2*>(ry + o);
+                    Z[c] = *reinterpret_cast<const ulonglong2*>(rz + o);
+                    I[c] = *reinterpret_cast<const int4*>(ri + o);
+                }
+                float d2[8];
+                int x[8];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const unsigned long long dx = rp_add2(h ? X[c].y : X[c].x, tx), dy = rp_add2(h ? Y[c].y : Y[c].x, ty),
+                                                 dz = rp_add2(h ? Z[c].y : Z[c].x, tz2);
+                        rp_unpack(rp_add2(rp_add2(rp_mul2(dx, dx, nz2), rp_mul2(dy, dy, nz2)), rp_mul2(dz, dz, nz2)),
+                                  d2[4 * c + 2 * h], d2[4 * c + 2 * h + 1]);
+                    }
+                    x[4 * c] = I[c].x;
+                    x[4 * c + 1] = I[c].y;
+                    x[4 * c + 2] = I[c].z;
+                    x[4 * c + 3] = I[c].w;
+                }
+                if (self) {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (x[u] == id) d2[u] = nan;   // the target itself
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float entry = Op::kIndex ? __int_as_float(x[u]) : d2[u];
+                    asm volatile(
+                        "{\n .reg .pred a;\n setp.lt.f32 a, %1, %2;\n @a st.shared.f32 [%0], %3;\n"
+                        " @a add.u32 %0, %0, 4;\n}\n"
+                        : "+r"(qa)
+                        : "f"(d2[u]), "f"(re2x), "f"(entry)
+                        : "memory");
+                }
+            }
+            cnt = (int)(qa - q0) >> 2;
+            if (__any_sync(~0u, cnt > kCap - 16)) flush(b);
+        };
+        auto drain = [&]() {   // the ring's last, incomplete 32
+            if (wp > rp) {
+                if (lane >= wp - rp) {
+                    rx[(rp & 32) + lane] = nan;
+                    ri[(rp & 32) + lane] = -1;
+                }
+                __syncwarp();
+                screen(rp & 32, true);
+                if (wp - rp > 16) screen((rp & 32) + 16, true);
+                __syncwarp();
+            }
+            wp = rp = own_until = 0;
+        };
+#pragma unroll 1
+        for (int up = -1; up <= (two ? 2 : 1); ++up) {   // layers of cells
+            if (up == -1 || two) {
+                // a layer's targets: those at most one layer away (two: each layer has its own)
+                in = mine && (tz == cz ? up <= 1 : up >= 0);
+                const Scalar3 p = in ? me.pos : s3(nan, nan, nan);
+                tx = rp_pack(-p.x, -p.x);
+                ty = rp_pack(-p.y, -p.y);
+                tz2 = rp_pack(-p.z, -p.z);
+                const float v[3] = {p.x, p.y, p.z};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = in ? v[a] : 3.4e38f;
+                    hi[a] = in ? v[a] : -3.4e38f;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        lo[a] = fminf(lo[a], __shfl_xor_sync(~0u, lo[a], o));
+                        hi[a] = fmaxf(hi[a], __shfl_xor_sync(~0u, hi[a], o));
+                    }
+                }
+            }
+            // lane m < 9: cell m of the layer (j outer, i inner)
+            int s = 0, len = 0;
+            if (lane < 9) {
+                const int m = cell_key(dims, (int)((unsigned)cx + (unsigned)(lane % 3 - 1)),
+                                       (int)((unsigned)cy + (unsigned)(lane / 3 - 1)), (int)((unsigned)cz + (unsigned)up));
+                if (m >= 0 && m < b.cell_num) {
+                    s = b.cell_start[m];
+                    if (s != -1) len = max(b.cell_end[m] - s, 0);
+                }
+            }
+            unsigned cells = __ballot_sync(~0u, len > 0);
+            int x0 = 0, e = 0;
+            auto fetch = [&](int x) {
+                return RpWarp<Op, 8>::fetch(b, x, e);
+            };
+            auto next_cell = [&]() {
+                if (!cells) return false;
+                const int m = __ffs(cells) - 1;
+                cells &= cells - 1u;
+                x0 = __shfl_sync(~0u, s, m);
+                e = x0 + __shfl_sync(~0u, len, m);
+                return true;
+            };
+            bool more = next_cell();
+            Scalar3 qn = s3(nan, nan, nan);
+            if (more) qn = fetch(x0 + lane);
+#pragma unroll 1
+            while (more) {
+                const Scalar3 q = qn;
+                const int x = x0 + lane;
+                const bool own = x0 < first + 32 && x0 + 32 > first;
+                x0 += 32;
+                if (x0 >= e) more = next_cell();
+                if (more) qn = fetch(x0 + lane);   // the next round's, under this one's work
+                const bool huge = fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))) > kRpHuge;
+                if (far_target || __any_sync(~0u, huge)) {
+                    // a squared distance may overflow (the reference accepts an infinite one)
+                    drain();
+#pragma unroll 1
+                    for (int c = 0; c < 32; ++c) {
+                        const int xc = __shfl_sync(~0u, x, c);
+                        const float dx = me.pos.x - __shfl_sync(~0u, q.x, c), dy = me.pos.y - __shfl_sync(~0u, q.y, c),
+                                    dz = me.pos.z - __shfl_sync(~0u, q.z, c);
+                        const float d2 = dx * dx + dy * dy + dz * dz;
+                        if (in && xc != id && d2 == d2 && !(d2 >= re2x && d2 <= 3.402823466e38f)) {
+                            sm[lane * kStride + cnt] = Op::kIndex ? __int_as_float(xc) : d2;
+                            ++cnt;
+                        }
+                        if (__any_sync(~0u, cnt > kCap - 16)) flush(b);
+                    }
+                    continue;
+                }
+                // the box in the order and rounding of a pair's squared distance: never above it
+                const float ax = fmaxf(fmaxf(lo[0] - q.x, q.x - hi[0]), 0.0f), ay = fmaxf(fmaxf(lo[1] - q.y, q.y - hi[1]), 0.0f),
+                            az = fmaxf(fmaxf(lo[2] - q.z, q.z - hi[2]), 0.0f);
+                const bool keep = q.x == q.x && !(ax * ax + ay * ay + az * az >= re2x);
+                const unsigned m = __ballot_sync(~0u, keep);
+                if (keep) {
+                    const int pos = (wp + __popc(m & ((1u << lane) - 1u))) & 63;
+                    rx[pos] = q.x;
+                    ry[pos] = q.y;
+                    rz[pos] = q.z;
+                    ri[pos] = x;
+                }
+                wp += __popc(m);
+                own_until = own ? wp : own_until;
+                if (wp - rp >= 32) {
+                    __syncwarp();
+                    const bool self = own_until > rp;
+                    screen(rp & 32, self);
+                    screen((rp & 32) + 16, self);
+                    rp += 32;
+                    __syncwarp();
+                }
+            }
+            if (two) drain();
+        }
+        drain();
+    }
+
+    // all targets of the warp: `live`, their cells (tx, ty, tz)
+    __device__ __forceinline__ void run(const RefBind& b, bool live, int tx, int ty, int tz) {
+        for (unsigned todo = __ballot_sync(~0u, live); todo;) {
+            const int l = __ffs(todo) - 1;
+            const int gx = __shfl_sync(~0u, tx, l), gy = __shfl_sync(~0u, ty, l), gz = __shfl_sync(~0u, tz, l);
+            const bool here = (todo >> lane & 1u) && tx == gx && ty == gy;
+            const unsigned up = __ballot_sync(~0u, here && gz != 0x7fffffff && tz == gz + 1);
+            const unsigned grp = __ballot_sync(~0u, here && tz == gz) | up;
+            walk(b, grp, gx, gy, gz, up != 0u, tz);
+            todo &= ~grp;
+        }
+        flush(b);
+    }
+    // sum c of this lane's target
+    __device__ __forceinline__ float sum(int c) const { return sm[kSum + c * 32 + lane]; }
 };
 
 // A lane per target, each walking its own 27 cells: the candidates four at a time from

@@ -122,3 +122,29 @@ def test_predictor_with_a_lane_per_target(misaligned):
 def test_turbulence_with_four_targets_per_warp():
     _compare(_scene(_block((47, 47, 46), seed=7), 7),
              ops=[("CalcTurbulenceViscosity", ORC.calc_turbulence_viscosity)])
+
+
+SLICE_OPS = [("CalcTemperatureFactor", ORC.calc_temperature_factor), ("CalcExplicitPressure", ORC.calc_explicit_pressure),
+             ("CalcExplicitPressureGradient", ORC.calc_explicit_pressure_gradient)]
+
+
+@pytest.mark.parametrize("shape,spacing,n", [((35, 35, 33), 1.0, 40001), ((36, 34, 33), 1.7, None), ((200, 1, 201), 1.0, None),
+                                             ((36, 34, 33), 0.6, 40030)], ids=["ragged", "sparse", "layer", "crowded"])
+def test_slices_of_32_targets(shape, spacing, n):
+    """k_ref_slices: a last slice of one target, slices over many cells, lists emptied within a
+    round, cells of a few and of 300 particles."""
+    _compare(_scene(_block(shape, spacing, seed=8)[:n], 8), ops=SLICE_OPS)
+
+
+@pytest.mark.parametrize("far", [3e18, 1e19, np.inf, np.nan])
+def test_slices_with_skipped_and_far_particles(far):
+    sc = _scene(_block((36, 35, 32), seed=9), 9)
+
+    def setup(st):
+        rng = np.random.default_rng(10)
+        away = rng.choice(st.n, 40, replace=False)
+        st.out_pos[away[:20], 0] = far
+        st.out_pos[away[20:], 2] = -far
+        st.out_id[away] = -1
+        st.out_id[rng.choice(st.n, 400, replace=False)] = -1
+    _compare(sc, setup, ops=SLICE_OPS)
