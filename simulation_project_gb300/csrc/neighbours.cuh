@@ -333,7 +333,7 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
     const int h = live ? d.key[i] : 0;
     const float4 p = live ? d.opos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float re = (float)d.c.re_lap, re2s = re * re, mind = (float)d.c.mind_lap;
-    const float reg = (float)d.c.re_grad, mindg = (float)d.c.mind_grad;
+    const float reg = (float)d.c.re_grad;
     const float cut = d.c.reach2, wmax = d.c.wmax_lap, wgmax = d.c.wmax_grad;
     const unsigned all = __ballot_sync(~0u, live);
     // first list position of this warp's lane and the step to the next one, in bytes

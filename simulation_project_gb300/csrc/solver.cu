@@ -27,6 +27,7 @@
 #include "native_kernels.cuh"
 #include "neighbours.cuh"
 #include "coarse.cuh"
+#include "cg_small.cuh"
 #include "../../include/mps_learned.h"
 
 namespace mps {
@@ -303,6 +304,14 @@ struct Solver {
         e = e ? e : mk(&d.r32, N); e = e ? e : mk(&d.z32, N); e = e ? e : mk(&d.pf32, N); e = e ? e : mk(&d.q32, N);
         e = e ? e : mk(&d.d32, N); e = e ? e : mk(&d.m32, N);
         e = e ? e : mk(&d.xs, N); e = e ? e : mk(&d.p32, N);
+        {   // k_cg_small: sizes it can have (see cg_small_slices)
+            const size_t rows = std::min(N32, (size_t)32 * kCgMaxSlices * 1024);
+            e = e ? e : mk(&cgs.zp, rows);
+            e = e ? e : mk(&cgs.part, 4 * 1024);
+            e = e ? e : mk(&cgs.coarse, kCgAgg + 1024);
+            e = e ? e : mk(&cgs.bar, 1);
+            if (!e) e = cudaMemset(cgs.bar, 0, sizeof(unsigned));
+        }
         e = e ? e : mk(&d.red, 4 * (size_t)kRedBlocks);
         e = e ? e : mk(&d.scal, (size_t)S_COUNT);
         e = e ? e : mk(&d.red_count, 16);
@@ -1450,6 +1459,46 @@ struct Solver {
         return inner16() && mg_ready ? 7e-4 : 2e-6;
     }
 
+    // ---- the inner CG in one launch (k_cg_small) ----
+    // The rows have to fit in the shared memory of the SMs (a CTA on each), and beside them the
+    // preconditioner's level 1, which has to be the last level or the one above it.
+    CgSmall cgs{};
+    int cg_sms = -1;
+    static constexpr size_t kCgSmem = 200 * 1024;   // beside 20 KB of static arrays
+    size_t cg_smem(int spc) const { return cg_small_smem(d.K, spc, mg_ready ? mg.levels : 0, mg_ready ? mg.L[1].n : 0); }
+    int cg_small_slices() {
+        if (cg_sms < 0) {
+            int dev = 0, coop = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&cg_sms, cudaDevAttrMultiProcessorCount, dev);
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+            if (!coop || !cgs.zp ||
+                cudaFuncSetAttribute(k_cg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmem) != cudaSuccess)
+                cg_sms = 0;
+        }
+        if (cg_sms <= 0 || !inner16() || prefer_wide || timer.on || (mg_ready && (mg.levels > 2 || mg.L[1].n > kCgAgg || fine_post() || opt.mg_sweeps > 1)))
+            return 0;
+        const int nsl = div_up(d.n, 32), spc = div_up(nsl, cg_sms);
+        return spc >= 1 && spc <= kCgMaxSlices && cg_smem(spc) <= kCgSmem ? spc : 0;
+    }
+    // A d = r / rn of one refinement pass to tol: d in d32; the iterations, -1 on failure
+    int cg_small(int spc, double rn, double tol) {
+        cgs.spc = spc;
+        cgs.levels = mg_ready ? mg.levels : 0;
+        cgs.flex = flex_step ? 1 : 0;
+        cgs.maxit = opt.cg_max_iter;
+        cgs.scale = 1.0 / rn;
+        cgs.tol = tol;
+        void* args[] = {(void*)&d, (void*)&mg, (void*)&cgs};
+        if (MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_cg_small, dim3(div_up(div_up(d.n, 32), spc)),
+                                                         dim3(kCgThreads), args, cg_smem(spc), st))
+            return -1;
+        if (pull_scal()) return -1;
+        const int it = (int)h_scal[S_ITER];
+        spmv_launches += std::max(it, 0);
+        return it;
+    }
+
     // FP32 Jacobi-PCG inside FP64 iterative refinement
     CCTStatusType solve_ir(MpsStepStats& S) {
         const float* w = (const float*)d.nbrw;
@@ -1487,16 +1536,22 @@ struct Solver {
             // 0.3 margin), but not below what FP32 CG reliably reaches (ir_inner_rtol)
             const double need = 0.3 * opt.cg_rtol * bnorm / rn;
             const double inner_tol = std::max(need, ir_inner_rtol());
-            MPS_COUNT_LAUNCH k_cg_start<float><<<red_blocks(d.n), 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,
-                                                          inner_tol, opt.cg_max_iter);
-            if (mg_ready) {
-                timer.mark(PH_PRECOND, st);
-                mg_apply(d.r32, d.z32, d.p32, 1);
-                timer.mark(PH_VEC, st);
-            }
             const int pi = outer < kPassMemory ? outer : kPassMemory - 1;
-            const int it = cg_loop<float, float, float>(d.d32, d.r32, d.z32, d.p32, d.q32, w, nullptr, d.m32,
-                                                        opt.cg_max_iter, pass_its[pi]);
+            const int small = cg_small_slices();
+            int it;
+            if (small > 0) {
+                it = cg_small(small, rn, inner_tol);
+            } else {
+                MPS_COUNT_LAUNCH k_cg_start<float><<<red_blocks(d.n), 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,
+                                                              inner_tol, opt.cg_max_iter);
+                if (mg_ready) {
+                    timer.mark(PH_PRECOND, st);
+                    mg_apply(d.r32, d.z32, d.p32, 1);
+                    timer.mark(PH_VEC, st);
+                }
+                it = cg_loop<float, float, float>(d.d32, d.r32, d.z32, d.p32, d.q32, w, nullptr, d.m32,
+                                                            opt.cg_max_iter, pass_its[pi]);
+            }
             if (it < 0) return CCT_CUDAERR;
             pass_its[pi] = it;
             S.cg_iterations += it;
