@@ -397,8 +397,33 @@ __device__ V3<T> closest_on_tri(const V3<T>& p, const V3<T>& a, const V3<T>& b, 
 // on a shared edge or vertex, whose distances differ only by rounding) resolve to the
 // lowest id instead of to the rounding of one implementation.  The choice matters for
 // drag bodies, whose drag acts along the chosen triangle's normal.
+//
+// The W warps of a CTA share 32 particles, a lane each: consecutive particles mostly have one
+// cell and so one list, whose triangle is then read once for all of them, and the warps
+// take kTriBatch triangles of every W * kTriBatch.  The first warp goes through the round's
+// distances in list order, so the choice is that of one lane going through the list.  Lists are a
+// handful of triangles in most cells and several hundred around a drag body; with a warp
+// per 32 particles the time was the longest list's chain.  (Lanes sharing a particle
+// instead of warps: its triangles' scattered loads cost what the shorter chain gains.)
+// The result is the first warp's; every thread of the CTA calls it.
+constexpr int kTriWarps = 8, kTriBatch = 4;
 template <class T>
-__device__ void nearest_tri(const Dev& d, const V3<T>& p, bool drag_only, T& md, V3<T>& mdir, int& mid) {
+__device__ __forceinline__ V3<T> tri_offset(const Dev& d, const V3<T>& p, int t) {
+    V3<T> q;
+    if constexpr (sizeof(T) == 4) {
+        const float* v = d.tri32 + 9 * (size_t)t;
+        q = closest_on_tri<T>(p, v3<T>(v[0], v[1], v[2]), v3<T>(v[3], v[4], v[5]), v3<T>(v[6], v[7], v[8]));
+    } else {
+        const double* v = d.tri + 9 * (size_t)t;
+        q = closest_on_tri<T>(p, v3<T>(v[0], v[1], v[2]), v3<T>(v[3], v[4], v[5]), v3<T>(v[6], v[7], v[8]));
+    }
+    return v3(p.x - q.x, p.y - q.y, p.z - q.z);
+}
+template <class T, int W>
+__device__ __forceinline__ void nearest_tri(const Dev& d, const V3<T>& p, bool live, bool drag_only, T& md, V3<T>& mdir,
+                                            int& mid) {
+    constexpr int N = W * kTriBatch;
+    __shared__ T dist[W > 1 ? 2 : 1][W > 1 ? N : 1][32];
     const T tol = sizeof(T) == 8 ? T(1e-12 * d.c.l0) : T(1e-5 * d.c.l0);
     md = T(1e8);
     mdir = v3(T(0), T(0), T(0));
@@ -407,7 +432,7 @@ __device__ void nearest_tri(const Dev& d, const V3<T>& p, bool drag_only, T& md,
     if constexpr (sizeof(T) == 4) {
         // FP32 path: cell of the candidate triangles in FP32 (the wall influence radius
         // is at most one cell, so the 27-cell neighbourhood covers it either way)
-        const float inv = (float)(1.0 / (double)d.box.m_CellSize);
+        const float inv = (float)d.c.ics;
         cx = f2i((p.x - d.box.m_BufferedZone.m_MinBound.x) * inv);
         cy = f2i((p.y - d.box.m_BufferedZone.m_MinBound.y) * inv);
         cz = f2i((p.z - d.box.m_BufferedZone.m_MinBound.z) * inv);
@@ -424,28 +449,53 @@ __device__ void nearest_tri(const Dev& d, const V3<T>& p, bool drag_only, T& md,
     cy = min(max(cy, 0), G.y - 1);
     cz = min(max(cz, 0), G.z - 1);
     const int key = 2 * cell_key(G, cx, cy, cz) + (drag_only ? 1 : 0);
-    const int s = d.tcs[key];
-    if (s < 0) return;
-    const int e = d.tcs[2 * d.cells + key];
-    for (int l = s; l < e; ++l) {
-        const int t = d.tids[l];
-        V3<T> q;
-        if constexpr (sizeof(T) == 4) {
-            const float* v = d.tri32 + 9 * (size_t)t;
-            q = closest_on_tri<T>(p, v3<T>(v[0], v[1], v[2]), v3<T>(v[3], v[4], v[5]), v3<T>(v[6], v[7], v[8]));
-        } else {
-            const double* v = d.tri + 9 * (size_t)t;
-            q = closest_on_tri<T>(p, v3<T>(v[0], v[1], v[2]), v3<T>(v[3], v[4], v[5]), v3<T>(v[6], v[7], v[8]));
+    const int s = live ? d.tcs[key] : -1;
+    const int len = s < 0 ? 0 : d.tcs[2 * d.cells + key] - s;
+    if constexpr (W == 1) {
+        for (int l = s; l < s + len; ++l) {
+            const int t = d.tids[l];
+            const V3<T> dv = tri_offset<T>(d, p, t);
+            const T dd = sqrt(dv.x * dv.x + dv.y * dv.y + dv.z * dv.z);
+            if (dd < md - tol) {
+                md = dd;
+                mdir = dv;
+                mid = t;
+            }
         }
-        const V3<T> dv = v3(p.x - q.x, p.y - q.y, p.z - q.z);
-        const T dd = sqrt(dv.x * dv.x + dv.y * dv.y + dv.z * dv.z);
-        if (dd < md - tol) {
-            md = dd;
-            mdir = dv;
-            mid = t;
+    } else {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int most = __reduce_max_sync(~0u, len);   // the same in every warp
+        int buf = 0;
+        for (int l0 = 0; l0 < most; l0 += N, buf ^= 1) {
+#pragma unroll
+            for (int u = 0; u < kTriBatch; ++u) {
+                const int l = l0 + warp * kTriBatch + u;
+                if (l < len) {
+                    const V3<T> dv = tri_offset<T>(d, p, d.tids[s + l]);
+                    dist[buf][warp * kTriBatch + u][lane] = sqrt(dv.x * dv.x + dv.y * dv.y + dv.z * dv.z);
+                }
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const int n = min(N, len - l0);
+                for (int r = 0; r < n; ++r) {
+                    const T dd = dist[buf][r][lane];
+                    if (dd < md - tol) {
+                        md = dd;
+                        mid = l0 + r;
+                    }
+                }
+            }
+        }
+        if (warp == 0 && mid >= 0) {
+            mid = d.tids[s + mid];
+            mdir = tri_offset<T>(d, p, mid);
         }
     }
 }
+// k_wall_distance and k_drag with W warps per 32 particles (W = 1: a CTA of 128 particles)
+template <int W> constexpr int tri_particles() { return W > 1 ? 32 : 128; }
+template <int W> constexpr int tri_threads() { return W > 1 ? W * 32 : 128; }
 
 template <class T>
 __device__ __forceinline__ V3<T> load_p(const Dev& d, int i) {
@@ -468,14 +518,15 @@ __device__ __forceinline__ V3<T> load_v(const Dev& d, int i) {
     }
 }
 
-template <class T>
-__global__ void k_wall_distance(const __grid_constant__ Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
+template <class T, int W>
+__global__ void __launch_bounds__(tri_threads<W>()) k_wall_distance(const __grid_constant__ Dev d) {
+    const int i = blockIdx.x * tri_particles<W>() + (W > 1 ? (int)threadIdx.x & 31 : (int)threadIdx.x);
+    const bool live = i < d.n;
     T md;
     V3<T> dir;
     int mid;
-    nearest_tri<T>(d, load_p<T>(d, i), false, md, dir, mid);
+    nearest_tri<T, W>(d, load_p<T>(d, live ? i : 0), live, false, md, dir, mid);
+    if (!live || (W > 1 && threadIdx.x >= 32)) return;
     d.wdist[i] = md;
     d.wdir[3 * (size_t)i] = dir.x;
     d.wdir[3 * (size_t)i + 1] = dir.y;
@@ -487,15 +538,16 @@ __global__ void k_wall_distance(const __grid_constant__ Dev d) {
 // reference's sorted/original index mix-up): nearest drag-model triangle within the
 // influence radius; 'E'+'V'/'B': velocity decrement k |u|^e n / permeability;
 // 'C': constant velocity; 'F': velocity factor.
-template <class T>
-__global__ void k_drag(const __grid_constant__ Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
+template <class T, int W>
+__global__ void __launch_bounds__(tri_threads<W>()) k_drag(const __grid_constant__ Dev d) {
+    const int i = blockIdx.x * tri_particles<W>() + (W > 1 ? (int)threadIdx.x & 31 : (int)threadIdx.x);
+    const bool live = i < d.n;
     double dv[3] = {0, 0, 0};
     T md;
     V3<T> dir;
     int mid;
-    nearest_tri<T>(d, load_p<T>(d, i), true, md, dir, mid);
+    nearest_tri<T, W>(d, load_p<T>(d, live ? i : 0), live, true, md, dir, mid);
+    if (!live || (W > 1 && threadIdx.x >= 32)) return;
     if (mid >= 0) {
         const DragParameter dp = d.drag[d.tparams[d.tmodel[mid]].DragTriangleID];
         if ((double)md <= (double)dp.CoefficientofInflueneRegion * d.c.l0) {

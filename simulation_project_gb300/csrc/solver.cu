@@ -858,10 +858,25 @@ struct Solver {
         d.rows_c32 = 1;
     }
 
+    // below it the warps of a CTA share the triangle lists of 32 particles (us, a warp per 32
+    // / kTriWarps: drag 113 / 65, walls 34 / 22 at 108,186 particles, 141 / 76 and 31 / 32 at 256,000,
+    // 86 / 110 and 36 / 85 at 882,080: there are warps enough and most CTAs find no triangles)
+    static constexpr int kTriSplit = 300000;
+    template <class T, int W>
+    void launch_tri(bool drag) {
+        const int grid = std::max(1, div_up(d.n, tri_particles<W>()));
+        if (drag) MPS_COUNT_LAUNCH k_drag<T, W><<<grid, tri_threads<W>(), 0, st>>>(d);
+        else MPS_COUNT_LAUNCH k_wall_distance<T, W><<<grid, tri_threads<W>(), 0, st>>>(d);
+    }
+    template <class T>
+    void launch_tri(bool drag) {
+        if (sizeof(T) == 4 && d.n < kTriSplit) launch_tri<T, sizeof(T) == 4 ? kTriWarps : 1>(drag);
+        else launch_tri<T, 1>(drag);
+    }
     template <class T>
     void walls_distance() {
         if (d.tri_n > 0) {
-            MPS_COUNT_LAUNCH k_wall_distance<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
+            launch_tri<T>(false);
         } else {
             cudaMemsetAsync(d.wid, 0xff, sizeof(int) * d.n, st);
         }
@@ -899,7 +914,7 @@ struct Solver {
             timer.mark(PH_WALLS, st);
             if (bins) cudaStreamWaitEvent(st, ev_bins, 0);
             walls_distance<T>();
-            if (d.drag_n > 0 && d.tri_n > 0) MPS_COUNT_LAUNCH k_drag<T><<<blocks_for(d.n), kBlock, 0, st>>>(d);
+            if (d.drag_n > 0 && d.tri_n > 0) launch_tri<T>(true);
             else cudaMemsetAsync(d.dragv, 0, sizeof(double) * 3 * d.n, st);
             timer.mark(PH_PRED, st);
             predict();
