@@ -17,8 +17,8 @@
 // Every CTA adds the CTAs' partial sums in the same order, so all hold the same scalars.
 // us, kernel chain -> here: an iteration 29 -> 13 (one coarse level), a step of 2,000 particles
 // 1,122 -> 853, of 9,248 (two levels) 1,542 -> 1,219, the Poisson solve of 8,000 particles
-// 901 -> 808, of 17,576 1,138 -> 988; above it stops fitting (four slices per CTA), so there is
-// no size at which the chain is the better one.  What bounds it: the three barriers with
+// 901 -> 808, of 17,576 1,138 -> 988; then it stops fitting, so there is no size at which the
+// chain is the better one.  What bounds it: the three barriers with
 // the partial sums behind them, 2 us each, and one round of gathers from L2.
 // The arithmetic per entry and row is the kernel chain's (k_spmv_ring_split, k_cg_update or
 // k_mg_update_restrict and k_mg_fine_z, k_cg_p); sums over rows are taken per warp in FP32 and
@@ -28,7 +28,7 @@
 namespace mps {
 
 constexpr int kCgThreads = 256;
-constexpr int kCgMaxSlices = 4;      // slices per CTA
+constexpr int kCgMaxSlices = 6;      // slices per CTA
 constexpr int kCgInv = 16;           // rows of the coarse inverse kept in shared memory
 constexpr int kCgAgg = 1024;         // level-1 aggregates at most
 struct CgSmall {
@@ -37,6 +37,7 @@ struct CgSmall {
     float* coarse;      // [aggregates + CTAs] share of aggregate I in CTA b at I + b
     unsigned* bar;
     int spc;            // slices per CTA
+    int K;              // room for a row's entries, whole chunks
     int levels, flex, maxit;   // levels of the preconditioner: 0 (Jacobi), 1, 2
     double scale, tol;  // r = scale * residual; stop at this norm of r
 };
@@ -80,10 +81,10 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg_small(const __grid_constan
     __shared__ double psum[2][kCgMaxSlices];
     const int R = c.spc * 32, b = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int sl0 = b * c.spc, row0 = sl0 * 32, nsl = (d.n + 31) >> 5;
-    // a slice's K x 32 columns and weights
+    // a slice's c.K x 32 columns and weights
     unsigned* const cols = (unsigned*)cg_sm;
-    unsigned* const wts = cols + (size_t)c.spc * d.K * 16;
-    float* const sx = (float*)(wts + (size_t)c.spc * d.K * 16);
+    unsigned* const wts = cols + (size_t)c.spc * c.K * 16;
+    float* const sx = (float*)(wts + (size_t)c.spc * c.K * 16);
     float* const sr = sx + R;
     float* const sp = sr + R;
     float* const sq = sp + R;
@@ -115,8 +116,8 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg_small(const __grid_constan
         const size_t e0 = (size_t)(sl0 + s) * d.K * 32;
         const uint4* const gc = (const uint4*)(d.nbr16 + e0);
         const uint4* const gw = (const uint4*)(d.w16 + e0);
-        uint4* const lc = (uint4*)(cols + (size_t)s * d.K * 16);
-        uint4* const lw = (uint4*)(wts + (size_t)s * d.K * 16);
+        uint4* const lc = (uint4*)(cols + (size_t)s * c.K * 16);
+        uint4* const lw = (uint4*)(wts + (size_t)s * c.K * 16);
         for (int k = t; k < n16; k += kCgThreads) {
             lc[k] = gc[k];
             lw[k] = gw[k];
@@ -224,8 +225,8 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg_small(const __grid_constan
             if (t < R) sp[t] = __fmaf_rn(beta, sp[t], zt);
             for (int s = 0; s < c.spc; ++s) {
                 const float2* const zr = c.zp + (sl0 + s) * 32;
-                const unsigned* const lc = cols + (size_t)s * d.K * 16;
-                const unsigned* const lw = wts + (size_t)s * d.K * 16;
+                const unsigned* const lc = cols + (size_t)s * c.K * 16;
+                const unsigned* const lw = wts + (size_t)s * c.K * 16;
                 const int nch = (km[s] + 15) >> 4;
                 float a0 = 0.f, a1 = 0.f;   // rows 2 (lane mod 16) and the next, every other entry
 #pragma unroll 2

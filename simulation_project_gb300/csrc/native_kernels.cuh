@@ -2025,6 +2025,7 @@ __global__ void __launch_bounds__(256) k_count_nnz(const __grid_constant__ Dev d
         d.scal[S_NNZ0] = out[0];
         d.scal[S_NNZ1] = out[1];
         d.scal[S_NINT] = out[2];
+        d.scal[S_MAXROW] = (double)d.istat[0];   // the longest row, from the list pass
     }
 }
 

@@ -1479,8 +1479,10 @@ struct Solver {
     // preconditioner's level 1, which has to be the last level or the one above it.
     CgSmall cgs{};
     int cg_sms = -1;
-    static constexpr size_t kCgSmem = 200 * 1024;   // beside 20 KB of static arrays
-    size_t cg_smem(int spc) const { return cg_small_smem(d.K, spc, mg_ready ? mg.levels : 0, mg_ready ? mg.L[1].n : 0); }
+    static constexpr size_t kCgSmem = 200 * 1024;   // beside 25 KB of static arrays
+    // entries of the longest row (k_count_nnz), in whole chunks
+    int cg_row_room() const { return std::min(d.K, ((int)h_scal[S_MAXROW] + 15) & ~15); }
+    size_t cg_smem(int spc) const { return cg_small_smem(cg_row_room(), spc, mg_ready ? mg.levels : 0, mg_ready ? mg.L[1].n : 0); }
     int cg_small_slices() {
         if (cg_sms < 0) {
             int dev = 0, coop = 0;
@@ -1499,6 +1501,7 @@ struct Solver {
     // A d = r / rn of one refinement pass to tol: d in d32; the iterations, -1 on failure
     int cg_small(int spc, double rn, double tol) {
         cgs.spc = spc;
+        cgs.K = cg_row_room();
         cgs.levels = mg_ready ? mg.levels : 0;
         cgs.flex = flex_step ? 1 : 0;
         cgs.maxit = opt.cg_max_iter;

@@ -1,6 +1,6 @@
 """The inner CG of a pass in one launch (k_cg_small) against the chain of kernels (which a
 profiling solver runs): fewer rows than a slice, slices over several coarse aggregates and
-aggregates over several CTAs, one to four slices per CTA, the size at which the chain takes
+aggregates over several CTAs, one to five slices per CTA, the size at which the chain takes
 over, flexible CG, and an iteration limit that ends it early."""
 import numpy as np
 import pytest
@@ -31,8 +31,8 @@ def _both(sc, njp, **kw):
 
 @pytest.mark.parametrize("njp,flexible", [(False, 0), (True, 0), (True, 1)], ids=["jacobi", "multilevel", "flexible"])
 @pytest.mark.parametrize("shape", [(5, 5, 5), (7, 7, 7), (9, 40, 5), (13, 12, 11), (17, 17, 16), (24, 24, 23), (27, 27, 26),
-                                   (27, 27, 27)],
-                         ids=["125", "343", "slab", "1716", "4624", "13248", "18954", "19683_chain"])
+                                   (27, 27, 27), (31, 31, 31)],
+                         ids=["125", "343", "slab", "1716", "4624", "13248", "18954", "19683", "29791_chain"])
 def test_against_the_kernel_chain(shape, njp, flexible):
     (a, pa, ra), (b, pb, rb) = _both(_block(shape), njp, flexible=flexible)
     assert a["error_flags"] == 0 and b["error_flags"] == 0 and a["inner16"] == 1
