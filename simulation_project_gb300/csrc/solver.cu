@@ -589,9 +589,9 @@ struct Solver {
             MPS_COUNT_LAUNCH k_mg_links<<<blocks_for(L[l].n), kBlock, 0, ss>>>(L[l], L[l < levels ? l + 1 : l], l < levels);
         for (int l = 1; l < levels; ++l)
             MPS_COUNT_LAUNCH k_mg_nbpar<<<blocks_for(27 * L[l].n), kBlock, 0, ss>>>(L[l]);
-        MPS_COUNT_LAUNCH k_mg_particles<<<blocks_for(d.n), kBlock, 0, ss>>>(d, mg);
         MPS_COUNT_LAUNCH k_mg_rows<<<blocks_for(L[1].n), kBlock, 0, ss>>>(d, mg);
-        if (rows_ready) cudaStreamWaitEvent(ss, rows_ready, 0);
+        if (rows_ready) cudaStreamWaitEvent(ss, rows_ready, 0);   // interior flags and rows
+        MPS_COUNT_LAUNCH k_mg_particles<<<blocks_for(d.n), kBlock, 0, ss>>>(d, mg);
         if (mg_assemble(ss, -1) != CCT_NOERR) return CCT_CUDAERR;
         for (int l = 1; l < levels; ++l)
             MPS_COUNT_LAUNCH k_mg_coarsen<<<div_up(L[l + 1].n, kMgCoarsenWarps), kMgCoarsenWarps * 32, 0, ss>>>(L[l], L[l + 1]);
@@ -926,6 +926,17 @@ struct Solver {
         if ((rc = grid())) return rc;
         timer.mark(PH_WALLS, st);
         if (pressure_only && d.tri_n > 0 && bins_dirty && (rc = bin_walls(st, h_int, scan_sums))) return rc;
+        // the multilevel setup runs on the second stream: its topology (which cells are
+        // occupied) beside the wall distances and the list pass, its operators from the rows
+        // on, beside the warm start, the first refinement residual and the learned guess
+        const bool overlap_mg = !fp64() && opt.pressure_mode != MPS_PRESSURE_EXPLICIT &&
+                                opt.preconditioner == MPS_PRECOND_MULTILEVEL;
+        mg_setup_done = false;
+        if (overlap_mg) {
+            cudaEventRecord(ev_setup, st);
+            cudaStreamWaitEvent(st2, ev_setup, 0);
+            if (mg_setup_topology(st2)) return CCT_CUDAERR;
+        }
         walls_distance<T>();
         timer.mark(PH_LIST, st);
         list_rows();
@@ -935,16 +946,6 @@ struct Solver {
         } else {
             MPS_COUNT_LAUNCH k_ppe_setup<<<blocks_for(d.n), kBlock, 0, st>>>(d);
             MPS_COUNT_LAUNCH k_count_nnz<<<red_blocks(d.n), 256, 0, st>>>(d, 4);
-            // the multilevel setup runs on the second stream: its topology (grid and
-            // interior flags only) beside the rows' transpose, its operators from the rows
-            // on, beside the warm start, the first refinement residual and the learned guess
-            const bool overlap_mg = !fp64() && opt.preconditioner == MPS_PRECOND_MULTILEVEL;
-            mg_setup_done = false;
-            if (overlap_mg) {
-                cudaEventRecord(ev_setup, st);
-                cudaStreamWaitEvent(st2, ev_setup, 0);
-                if (mg_setup_topology(st2)) return CCT_CUDAERR;
-            }
             if (fp64()) {
                 const int flags = row_flags();
                 rows_sell(flags);
