@@ -1499,8 +1499,9 @@ struct Solver {
         const int nsl = div_up(d.n, 32), spc = div_up(nsl, cg_sms);
         return spc >= 1 && spc <= kCgMaxSlices && cg_smem(spc) <= kCgSmem ? spc : 0;
     }
-    // A d = r / rn of one refinement pass to tol: d in d32; the iterations, -1 on failure
-    int cg_small(int spc, double rn, double tol) {
+    // A d = r / rn of one refinement pass to tol: d in d32.  Nothing is read back: the count of
+    // iterations (S_ITER, -1 on failure) comes with the next residual's norms.
+    bool cg_small(int spc, double rn, double tol) {
         cgs.spc = spc;
         cgs.K = cg_row_room();
         cgs.levels = mg_ready ? mg.levels : 0;
@@ -1511,11 +1512,8 @@ struct Solver {
         void* args[] = {(void*)&d, (void*)&mg, (void*)&cgs};
         if (MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_cg_small, dim3(div_up(div_up(d.n, 32), spc)),
                                                          dim3(kCgThreads), args, cg_smem(spc), st))
-            return -1;
-        if (pull_scal()) return -1;
-        const int it = (int)h_scal[S_ITER];
-        spmv_launches += std::max(it, 0);
-        return it;
+            return false;
+        return true;
     }
 
     // FP32 Jacobi-PCG inside FP64 iterative refinement
@@ -1529,7 +1527,7 @@ struct Solver {
         S.mg_level1 = mg_ready ? mg.L[1].n : 0;
         timer.mark(PH_VEC, st);
         double bnorm = 0.0;
-        int outer = 0;
+        int outer = 0, small_pass = -1;
         for (;;) {
             // the residual is already there for the first pass when the step computed it
             // before the solve (or from the learned guess), and for the later passes when
@@ -1537,6 +1535,14 @@ struct Solver {
             const bool have = residual_ready;
             if (!have) residual_df(w, true, residual_by_update());
             if (stream_failed || pull_scal()) return CCT_CUDAERR;
+            if (small_pass >= 0) {   // the last pass's inner solve
+                const int it = (int)h_scal[S_ITER];
+                if (it < 0) return CCT_CUDAERR;
+                pass_its[small_pass] = it;
+                S.cg_iterations += it;
+                spmv_launches += it;
+                small_pass = -1;
+            }
             if (outer == 0) {
                 h_nnz[0] = h_scal[S_NNZ0];
                 h_nnz[1] = h_scal[S_NNZ1];
@@ -1557,9 +1563,9 @@ struct Solver {
             const double inner_tol = std::max(need, ir_inner_rtol());
             const int pi = outer < kPassMemory ? outer : kPassMemory - 1;
             const int small = cg_small_slices();
-            int it;
             if (small > 0) {
-                it = cg_small(small, rn, inner_tol);
+                if (!cg_small(small, rn, inner_tol)) return CCT_CUDAERR;
+                small_pass = pi;
             } else {
                 MPS_COUNT_LAUNCH k_cg_start<float><<<red_blocks(d.n), 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,
                                                               inner_tol, opt.cg_max_iter);
@@ -1568,12 +1574,12 @@ struct Solver {
                     mg_apply(d.r32, d.z32, d.p32, 1);
                     timer.mark(PH_VEC, st);
                 }
-                it = cg_loop<float, float, float>(d.d32, d.r32, d.z32, d.p32, d.q32, w, nullptr, d.m32,
+                const int it = cg_loop<float, float, float>(d.d32, d.r32, d.z32, d.p32, d.q32, w, nullptr, d.m32,
                                                             opt.cg_max_iter, pass_its[pi]);
+                if (it < 0) return CCT_CUDAERR;
+                pass_its[pi] = it;
+                S.cg_iterations += it;
             }
-            if (it < 0) return CCT_CUDAERR;
-            pass_its[pi] = it;
-            S.cg_iterations += it;
             if (residual_by_update()) {
                 // x += rn d and the next pass's residual r -= rn A d, one pass over the rows
                 residual_update(w, rn);
