@@ -64,9 +64,9 @@ STEP_FIXED_B, STEP_ITER_B, STEP_IR_B = 760.0, 72.0, 48.0
 SPMV_DRAM_BYTES_PER_ENTRY = (1.33758e9 + 2.24e6) / 201.362e6
 # warp instructions per particle of the two FP32 neighbour passes, counted by ncu
 # (smsp__inst_executed.sum, one launch on the bucket at l0 = 0.004, 108,186 particles):
-# the list pass 233.67M, the predictor 213.7M
-NB_LIST_INST_PER_PARTICLE = 233.67e6 / 108186
-NB_PRED_INST_PER_PARTICLE = 213.7e6 / 108186
+# the list pass (k_list) 106.83M, the predictor (k_predict) 77.81M
+NB_LIST_INST_PER_PARTICLE = 106.83e6 / 108186
+NB_PRED_INST_PER_PARTICLE = 77.81e6 / 108186
 # the same for the FP16-weight kernel of the inner CG (k_spmv_stream<..., __half>):
 # 898.3 MB read + 1.8 MB written for 201.36M entries
 SPMV16_DRAM_BYTES_PER_ENTRY = (898.3e6 + 1.8e6) / 201.362e6
