@@ -48,3 +48,26 @@ def test_iteration_limit(limit):
     (a, pa, _), (b, pb, _) = _both(_block((13, 12, 11)), True, cg_max_iter=limit, ir_max_outer=2)
     assert a["error_flags"] == b["error_flags"] and a["cg_iterations"] == b["cg_iterations"] == 2 * limit
     assert np.abs(pa - pb).max() <= 1e-5 * np.abs(pb).max()
+
+
+def test_solvers_in_threads():
+    """Cooperative launches of several solvers at once: each finds its CTAs together or waits."""
+    import threading
+    shapes = [(24, 24, 23), (17, 17, 16), (24, 23, 22), (13, 12, 11)]
+    out = [[None] * len(shapes) for _ in range(2)]
+
+    def work(k, into):
+        s = Solver(_block(shapes[k], seed=k), precision="fp32_ir")
+        st = [s.step(i) for i in range(15)]
+        into[k] = ([(q["error_flags"], q["cg_iterations"]) for q in st], s.state()["press"])
+        s.close()
+    for k in range(len(shapes)):
+        work(k, out[0])
+    threads = [threading.Thread(target=work, args=(k, out[1])) for k in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(*out):
+        assert all(f == 0 for f, _ in a[0]) and a[0] == b[0]
+        assert np.array_equal(a[1], b[1])
