@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(S == 1 ? kNpWarps * 32 : S * 32, S == 1 ? 6 : 
 // shared memory of a k_list CTA: the lists of accepted candidates [K + 16][32], the gradient
 // lists (the rings of candidates lie there before the first of them is written), the first
 // particle of each run of each piece, what the second warp hands to the first
-constexpr int kNbPieces = 8, kNbHand = 9;
+constexpr int kNbPieces = 32, kNbHand = 9;   // a slice has at most as many pieces as targets
 static_assert(2 * sizeof(NbRing<true>) <= 32 * kGradStride * 2, "the rings lie in the gradient lists");
 inline size_t nb_list_smem(int L) {
     return (size_t)(L + 16) * 64 + 32 * kGradStride * 2 + kNbPieces * 9 * 4 + kNbHand * 32 * 4;
@@ -316,9 +316,9 @@ inline size_t nb_list_smem(int L) {
 // bytes of shared memory per entry.  L: entries that a list has room for (25 KB per slice with
 // 296, 31 KB with 384; sixteen or fourteen warps per SM).  112 registers, 8 candidates and 4
 // entries at a time: 16 and 8 of them spilled (1620 us instead of 1360 at 882,080 particles).
-// Bit 4 of flags, a row longer than L, a run too long for the codes or more than kNbPieces
-// pieces: the candidates are walked twice by one warp, once for the rows' lengths and ends and
-// once for the entries, with no list; same rows and sums, bit for bit.
+// Bit 4 of flags, a row longer than L or a run too long for the codes: the candidates are walked
+// twice by one warp, once for the rows' lengths and ends and once for the entries, with no
+// list; same rows and sums, bit for bit.
 __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags, int L) {
     extern __shared__ __align__(16) unsigned char nb_sm[];
     unsigned short* const list = (unsigned short*)nb_sm;
@@ -348,7 +348,7 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
     for (unsigned todo = direct ? 0u : all; todo; ++piece) {
         const NbPiece s = nb_piece(d, todo, h, p);
         todo &= ~s.mem;
-        if (piece == kNbPieces || __any_sync(~0u, s.rl > kNbOff)) {
+        if (__any_sync(~0u, s.rl > kNbOff)) {
             direct = true;   // in both warps
             break;
         }

@@ -102,7 +102,7 @@ struct Solver {
     int models = 0;
     int walls_move = 0;
     cudaStream_t st = nullptr;
-    // second stream: the multilevel setup runs there beside the rows' transpose, the first
+    // second stream: the multilevel setup runs there beside the list pass, the first
     // refinement residual and the learned guess
     cudaStream_t st2 = nullptr;
     cudaEvent_t ev_setup = nullptr, ev_rows = nullptr, ev_mg = nullptr, ev_walls = nullptr, ev_bins = nullptr;
@@ -260,7 +260,7 @@ struct Solver {
             if (cudaEventCreate(&e) != cudaSuccess) return CCT_CUDAERR;
         // the second stream at a higher priority: the work it takes (wall bins, multilevel
         // setup) is on the step's critical path, and the solver-stream kernels beside it
-        // (compaction, grid, transpose, first residual) fill the SMs it leaves
+        // (compaction, grid, list, first residual) fill the SMs it leaves
         int prio_low = 0, prio_high = 0;
         cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
         if (cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
@@ -839,10 +839,12 @@ struct Solver {
             return;
         }
         const int slices = (d.n + 31) / 32, flags = row_flags();
-        // room for an eighth more entries than the last step's longest row had: less shared memory
-        // per slice, eight CTAs on an SM instead of seven (1359 us instead of 1445 at 882,080
+        // room for an eighth more entries than the last step's longest row had, and for 256 at
+        // least (fluid that comes together again fills its rows within a step): less shared memory per slice
+        // than for K, eight CTAs on an SM instead of seven (1359 us instead of 1445 at 882,080
         // particles); a slice with a longer row takes the direct walk, with the same rows
-        const int room = last.max_row > 0 ? (last.max_row + last.max_row / 8 + 15) / 8 * 8 : d.K;
+        // (250 us for one such slice in 9,248 particles)
+        const int room = last.max_row > 0 ? std::max(256, (last.max_row + last.max_row / 8 + 15) / 8 * 8) : d.K;
         const int L = std::min(room, d.K);
         if (slices > 0)
             MPS_COUNT_LAUNCH k_list<<<slices, 64, nb_list_smem(L), st>>>(d, flags | (opt.rows_sell == 1 ? 16 : 0), L);
