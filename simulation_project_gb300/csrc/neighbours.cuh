@@ -629,7 +629,25 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
         hand[(6 + warp) * 32 + lane] = gcnt;
         __syncthreads();
         // gradient rows, four targets at a time (a row is contiguous)
-        const int g0 = hand[6 * 32 + lane], g1 = hand[7 * 32 + lane], glow = min(g0, d.KG), gc = min(g0 + g1, d.KG);
+        const int g0 = hand[6 * 32 + lane], g1 = hand[7 * 32 + lane], gc = min(g0 + g1, d.KG);
+        int glow = min(g0, d.KG);
+        if (__any_sync(~0u, g0 + g1 > d.KG)) {   // in both warps
+            // the halves of a full list have met and overwritten each other: the first KG
+            // entries of every row again, from the whole list in its order
+            if (warp == 0) {
+                int g = 0;
+                for (int k = 0; k < cap && g < d.KG; ++k) {
+                    const unsigned cg = code_of(k);
+                    const float4 qg = __ldg(d.opos + decode(cg));
+                    float ri, rr;
+                    lap_weight_f32(dist2_f32(__fsub_rn(qg.x, p.x), __fsub_rn(qg.y, p.y), __fsub_rn(qg.z, p.z)), re, mind,
+                                   wmax, ri, rr);
+                    if (rr < reg) glist[lane * kGradStride + g++] = (unsigned short)cg;
+                }
+            }
+            __syncthreads();
+            glow = gc;
+        }
         for (int t0 = 16 * warp; t0 < 16 * warp + 16; t0 += 4) {
             int tj[8];
             float4 tq[8];
