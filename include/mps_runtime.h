@@ -44,6 +44,9 @@ const char* mps_last_error(void);
 void mps_clear_error(void);
 /* bytes of library-owned scratch currently held by the reference-named entry points */
 size_t mps_scratch_bytes(void);
+/* Test hook: polls after which a grid barrier of the cooperative kernels (sorts, inner CG of
+ * small systems, coarse V-cycle) gives up; negative: the default.  Waits for the device. */
+CCTStatusType mps_debug_barrier_polls(int polls);
 /* build identification: "sm_103a" and the library version */
 const char* mps_build_info(void);
 /* kernels this library has launched since it was loaded (all threads, all devices) */

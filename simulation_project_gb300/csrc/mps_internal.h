@@ -29,6 +29,9 @@ int radix_bits(unsigned range);
 // hold the pairs in no particular order.
 cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, cudaStream_t st,
                              int max_ctas = kRadixMaxCtas);
+// polls of a grid barrier's wait, in the kernels of sort.cu and of solver.cu
+cudaError_t sort_barrier_polls(int polls);
+cudaError_t solver_barrier_polls(int polls);
 // in-place exclusive scan of len unsigned values, total to *total_dev (if not NULL);
 // tile_sums (scan_tile_sums_capacity() values, or NULL: single-CTA scan) lets it
 // run on many CTAs

@@ -5,6 +5,7 @@
 
 #include <mutex>
 
+#include "mps_common.cuh"
 #include "mps_internal.h"
 #include "../../include/mps_runtime.h"
 
@@ -142,6 +143,13 @@ size_t mps_scratch_bytes(void) {
     size_t s = 0;
     for (auto& x : mps::g_slots) s += x.bytes;
     return s;
+}
+CCTStatusType mps_debug_barrier_polls(int polls) {
+    const int v = polls < 0 ? mps::kCoopPolls : polls;
+    cudaError_t e = cudaDeviceSynchronize();
+    if (!e) e = mps::sort_barrier_polls(v);
+    if (!e) e = mps::solver_barrier_polls(v);
+    return rec(e);
 }
 const char* mps_build_info(void) { return "gb300-mps 0.1 sm_103a"; }
 

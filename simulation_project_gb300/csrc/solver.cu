@@ -31,6 +31,8 @@
 #include "../../include/mps_learned.h"
 
 namespace mps {
+
+cudaError_t solver_barrier_polls(int polls) { return cudaMemcpyToSymbol(c_coop_polls, &polls, sizeof(polls)); }
 cudaError_t mlp_forward(MpsMlp* m, int M, const float* X, float* Y, cudaStream_t st, unsigned* err);
 
 namespace {
@@ -102,6 +104,11 @@ struct Solver {
     int models = 0;
     int walls_move = 0;
     cudaStream_t st = nullptr;
+    // the error word's allocation: the error bits, then the grid barriers' words of k_cg_small
+    // and k_mg_coarse_cycle.  One memset at the start of a step clears all: after a wait that
+    // ran out a barrier's word is a part of a count
+    static constexpr int kErrWords = 3;
+    unsigned* coop_bar = nullptr;
     // second stream: the multilevel setup runs there beside the list pass, the first
     // refinement residual and the learned guess
     cudaStream_t st2 = nullptr;
@@ -309,13 +316,13 @@ struct Solver {
             e = e ? e : mk(&cgs.zp, rows);
             e = e ? e : mk(&cgs.part, 4 * 1024);
             e = e ? e : mk(&cgs.coarse, kCgAgg + 1024);
-            e = e ? e : mk(&cgs.bar, 1);
-            if (!e) e = cudaMemset(cgs.bar, 0, sizeof(unsigned));
         }
         e = e ? e : mk(&d.red, 4 * (size_t)kRedBlocks);
         e = e ? e : mk(&d.scal, (size_t)S_COUNT);
         e = e ? e : mk(&d.red_count, 16);
-        e = e ? e : mk(&d.err, 1);
+        e = e ? e : mk(&d.err, kErrWords);
+        cgs.bar = d.err + 1;
+        coop_bar = d.err + 2;
         e = e ? e : mk(&d.istat, 4);
         e = e ? e : mk(&stage, 7 * N);
         e = e ? e : mk(&d.pprev, N);
@@ -339,7 +346,7 @@ struct Solver {
         }
         cudaMemset(d.red_count, 0, sizeof(unsigned) * 16);
         cudaMemset(d.scal, 0, sizeof(double) * S_COUNT);
-        cudaMemset(d.err, 0, sizeof(unsigned));
+        cudaMemset(d.err, 0, sizeof(unsigned) * kErrWords);
         return cudaDeviceSynchronize() == cudaSuccess ? CCT_NOERR : CCT_CUDAERR;
     }
 
@@ -502,8 +509,8 @@ struct Solver {
         mg_grid_levels = std::min(l, kMgMaxLevels);
         e = e ? e : mk(&mg.ainv, (size_t)kMgMaxDense * kMgMaxDense);
         // [0]: k_mg_down's finished CTAs; [1], [2]: k_mg_coarse_cycle's grid barrier
-        e = e ? e : mk(&mg.done, 3);
-        if (!e) e = cudaMemset(mg.done, 0, 3 * sizeof(unsigned));
+        e = e ? e : mk(&mg.done, 1);
+        if (!e) e = cudaMemset(mg.done, 0, sizeof(unsigned));
         e = e ? e : mk(&mg.agg1, (size_t)nmax); e = e ? e : mk(&mg.pcc, (size_t)nmax);
         e = e ? e : mk(&mg.part, 27 * (size_t)nmax); e = e ? e : mk(&mg.partd, (size_t)nmax);
         e = e ? e : mk(&mg.rb, (size_t)d.cells + 1);
@@ -621,7 +628,6 @@ struct Solver {
     // CTAs of the cooperative coarse V-cycle: all resident (SMs x the CTAs that fit),
     // no more than the level-2 aggregates need (a warp each); 0: not available
     int coop_resident = -1;
-    unsigned* coop_bar = nullptr;
     int coarse_cycle_grid() {
         if (coop_resident < 0) {
             int dev = 0, sms = 0, per_sm = 0, coop = 0;
@@ -631,7 +637,6 @@ struct Solver {
             if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_coarse_cycle, 256, 0) != cudaSuccess)
                 per_sm = 0;
             coop_resident = sms * per_sm;
-            coop_bar = mg.done + 1;
         }
         if (coop_resident <= 0) return 0;
         return std::max(1, std::min(coop_resident, div_up(mg.L[2].n, 8)));
@@ -897,7 +902,7 @@ struct Solver {
         d.rows_w16 = 0;
         d.rows_c32 = 0;
         timer.mark(PH_GRID, st);
-        cudaMemsetAsync(d.err, 0, sizeof(unsigned), st);
+        cudaMemsetAsync(d.err, 0, sizeof(unsigned) * kErrWords, st);
         cudaMemsetAsync(d.istat, 0, 2 * sizeof(int), st);
         CCTStatusType rc;
         if (!pressure_only) {

@@ -379,6 +379,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
     }
 }
 
+cudaError_t sort_barrier_polls(int polls) { return cudaMemcpyToSymbol(c_coop_polls, &polls, sizeof(polls)); }
+
 int radix_bits(unsigned range) {
     int bits = 0;
     while (bits < 32 && (range >> bits) != 0u) ++bits;

@@ -41,6 +41,7 @@ _SIGS = {
     "mps_clear_error": (None, []),
     "mps_scratch_bytes": (C.c_size_t, []),
     "mps_build_info": (C.c_char_p, []),
+    "mps_debug_barrier_polls": (I, [I]),
     "mps_kernel_launches": (C.c_ulonglong, []),
     # reference-named launcher API (include/mps_device_process.h)
     "CalcTurbulenceViscosity": (I, [C.POINTER(P), I]),
