@@ -34,14 +34,14 @@ __host__ __device__ inline int div_up(long long a, int b) { return (int)((a + b 
 // The arrivals of one barrier add 2^31 to *bar in all (CTA 0 adds what the others leave),
 // so its top bit flips when the last one arrives and the word needs no reset between
 // barriers or launches: it starts at 0 and is used by one launch at a time.  A wait that runs
-// out (c_coop_polls polls) sets MPS_ERR_STAGE_TIMEOUT and returns false (the CTA then stops,
+// out (c_coop_polls polls) sets `bit` in *err and returns false (the CTA then stops,
 // so the others run out too, or pass a barrier that it had arrived at); the word then keeps a
 // part of a count and has to be cleared before the next launch.  Release on arrival,
 // acquire while polling: 1.15 us on 16 to 304 CTAs; a counter with a separate generation
 // word, full fences and a relaxed poll took 2.3 to 2.7.
 constexpr int kCoopPolls = 1 << 20;
 static __constant__ int c_coop_polls = kCoopPolls;   // each translation unit's (mps_debug_barrier_polls)
-__device__ __forceinline__ bool coop_barrier(unsigned* bar, unsigned* err) {
+__device__ __forceinline__ bool coop_barrier(unsigned* bar, unsigned* err, unsigned bit = 32u) {   // MPS_ERR_STAGE_TIMEOUT
     __shared__ int ok;
     __syncthreads();
     if (gridDim.x == 1) return true;
@@ -53,7 +53,7 @@ __device__ __forceinline__ bool coop_barrier(unsigned* bar, unsigned* err) {
         for (int k = 0; ((now ^ old) & 0x80000000u) == 0u && k < c_coop_polls; ++k)
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
         ok = ((now ^ old) & 0x80000000u) != 0u;
-        if (!ok && err) atomicOr(err, 32u);   // MPS_ERR_STAGE_TIMEOUT
+        if (!ok && err) atomicOr(err, bit);
     }
     __syncthreads();
     return ok != 0;

@@ -24,11 +24,15 @@ constexpr size_t radix_scratch_bytes_for(long long n, int max_ctas = kRadixMaxCt
 inline size_t radix_scratch_bytes(int n) { return radix_scratch_bytes_for(n); }
 // bits of the keys 0 .. range
 int radix_bits(unsigned range);
+// Bits of a solver's error word that its host side keeps to itself (not MPS_ERR_*): a grid
+// barrier of the sort of its particles, of its wall bins ran out.
+constexpr unsigned kErrSortParticles = 1u << 30, kErrSortBins = 1u << 29;
 // stable sort of (keys, vals) by key; bits: the keys lie in [0, 2^bits), < 0: any int range.
-// err (may be NULL) gets MPS_ERR_STAGE_TIMEOUT if a grid barrier runs out; the arrays then
-// hold the pairs in no particular order.
-cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, cudaStream_t st,
-                             int max_ctas = kRadixMaxCtas);
+// *err gets `bit` if a grid barrier runs out.  The arrays' contents are then undefined (pairs
+// lost, repeated or never written): nothing may use them as indexes before it has seen that
+// *err is clear.
+cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, unsigned bit,
+                             cudaStream_t st, int max_ctas = kRadixMaxCtas);
 // polls of a grid barrier's wait, in the kernels of sort.cu and of solver.cu
 cudaError_t sort_barrier_polls(int polls);
 cudaError_t solver_barrier_polls(int polls);

@@ -260,7 +260,10 @@ __global__ void k_hash(const __grid_constant__ Dev d) {
 __global__ void k_gather(const __grid_constant__ Dev d) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
-    const int s = d.idx[i];
+    // after a sort that gave up neither the indexes nor the keys mean anything: the particles
+    // keep their places, without cells and neighbours, and the tables stay empty (the step fails)
+    const bool sorted = (*d.err & kErrSortParticles) == 0u;
+    const int s = sorted ? d.idx[i] : i;
     const dbl4 p = d.pos[s], v = d.vel[s];
     d.pos2[i] = p;
     d.vel2[i] = v;
@@ -270,13 +273,18 @@ __global__ void k_gather(const __grid_constant__ Dev d) {
     d.id2[i] = d.id[s];
     d.dph1b[i] = d.dph1[s];
     d.dph2b[i] = d.dph2[s];
-    const int sk = d.skey[i];
+    const int sk = sorted ? d.skey[i] : 0;
     const int h = sk >> d.zbits;
     // global z bin (cell z * 64 + bin inside the cell), exact in a float
     const float zbin = (float)((h % d.box.m_GridSize.z) * 64 + ((sk & ((1 << d.zbits) - 1)) << (6 - d.zbits)));
     d.opos[i] = make_float4((float)p.x, (float)p.y, (float)p.z, zbin);
     d.ovel[i] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
     d.key[i] = h;
+    if (!sorted) {
+        d.nbr_cnt[i] = d.gcnt[i] = 0;
+        d.pnd[i] = d.sumw[i] = 0.0;
+        return;
+    }
     const int hp = i > 0 ? (d.skey[i - 1] >> d.zbits) : -1;
     if (i == 0 || h != hp) {
         d.cstart[h] = i;
@@ -346,9 +354,9 @@ __global__ void k_bin_fill(const __grid_constant__ Dev d, const unsigned* off, i
         vtri[o + q] = t;
     }
 }
-__global__ void k_bin_bounds(int nv, const int* vcell, int* ts, int* te) {
+__global__ void k_bin_bounds(int nv, const int* vcell, int* ts, int* te, const unsigned* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
+    if (i >= nv || (*err & kErrSortBins) != 0u) return;   // a sort that gave up: no lists (the step fails)
     const int c = vcell[i];
     if (i == 0 || c != vcell[i - 1]) {
         ts[c] = i;

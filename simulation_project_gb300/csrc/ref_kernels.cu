@@ -1136,7 +1136,7 @@ CCTStatusType SortUsingThrust(Integer MaxParticleNum, Integer* daNumberHash, Int
     void* scr = scratch_get(1, radix_scratch_bytes(n));
     if (!scr) return CCT_MEMERR;
     unsigned* const err = sort_error();
-    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, st));
+    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, 1u, st));
     // thrust::sort_by_key with the default policy returns after the sort completed;
     // callers rely on that (they launch the reorder on their own stream next).
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1206,7 +1206,7 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
         MPS_COUNT_LAUNCH k_tri_fill<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
     else
         MPS_COUNT_LAUNCH k_tri_fill<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
-    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, radix_bits((unsigned)CellNum), sscr, sort_error(), Stream));
+    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, radix_bits((unsigned)CellNum), sscr, sort_error(), 1u, Stream));
     MPS_CUDA_TRY(cudaMemsetAsync(vrange, 0xff, sizeof(int) * (size_t)CellNum * 2, Stream));
     MPS_COUNT_LAUNCH k_tri_bounds<<<grid_of((int)nv), kBlock, 0, Stream>>>((int)nv, vcell, vrange, vrange + CellNum);
     MPS_COUNT_LAUNCH k_tri_cells<<<div_up(32ll * CellNum, kBlock), kBlock, 0, Stream>>>(CellNum, vrange, vrange + CellNum, vtri, daCell);

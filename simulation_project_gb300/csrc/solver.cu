@@ -738,7 +738,7 @@ struct Solver {
         }
         MPS_COUNT_LAUNCH k_hash<<<blocks_for(n), kBlock, 0, st>>>(d);
         const unsigned krange = ((unsigned)d.cells << d.zbits) - 1u;
-        if (radix_sort_pairs(n, d.skey, d.idx, radix_bits(krange), sort_scratch, d.err, st)) return CCT_CUDAERR;
+        if (radix_sort_pairs(n, d.skey, d.idx, radix_bits(krange), sort_scratch, d.err, kErrSortParticles, st)) return CCT_CUDAERR;
         cudaMemsetAsync(d.cstart, 0xff, sizeof(int) * d.cells, st);
         cudaMemsetAsync(d.cend, 0xff, sizeof(int) * d.cells, st);
         cudaMemsetAsync(d.cell_count, 0, sizeof(int), st);
@@ -747,11 +747,22 @@ struct Solver {
         return cuda_status(cudaGetLastError());
     }
 
+    // whether a sort gave up, by the error word in h_int[0]
+    bool sort_failed() {
+        const unsigned f = (unsigned)h_int[0];
+        bins_checked = (f & kErrSortBins) == 0u;
+        if ((f & (kErrSortParticles | kErrSortBins)) == 0u) return false;
+        note_message("a grid barrier of the sort of the particles or of the wall bins ran out");
+        return true;
+    }
+
+    bool bins_checked = true;   // the sort of the wall bins is known to have ended well
     // on stream ss with its own host buffer and scan scratch (the second stream, beside
     // the particles' compaction, in a step)
     CCTStatusType bin_walls(cudaStream_t ss, int* hb, unsigned* scr) {
         const int t = d.tri_n;
         if (t <= 0) return CCT_NOERR;
+        bins_checked = false;
         // counts (t + 1 with the scan's total) and the 64-bit sum of the counts behind them
         if ((size_t)t > bin_off_cap) {   // sized for the largest wall set seen
             if (bin_off) cudaFree(bin_off);
@@ -796,11 +807,12 @@ struct Solver {
         int* vcell = bin_visit;
         d.tids = bin_visit + bin_visit_cap;
         MPS_COUNT_LAUNCH k_bin_fill<<<div_up(t * 32, 256), 256, 0, ss>>>(d, bin_off, vcell, d.tids);
-        if (radix_sort_pairs((int)nv, vcell, d.tids, radix_bits((unsigned)(2 * d.cells - 1)), bin_sort, d.err, ss))
+        if (radix_sort_pairs((int)nv, vcell, d.tids, radix_bits((unsigned)(2 * d.cells - 1)), bin_sort, d.err,
+                             kErrSortBins, ss))
             return CCT_CUDAERR;
         cudaMemsetAsync(d.tcs, 0xff, sizeof(int) * 4 * d.cells, ss);
         MPS_COUNT_LAUNCH k_bin_bounds<<<blocks_for((int)nv), kBlock, 0, ss>>>((int)nv, vcell, d.tcs,
-                                                                               d.tcs + 2 * d.cells);
+                                                                               d.tcs + 2 * d.cells, d.err);
         bins_dirty = 0;
         return cuda_status(cudaGetLastError());
     }
@@ -905,6 +917,7 @@ struct Solver {
         cudaMemsetAsync(d.err, 0, sizeof(unsigned) * kErrWords, st);
         cudaMemsetAsync(d.istat, 0, 2 * sizeof(int), st);
         CCTStatusType rc;
+        if (!bins_checked) bins_dirty = 1;   // the step that made them did not end well
         if (!pressure_only) {
             // the wall bins (the triangles moved at the end of the last step) on the second
             // stream, their host waits and kernels beside the compaction and the grid
@@ -1064,6 +1077,7 @@ struct Solver {
             gate_update(S, gate_pending == 2);
             gate_pending = 0;
         }
+        if (sort_failed()) return CCT_CUDAERR;
         S.error_flags |= (unsigned)h_int[0];
         S.max_row = h_int[1];
         S.nnz_wide = h_int[2];
@@ -1957,9 +1971,12 @@ CCTStatusType mps_solver_debug_wall_bins(MpsSolver* s, int* bounds, int* tids, i
     mps::Dev& d = S.d;
     *entries = 0;
     if (d.tri_n <= 0) return CCT_NOERR;
-    if (S.bins_dirty) {
+    if (S.bins_dirty || !S.bins_checked) {
+        cudaMemsetAsync(d.err, 0, sizeof(unsigned) * mps::Solver::kErrWords, S.st);
         const CCTStatusType rc = S.bin_walls(S.st, S.h_int, S.scan_sums);
         if (rc != CCT_NOERR) return rc;
+        cudaMemcpyAsync(S.h_int, d.err, sizeof(unsigned), cudaMemcpyDeviceToHost, S.st);
+        if (cudaStreamSynchronize(S.st) || S.sort_failed()) return CCT_CUDAERR;
     }
     if (cudaStreamSynchronize(S.st)) return CCT_CUDAERR;
     const int nv = S.bin_entries;

@@ -175,7 +175,7 @@ struct SortScratch {
 
 // bits: the keys lie in [0, 2^bits); < 0: any int range (found first)
 __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* keys, int* vals, int bits, SortScratch s,
-                                                       unsigned* err) {
+                                                       unsigned* err, unsigned bit) {
     __shared__ unsigned wcount[kSortWarps][kRadix];
     __shared__ unsigned off[kRadix];
     __shared__ unsigned wsum[32];
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                 s.range[ctas + c] = h2;
             }
         }
-        if (!coop_barrier(s.bar, err)) return;
+        if (!coop_barrier(s.bar, err, bit)) return;
         lo = INT_MAX;
         hi = INT_MIN;
         for (int i = lane; i < ctas; i += 32) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
         const unsigned mine = off[tid];
         if (ctas > 1) {
             s.counts[(size_t)c * kRadix + tid] = mine;
-            if (!coop_barrier(s.bar, err)) return;
+            if (!coop_barrier(s.bar, err, bit)) return;
             // ---- prefix over the CTAs, a warp per digit, a run of CTAs per lane ----
             constexpr int kRun = (kRadixMaxCtas + 31) / 32;
             for (int d = w * ctas + c; d < kRadix; d += ctas * kSortWarps) {   // spread over the SMs
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                 }
                 if (lane == 31) s.total[d] = inc;
             }
-            if (!coop_barrier(s.bar, err)) return;
+            if (!coop_barrier(s.bar, err, bit)) return;
         }
         // ---- first position of each digit's keys of this CTA ----
         {
@@ -360,14 +360,16 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                     const unsigned d = at[r] & 1023u;
                     if (d < (unsigned)kRadix) {
                         const unsigned dst = wcount[w][d] + (at[r] >> 10);
-                        kb[dst] = key[r];
-                        vb[dst] = val[r];
+                        if (dst < (unsigned)n) {   // not where another CTA gave up at a barrier
+                            kb[dst] = key[r];
+                            vb[dst] = val[r];
+                        }
                     }
                 }
             }
             __syncthreads();
         }
-        if (!coop_barrier(s.bar, err)) return;
+        if (!coop_barrier(s.bar, err, bit)) return;
         int* t = ka; ka = kb; kb = t;
         t = va; va = vb; vb = t;
     }
@@ -387,8 +389,8 @@ int radix_bits(unsigned range) {
     return bits;
 }
 
-cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, cudaStream_t st,
-                             int max_ctas) {
+cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratch, unsigned* err, unsigned bit,
+                             cudaStream_t st, int max_ctas) {
     if (n <= 1 || bits == 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -409,7 +411,7 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
         const cudaError_t e = cudaMemsetAsync(s.bar, 0, sizeof(unsigned), st);
         if (e) return e;
     }
-    void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err};
+    void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err, (void*)&bit};
     return MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_sort, dim3(ctas), dim3(kSortThreads), args, 0, st);
 }
 

@@ -77,7 +77,7 @@ extern "C" CCTStatusType SortUsingThrustNoAlloc(Integer MaxParticleNum, Integer*
     cudaStream_t st = 0;
     unsigned failed = 0;
     MPS_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
-    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, st, kNoAllocCtas));
+    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, 1u, st, kNoAllocCtas));
     MPS_CUDA_TRY(cudaMemcpyAsync(&failed, err, sizeof(failed), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
     if (failed) return CCT_CUDAERR;

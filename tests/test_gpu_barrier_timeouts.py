@@ -6,10 +6,10 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from simulation_project_gb300 import scenes
-from simulation_project_gb300.lib import call
+from simulation_project_gb300 import lib, scenes
+from simulation_project_gb300.lib import DeviceArray, call
 from simulation_project_gb300.solver import Solver, _lib
-from simulation_project_gb300.types import MpsError
+from simulation_project_gb300.types import CTriangleParameters, MpsError
 
 pytestmark = pytest.mark.gpu
 STAGE_TIMEOUT = 32
@@ -39,12 +39,23 @@ def _reset(s):
                                                  (s.scene.press, np.float64), (s.scene.visc, np.float64),
                                                  (s.scene.ptype, np.int32))]
     assert _lib().mps_solver_set_particles(s.h, s.scene.n, *[x.ctypes.data for x in a]) == 0
+    if s.scene.t:
+        v = np.ascontiguousarray(s.scene.tri_vertices.reshape(-1, 9))
+        tp = (CTriangleParameters * len(s.scene.tri_params))(*s.scene.tri_params)
+        assert _lib().mps_solver_set_triangles(s.h, s.scene.t, v.ctypes.data, s.scene.tri_model.ctypes.data,
+                                               len(s.scene.tri_params), C.addressof(tp)) == 0
 
 
 def _three_steps(s):
     st = [s.step(i) for i in range(3)]
     assert all(q["error_flags"] == 0 for q in st)
     return [q["cg_iterations"] for q in st], s.state()
+
+
+def _same(a, b):
+    assert a[0] == b[0]
+    for k in ("pos", "vel", "press"):
+        assert np.array_equal(a[1][k], b[1][k]), k
 
 
 # up to 4,096 particles, whose sort has no barrier: the small system's CG (1,716 rows, 54 CTAs)
@@ -66,8 +77,58 @@ def test_solve_after_a_barrier_ran_out(shape, profile):
             else:
                 assert profile
         _reset(s)
-    its, state = _three_steps(s)
+    got = _three_steps(s)
     s.close()
-    assert its == want[0]
-    for k in ("pos", "vel", "press"):
-        assert np.array_equal(state[k], want[1][k]), k
+    _same(got, want)
+
+
+@pytest.mark.parametrize("precision", ["fp32_ir", "fp64"])
+@pytest.mark.parametrize("scene", [lambda: _block((24, 24, 23)), lambda: scenes.dam_break(l0=0.01),
+                                   lambda: scenes.rotating_bucket(l0=0.008, n_drag=4)],
+                         ids=["no_walls", "resting_walls", "moving_walls"])
+def test_step_after_a_sort_gave_up(scene, precision):
+    """The sorts of the particles and of the wall bins (over 4,096 keys each): the step fails
+    with an error, and so does the next as long as the limit holds."""
+    sc = scene()
+    fresh = Solver(sc, precision=precision)
+    if sc.t:
+        assert sum(map(len, fresh.debug_wall_bins().values())) > 4096
+    want = _three_steps(fresh)
+    fresh.close()
+    s = Solver(sc, precision=precision)
+    for first in (True, False):   # as a solver's first step, and after good ones
+        with no_polls():
+            for _ in range(2):
+                with pytest.raises(MpsError):
+                    s.step(0)
+            with pytest.raises(MpsError):
+                s.pressure()
+        _reset(s)
+        if first:
+            _three_steps(s)
+    got = _three_steps(s)
+    s.close()
+    _same(got, want)
+
+
+def test_wall_bins_alone_after_a_sort_gave_up():
+    sc = scenes.dam_break(l0=0.01)
+    s, fresh = Solver(sc, precision="fp32_ir"), Solver(sc, precision="fp32_ir")
+    with no_polls(), pytest.raises(MpsError):
+        s.debug_wall_bins()
+    assert s.debug_wall_bins() == fresh.debug_wall_bins()
+
+
+def test_sorts_that_give_up():
+    """SortUsingThrust and its variant without allocation report it and work again afterwards."""
+    keys = np.random.default_rng(0).integers(-10 ** 6, 10 ** 6, 50_000).astype(np.int32)
+    order = np.argsort(keys, kind="stable")
+    lib.load().SortUsingThrustNoAlloc.argtypes = [C.c_int, C.c_void_p, C.c_void_p]
+    for name in ("SortUsingThrust", "SortUsingThrustNoAlloc"):
+        dk, dv = DeviceArray.from_host(keys), DeviceArray.from_host(np.arange(len(keys), dtype=np.int32))
+        with no_polls(), pytest.raises(MpsError):
+            call(name, len(keys), dk.ptr, dv.ptr)
+        dk.upload(keys)
+        dv.upload(np.arange(len(keys), dtype=np.int32))
+        call(name, len(keys), dk.ptr, dv.ptr)
+        assert np.array_equal(dk.download(), keys[order]) and np.array_equal(dv.download(), order)
