@@ -19,6 +19,8 @@
 #include <cfloat>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "mps_common.cuh"
 #include "mps_internal.h"
 #include "../../include/mps_device_process.h"
@@ -299,7 +301,8 @@ struct StoreVisit {
 template <int G>
 __global__ void __launch_bounds__(kBlock) k_tri_count(int t, const CTriangle* __restrict__ tri,
                                                       const __grid_constant__ CGridBox box, int cells,
-                                                      unsigned* __restrict__ count) {
+                                                      unsigned* __restrict__ count, unsigned* __restrict__ failed) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *failed = 0u;   // the sort's error word
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G, lane = threadIdx.x % G;
     if (i >= t) return;   // the G lanes of a triangle leave together
     const unsigned group = G == 32 ? ~0u : ((1u << (G % 32)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
@@ -325,10 +328,16 @@ __global__ void __launch_bounds__(kBlock) k_tri_fill(int t, const CTriangle* __r
     const CTriangle T = tri[i];
     ref_walk_triangle<G>(box, T, cells, v.group, lane, v);
 }
-// visits sorted (stably) by cell: unique triangle ids per cell, ascending, first 100
-__global__ void k_tri_bounds(int nv, const int* __restrict__ vcell, int* __restrict__ vs, int* __restrict__ ve) {
+// visits sorted (stably) by cell: unique triangle ids per cell, ascending, first 100.  After a
+// sort that gave up no cell gets a triangle and the host hears of it (*report).
+__global__ void k_tri_bounds(int nv, const int* __restrict__ vcell, int* __restrict__ vs, int* __restrict__ ve,
+                             const unsigned* __restrict__ failed, volatile unsigned* report) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nv) return;
+    if (*failed) {
+        if (i == 0) *report = 1u;
+        return;
+    }
     const int c = vcell[i];
     if (i == 0 || c != vcell[i - 1]) {
         vs[c] = i;
@@ -1111,19 +1120,29 @@ CCTStatusType reorderDataAndFindCellStart(cudaStream_t& Stream, Integer numParti
 // tile sums of the multi-CTA scan (NULL when the slot cannot be had: one-CTA scan)
 static unsigned* scan_sums() { return (unsigned*)scratch_get(8, sizeof(unsigned) * scan_tile_sums_capacity()); }
 
-// Error word of the sorts in host memory that the GPU can write: read without a copy once
-// the stream has been waited for.  NULL when it cannot be had (errors then go unseen).
-static unsigned* sort_error() {
-    static unsigned* const word = [] {
+// Error words in host memory that the GPU can write: read without a copy once the stream
+// has been waited for.  NULL when they cannot be had.
+enum { kErrSort = 0, kErrTriangles, kErrWords };
+static std::atomic<unsigned*> g_errors{nullptr};
+static volatile unsigned* host_error(int which) {
+    static unsigned* const words = [] {
         void* p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocMapped) != cudaSuccess) {
+        if (cudaHostAlloc(&p, sizeof(unsigned) * kErrWords, cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
             return (unsigned*)nullptr;
         }
-        *(unsigned*)p = 0u;
+        for (int k = 0; k < kErrWords; ++k) ((unsigned*)p)[k] = 0u;
+        g_errors.store((unsigned*)p);
         return (unsigned*)p;
     }();
-    return word;
+    return words ? words + which : nullptr;
+}
+// the triangle cells that an earlier RegisterTriangleTopology made are incomplete
+static bool triangles_failed() {
+    volatile unsigned* const e = g_errors.load(std::memory_order_relaxed);
+    if (!e || !e[kErrTriangles]) return false;
+    note_message("RegisterTriangleTopology: a grid barrier of its sort ran out, the triangle cells are incomplete");
+    return true;
 }
 
 // thrust::sort_by_key replacement: stable LSD radix sort on the legacy default
@@ -1135,14 +1154,15 @@ CCTStatusType SortUsingThrust(Integer MaxParticleNum, Integer* daNumberHash, Int
     cudaStream_t st = 0;
     void* scr = scratch_get(1, radix_scratch_bytes(n));
     if (!scr) return CCT_MEMERR;
-    unsigned* const err = sort_error();
-    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, err, 1u, st));
+    volatile unsigned* const err = host_error(kErrSort);
+    if (!err) return CCT_MEMERR;
+    MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, (unsigned*)err, 1u, st));
     // thrust::sort_by_key with the default policy returns after the sort completed;
     // callers rely on that (they launch the reorder on their own stream next).
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (err && *(volatile unsigned*)err) {   // this sort's, or that of an earlier triangle binning
-        *(volatile unsigned*)err = 0u;
-        note_message("SortUsingThrust: a grid barrier of a sort ran out");
+    if (*err) {
+        *err = 0u;
+        note_message("SortUsingThrust: a grid barrier of the sort ran out");
         return CCT_CUDAERR;
     }
     return launch_status();
@@ -1186,16 +1206,22 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
     const ScratchTurn turn(Stream);
     unsigned* off = (unsigned*)scratch_get(4, sizeof(unsigned) * ((size_t)t + 4));
     if (!off) return CCT_MEMERR;
-    unsigned* total_dev = off + t;
+    unsigned *const total_dev = off + t, *const failed = off + t + 1;
+    volatile unsigned* const report = host_error(kErrTriangles);
+    if (!report) return CCT_MEMERR;
     const bool few = t < kTriFew;
     if (few)
-        MPS_COUNT_LAUNCH k_tri_count<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off);
+        MPS_COUNT_LAUNCH k_tri_count<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, failed);
     else
-        MPS_COUNT_LAUNCH k_tri_count<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off);
+        MPS_COUNT_LAUNCH k_tri_count<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, failed);
     MPS_CUDA_TRY(scan_exclusive(off, t, total_dev, Stream, scan_sums()));
     unsigned nv = 0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&nv, total_dev, sizeof(unsigned), cudaMemcpyDeviceToHost, Stream));
     MPS_CUDA_TRY(cudaStreamSynchronize(Stream));
+    if (triangles_failed()) {   // in an earlier call: said once here, in the wall launchers until then
+        *report = 0u;
+        return CCT_CUDAERR;
+    }
     if (nv == 0) return launch_status();
     int* vcell = (int*)scratch_get(5, sizeof(int) * (size_t)nv * 2);
     int* vrange = (int*)scratch_get(6, sizeof(int) * (size_t)CellNum * 2);
@@ -1206,9 +1232,9 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
         MPS_COUNT_LAUNCH k_tri_fill<32><<<div_up(32ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
     else
         MPS_COUNT_LAUNCH k_tri_fill<8><<<div_up(8ll * t, kBlock), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, vcell, vtri);
-    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, radix_bits((unsigned)CellNum), sscr, sort_error(), 1u, Stream));
+    MPS_CUDA_TRY(radix_sort_pairs((int)nv, vcell, vtri, radix_bits((unsigned)CellNum), sscr, failed, 1u, Stream));
     MPS_CUDA_TRY(cudaMemsetAsync(vrange, 0xff, sizeof(int) * (size_t)CellNum * 2, Stream));
-    MPS_COUNT_LAUNCH k_tri_bounds<<<grid_of((int)nv), kBlock, 0, Stream>>>((int)nv, vcell, vrange, vrange + CellNum);
+    MPS_COUNT_LAUNCH k_tri_bounds<<<grid_of((int)nv), kBlock, 0, Stream>>>((int)nv, vcell, vrange, vrange + CellNum, failed, report);
     MPS_COUNT_LAUNCH k_tri_cells<<<div_up(32ll * CellNum, kBlock), kBlock, 0, Stream>>>(CellNum, vrange, vrange + CellNum, vtri, daCell);
     return launch_status();
 }
@@ -1235,12 +1261,14 @@ CCTStatusType ResetWallPosition(cudaStream_t& Stream, const Integer TriangleNum,
 
 CCTStatusType CalcSTLDistance(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
+    if (triangles_failed()) return CCT_CUDAERR;
     MPS_COUNT_LAUNCH k_ref_stl_distance<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
     return launch_status();
 }
 
 CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
+    if (triangles_failed()) return CCT_CUDAERR;
     MPS_COUNT_LAUNCH k_ref_drag<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
     return launch_status();
 }

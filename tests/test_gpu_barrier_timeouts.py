@@ -6,6 +6,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
+import gpu_ref
+import orc
 from simulation_project_gb300 import lib, scenes
 from simulation_project_gb300.lib import DeviceArray, call
 from simulation_project_gb300.solver import Solver, _lib
@@ -132,3 +134,31 @@ def test_sorts_that_give_up():
         dv.upload(np.arange(len(keys), dtype=np.int32))
         call(name, len(keys), dk.ptr, dv.ptr)
         assert np.array_equal(dk.download(), keys[order]) and np.array_equal(dv.download(), order)
+
+
+def test_triangle_cells_whose_sort_gave_up():
+    """The cells hold no triangle then (not stale or half sorted ones); the wall launchers
+    report it until the next RegisterTriangleTopology has, and the one after works."""
+    st = orc.RefState(scenes.rotating_bucket(l0=0.008, n_drag=4))
+    g = gpu_ref.GpuRef(st)
+    g.topology(st.n)
+    s = g.stream.ref()
+    g.walls()
+    want = g.download()["cells"]
+    assert want["m_TriangleNum"].sum() > 4096
+    with no_polls():
+        g.walls()
+        got = g.download()["cells"]
+        assert not got["m_TriangleNum"].any()
+        for name in ("CalcSTLDistance", "CalcDragEffect"):
+            with pytest.raises(MpsError):
+                call(name, s, st.n)
+    keys = DeviceArray.from_host(np.array([3, 1, 2], np.int32))
+    call("SortUsingThrust", 3, keys.ptr, DeviceArray.from_host(np.zeros(3, np.int32)).ptr)   # its own sort was fine
+    with pytest.raises(MpsError):
+        g.walls()
+    g.walls()
+    got = g.download()["cells"]
+    assert np.array_equal(got["m_TriangleNum"], want["m_TriangleNum"])
+    for name in ("CalcSTLDistance", "CalcDragEffect"):
+        g.run(name, st.n)
