@@ -904,14 +904,23 @@ struct RefOp<RpGradient> {
     }
 };
 
+// Two launches share a large call: one of k_ref_pairs and k_ref_slices takes it in dense fluid,
+// k_ref_walk after it in sparse fluid, and the other one of the two has nothing to do
+// (rp_sparse).  k_ref_walk may start once every CTA of the first has (programmatic dependent
+// launch: neither reads what the other writes), and every thread of it ends after the
+// first launch has, so what follows in the stream follows both.
+__device__ __forceinline__ void ref_beside_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void ref_beside_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // one operator over targets 0 .. n-1, T per warp
 template <class Op, int T>
-__global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::NS > 3 ? 5 : 7) k_ref_pairs(int n, float coef, float minus_zero, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::NS > 3 ? 5 : 7) k_ref_pairs(int n, float coef, float minus_zero, int sparse, const __grid_constant__ RefBind b) {
     using W = RpWarp<Op, T>;
     __shared__ __align__(16) float sm[kRpWarps * W::kFloats];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = (blockIdx.x * kRpWarps + warp) * T;
-    if (first >= n) return;
+    ref_beside_start();
+    if ((sparse > 0 && rp_sparse(b, n, sparse)) || first >= n) return;
     const int id = first + lane;
     RpTarget t{};
     int cx = 0, cy = 0, cz = 0;
@@ -932,32 +941,37 @@ __global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::
     if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
-// the same, a lane per target
+// a lane per target: those that the kernels beside it leave (sparse > 0), or all
 template <class Op>
-__global__ void __launch_bounds__(128) k_ref_lanes(int n, float coef, float minus_zero, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(128) k_ref_walk(int n, float coef, int sparse, const __grid_constant__ RefBind b) {
+    __shared__ int2 run[9][128];
     const int id = blockIdx.x * 128 + threadIdx.x;
-    RpTarget t{};
-    int cx = 0, cy = 0, cz = 0;
-    bool walk = false, fin = false;
-    if (id < n) {
+    if ((sparse <= 0 || rp_sparse(b, n, sparse)) && id < n) {
+        RpTarget t{};
+        int cx = 0, cy = 0, cz = 0;
+        bool walk = false;
         t.pos = b.pos[id];
-        fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
+        if (RefOp<Op>::begin(b, id, t, cx, cy, cz, walk)) {
+            float sum[Op::NS], rare[RpShape<Op>::NXR];
+            rp_walk_sums<Op>(b, t, id, walk, cx, cy, cz, RefOp<Op>::radius(b.param), &run[0][threadIdx.x], 128, sum, rare);
+            RefOp<Op>::finish(b, id, t, sum, rare, coef);
+        }
     }
-    float sum[Op::NS], rare[RpShape<Op>::NXR];
-    rl_sums<Op>(b, t, n, id, walk && fin, cx, cy, cz, RefOp<Op>::radius(b.param), minus_zero, sum, rare);
-    if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
+    ref_beside_end();
 }
 
 // 32 targets per warp, operators without rarer pairs
 template <class Op>
 constexpr int rs_warps() { return Op::NS == 1 ? 4 : 2; }
 template <class Op>
-__global__ void __launch_bounds__(rs_warps<Op>() * 32) k_ref_slices(int n, float minus_zero, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(rs_warps<Op>() * 32) k_ref_slices(int n, float minus_zero, int sparse,
+                                                                  const __grid_constant__ RefBind b) {
     using W = RpSlice<Op>;
     __shared__ __align__(16) float sm[rs_warps<Op>() * W::kFloats];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = (blockIdx.x * rs_warps<Op>() + warp) * 32;
-    if (first >= n) return;
+    ref_beside_start();
+    if (rp_sparse(b, n, sparse) || first >= n) return;
     const int id = first + lane;
     RpTarget t{};
     int cx = 0, cy = 0, cz = 0;
@@ -984,6 +998,44 @@ inline int grid_of(int n) { return div_up(n, kBlock); }
 // often (3,120 / 3,514 at 884,736); the turbulence has nine sums.
 constexpr int kRefSlices = 40000;
 
+// From here on a call asks first whether the fluid is sparse and leaves it to k_ref_walk if so.
+// The kernels that share candidates between targets have little to share there, and a warp
+// per few targets is 8 to 32 times fewer targets at a time (us, without and with k_ref_walk,
+// 0.03 particles per cube of the particle distance): pressure 1,262 / 175 at 882,000
+// particles, 198 / 33 at 50,000, 50 / 30 at 19,000, 38 / 32 at 10,000; turbulence 2,353 / 296 at
+// 882,000, predictor 311 / 69 at 110,000.  In dense fluid the question and the second launch
+// cost 1 to 4 % (pressure 77.7 / 79.5 at 103,823, gradient 151 / 153, turbulence 2,215 / 2,269 at
+// 884,736); at 15,625 they would cost 8 % of the pressure.
+constexpr int kRefSplit = 16384;
+// Particles per cell below which k_ref_walk is the faster one.  Measured on random fluid of
+// 0.004 to 1 per cube of the distance (64 such cubes are a cell), us at the densities on both
+// sides of the line, kernel that shares / k_ref_walk: pressure (slices) 0.15: 581 / 410, 0.3:
+// 383 / 670 at 882,000; eight targets per warp 0.06: 65 / 42, 0.15: 48 / 71 at 30,000;
+// turbulence (four per warp) 0.5: 2,015 / 1,605, 1.0: 2,882 / 2,885 at 882,000; predictor 0.1:
+// 96 / 95 at 30,000 and 0.2: 257 / 210, 0.3: 280 / 282 at 110,000.
+template <class Op>
+int rp_few(int n, bool slices, bool pairs2) {
+    if (slices) return 15;
+    if (std::is_same<Op, RpTurbulence>::value && !pairs2) return 40;
+    if (n < 40000) return 7;
+    return std::is_same<Op, RpExplicitly>::value && n >= 64000 ? 16 : 10;
+}
+
+// all targets (sparse 0), or beside the launch before it
+template <class Op>
+cudaError_t ref_walk_launch(cudaStream_t st, int n, float coef, int sparse) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)div_up(n, 128));
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = sparse > 0 ? 1 : 0;
+    return MPS_COUNT_LAUNCH cudaLaunchKernelEx(&cfg, k_ref_walk<Op>, n, coef, sparse, (const RefBind)g_bind);
+}
+
 // Targets per warp of an operator: kMany share each round's candidates; below `few` of
 // them that leaves too few warps per SM and two per warp finish sooner.  Measured in us,
 // two against kMany, on a jittered block: pressure 50 / 54 at 15,625 particles, 72 / 54
@@ -992,27 +1044,29 @@ template <class Op, int kMany>
 cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
     constexpr bool kSlices = std::is_same<Op, RpPressure>::value || std::is_same<Op, RpGradient>::value ||
                              std::is_same<Op, RpTemperature>::value;
+    const int sparse = n < kRefSplit ? 0 : rp_few<Op>(n, kSlices && n >= kRefSlices, n < few);
     if (n < few) {
-        MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, g_bind);
-        return cudaGetLastError();
-    }
-    if constexpr (kSlices) {
-        if (n >= kRefSlices) {
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse, g_bind);
+    } else if (kSlices && n >= kRefSlices) {
+        if constexpr (kSlices) {
             constexpr int W = rs_warps<Op>();
-            MPS_COUNT_LAUNCH k_ref_slices<Op><<<div_up(n, W * 32), W * 32, 0, st>>>(n, -0.0f, g_bind);
-            return cudaGetLastError();
+            MPS_COUNT_LAUNCH k_ref_slices<Op><<<div_up(n, W * 32), W * 32, 0, st>>>(n, -0.0f, sparse, g_bind);
         }
+    } else {
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse,
+                                                                                                        g_bind);
     }
-    MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, g_bind);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    return e || sparse == 0 ? e : ref_walk_launch<Op>(st, n, coef, sparse);
 }
 // Below it a triangle is walked by 32 lanes (few triangles are large ones), else by 8.
 constexpr int kTriFew = 2048;
 constexpr int kRefFew = 20000, kRefFewTurbulence = 100000;
 // From here on the predictor, whose radius is the cell size (250 of 1,728 candidates
-// accepted), runs a lane per target: 2.83 against 2.99 ms at 884,736 particles, 772
-// against 759 us at 216,000.  Its 16-byte loads need aligned arrays.
-constexpr int kRefLanes = 300000;
+// accepted), runs a lane per target whatever the density (us, eight targets per warp / a lane
+// each, with turbulence): 642 / 707 at 157,464 particles, 876 / 885 at 216,000, 3,096 / 2,993
+// at 884,736.
+constexpr int kRefLanes = 216000;
 
 CCTStatusType launch_status() { return cuda_status(cudaGetLastError()); }
 
@@ -1286,9 +1340,8 @@ CCTStatusType CalcExplicitly(cudaStream_t& Stream, Integer ParticleNum) {
     if (g_bind.param.bTurbulance && (!g_bind.turb_visc || !g_bind.strain)) return CCT_PARAMERR;
     const CParameter& P = g_bind.param;
     const float coef = (float)((2.0 * P.Dimension) / (double)(P.LambdaValue * P.ConstantParticleDensity));
-    if (ParticleNum >= kRefLanes && (((uintptr_t)g_bind.pos | (uintptr_t)g_bind.out_id) & 15) == 0)
-        MPS_COUNT_LAUNCH k_ref_lanes<RpExplicitly><<<div_up(ParticleNum, 128), 128, 0, Stream>>>(ParticleNum, coef, -0.0f,
-                                                                                                  g_bind);
+    if (ParticleNum >= kRefLanes)
+        MPS_CUDA_TRY(ref_walk_launch<RpExplicitly>(Stream, ParticleNum, coef, 0));
     else
         MPS_CUDA_TRY((ref_op_launch<RpExplicitly, 8>(Stream, ParticleNum, kRefFew, coef)));
     return launch_status();

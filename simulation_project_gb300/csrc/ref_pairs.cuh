@@ -24,6 +24,7 @@
 // and after: 15,625 particles pressure 312 / 50, heat 324 / 53, turbulence 414 / 62,
 // predictor 531 / 94; 103,823 pressure 334 / 137, gradient 462 / 177; 884,736 pressure
 // 1,520 / 1,160, gradient 2,450 / 1,406 (from 40,000 particles on RpSlice takes over these).
+// In sparse fluid there is little to share; a lane per target is faster there (rp_walk_sums).
 #pragma once
 
 namespace mps {
@@ -838,102 +839,71 @@ struct RpSlice {
     __device__ __forceinline__ float sum(int c) const { return sm[kSum + c * 32 + lane]; }
 };
 
-// A lane per target, each walking its own 27 cells: the candidates four at a time from
-// 16-byte loads (the lanes of a warp mostly share a cell, so one address), the next four
-// loaded before these are tested, an accepted pair's terms added at once.  It needs no
-// votes, ranks and second pass per pair, but runs the terms of every candidate that any
-// of 32 targets accepts, and has 1/32 warp per target: only for many accepted pairs per
-// candidate and many targets.
+// Sparse fluid: a cell holds fewer than about `few` particles, seen from 16 targets spread over
+// the sorted order, half of which at least have the target `few` places on more than a cell
+// away.  Every warp of a call comes to the same answer, from one round of loads.
+__device__ __forceinline__ bool rp_sparse(const RefBind& b, int n, int few) {
+    const int lane = threadIdx.x & 31;
+    bool near = false;
+    if (lane < 16) {
+        const int x = (int)((long long)n * (2 * lane + 1) / 32);
+        const Scalar3 p = b.pos[x], q = b.pos[min(x + few, n - 1)];
+        near = fmaxf(fabsf(p.x - q.x), fmaxf(fabsf(p.y - q.y), fabsf(p.z - q.z))) < b.box.m_CellSize;
+    }
+    return __popc(__ballot_sync(~0u, near)) < 8;
+}
+
+// A lane per target, each walking its own 27 cells.  The bounds of a layer's nine cells are
+// loaded together into `run` (a column of shared memory per thread), so a target without
+// neighbours waits for memory six times, not 54.  It needs no votes, ranks and second pass per
+// pair and no warp per few targets, but runs the terms of every candidate that any of 32
+// targets accepts: for many accepted pairs per candidate or few candidates per cell.
 template <class Op>
-__device__ __forceinline__ void rl_sums(const RefBind& b, const RpTarget& t, int n, int id, bool walk, int cx, int cy,
-                                        int cz, float re, float minus_zero, float (&acc)[Op::NS],
-                                        float (&xacc)[RpShape<Op>::NXR]) {
+__device__ __forceinline__ void rp_walk_sums(const RefBind& b, const RpTarget& t, int id, bool walk, int cx, int cy, int cz,
+                                             float re, int2* run, int stride, float (&acc)[Op::NS],
+                                             float (&xacc)[RpShape<Op>::NXR]) {
     const float mind = (float)(re * 1e-3), re2x = ref_screen2(re);
     float rare_re = 0.0f;
     if constexpr (Op::NX > 0) rare_re = Op::rare_radius(b.param);
-    const unsigned long long nz2 = rp_pack(minus_zero, minus_zero);
-    // differences in the order that the components lie in memory (a square has no sign)
-    const unsigned long long txy = rp_pack(-t.pos.x, -t.pos.y), tzx = rp_pack(-t.pos.z, -t.pos.x),
-                             tyz = rp_pack(-t.pos.y, -t.pos.z);
 #pragma unroll
     for (int c = 0; c < Op::NS; ++c) acc[c] = 0.0f;
 #pragma unroll
     for (int c = 0; c < RpShape<Op>::NXR; ++c) xacc[c] = 0.0f;
-    const Integer3 G = b.box.m_GridSize;
-    const ulonglong2* const pos16 = reinterpret_cast<const ulonglong2*>(b.pos);
-    const int4* const oid4 = reinterpret_cast<const int4*>(b.out_id);
+    if (!walk) return;
 #pragma unroll 1
-    for (int m = 0; m < 27; ++m) {
-        const int i = m % 3 - 1, j = (m / 3) % 3 - 1, k = m / 9 - 1;
-        const int cell = cell_key(G, (int)((unsigned)cx + (unsigned)i), (int)((unsigned)cy + (unsigned)j),
-                                  (int)((unsigned)cz + (unsigned)k));
-        int s = 0, e = 0;
-        if (walk && cell >= 0 && cell < b.cell_num) {
-            s = b.cell_start[cell];
-            e = s == -1 ? s : b.cell_end[cell];
+    for (int k = -1; k <= 1; ++k) {
+        int s[9], m[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            m[q] = cell_key(b.box.m_GridSize, (int)((unsigned)cx + (unsigned)(q % 3 - 1)),
+                            (int)((unsigned)cy + (unsigned)(q / 3 - 1)), (int)((unsigned)cz + (unsigned)k));
+            s[q] = m[q] >= 0 && m[q] < b.cell_num ? b.cell_start[m[q]] : -1;
         }
-        if (s >= e) continue;
-        const int g1 = (e + 3) >> 2;
-        int g = s >> 2;
-        int4 on = make_int4(0, 0, 0, 0);
-        ulonglong2 n0{}, n1{}, n2{};
-        if (4 * g + 4 <= n) {   // 16-byte loads stay inside the arrays
-            on = oid4[g];
-            n0 = pos16[3 * (size_t)g];
-            n1 = pos16[3 * (size_t)g + 1];
-            n2 = pos16[3 * (size_t)g + 2];
-        }
+#pragma unroll
+        for (int q = 0; q < 9; ++q) run[q * stride] = make_int2(s[q], s[q] != -1 ? b.cell_end[m[q]] : -1);
 #pragma unroll 1
-        for (; g < g1; ++g) {
-            const int4 o = on;
-            const ulonglong2 p0 = n0, p1 = n1, p2 = n2;
-            const bool safe = 4 * g + 4 <= n;
-            if (g + 1 < g1 && 4 * g + 8 <= n) {
-                on = oid4[g + 1];
-                n0 = pos16[3 * (size_t)g + 3];
-                n1 = pos16[3 * (size_t)g + 4];
-                n2 = pos16[3 * (size_t)g + 5];
-            }
-            const unsigned long long c[6] = {rp_add2(p0.x, txy), rp_add2(p0.y, tzx), rp_add2(p1.x, tyz),
-                                             rp_add2(p1.y, txy), rp_add2(p2.x, tzx), rp_add2(p2.y, tyz)};
-            float f[12], d2[4];
-#pragma unroll
-            for (int h = 0; h < 6; ++h) rp_unpack(rp_mul2(c[h], c[h], nz2), f[2 * h], f[2 * h + 1]);
-#pragma unroll
-            for (int h = 0; h < 4; ++h) d2[h] = f[3 * h] + f[3 * h + 1] + f[3 * h + 2];
-            if (!safe || 4 * g < s || 4 * g + 4 > e || ((o.x | o.y) | (o.z | o.w)) < 0) {
-                // a cell's first or last group, or particles to be skipped
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int x = 4 * g + h;
-                    const bool valid = x >= s && x < e;
-                    int oid = h == 0 ? o.x : h == 1 ? o.y : h == 2 ? o.z : o.w;
-                    if (!safe && valid) {
-                        oid = b.out_id[x];
-                        const Scalar3 p = b.pos[x];
-                        const float dx = t.pos.x - p.x, dy = t.pos.y - p.y, dz = t.pos.z - p.z;
-                        d2[h] = dx * dx + dy * dy + dz * dz;
-                    }
-                    if (!valid || oid < 0) d2[h] = 3.402823466e38f;   // screened out
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                if (d2[h] >= re2x && d2[h] <= 3.402823466e38f) continue;
-                const int x = 4 * g + h;
-                float d = ref_sqrt(d2[h]);
-                if (!(Op::kLe ? d <= re : d < re) || x == id) continue;
+        for (int q = 0; q < 9; ++q) {
+            const int2 r = run[q * stride];
+#pragma unroll 1
+            for (int x = r.x; x < r.y; ++x) {
+                const int out = b.out_id[x];
+                const Scalar3 p = b.pos[x];
+                const float dx = t.pos.x - p.x, dy = t.pos.y - p.y, dz = t.pos.z - p.z;
+                const float d2 = dx * dx + dy * dy + dz * dz;
+                if (out < 0 || x == id || (d2 >= re2x && d2 <= 3.402823466e38f)) continue;
+                float d = ref_sqrt(d2);
+                if (!(Op::kLe ? d <= re : d < re)) continue;
                 if (d < mind) d = mind;
                 float v[Op::NS];
                 Op::terms(b, re, t, x, d, v);
 #pragma unroll
-                for (int q = 0; q < Op::NS; ++q) acc[q] += v[q];
+                for (int c = 0; c < Op::NS; ++c) acc[c] += v[c];
                 if constexpr (Op::NX > 0) {
                     if (d < rare_re) {
                         float ex[Op::NX];
                         Op::rare_terms(b, re, t, x, d, ex);
 #pragma unroll
-                        for (int q = 0; q < Op::NX; ++q) xacc[q] += ex[q];
+                        for (int c = 0; c < Op::NX; ++c) xacc[c] += ex[c];
                     }
                 }
             }
