@@ -449,7 +449,8 @@ __global__ void k_tri_reset_wall(int t, int step, const CTriangle* __restrict__ 
 // Bound by the latency of long lists: particles beside drag spheres meet hundreds of
 // entries while most meet none, and a thread per particle ran them one after another, each
 // with three FP64 divisions: 535 us for 108,186 particles and 9,216 triangles, DRAM idle.
-// A warp for four: 184 us (drag 548 -> 179); 882,080 particles 478 -> 367 (376 -> 314).
+// A warp for four: 184 us (drag 548 -> 179); 882,080 particles 478 -> 367 (376 -> 314).  Where
+// most particles see few triangles a lane per particle goes first (near_short_first).
 constexpr int kNearT = 4;
 template <bool DRAG>
 __device__ __forceinline__ void ref_nearest(const RefBind& b, const Scalar3& p, bool live, CDistance& nd, int& nid) {
@@ -541,30 +542,102 @@ __device__ __forceinline__ void ref_nearest(const RefBind& b, const Scalar3& p, 
     if (nid != -1) nd.Magnitude = ref_tri_distance(ref_tri(b.triangles[nid]), p, nd.Direction);
 }
 
-// CalcSTLDistance_Kernel (DeviceProcess_Kernel.h:853-919)
+// A lane per particle: the serial loop itself where its lists hold at most kNearShort entries in
+// all (false: more, nothing done).  The 27 lengths are loaded nine at a time.
+constexpr unsigned kNearShort = 32;
+template <bool DRAG>
+__device__ __forceinline__ bool ref_nearest_short(const RefBind& b, const Scalar3& p, bool live, CDistance& nd, int& nid) {
+    nd.Magnitude = 1e8f;
+    nd.Direction = s3(0, 0, 0);
+    nid = -1;
+    int cx, cy, cz;
+    const int cid = ref_cell(b.box, p, cx, cy, cz);
+    if (!live || cid < 0 || cid >= b.cell_num) return true;
+    auto key = [&](int c) {
+        return cell_key(b.box.m_GridSize, (int)((unsigned)cx + (unsigned)(c % 3) - 1u),
+                        (int)((unsigned)cy + (unsigned)(c / 3 % 3) - 1u), (int)((unsigned)cz + (unsigned)(c / 9) - 1u));
+    };
+    unsigned held = 0, some = 0;
+#pragma unroll 9
+    for (int c = 0; c < 27; ++c) {
+        const int m = key(c);
+        const unsigned len = m >= 0 && m < b.cell_num ? min(b.cells[m].m_TriangleNum, (unsigned)CELLMAXTRIANGLENUM) : 0u;
+        held += len;
+        if (len) some |= 1u << c;
+    }
+    if (held > kNearShort) return false;
+    while (some) {
+        const CCell& cell = b.cells[key(__ffs(some) - 1)];
+        some &= some - 1u;
+        const int len = (int)min(cell.m_TriangleNum, (unsigned)CELLMAXTRIANGLENUM);
+        for (int l = 0; l < len; ++l) {
+            const int t = cell.m_TriangleID[l];
+            if (t < 0 || t >= b.triangle_num || (DRAG && !b.tri_params[b.triangles[t].ModelIDNumber].isDrag)) continue;
+            Scalar3 dir;
+            const float d = ref_tri_distance(ref_tri(b.triangles[t]), p, dir);
+            if (d < nd.Magnitude) {
+                nd.Magnitude = d;
+                nd.Direction = dir;
+                nid = t;
+            }
+        }
+    }
+    return true;
+}
+constexpr int kNearLeft = -2;   // mark of the particles that the lane per particle leaves
+
+// particles of a CTA of four warps, kNearT to a warp at a time
+template <bool LEFT>
+constexpr int near_particles() { return LEFT ? 32 : 4 * kNearT; }
+// work(id, mine): a warp's kNearT particles, one in each of its first lanes; LEFT: those with
+// the mark alone (mark[id] == kNearLeft)
+template <bool LEFT, class Work>
+__device__ __forceinline__ void near_groups(int n, const int* mark, Work&& work) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = blockIdx.x * near_particles<LEFT>();
+    if constexpr (!LEFT) {
+        const int id = first + warp * kNearT + lane;
+        work(id, lane < kNearT && id < n);
+    } else {
+        __shared__ int list[32];
+        const bool on = first + lane < n && mark[first + lane] == kNearLeft;
+        const unsigned found = __ballot_sync(~0u, on);   // the same in every warp
+        const int count = __popc(found);
+        if (on && warp == 0) list[__popc(found & ((1u << lane) - 1u))] = first + lane;
+        if (count == 0) return;
+        __syncthreads();
+        for (int g = warp * kNearT; g < count; g += 4 * kNearT) {
+            const bool mine = lane < kNearT && g + lane < count;
+            work(mine ? list[g + lane] : 0, mine);
+        }
+    }
+}
+
+// CalcSTLDistance_Kernel (DeviceProcess_Kernel.h:853-919): a warp for kNearT particles, those
+// that k_ref_stl_short has left, or all
+template <bool LEFT>
 __global__ void __launch_bounds__(128, 8) k_ref_stl_distance(int n, const __grid_constant__ RefBind b) {
-    const int lane = threadIdx.x & 31;
-    const int id = (blockIdx.x * 4 + (threadIdx.x >> 5)) * kNearT + lane;
-    const bool mine = lane < kNearT && id < n;
+    near_groups<LEFT>(n, b.stl_id, [&](int id, bool mine) {
+        CDistance nd;
+        int nid;
+        ref_nearest<false>(b, mine ? b.pos[id] : s3(0, 0, 0), mine, nd, nid);
+        if (!mine) return;
+        b.stl_distance[id] = nd;
+        b.stl_id[id] = nid;
+    });
+}
+__global__ void __launch_bounds__(128) k_ref_stl_short(int n, const __grid_constant__ RefBind b) {
+    const int id = blockIdx.x * 128 + threadIdx.x;
+    if (id >= n) return;
     CDistance nd;
     int nid;
-    ref_nearest<false>(b, mine ? b.pos[id] : s3(0, 0, 0), mine, nd, nid);
-    if (!mine) return;
-    b.stl_distance[id] = nd;
+    if (ref_nearest_short<false>(b, b.pos[id], true, nd, nid)) b.stl_distance[id] = nd;
+    else nid = kNearLeft;
     b.stl_id[id] = nid;
 }
 
 // CalcDragEffect_Kernel and mode helpers (DeviceProcess_Kernel.h:125-389), with the
 // reference's index use and brace placement (mode 'F' acts outside the region).
-__global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constant__ RefBind b) {
-    const int lane = threadIdx.x & 31;
-    const int id = (blockIdx.x * 4 + (threadIdx.x >> 5)) * kNearT + lane;
-    const bool mine = lane < kNearT && id < n;
-    const bool gone = mine && b.out_id[id] < -1;
-    CDistance nd;
-    int nid;
-    ref_nearest<true>(b, mine ? b.pos[id] : s3(0, 0, 0), mine && !gone, nd, nid);
-    if (!mine) return;
+__device__ __forceinline__ void ref_drag_finish(const RefBind& b, int id, bool gone, const CDistance& nd, int nid) {
     const CParameter& P = b.param;
     if (b.magnifier_count[id] > 0) b.magnifier_count[id]++;
     if (b.magnifier_count[id] == 10) b.magnifier_count[id] = 0;
@@ -610,6 +683,26 @@ __global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constan
             b.out_vel[id].x *= f; b.out_vel[id].y *= f; b.out_vel[id].z *= f;
         }
     }
+}
+// as k_ref_stl_distance and k_ref_stl_short
+template <bool LEFT>
+__global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constant__ RefBind b) {
+    near_groups<LEFT>(n, b.out_type, [&](int id, bool mine) {
+        const bool gone = mine && b.out_id[id] < -1;
+        CDistance nd;
+        int nid;
+        ref_nearest<true>(b, mine ? b.pos[id] : s3(0, 0, 0), mine && !gone, nd, nid);
+        if (mine) ref_drag_finish(b, id, gone, nd, nid);
+    });
+}
+__global__ void __launch_bounds__(128) k_ref_drag_short(int n, const __grid_constant__ RefBind b) {
+    const int id = blockIdx.x * 128 + threadIdx.x;
+    if (id >= n) return;
+    const bool gone = b.out_id[id] < -1;
+    CDistance nd;
+    int nid;
+    if (ref_nearest_short<true>(b, b.pos[id], !gone, nd, nid)) ref_drag_finish(b, id, gone, nd, nid);
+    else b.out_type[id] = kNearLeft;
 }
 
 // ---------------------------------------------------------------------------
@@ -1061,6 +1154,15 @@ cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
 }
 // Below it a triangle is walked by 32 lanes (few triangles are large ones), else by 8.
 constexpr int kTriFew = 2048;
+// Wall distance and drag: most particles of a large set see few triangles or none, and a warp
+// per four of them is then most of the time.  With 64,000 particles and 100 for every
+// triangle a lane per particle does the short lists first.  us, a thread per particle (its
+// divisions in FP64) / a warp per four / both in turn: no triangles near 882,000 particles 44 / 101 /
+// 38, 110,000 15 / 17 / 12, 16,000 14 / 7 / 10; 12 triangles around 1,024,000 65 / 175 / 74, around
+// 250,000 42 / 58 / 48; 4,096 around 882,080 177 / 196 / 169 (drag, none of them: 58 / 118 / 67);
+// the line: 9,216 with drag spheres among 882,080 (96 to one) 539 / 347 / 350, 4,176 among 513,279
+// (123 to one) 211 / 136 / 135, among 318,675 (76 to one) 240 / 108 / 125.
+bool near_short_first(int n) { return n >= 64000 && n / 100 >= g_bind.triangle_num; }
 constexpr int kRefFew = 20000, kRefFewTurbulence = 100000;
 // From here on the predictor, whose radius is the cell size (250 of 1,728 candidates
 // accepted), runs a lane per target whatever the density (us, eight targets per warp / a lane
@@ -1324,14 +1426,26 @@ CCTStatusType ResetWallPosition(cudaStream_t& Stream, const Integer TriangleNum,
 CCTStatusType CalcSTLDistance(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (triangles_failed()) return CCT_CUDAERR;
-    MPS_COUNT_LAUNCH k_ref_stl_distance<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
+    const int n = ComputeParticleNum;
+    if (near_short_first(n)) {
+        MPS_COUNT_LAUNCH k_ref_stl_short<<<div_up(n, 128), 128, 0, Stream>>>(n, g_bind);
+        MPS_COUNT_LAUNCH k_ref_stl_distance<true><<<div_up(n, near_particles<true>()), 128, 0, Stream>>>(n, g_bind);
+    } else {
+        MPS_COUNT_LAUNCH k_ref_stl_distance<false><<<div_up(n, near_particles<false>()), 128, 0, Stream>>>(n, g_bind);
+    }
     return launch_status();
 }
 
 CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (triangles_failed()) return CCT_CUDAERR;
-    MPS_COUNT_LAUNCH k_ref_drag<<<div_up(ComputeParticleNum, 4 * kNearT), 128, 0, Stream>>>(ComputeParticleNum, g_bind);
+    const int n = ComputeParticleNum;
+    if (near_short_first(n)) {
+        MPS_COUNT_LAUNCH k_ref_drag_short<<<div_up(n, 128), 128, 0, Stream>>>(n, g_bind);
+        MPS_COUNT_LAUNCH k_ref_drag<true><<<div_up(n, near_particles<true>()), 128, 0, Stream>>>(n, g_bind);
+    } else {
+        MPS_COUNT_LAUNCH k_ref_drag<false><<<div_up(n, near_particles<false>()), 128, 0, Stream>>>(n, g_bind);
+    }
     return launch_status();
 }
 
