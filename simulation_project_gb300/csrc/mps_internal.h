@@ -11,14 +11,17 @@ namespace mps {
 // radix sort (sort.cu).  Scratch: barrier words, key ranges, digit totals, digit counts of
 // every CTA, alternate key and value arrays.
 constexpr int kRadixDigitBits = 9;
-constexpr int kRadixMaxCtas = 152;
-// CTAs of a sort: up to 4,096 keys one (no grid barriers), then one per 1,024 keys
+constexpr int kRadixMaxCtas = 304;
+constexpr long long kRadixTwoPerSm = 2500000;
+// CTAs of a sort: up to 4,096 keys one (no grid barriers), then one per 1,024 keys, one per SM
+// at most, or two where memory bounds it
 constexpr int radix_ctas_for(long long n) {
-    return n <= 4096 ? 1 : (n + 1023) / 1024 < kRadixMaxCtas ? (int)((n + 1023) / 1024) : kRadixMaxCtas;
+    const int most = n < kRadixTwoPerSm ? kRadixMaxCtas / 2 : kRadixMaxCtas;
+    return n <= 4096 ? 1 : (n + 1023) / 1024 < most ? (int)((n + 1023) / 1024) : most;
 }
 constexpr size_t radix_scratch_bytes_for(long long n, int max_ctas = kRadixMaxCtas) {
     const size_t ctas = (size_t)(radix_ctas_for(n) < max_ctas ? radix_ctas_for(n) : max_ctas);
-    return sizeof(unsigned) * (8 + 2 * (size_t)kRadixMaxCtas + ((size_t)1 << kRadixDigitBits) * (ctas + 1)) +
+    return sizeof(unsigned) * (8 + 2 * ctas + ((size_t)1 << kRadixDigitBits) * (ctas + 1)) +
            sizeof(int) * 2 * (size_t)(n > 0 ? n : 0);
 }
 inline size_t radix_scratch_bytes(int n) { return radix_scratch_bytes_for(n); }

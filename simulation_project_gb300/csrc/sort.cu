@@ -25,7 +25,9 @@
 // and values stay in L2.  882,080 nearly sorted keys of 17 bits, in us: range 6, then per
 // pass count 2.6, prefix 1, scan 0.6, scatter 4.4 and three barriers of 1.2 to 2.2; 34 in
 // all (random keys 68: their scatter takes 14, 16,000 keys 21 to 26).  Two CTAs per SM took
-// 40 and 72.  It replaces three launches per 8-bit pass, 13 to 16 per sort with
+// 40 and 72; from 2.5 million keys on they are the faster (us, a call with one / two per SM:
+// 2,000,000 nearly sorted 92 / 97, random 226 / 223; 5,000,000 236 / 195 and 467 / 437; 30,000,000
+// 1,540 / 1,172 and 2,778 / 2,488).  It replaces three launches per 8-bit pass, 13 to 16 per sort with
 // the range's and those of passes beyond the range, which returned at once; finding the
 // range alone took 27 us at 882,080 keys (19,456 atomics on one address).
 #include <limits.h>
@@ -233,14 +235,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
         // these pairs in this launch: through L2)
         const bool one = end - beg <= kSortTile;
         int key[kSortRounds], val[kSortRounds];
-        auto load = [&](int t0, int tend, int rounds) {
+        auto load = [&](int t0, int tend, int rounds, bool values) {
             const int base = t0 + w * 32 * rounds + lane;
 #pragma unroll
             for (int r = 0; r < kSortRounds; ++r) {
                 if (r < rounds) {
                     const int i = base + 32 * r;
                     key[r] = i < tend ? __ldcg(ka + i) : 0;
-                    val[r] = i < tend ? __ldcg(va + i) : 0;
+                    if (values) val[r] = i < tend ? __ldcg(va + i) : 0;
                 }
             }
         };
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
         for (int t0 = beg; t0 < end; t0 += kSortTile) {
             const int tend = min(end, t0 + kSortTile);
             const int rounds = (tend - t0 + kSortThreads - 1) / kSortThreads;   // of 32 keys per warp
-            load(t0, tend, rounds);
+            load(t0, tend, rounds, one);
 #pragma unroll
             for (int r = 0; r < kSortRounds; ++r) {
                 if (r < rounds) {
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
             for (int q = 0; q < kSortWarps; ++q) wcount[q][tid] = 0;
             __syncthreads();
             const int base = t0 + w * 32 * rounds + lane;
-            if (!one) load(t0, tend, rounds);
+            if (!one) load(t0, tend, rounds, true);
             unsigned at[kSortRounds];   // digit | rank << 10
 #pragma unroll
             for (int r = 0; r < kSortRounds; ++r) {
@@ -395,7 +397,7 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), sms));   // one per SM at most: all resident
+    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), n < kRadixTwoPerSm ? sms : 2 * sms));   // all resident
     int part = div_up(n, most);
     part = (part + kSortThreads - 1) / kSortThreads * kSortThreads;
     const int ctas = div_up(n, part);
@@ -403,7 +405,7 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
     unsigned* p = (unsigned*)scratch;
     s.bar = p;
     s.range = (int*)(p + 8);
-    s.total = p + 8 + 2 * kRadixMaxCtas;
+    s.total = p + 8 + 2 * ctas;
     s.counts = s.total + kRadix;
     s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
     s.vals = s.keys + n;
