@@ -75,6 +75,14 @@ extern unsigned long long g_kernel_launches;
 #define MPS_COUNT_LAUNCH __atomic_fetch_add(&::mps::g_kernel_launches, 1ull, __ATOMIC_RELAXED),
 void scratch_release_all();
 
+// a cooperative launch that its stream or context has no room for (its SMs are a part of the
+// GPU's) or does not do: not an error of the call, which then takes another way
+inline bool coop_refused(cudaError_t e) {
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+    cudaGetLastError();
+    return true;
+}
+
 inline CCTStatusType cuda_status(cudaError_t e) { return e == cudaSuccess ? CCT_NOERR : CCT_CUDAERR; }
 
 }  // namespace mps

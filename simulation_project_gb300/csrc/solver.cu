@@ -642,6 +642,21 @@ struct Solver {
         return std::max(1, std::min(coop_resident, div_up(mg.L[2].n, 8)));
     }
 
+    // levels 2 .. last in one cooperative launch (grid barriers between stages); false: not available
+    bool coarse_cycle() {
+        const int grid = coarse_cycle_grid();
+        if (grid <= 0) return false;
+        void* args[] = {(void*)&d.scal, (void*)&mg, (void*)&coop_bar, (void*)&d.err};
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_mg_coarse_cycle, dim3(grid), dim3(256), args, 0, st);
+        if (coop_refused(e)) {
+            coop_resident = 0;
+            return false;
+        }
+        if (e) stream_failed = true;
+        MPS_COUNT_LAUNCH 0;
+        return true;
+    }
+
     void mg_apply(const float* r, float* z, float* p, int mode, bool restricted = false) {
         MgLevel* L = mg.L;
         const int lv = mg.levels;
@@ -661,13 +676,7 @@ struct Solver {
         // the reduction buffer holds 2 partials per CTA of the fused kernel
         const bool fuse = !post && lv >= 2 && extra == 0 && up1_blocks <= 2 * kRedBlocks;
         const float* qf = (flex_step && mode == 0) ? d.q32 : nullptr;
-        const int cg = fuse ? coarse_cycle_grid() : 0;
-        if (cg > 0) {
-            // levels 2 .. last in one cooperative launch (grid barriers between stages)
-            void* args[] = {(void*)&d.scal, (void*)&mg, (void*)&coop_bar, (void*)&d.err};
-            MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_mg_coarse_cycle, dim3(cg), dim3(256), args, 0,
-                                                         st);
-        } else {
+        if (!fuse || !coarse_cycle()) {
             // the last restriction also solves the last level densely (its last CTA, of
             // 1024 threads like the stand-alone dense solve)
             for (int l = 1; l < lv; ++l) {
@@ -1521,8 +1530,9 @@ struct Solver {
         return spc >= 1 && spc <= kCgMaxSlices && cg_smem(spc) <= kCgSmem ? spc : 0;
     }
     // A d = r / rn of one refinement pass to tol: d in d32.  Nothing is read back: the count of
-    // iterations (S_ITER, -1 on failure) comes with the next residual's norms.
-    bool cg_small(int spc, double rn, double tol) {
+    // iterations (S_ITER, -1 on failure) comes with the next residual's norms.  Returns 1, 0 if
+    // the launch is refused (the kernel chain then, from now on) and -1 on an error.
+    int cg_small(int spc, double rn, double tol) {
         cgs.spc = spc;
         cgs.K = cg_row_room();
         cgs.levels = mg_ready ? mg.levels : 0;
@@ -1531,10 +1541,12 @@ struct Solver {
         cgs.scale = 1.0 / rn;
         cgs.tol = tol;
         void* args[] = {(void*)&d, (void*)&mg, (void*)&cgs};
-        if (MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_cg_small, dim3(div_up(div_up(d.n, 32), spc)),
-                                                         dim3(kCgThreads), args, cg_smem(spc), st))
-            return false;
-        return true;
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_cg_small, dim3(div_up(div_up(d.n, 32), spc)),
+                                                          dim3(kCgThreads), args, cg_smem(spc), st);
+        if (coop_refused(e)) return cg_sms = 0;
+        if (e) return -1;
+        MPS_COUNT_LAUNCH 0;
+        return 1;
     }
 
     // FP32 Jacobi-PCG inside FP64 iterative refinement
@@ -1583,9 +1595,9 @@ struct Solver {
             const double need = 0.3 * opt.cg_rtol * bnorm / rn;
             const double inner_tol = std::max(need, ir_inner_rtol());
             const int pi = outer < kPassMemory ? outer : kPassMemory - 1;
-            const int small = cg_small_slices();
+            const int spc = cg_small_slices(), small = spc > 0 ? cg_small(spc, rn, inner_tol) : 0;
+            if (small < 0) return CCT_CUDAERR;
             if (small > 0) {
-                if (!cg_small(small, rn, inner_tol)) return CCT_CUDAERR;
                 small_pass = pi;
             } else {
                 MPS_COUNT_LAUNCH k_cg_start<float><<<red_blocks(d.n), 256, 0, st>>>(d, d.r32, d.z32, d.p32, d.r, 1.0 / rn, nullptr, d.m32, d.d32, 3,

@@ -397,24 +397,33 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int most = max(1, min(min(max_ctas, radix_ctas_for(n)), n < kRadixTwoPerSm ? sms : 2 * sms));   // all resident
-    int part = div_up(n, most);
-    part = (part + kSortThreads - 1) / kSortThreads * kSortThreads;
-    const int ctas = div_up(n, part);
-    SortScratch s;
-    unsigned* p = (unsigned*)scratch;
-    s.bar = p;
-    s.range = (int*)(p + 8);
-    s.total = p + 8 + 2 * ctas;
-    s.counts = s.total + kRadix;
-    s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
-    s.vals = s.keys + n;
-    if (ctas > 1) {
-        const cudaError_t e = cudaMemsetAsync(s.bar, 0, sizeof(unsigned), st);
+    // all resident on the whole GPU; a stream or context with a part of its SMs refuses such a
+    // launch and gets half as many until one fits.  One CTA has no barriers and is an
+    // ordinary launch.
+    for (int most = max(1, min(min(max_ctas, radix_ctas_for(n)), n < kRadixTwoPerSm ? sms : 2 * sms));; most /= 2) {
+        int part = div_up(n, most);
+        part = (part + kSortThreads - 1) / kSortThreads * kSortThreads;
+        const int ctas = div_up(n, part);
+        SortScratch s;
+        unsigned* p = (unsigned*)scratch;
+        s.bar = p;
+        s.range = (int*)(p + 8);
+        s.total = p + 8 + 2 * ctas;
+        s.counts = s.total + kRadix;
+        s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
+        s.vals = s.keys + n;
+        if (ctas == 1) {
+            MPS_COUNT_LAUNCH k_sort<<<1, kSortThreads, 0, st>>>(n, part, keys, vals, bits, s, err, bit);
+            return cudaGetLastError();
+        }
+        cudaError_t e = cudaMemsetAsync(s.bar, 0, sizeof(unsigned), st);
         if (e) return e;
+        void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err, (void*)&bit};
+        e = cudaLaunchCooperativeKernel((const void*)k_sort, dim3(ctas), dim3(kSortThreads), args, 0, st);
+        if (e == cudaSuccess) MPS_COUNT_LAUNCH 0;
+        if (!coop_refused(e)) return e;
+        if (e == cudaErrorNotSupported) most = 2;   // one CTA next
     }
-    void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err, (void*)&bit};
-    return MPS_COUNT_LAUNCH cudaLaunchCooperativeKernel((const void*)k_sort, dim3(ctas), dim3(kSortThreads), args, 0, st);
 }
 
 cudaError_t scan_exclusive(unsigned* a, int len, unsigned* total_dev, cudaStream_t st, unsigned* tile_sums) {
