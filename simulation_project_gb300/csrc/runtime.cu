@@ -60,12 +60,23 @@ void* scratch_get(int slot, size_t bytes) {
 ScratchTurn::ScratchTurn() { g_turn.lock(); }
 ScratchTurn::ScratchTurn(cudaStream_t st) : st_(st), on_stream_(true) {
     g_turn.lock();
-    if (g_turn_done) cudaStreamWaitEvent(st, g_turn_done, 0);
-    else if (cudaEventCreateWithFlags(&g_turn_done, cudaEventDisableTiming) != cudaSuccess) g_turn_done = nullptr;
+    // an event that cannot be had or waited for costs a host wait, and its error is not the call's
+    if (!g_turn_done) {
+        if (cudaEventCreateWithFlags(&g_turn_done, cudaEventDisableTiming) == cudaSuccess) return;
+        g_turn_done = nullptr;
+        cudaGetLastError();
+    } else if (cudaStreamWaitEvent(st, g_turn_done, 0) != cudaSuccess) {
+        cudaGetLastError();
+        cudaEventSynchronize(g_turn_done);
+    }
 }
 ScratchTurn::~ScratchTurn() {
-    // without an event (none could be created) the turn ends when its work does
-    if (on_stream_ && (!g_turn_done || cudaEventRecord(g_turn_done, st_) != cudaSuccess)) cudaStreamSynchronize(st_);
+    // without an event (none could be created, or it is another device's) the turn ends when
+    // its work does
+    if (on_stream_ && (!g_turn_done || cudaEventRecord(g_turn_done, st_) != cudaSuccess)) {
+        if (g_turn_done) cudaGetLastError();
+        cudaStreamSynchronize(st_);
+    }
     g_turn.unlock();
 }
 
