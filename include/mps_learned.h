@@ -61,18 +61,21 @@ CCTStatusType mps_mlp_forward_variant(MpsMlp* m, int M, const float* X, float* Y
 /* nonzero if an MMA completion wait of the tcgen05 kernel ever ran out (the kernel then
  * stops early; its outputs are incomplete) */
 CCTStatusType mps_mlp_tc_timeouts(unsigned* out);
-/* debugging and tests: the number of polls of the inference kernel's MMA completion
- * waits (negative: the default, 4,194,304; 0: every such wait runs out at once, so the
- * kernel's stop path runs: each 128-row tile stops after issuing its first layer and
- * writes no output, the MMAs in flight drain before TMEM is freed).  Synchronises the
+/* debugging and tests: the number of polls of the MMA completion waits of the inference
+ * and the training kernel (negative: the default, 4,194,304; 0: every such wait runs out at
+ * once, so the kernels' stop paths run: each 128-row tile stops after issuing its first
+ * layer and writes no output, the MMAs in flight drain before TMEM is freed).  Synchronises the
  * device and clears the mps_mlp_tc_timeouts flag. */
 CCTStatusType mps_mlp_debug_wait_spins(long long spins);
 /* loss = mean over rows of (y0-t0)^2 + w1 (y1-t1)^2 and the gradient of every
  * parameter (device FP32, MPS_MLP_PARAMS floats), forward and backward pass in one kernel
- * on the tensor cores (an array that is not 16-byte aligned costs a copy) */
+ * on the tensor cores (an array that is not 16-byte aligned costs a copy).  CCT_CUDAERR if
+ * a wait of the kernel ran out: loss and gradient are incomplete then */
 CCTStatusType mps_mlp_loss_grad(MpsMlp* m, int M, const float* X, const float* T, float w1, float* grad,
                                 float* host_loss, void* stream);
-/* one Adam step (lr, beta1 0.9, beta2 0.999, eps 1e-8) on a mini-batch */
+/* one Adam step (lr, beta1 0.9, beta2 0.999, eps 1e-8) on a mini-batch.  A step whose kernel
+ * ran into its wait limit leaves the parameters as they are; it returns CCT_CUDAERR if it
+ * waits for the loss, else the next call does */
 CCTStatusType mps_mlp_train_step(MpsMlp* m, int M, const float* X, const float* T, float w1, float lr,
                                  float* host_loss, void* stream);
 

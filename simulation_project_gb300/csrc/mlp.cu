@@ -1031,8 +1031,9 @@ __global__ void __launch_bounds__(TcShape<NS>::Threads, 1) k_mlp_infer_tc(int M,
 // wait), 52 us from 512 to 16,384 rows, 57 us at 19,456.  Bound by the latency of its chain
 // of stages (eight MMA stages with SiLU or its derivative between them), 64 CTAs at 8,192
 // rows.
-// Every wait is bounded; when one runs out the CTA flags it, waits (bounded) for its MMAs
-// and leaves its gradients out.
+// Every wait is bounded (g_mlp_tc_wait_spins polls); when one runs out the CTA sets *failed,
+// waits (bounded) for its MMAs and stops.  Loss and gradients are then
+// incomplete: Adam leaves the parameters as they are and the host returns an error.
 // ---------------------------------------------------------------------------
 constexpr int kTrRows = 128, kTrThreads = 512;
 constexpr int kTrWide = kTrRows * H * 2;       // bytes of a [128][128] BF16 tile
@@ -1070,10 +1071,10 @@ __device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
     return v[0];
 }
 
-// g: MPS_MLP_PARAMS floats, 16-byte aligned, zero on entry, as is *loss
+// g: MPS_MLP_PARAMS floats, 16-byte aligned, zero on entry, as are *loss and *failed
 __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(int M, const float* __restrict__ X, const float* __restrict__ T,
                                                              float w1, Layers L, float* __restrict__ g,
-                                                             double* __restrict__ loss) {
+                                                             double* __restrict__ loss, unsigned* failed_word) {
     extern __shared__ unsigned char tr_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((uintptr_t)tr_raw + 1023) & ~(uintptr_t)1023);
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(sm + kTrBar);
@@ -1120,6 +1121,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(int M, const float*
     constexpr int o1 = FIN * H, o2 = o1 + H, o3 = o2 + H * H, o4 = o3 + H, o5 = o4 + H * H, o6 = o5 + H, o7 = o6 + H * FOUT;
     const unsigned sa = tc_smem(sm);
     const unsigned wide = tc_idesc(128, 128), narrow = tc_idesc(128, 16);
+    const long long spins = g_mlp_tc_wait_spins;
     unsigned parity = 0u;
     bool failed = false;
     // what every thread wrote to shared memory and read from TMEM comes before the next
@@ -1131,9 +1133,12 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(int M, const float*
     };
     // the stage's MMAs are done (false: the wait ran out, for all threads alike)
     auto done = [&]() {
-        const bool ok = tc_bar_wait(bar, parity, 1ll << 22);
+        const bool ok = tc_bar_wait(bar, parity, spins);
         if (__syncthreads_or(!ok)) {
-            if (tid == 0) atomicOr(&g_mlp_tc_timeout, 1u);
+            if (tid == 0) {
+                atomicOr(&g_mlp_tc_timeout, 1u);
+                atomicOr(failed_word, 1u);
+            }
             tc_bar_wait(bar, parity, 1ll << 24);
             failed = true;
             return false;
@@ -1295,9 +1300,14 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(int M, const float*
     }
 }
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1t, float b2t) {
+                       float* __restrict__ v, float lr, float b1t, float b2t, const unsigned* __restrict__ failed,
+                       volatile unsigned* skipped) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (*failed) {   // the gradient is incomplete: no step, and the host counts it
+        if (i == 0) *skipped = *skipped + 1u;
+        return;
+    }
     const float gi = g[i];
     const float mi = 0.9f * m[i] + 0.1f * gi;
     const float vi = 0.999f * v[i] + 0.001f * gi * gi;
@@ -1316,9 +1326,13 @@ struct MpsMlp {
     int nparams = MPS_MLP_PARAMS;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     Layers L{};
+    // loss and, in the low word of the second, whether a wait of the pass ran out; their host
+    // copies, and in the third the number of steps that were not taken for it
     double* loss = nullptr;
     double* h_loss = nullptr;
     int t = 0;
+    unsigned* failed() const { return reinterpret_cast<unsigned*>(loss + 1); }
+    volatile unsigned* skipped() const { return reinterpret_cast<volatile unsigned*>(h_loss + 2); }
     std::vector<void*> allocs;
 
     template <class T>
@@ -1335,9 +1349,10 @@ struct MpsMlp {
         e = e ? e : mk(&L.W4, H * FOUTP);
         e = e ? e : mk(&L.b1, H); e = e ? e : mk(&L.b2, H); e = e ? e : mk(&L.b3, H); e = e ? e : mk(&L.b4, FOUTP);
         e = e ? e : mk(&L.tc, (size_t)kTcImage);
-        e = e ? e : mk(&loss, 1);
+        e = e ? e : mk(&loss, 2);
         if (e) return e;
-        if ((e = cudaMallocHost((void**)&h_loss, sizeof(double)))) return e;
+        if ((e = cudaMallocHost((void**)&h_loss, 3 * sizeof(double)))) return e;
+        *skipped() = 0u;
         cudaMemset(m, 0, sizeof(float) * nparams);
         cudaMemset(v, 0, sizeof(float) * nparams);
         return cudaDeviceSynchronize();
@@ -1367,11 +1382,26 @@ struct MpsMlp {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if ((e = cudaMemsetAsync(out, 0, sizeof(float) * MPS_MLP_PARAMS, st))) return e;
-        if ((e = cudaMemsetAsync(loss, 0, sizeof(double), st))) return e;
+        if ((e = cudaMemsetAsync(loss, 0, 2 * sizeof(double), st))) return e;
         MPS_COUNT_LAUNCH k_mlp_train<<<std::max(1, std::min(div_up(M, kTrRows), sms)), kTrThreads, kTrSmem, st>>>(
-            M, X, T, w1, L, out, loss);
+            M, X, T, w1, L, out, loss, failed());
         return cudaGetLastError();
     }
+    // the pass's loss to the host, with a wait
+    cudaError_t pull_loss(cudaStream_t st) {
+        cudaError_t e = cudaMemcpyAsync(h_loss, loss, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
+        return e ? e : cudaStreamSynchronize(st);
+    }
+    // steps that were not taken, unsaid so far: out of the count of Adam's steps
+    bool ran_out() {
+        const unsigned k = *skipped();
+        if (!k) return false;
+        t -= (int)k;
+        *skipped() = 0u;
+        note_message(kRanOut);
+        return true;
+    }
+    static constexpr const char* kRanOut = "mlp training: a wait for the tensor cores ran out, the pass is incomplete";
 };
 
 namespace mps {
@@ -1498,6 +1528,7 @@ CCTStatusType mps_mlp_set_params(MpsMlp* m, const float* host_params) {
     if (!e) e = m->sync_layers(0);
     if (!e) e = cudaDeviceSynchronize();
     m->t = 0;
+    *m->skipped() = 0u;
     cudaMemset(m->m, 0, sizeof(float) * MPS_MLP_PARAMS);
     cudaMemset(m->v, 0, sizeof(float) * MPS_MLP_PARAMS);
     return cuda_status(e);
@@ -1551,11 +1582,11 @@ CCTStatusType mps_mlp_loss_grad(MpsMlp* m, int M, const float* X, const float* T
         note_error(what, e);
         return CCT_CUDAERR;
     }
-    if ((e = cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st))) {
-        note_error("loss copy", e);
+    if ((e = m->pull_loss(st))) { note_error("mps_mlp_loss_grad: loss copy", e); return CCT_CUDAERR; }
+    if (*reinterpret_cast<const unsigned*>(m->h_loss + 1)) {
+        note_message(MpsMlp::kRanOut);
         return CCT_CUDAERR;
     }
-    if ((e = cudaStreamSynchronize(st))) { note_error("mps_mlp_loss_grad sync", e); return CCT_CUDAERR; }
     if (host_loss) *host_loss = (float)(*m->h_loss / M);
     return CCT_NOERR;
 }
@@ -1564,15 +1595,17 @@ CCTStatusType mps_mlp_train_step(MpsMlp* m, int M, const float* X, const float* 
                                  float* host_loss, void* stream) {
     if (!m || M <= 0 || M > m->maxb) return CCT_PARAMERR;
     cudaStream_t st = (cudaStream_t)stream;
+    if (m->ran_out()) return CCT_CUDAERR;   // an earlier step that did not wait for its loss
     cudaError_t e = m->loss_grad(M, X, T, w1, m->g, st);
     if (e) return cuda_status(e);
     m->t += 1;
     const float b1t = powf(0.9f, (float)m->t), b2t = powf(0.999f, (float)m->t);
-    MPS_COUNT_LAUNCH k_adam<<<div_up(MPS_MLP_PARAMS, 256), 256, 0, st>>>(MPS_MLP_PARAMS, m->p, m->g, m->m, m->v, lr, b1t, b2t);
+    MPS_COUNT_LAUNCH k_adam<<<div_up(MPS_MLP_PARAMS, 256), 256, 0, st>>>(MPS_MLP_PARAMS, m->p, m->g, m->m, m->v, lr, b1t, b2t,
+                                                                        m->failed(), m->skipped());
     e = m->sync_layers(st);
     if (!e && host_loss) {
-        e = cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st);
-        if (!e) e = cudaStreamSynchronize(st);
+        e = m->pull_loss(st);
+        if (!e && m->ran_out()) return CCT_CUDAERR;
         if (!e) *host_loss = (float)(*m->h_loss / M);
     }
     return cuda_status(e ? e : cudaGetLastError());
