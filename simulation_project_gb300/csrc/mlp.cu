@@ -25,6 +25,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "mps_common.cuh"
@@ -33,6 +35,22 @@
 #include "../../include/mps_solver.h"
 
 namespace mps {
+
+// A kernel's dynamic shared memory above 48 KB: an attribute of the function on each device,
+// set on a device's first launch, by any thread.
+struct SmemOptIn {
+    std::atomic<unsigned long long> devices{0};
+    template <class K>
+    cudaError_t operator()(K kernel, int bytes) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+        if (e || (devices.load(std::memory_order_acquire) & bit)) return e;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (!e) devices.fetch_or(bit, std::memory_order_release);
+        return e;
+    }
+};
 
 typedef __nv_bfloat16 bf16;
 constexpr int GT_M = 64, GT_N = 64, GT_K = 32, GT_PAD = 8;
@@ -687,12 +705,8 @@ __global__ void __launch_bounds__(kGtThreads) k_gemm_tc(int M, int N, int K, con
 cudaError_t gemm(int M, int N, int K, const bf16* A, int lda, int ta, const bf16* B, int ldb, int tb, float* C, int ldc,
                  bf16* Cb, int ldcb, float* Cz, const float* bias, int act, float beta, int split, cudaStream_t st) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
-    static bool smem_set = false;
-    if (!smem_set) {
-        const cudaError_t e = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtSmem);
-        if (e) return e;
-        smem_set = true;
-    }
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(k_gemm_tc, (int)kGtSmem)) return e;
     split = max(1, split);
     int kchunk = (K + split - 1) / split;
     kchunk = (kchunk + kGtBK - 1) / kGtBK * kGtBK;
@@ -1372,12 +1386,9 @@ struct MpsMlp {
     // loss (h_loss after a copy) and gradients (out: MPS_MLP_PARAMS floats, 16-byte aligned)
     // of M rows
     cudaError_t loss_grad(int M, const float* X, const float* T, float w1, float* out, cudaStream_t st) {
-        static bool set = false;   // the attribute is per function, set once
-        cudaError_t e = cudaSuccess;
-        if (!set) {
-            if ((e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrSmem))) return e;
-            set = true;
-        }
+        static SmemOptIn opt_in;
+        cudaError_t e = opt_in(k_mlp_train, (int)kTrSmem);
+        if (e) return e;
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1408,14 +1419,8 @@ namespace mps {
 // the tcgen05 inference kernel with POLY's columns on the FMA pipe
 template <int POLY>
 cudaError_t mlp_forward_tc(MpsMlp* m, int M, const float* X, float* Y, cudaStream_t st, unsigned* err, int sms) {
-    static bool tc_set = false;   // the attribute is per function, set once
-    if (!tc_set) {
-        const cudaError_t e = cudaFuncSetAttribute(k_mlp_infer_tc<kTcSlots, POLY>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)TcShape<kTcSlots>::Smem);
-        if (e) return e;
-        tc_set = true;
-    }
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(k_mlp_infer_tc<kTcSlots, POLY>, (int)TcShape<kTcSlots>::Smem)) return e;
     const int tiles = (M + kTcRows - 1) / kTcRows;
     const int grid = std::max(1, std::min(div_up(tiles, kTcSlots), std::max(sms, 1)));   // one CTA per SM
     MPS_COUNT_LAUNCH k_mlp_infer_tc<kTcSlots, POLY>
@@ -1433,7 +1438,7 @@ constexpr int kTcPolyDefault = 0x8;
 cudaError_t mlp_forward_variant(MpsMlp* m, int M, const float* X, float* Y, cudaStream_t st, int variant,
                                 unsigned* err) {
     if (M <= 0) return cudaSuccess;
-    static bool smem_set = false;   // the attribute is per function, set once
+    static SmemOptIn opt_in;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1445,11 +1450,7 @@ cudaError_t mlp_forward_variant(MpsMlp* m, int M, const float* X, float* Y, cuda
         case 5: return mlp_forward_tc<0xE>(m, M, X, Y, st, err, sms);
         default: break;
     }
-    if (!smem_set) {
-        const cudaError_t e = cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMiSmem);
-        if (e) return e;
-        smem_set = true;
-    }
+    if (const cudaError_t e = opt_in(k_mlp_infer, (int)kMiSmem)) return e;
     const int tiles = (M + 15) / 16;
     const int grid = std::max(1, std::min(div_up(tiles, kMiWarps), 2 * std::max(sms, 1)));
     MPS_COUNT_LAUNCH k_mlp_infer<<<grid, kMiWarps * 32, kMiSmem, st>>>(M, X, Y, m->L);
