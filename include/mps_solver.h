@@ -203,6 +203,12 @@ CCTStatusType mps_solver_debug_history(MpsSolver* s, float* dph1, float* dph2, u
  * triangle order (the 27-cell candidate set of the cell; CCell lists of
  * RegisterTriangleTopology, Utility_Inline.h:1745-1855, in the reference). */
 CCTStatusType mps_solver_debug_wall_bins(MpsSolver* s, int* bounds, int* tids, int cap, int* entries);
+/* The inner CG in one launch with the rows in shared memory: slices of 32 rows per CTA for
+ * so many rows, the longest of so many entries, on so many SMs, with 0 to 2 levels of the
+ * preconditioner and so many level-1 aggregates (0: they do not fit, or a row's columns
+ * could need 32 bits; no GPU needed), and what the last solve ran with (0: the kernel chain). */
+int mps_debug_cg_small_slices(int rows, int longest_row, int sms, int levels, int aggregates);
+CCTStatusType mps_solver_debug_cg_small(MpsSolver* s, int* slices);
 /* refinement residual r = b - A p of the current state (FP32_IR solvers; host
  * array of n doubles, may be NULL) and ||r|| / ||b||: variant 0 with FP64
  * products and sums, variant 1 with the double-float kernel the solver uses (rows

@@ -17,8 +17,10 @@
 // Every CTA adds the CTAs' partial sums in the same order, so all hold the same scalars.
 // us, kernel chain -> here: an iteration 29 -> 13 (one coarse level), a step of 2,000 particles
 // 1,122 -> 853, of 9,248 (two levels) 1,542 -> 1,219, the Poisson solve of 8,000 particles
-// 901 -> 808, of 17,576 1,138 -> 988; then it stops fitting, so there is no size at which the
-// chain is the better one.  What bounds it: the three barriers with
+// 901 -> 808, of 17,576 1,138 -> 988; then it stops fitting (cg_small_slices_for: with rows of
+// 256 entries 24,320 rows for Jacobi or one coarse level, 19,456 with two levels of up to 368
+// aggregates; with rows of 240 entries 29,184), so there is no size at which the chain is the
+// better one.  What bounds it: the three barriers with
 // the partial sums behind them, 2 us each, and one round of gathers from L2.
 // The arithmetic per entry and row is the kernel chain's (k_spmv_ring_split, k_cg_update or
 // k_mg_update_restrict and k_mg_fine_z, k_cg_p); sums over rows are taken per warp in FP32 and
@@ -47,6 +49,15 @@ struct CgSmall {
 inline size_t cg_small_smem(int K, int spc, int levels, int n1) {
     return (size_t)spc * K * 128 + (size_t)spc * 32 * (5 + kCgThreads / 32) * 4 +
            (levels ? (size_t)((n1 + 7) & ~7) * (levels > 1 ? 4 * 4 + 4 + 27 * 6 : 3 * 4) : 0);
+}
+
+constexpr size_t kCgSmem = 200 * 1024;   // shared memory that the rows can take, beside 25 KB of static arrays
+// Slices per CTA for n rows with room for `row` entries each on `sms` SMs, 0: they do not fit.
+// A slice with 32-bit columns would be read as empty: with at most 32,768 rows there is none.
+inline int cg_small_slices_for(int n, int row, int sms, int levels, int n1) {
+    if (n <= 0 || n > 32768 || sms <= 0 || levels > 2 || (levels > 0 && n1 > kCgAgg)) return 0;
+    const int spc = div_up(div_up(n, 32), sms);
+    return spc <= kCgMaxSlices && cg_small_smem(row, spc, levels, n1) <= kCgSmem ? spc : 0;
 }
 
 // The CTAs' partial sums `part` added in order by warp 0; valid in every thread.  SLOT: place

@@ -1507,10 +1507,11 @@ struct Solver {
 
     // ---- the inner CG in one launch (k_cg_small) ----
     // The rows have to fit in the shared memory of the SMs (a CTA on each), and beside them the
-    // preconditioner's level 1, which has to be the last level or the one above it.
+    // preconditioner's level 1, which has to be the last level or the one above it
+    // (cg_small_slices_for).
     CgSmall cgs{};
     int cg_sms = -1;
-    static constexpr size_t kCgSmem = 200 * 1024;   // beside 25 KB of static arrays
+    int cg_last = 0;   // slices per CTA of the last solve's k_cg_small, 0: the kernel chain
     // entries of the longest row (k_count_nnz), in whole chunks
     int cg_row_room() const { return std::min(d.K, ((int)h_scal[S_MAXROW] + 15) & ~15); }
     size_t cg_smem(int spc) const { return cg_small_smem(cg_row_room(), spc, mg_ready ? mg.levels : 0, mg_ready ? mg.L[1].n : 0); }
@@ -1524,10 +1525,8 @@ struct Solver {
                 cudaFuncSetAttribute(k_cg_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmem) != cudaSuccess)
                 cg_sms = 0;
         }
-        if (cg_sms <= 0 || !inner16() || prefer_wide || timer.on || (mg_ready && (mg.levels > 2 || mg.L[1].n > kCgAgg || fine_post() || opt.mg_sweeps > 1)))
-            return 0;
-        const int nsl = div_up(d.n, 32), spc = div_up(nsl, cg_sms);
-        return spc >= 1 && spc <= kCgMaxSlices && cg_smem(spc) <= kCgSmem ? spc : 0;
+        if (!inner16() || prefer_wide || timer.on || (mg_ready && (fine_post() || opt.mg_sweeps > 1))) return 0;
+        return cg_small_slices_for(d.n, cg_row_room(), cg_sms, mg_ready ? mg.levels : 0, mg_ready ? mg.L[1].n : 0);
     }
     // A d = r / rn of one refinement pass to tol: d in d32.  Nothing is read back: the count of
     // iterations (S_ITER, -1 on failure) comes with the next residual's norms.  Returns 1, 0 if
@@ -1597,6 +1596,7 @@ struct Solver {
             const int pi = outer < kPassMemory ? outer : kPassMemory - 1;
             const int spc = cg_small_slices(), small = spc > 0 ? cg_small(spc, rn, inner_tol) : 0;
             if (small < 0) return CCT_CUDAERR;
+            cg_last = small > 0 ? spc : 0;
             if (small > 0) {
                 small_pass = pi;
             } else {
@@ -2001,6 +2001,16 @@ CCTStatusType mps_solver_debug_wall_bins(MpsSolver* s, int* bounds, int* tids, i
         if (cap < nv) return CCT_PARAMERR;
         if (cudaMemcpy(tids, d.tids, sizeof(int) * (size_t)nv, cudaMemcpyDeviceToHost)) return CCT_CUDAERR;
     }
+    return CCT_NOERR;
+}
+
+int mps_debug_cg_small_slices(int rows, int longest_row, int sms, int levels, int aggregates) {
+    return mps::cg_small_slices_for(rows, (longest_row + 15) & ~15, sms, levels, aggregates);
+}
+
+CCTStatusType mps_solver_debug_cg_small(MpsSolver* s, int* slices) {
+    if (!s || !slices) return CCT_PARAMERR;
+    *slices = s->s.cg_last;
     return CCT_NOERR;
 }
 

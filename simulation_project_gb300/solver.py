@@ -66,6 +66,8 @@ _SIGS = {
     "mps_solver_get_particles": (C.c_int, [P, C.POINTER(C.c_int), P, P, P, P, P]),
     "mps_solver_get_triangles": (C.c_int, [P, P]),
     "mps_solver_debug_residual": (C.c_int, [P, C.c_int, P, C.POINTER(C.c_double)]),
+    "mps_debug_cg_small_slices": (C.c_int, [C.c_int] * 5),
+    "mps_solver_debug_cg_small": (C.c_int, [P, C.POINTER(C.c_int)]),
     "mps_solver_debug_ppe": (C.c_int, [P, P, P, P, P, P, P, P]),
     "mps_solver_debug_history": (C.c_int, [P, P, P, P, P, P]),
     "mps_solver_debug_spmv": (C.c_int, [P, C.c_int, P, P]),
@@ -201,6 +203,12 @@ class Solver:
         out["id"] = ids[:n]
         out["nbr_count"] = cnt[:n]
         return out
+
+    def debug_cg_small(self) -> int:
+        """Slices per CTA of the last solve's inner CG in one launch (0: the kernel chain)."""
+        k = C.c_int()
+        _check(_lib().mps_solver_debug_cg_small(self.h, C.byref(k)), "mps_solver_debug_cg_small")
+        return k.value
 
     def debug_history(self) -> dict:
         """Warm-start pressure history in solver order: dph1 = P_n - P_{n-1}, dph2 =
