@@ -737,7 +737,9 @@ struct Solver {
         return cuda_status(cudaGetLastError());
     }
 
-    int correct_share() const { return d.n < 20000 ? 4 : d.n < 200000 ? 16 : 32; }
+    // particles per warp of the correction (us, 4 / 16 / 32: 2,000 particles 17 / 32 / 48, 12,635
+    // 25 / 26 / 40, 20,496 34 / 30 / 40, 40,121 44 / 34 / 45, 108,186 83 / 60 / 52, 194,376 127 / 80 / 60)
+    int correct_share() const { return d.n < 20000 ? 4 : d.n < 80000 ? 16 : 32; }
 
     CCTStatusType grid() {
         const int n = d.n;

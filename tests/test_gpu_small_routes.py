@@ -1,7 +1,8 @@
 """Which kernel the inner CG of a small system runs on, and that kernel at the sizes it then
 has: k_cg_small with one to six slices per CTA and at the size at which the chain takes over,
 each against the chain (a profiling solver), and the chain's k_spmv_ring_split on fewer rows
-than a slice and on ragged last slices, which a default solver no longer gives it."""
+than a slice and on ragged last slices, which a default solver no longer gives it; and the
+size at which a warp of the correction takes 32 particles."""
 import numpy as np
 import pytest
 
@@ -57,3 +58,16 @@ def test_small_systems_on_the_chain(shape, njp):
         passes.append(st["ir_passes"])
         s.close()
     assert passes[0] <= passes[1] + 2
+
+
+@pytest.mark.parametrize("side", [43, 44])
+def test_correction_shares(side):
+    """16 and 32 particles per warp of the correction: the velocities of a step against the
+    FP64 solver's, to the FP32 operators' accuracy over one step."""
+    out = []
+    for precision in ("fp32_ir", "fp64"):
+        s = Solver(_block((side,) * 3), precision=precision)
+        assert s.step(0)["error_flags"] == 0
+        out.append(s.state()["vel"])
+        s.close()
+    assert np.abs(out[0] - out[1]).max() <= 2e-3 * np.abs(out[1]).max()
