@@ -998,8 +998,8 @@ struct RefOp<RpGradient> {
 };
 
 // Two launches share a large call: one of k_ref_pairs and k_ref_slices takes it in dense fluid,
-// k_ref_walk after it in sparse fluid, and the other one of the two has nothing to do
-// (rp_sparse).  k_ref_walk may start once every CTA of the first has (programmatic dependent
+// k_ref_walk_sparse after it in sparse fluid, and the other one of the two has nothing to do
+// (rp_sparse).  k_ref_walk_sparse may start once every CTA of the first has (programmatic dependent
 // launch: neither reads what the other writes), and every thread of it ends after the
 // first launch has, so what follows in the stream follows both.
 __device__ __forceinline__ void ref_beside_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -1034,22 +1034,31 @@ __global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::
     if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
-// a lane per target: those that the kernels beside it leave (sparse > 0), or all
+// a lane per target
 template <class Op>
-__global__ void __launch_bounds__(128) k_ref_walk(int n, float coef, int sparse, const __grid_constant__ RefBind b) {
+__device__ __forceinline__ void ref_walk(const RefBind& b, int id, float coef, int2* run) {
+    RpTarget t{};
+    int cx = 0, cy = 0, cz = 0;
+    bool walk = false;
+    t.pos = b.pos[id];
+    if (!RefOp<Op>::begin(b, id, t, cx, cy, cz, walk)) return;
+    float sum[Op::NS], rare[RpShape<Op>::NXR];
+    rp_walk_sums<Op>(b, t, id, walk, cx, cy, cz, RefOp<Op>::radius(b.param), run, 128, sum, rare);
+    RefOp<Op>::finish(b, id, t, sum, rare, coef);
+}
+template <class Op>
+__global__ void __launch_bounds__(128) k_ref_walk(int n, float coef, const __grid_constant__ RefBind b) {
     __shared__ int2 run[9][128];
     const int id = blockIdx.x * 128 + threadIdx.x;
-    if ((sparse <= 0 || rp_sparse(b, n, sparse)) && id < n) {
-        RpTarget t{};
-        int cx = 0, cy = 0, cz = 0;
-        bool walk = false;
-        t.pos = b.pos[id];
-        if (RefOp<Op>::begin(b, id, t, cx, cy, cz, walk)) {
-            float sum[Op::NS], rare[RpShape<Op>::NXR];
-            rp_walk_sums<Op>(b, t, id, walk, cx, cy, cz, RefOp<Op>::radius(b.param), &run[0][threadIdx.x], 128, sum, rare);
-            RefOp<Op>::finish(b, id, t, sum, rare, coef);
-        }
-    }
+    if (id < n) ref_walk<Op>(b, id, coef, &run[0][threadIdx.x]);
+}
+// ... if the kernel beside it leaves them
+template <class Op>
+__global__ void __launch_bounds__(128) k_ref_walk_sparse(int n, float coef, int sparse, const __grid_constant__ RefBind b) {
+    __shared__ int2 run[9][128];
+    if (rp_sparse(b, n, sparse))
+        for (int id = blockIdx.x * 128 + threadIdx.x; id < n; id += gridDim.x * 128)
+            ref_walk<Op>(b, id, coef, &run[0][threadIdx.x]);
     ref_beside_end();
 }
 
@@ -1064,7 +1073,7 @@ __global__ void __launch_bounds__(rs_warps<Op>() * 32) k_ref_slices(int n, float
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = (blockIdx.x * rs_warps<Op>() + warp) * 32;
     ref_beside_start();
-    if (rp_sparse(b, n, sparse) || first >= n) return;
+    if ((sparse > 0 && rp_sparse(b, n, sparse)) || first >= n) return;
     const int id = first + lane;
     RpTarget t{};
     int cx = 0, cy = 0, cz = 0;
@@ -1114,19 +1123,19 @@ int rp_few(int n, bool slices, bool pairs2) {
     return std::is_same<Op, RpExplicitly>::value && n >= 64000 ? 16 : 10;
 }
 
-// all targets (sparse 0), or beside the launch before it
+// beside the launch before it; one wave of CTAs, which mostly find that there is nothing to do
 template <class Op>
-cudaError_t ref_walk_launch(cudaStream_t st, int n, float coef, int sparse) {
+cudaError_t ref_walk_beside(cudaStream_t st, int n, float coef, int sparse) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)div_up(n, 128));
+    cfg.gridDim = dim3((unsigned)std::min(div_up(n, 128), 152 * 16));
     cfg.blockDim = dim3(128);
     cfg.stream = st;
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = sparse > 0 ? 1 : 0;
-    return MPS_COUNT_LAUNCH cudaLaunchKernelEx(&cfg, k_ref_walk<Op>, n, coef, sparse, (const RefBind)g_bind);
+    cfg.numAttrs = 1;
+    return MPS_COUNT_LAUNCH cudaLaunchKernelEx(&cfg, k_ref_walk_sparse<Op>, n, coef, sparse, (const RefBind)g_bind);
 }
 
 // Targets per warp of an operator: kMany share each round's candidates; below `few` of
@@ -1137,7 +1146,9 @@ template <class Op, int kMany>
 cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
     constexpr bool kSlices = std::is_same<Op, RpPressure>::value || std::is_same<Op, RpGradient>::value ||
                              std::is_same<Op, RpTemperature>::value;
-    const int sparse = n < kRefSplit ? 0 : rp_few<Op>(n, kSlices && n >= kRefSlices, n < few);
+    // 0: not asked, since the call is small or all cells of the grid hold that many on average
+    int sparse = n < kRefSplit ? 0 : rp_few<Op>(n, kSlices && n >= kRefSlices, n < few);
+    if ((long long)n >= (long long)sparse * g_bind.cell_num) sparse = 0;
     if (n < few) {
         MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse, g_bind);
     } else if (kSlices && n >= kRefSlices) {
@@ -1150,7 +1161,7 @@ cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
                                                                                                         g_bind);
     }
     const cudaError_t e = cudaGetLastError();
-    return e || sparse == 0 ? e : ref_walk_launch<Op>(st, n, coef, sparse);
+    return e || sparse == 0 ? e : ref_walk_beside<Op>(st, n, coef, sparse);
 }
 // Below it a triangle is walked by 32 lanes (few triangles are large ones), else by 8.
 constexpr int kTriFew = 2048;
@@ -1455,7 +1466,7 @@ CCTStatusType CalcExplicitly(cudaStream_t& Stream, Integer ParticleNum) {
     const CParameter& P = g_bind.param;
     const float coef = (float)((2.0 * P.Dimension) / (double)(P.LambdaValue * P.ConstantParticleDensity));
     if (ParticleNum >= kRefLanes)
-        MPS_CUDA_TRY(ref_walk_launch<RpExplicitly>(Stream, ParticleNum, coef, 0));
+        MPS_COUNT_LAUNCH k_ref_walk<RpExplicitly><<<div_up(ParticleNum, 128), 128, 0, Stream>>>(ParticleNum, coef, g_bind);
     else
         MPS_CUDA_TRY((ref_op_launch<RpExplicitly, 8>(Stream, ParticleNum, kRefFew, coef)));
     return launch_status();

@@ -270,12 +270,13 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
             if (!coop_barrier(s.bar, err, bit)) return;
             // ---- prefix over the CTAs, a warp per digit, a run of CTAs per lane ----
             constexpr int kRun = (kRadixMaxCtas + 31) / 32;
+            const int each = (ctas + 31) / 32;
             for (int d = w * ctas + c; d < kRadix; d += ctas * kSortWarps) {   // spread over the SMs
                 unsigned x[kRun], sum = 0;
 #pragma unroll
                 for (int q = 0; q < kRun; ++q) {
-                    const int k = lane * kRun + q;
-                    x[q] = k < ctas ? __ldcg(s.counts + (size_t)k * kRadix + d) : 0u;
+                    const int k = lane * each + q;
+                    x[q] = q < each && k < ctas ? __ldcg(s.counts + (size_t)k * kRadix + d) : 0u;
                 }
 #pragma unroll
                 for (int q = 0; q < kRun; ++q) sum += x[q];
@@ -288,8 +289,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                 unsigned run = inc - sum;
 #pragma unroll
                 for (int q = 0; q < kRun; ++q) {
-                    const int k = lane * kRun + q;
-                    if (k < ctas) s.counts[(size_t)k * kRadix + d] = run;
+                    const int k = lane * each + q;
+                    if (q < each && k < ctas) s.counts[(size_t)k * kRadix + d] = run;
                     run += x[q];
                 }
                 if (lane == 31) s.total[d] = inc;
