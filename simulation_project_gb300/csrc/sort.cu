@@ -32,6 +32,8 @@
 // range alone took 27 us at 882,080 keys (19,456 atomics on one address).
 #include <limits.h>
 
+#include <type_traits>
+
 #include "mps_common.cuh"
 #include "mps_internal.h"
 
@@ -269,32 +271,36 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
             s.counts[(size_t)c * kRadix + tid] = mine;
             if (!coop_barrier(s.bar, err, bit)) return;
             // ---- prefix over the CTAs, a warp per digit, a run of CTAs per lane ----
-            constexpr int kRun = (kRadixMaxCtas + 31) / 32;
-            const int each = (ctas + 31) / 32;
-            for (int d = w * ctas + c; d < kRadix; d += ctas * kSortWarps) {   // spread over the SMs
-                unsigned x[kRun], sum = 0;
+            auto prefix = [&](auto run_of) {
+                constexpr int kRun = run_of.value;
+                for (int d = w * ctas + c; d < kRadix; d += ctas * kSortWarps) {   // spread over the SMs
+                    unsigned x[kRun], sum = 0;
 #pragma unroll
-                for (int q = 0; q < kRun; ++q) {
-                    const int k = lane * each + q;
-                    x[q] = q < each && k < ctas ? __ldcg(s.counts + (size_t)k * kRadix + d) : 0u;
+                    for (int q = 0; q < kRun; ++q) {
+                        const int k = lane * kRun + q;
+                        x[q] = k < ctas ? __ldcg(s.counts + (size_t)k * kRadix + d) : 0u;
+                    }
+#pragma unroll
+                    for (int q = 0; q < kRun; ++q) sum += x[q];
+                    unsigned inc = sum;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+                        if (lane >= o) inc += v;
+                    }
+                    unsigned run = inc - sum;
+#pragma unroll
+                    for (int q = 0; q < kRun; ++q) {
+                        const int k = lane * kRun + q;
+                        if (k < ctas) s.counts[(size_t)k * kRadix + d] = run;
+                        run += x[q];
+                    }
+                    if (lane == 31) s.total[d] = inc;
                 }
-#pragma unroll
-                for (int q = 0; q < kRun; ++q) sum += x[q];
-                unsigned inc = sum;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
-                }
-                unsigned run = inc - sum;
-#pragma unroll
-                for (int q = 0; q < kRun; ++q) {
-                    const int k = lane * each + q;
-                    if (q < each && k < ctas) s.counts[(size_t)k * kRadix + d] = run;
-                    run += x[q];
-                }
-                if (lane == 31) s.total[d] = inc;
-            }
+            };
+            constexpr int kHalf = (kRadixMaxCtas / 2 + 31) / 32;
+            if (ctas <= kRadixMaxCtas / 2) prefix(std::integral_constant<int, kHalf>());
+            else prefix(std::integral_constant<int, 2 * kHalf>());
             if (!coop_barrier(s.bar, err, bit)) return;
         }
         // ---- first position of each digit's keys of this CTA ----
