@@ -890,7 +890,9 @@ struct Solver {
 
     // below it the warps of a CTA share the triangle lists of 32 particles (us, a warp per 32
     // / kTriWarps: drag 113 / 65, walls 34 / 22 at 108,186 particles, 141 / 76 and 31 / 32 at 256,000,
-    // 86 / 110 and 36 / 85 at 882,080: there are warps enough and most CTAs find no triangles)
+    // 86 / 110 and 36 / 85 at 882,080: there are warps enough and most CTAs find no triangles;
+    // all wall work of a step with 64 drag bodies 205 / 186 at 255,976, 208 / 214 at 361,444, 192 / 241
+    // at 513,279; without drag 113 / 102 at 194,376, 103 / 105 at 255,976, 110 / 127 at 361,444)
     static constexpr int kTriSplit = 300000;
     template <class T, int W>
     void launch_tri(bool drag) {
@@ -1235,7 +1237,10 @@ struct Solver {
             MPS_COUNT_LAUNCH k<<<spmv16_grid, kSsWarps * 32, kS16Smem, st>>>(d, d.w16, x, y, nullptr, 0);
         }
     }
-    // the same for systems with few slices per warp (k_spmv_ring_split)
+    // the same for systems with few slices per warp (k_spmv_ring_split, which has its times on
+    // both sides of the line; vectors and residuals of a step, us, shared / whole slices: 663 / 704
+    // at 108,186 particles, 967 / 987 at 255,976, 1,311 / 1,320 at 453,356, 1,512 / 1,521 at 581,376,
+    // 2,017 / 1,911 at 882,080)
     static constexpr int kSplitRows = 400000, kSplit = 4;
     // below it three warps share a slice of the predictor (k_predict<3> / <1>, us: 22.8 / 34.6
     // at 2,000 particles, 35 / 49 at 12,635, 53 / 55 at 29,500, 108 / 77 at 53,000)
