@@ -317,8 +317,10 @@ inline size_t nb_list_smem(int L) {
 // 296, 31 KB with 384; sixteen or fourteen warps per SM).  112 registers, 8 candidates and 4
 // entries at a time: 16 and 8 of them spilled (1620 us instead of 1360 at 882,080 particles).
 // Bit 4 of flags, a row longer than L or a run too long for the codes: the candidates are walked
-// twice by one warp, once for the rows' lengths and ends and once for the entries, with no
-// list; same rows and sums, bit for bit.
+// twice by one warp, once for the rows' lengths and ends and once for the entries, 32 at a time
+// culled against the box around the targets, with no list; same rows and sums, bit for bit (cells
+// three times the radius, 216,000 particles: 5.7 ms with a warp per target, 24 without the cull,
+// 3.8 now).
 __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags, int L) {
     extern __shared__ __align__(16) unsigned char nb_sm[];
     unsigned short* const list = (unsigned short*)nb_sm;
@@ -422,11 +424,19 @@ __global__ void __maxnreg__(112) k_list(const __grid_constant__ Dev d, int flags
             todo &= ~s.mem;
             const bool in = s.mem >> lane & 1u;
             for (int r = 0; r < 9; ++r) {
-                const int len = __shfl_sync(~0u, s.rl, r), start = __shfl_sync(~0u, s.rs, r);
-                for (int j = start; j < start + len; ++j) {
-                    const float4 q = d.opos[j];
-                    const float d2 = dist2_f32(__fsub_rn(q.x, p.x), __fsub_rn(q.y, p.y), __fsub_rn(q.z, p.z));
-                    if (in && j != i && d2 < re2s) f(j, d2);
+                const int start = __shfl_sync(~0u, s.rs, r), end = start + __shfl_sync(~0u, s.rl, r);
+                for (int b = start; b < end; b += 32) {   // 32 candidates, those in reach of the box
+                    const float4 c = d.opos[min(b + lane, end - 1)];
+                    const float dx = fmaxf(fmaxf(__fsub_rn(s.lo[0], c.x), __fsub_rn(c.x, s.hi[0])), 0.f),
+                                dy = fmaxf(fmaxf(__fsub_rn(s.lo[1], c.y), __fsub_rn(c.y, s.hi[1])), 0.f),
+                                dz = fmaxf(fmaxf(__fsub_rn(s.lo[2], c.z), __fsub_rn(c.z, s.hi[2])), 0.f);
+                    for (unsigned m = __ballot_sync(~0u, b + lane < end && dist2_f32(dx, dy, dz) < cut); m; m &= m - 1u) {
+                        const int u = __ffs(m) - 1;
+                        const float d2 = dist2_f32(__fsub_rn(__shfl_sync(~0u, c.x, u), p.x),
+                                                   __fsub_rn(__shfl_sync(~0u, c.y, u), p.y),
+                                                   __fsub_rn(__shfl_sync(~0u, c.z, u), p.z));
+                        if (in && b + u != i && d2 < re2s) f(b + u, d2);
+                    }
                 }
             }
         }
