@@ -46,21 +46,25 @@ cudaError_t scan_exclusive(unsigned* a, int len, unsigned* total_dev, cudaStream
 size_t scan_tile_sums_capacity();
 
 // library-owned scratch for the reference-named entry points, which take no scratch
-// argument (runtime.cu).  Grows on demand; one buffer per slot.
+// argument (runtime.cu).  Grows on demand; one buffer per slot, and no slot belongs to two
+// of the users below.
 void* scratch_get(int slot, size_t bytes);
-// A call's turn with that scratch: one host thread at a time, and on the GPU after the
+// A call's turn with its user's scratch: one host thread at a time, and on the GPU after the
 // work that the turn before queued on its own stream, so calls on several streams do not
 // overwrite each other's buffers.  Without a stream only the host threads take turns (the
-// call has waited for its own work by then).
+// call has waited for its own work by then).  A turn lasts through the call's host waits, so
+// each user has its own: a thread that sorts does not wait for one that bins triangles.
 class ScratchTurn {
 public:
-    ScratchTurn();
-    explicit ScratchTurn(cudaStream_t st);
+    enum User { kSort, kOutside, kTriangles, kUsers };
+    explicit ScratchTurn(User user);
+    ScratchTurn(User user, cudaStream_t st);
     ~ScratchTurn();
     ScratchTurn(const ScratchTurn&) = delete;
     ScratchTurn& operator=(const ScratchTurn&) = delete;
 
 private:
+    User user_;
     cudaStream_t st_ = nullptr;
     bool on_stream_ = false;
 };

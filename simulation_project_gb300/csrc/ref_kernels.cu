@@ -1294,20 +1294,24 @@ CCTStatusType reorderDataAndFindCellStart(cudaStream_t& Stream, Integer numParti
 }
 
 // tile sums of the multi-CTA scan (NULL when the slot cannot be had: one-CTA scan)
-static unsigned* scan_sums() { return (unsigned*)scratch_get(8, sizeof(unsigned) * scan_tile_sums_capacity()); }
+static unsigned* scan_sums(int slot) {
+    return (unsigned*)scratch_get(slot, sizeof(unsigned) * scan_tile_sums_capacity());
+}
 
-// Error words in host memory that the GPU can write: read without a copy once the stream
-// has been waited for.  NULL when they cannot be had.
-enum { kErrSort = 0, kErrTriangles, kErrWords };
+// Words in host memory that the GPU can write: errors, read without a copy once the stream has
+// been waited for, and counts that a call copies to the host (a copy to pageable memory
+// waits for its stream inside the driver, where other threads' calls then wait too).
+// NULL when they cannot be had.
+enum { kErrSort = 0, kErrTriangles, kVisits, kRemoved, kHostWords };
 static std::atomic<unsigned*> g_errors{nullptr};
-static volatile unsigned* host_error(int which) {
+static volatile unsigned* host_word(int which) {
     static unsigned* const words = [] {
         void* p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(unsigned) * kErrWords, cudaHostAllocMapped) != cudaSuccess) {
+        if (cudaHostAlloc(&p, sizeof(unsigned) * kHostWords, cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
             return (unsigned*)nullptr;
         }
-        for (int k = 0; k < kErrWords; ++k) ((unsigned*)p)[k] = 0u;
+        for (int k = 0; k < kHostWords; ++k) ((unsigned*)p)[k] = 0u;
         g_errors.store((unsigned*)p);
         return (unsigned*)p;
     }();
@@ -1326,11 +1330,11 @@ static bool triangles_failed() {
 CCTStatusType SortUsingThrust(Integer MaxParticleNum, Integer* daNumberHash, Integer* daNumberIndex) {
     const int n = MaxParticleNum;
     if (n <= 1) return CCT_NOERR;
-    const ScratchTurn turn;
+    const ScratchTurn turn(ScratchTurn::kSort);
     cudaStream_t st = 0;
     void* scr = scratch_get(1, radix_scratch_bytes(n));
     if (!scr) return CCT_MEMERR;
-    volatile unsigned* const err = host_error(kErrSort);
+    volatile unsigned* const err = host_word(kErrSort);
     if (!err) return CCT_MEMERR;
     MPS_CUDA_TRY(radix_sort_pairs(n, daNumberHash, daNumberIndex, -1, scr, (unsigned*)err, 1u, st));
     // thrust::sort_by_key with the default policy returns after the sort completed;
@@ -1351,19 +1355,20 @@ CCTStatusType StableSortUsingThrust(Integer MaxParticleNum, Integer* daNumberHas
 CCTStatusType CheckParticleOutsideComputeZone(cudaStream_t& Stream, Integer* ParticleNum) {
     const int n = *ParticleNum;
     if (n <= 0) return CCT_NOERR;
-    const ScratchTurn turn(Stream);
+    const ScratchTurn turn(ScratchTurn::kOutside, Stream);
     unsigned* flag = (unsigned*)scratch_get(2, sizeof(unsigned) * ((size_t)n + 4));
     unsigned* rank = (unsigned*)scratch_get(3, sizeof(unsigned) * ((size_t)n + 4));
-    if (!flag || !rank) return CCT_MEMERR;
+    volatile unsigned* const gone = host_word(kRemoved);
+    if (!flag || !rank || !gone) return CCT_MEMERR;
     int* removed = (int*)(rank + n);
     MPS_CUDA_TRY(cudaMemsetAsync(removed, 0, sizeof(int), Stream));
     MPS_COUNT_LAUNCH k_ref_outside_flags<<<grid_of(n), kBlock, 0, Stream>>>(n, g_bind, flag);
     MPS_CUDA_TRY(cudaMemcpyAsync(rank, flag, sizeof(unsigned) * (size_t)n, cudaMemcpyDeviceToDevice, Stream));
-    MPS_CUDA_TRY(scan_exclusive(rank, n, nullptr, Stream, scan_sums()));
+    MPS_CUDA_TRY(scan_exclusive(rank, n, nullptr, Stream, scan_sums(9)));
     MPS_COUNT_LAUNCH k_ref_compact<<<grid_of(n), kBlock, 0, Stream>>>(n, g_bind, flag, rank, removed);
-    int r = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&r, removed, sizeof(int), cudaMemcpyDeviceToHost, Stream));
+    MPS_CUDA_TRY(cudaMemcpyAsync((void*)gone, removed, sizeof(int), cudaMemcpyDeviceToHost, Stream));
     MPS_CUDA_TRY(cudaStreamSynchronize(Stream));
+    const int r = (int)*gone;
     *ParticleNum = n - r;
     g_bind.particle_num = n - r;
     return launch_status();
@@ -1379,21 +1384,22 @@ CCTStatusType RegisterTriangleTopology(cudaStream_t& Stream, CTriangle* daTriang
                                        Integer CellNum) {
     const int t = TriangleNum;
     if (t <= 0 || CellNum <= 0) return CCT_NOERR;
-    const ScratchTurn turn(Stream);
+    const ScratchTurn turn(ScratchTurn::kTriangles, Stream);
     unsigned* off = (unsigned*)scratch_get(4, sizeof(unsigned) * ((size_t)t + 4));
     if (!off) return CCT_MEMERR;
     unsigned *const total_dev = off + t, *const failed = off + t + 1;
-    volatile unsigned* const report = host_error(kErrTriangles);
+    volatile unsigned* const report = host_word(kErrTriangles);
     if (!report) return CCT_MEMERR;
     const bool few = t < kTriFew;
     if (few)
         MPS_COUNT_LAUNCH k_tri_count<32><<<div_up(t, kBlock / 32), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, failed);
     else
         MPS_COUNT_LAUNCH k_tri_count<8><<<div_up(t, kBlock / 8), kBlock, 0, Stream>>>(t, daTriangle, g_bind.box, CellNum, off, failed);
-    MPS_CUDA_TRY(scan_exclusive(off, t, total_dev, Stream, scan_sums()));
-    unsigned nv = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&nv, total_dev, sizeof(unsigned), cudaMemcpyDeviceToHost, Stream));
+    MPS_CUDA_TRY(scan_exclusive(off, t, total_dev, Stream, scan_sums(8)));
+    volatile unsigned* const visits = host_word(kVisits);
+    MPS_CUDA_TRY(cudaMemcpyAsync((void*)visits, total_dev, sizeof(unsigned), cudaMemcpyDeviceToHost, Stream));
     MPS_CUDA_TRY(cudaStreamSynchronize(Stream));
+    const unsigned nv = *visits;
     if (triangles_failed()) {   // in an earlier call: said once here, in the wall launchers until then
         *report = 0u;
         return CCT_CUDAERR;

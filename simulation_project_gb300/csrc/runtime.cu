@@ -18,8 +18,11 @@ struct Slot {
 };
 constexpr int kSlots = 16;
 Slot g_slots[kSlots];
-std::mutex g_turn;
-cudaEvent_t g_turn_done = nullptr;   // end of the last turn's work on its stream
+struct Turn {
+    std::mutex lock;
+    cudaEvent_t done = nullptr;   // end of the last turn's work on its stream
+};
+Turn g_turns[ScratchTurn::kUsers];
 thread_local char g_err[256] = "no error";
 
 CCTStatusType rec(cudaError_t e) {
@@ -57,27 +60,29 @@ void* scratch_get(int slot, size_t bytes) {
     return s.ptr;
 }
 
-ScratchTurn::ScratchTurn() { g_turn.lock(); }
-ScratchTurn::ScratchTurn(cudaStream_t st) : st_(st), on_stream_(true) {
-    g_turn.lock();
+ScratchTurn::ScratchTurn(User user) : user_(user) { g_turns[user].lock.lock(); }
+ScratchTurn::ScratchTurn(User user, cudaStream_t st) : user_(user), st_(st), on_stream_(true) {
+    Turn& t = g_turns[user];
+    t.lock.lock();
     // an event that cannot be had or waited for costs a host wait, and its error is not the call's
-    if (!g_turn_done) {
-        if (cudaEventCreateWithFlags(&g_turn_done, cudaEventDisableTiming) == cudaSuccess) return;
-        g_turn_done = nullptr;
+    if (!t.done) {
+        if (cudaEventCreateWithFlags(&t.done, cudaEventDisableTiming) == cudaSuccess) return;
+        t.done = nullptr;
         cudaGetLastError();
-    } else if (cudaStreamWaitEvent(st, g_turn_done, 0) != cudaSuccess) {
+    } else if (cudaStreamWaitEvent(st, t.done, 0) != cudaSuccess) {
         cudaGetLastError();
-        cudaEventSynchronize(g_turn_done);
+        cudaEventSynchronize(t.done);
     }
 }
 ScratchTurn::~ScratchTurn() {
+    Turn& t = g_turns[user_];
     // without an event (none could be created, or it is another device's) the turn ends when
     // its work does
-    if (on_stream_ && (!g_turn_done || cudaEventRecord(g_turn_done, st_) != cudaSuccess)) {
-        if (g_turn_done) cudaGetLastError();
+    if (on_stream_ && (!t.done || cudaEventRecord(t.done, st_) != cudaSuccess)) {
+        if (t.done) cudaGetLastError();
         cudaStreamSynchronize(st_);
     }
-    g_turn.unlock();
+    t.lock.unlock();
 }
 
 void scratch_release_all() {
