@@ -311,7 +311,8 @@ CCTStatusType CalculatePressureNJPCG(MpsSolver* s, MpsStepStats* stats);
  * (stats, may be NULL, has the details). */
 CCTStatusType CalcPoisson(void* Stream, MpsSolver* s, Integer ParticleNum, Scalar* dA, Scalar* dB, Scalar* dX,
                           const Scalar* dX0, MpsStepStats* stats);
-/* switches between MPS_PREC_FP64 and MPS_PREC_FP32_IR for the following steps */
+/* switches between MPS_PREC_FP64 and MPS_PREC_FP32_IR for the following steps (a solver's
+ * first use of FP64 allocates 12 bytes per row entry: CCT_MEMERR, the precision as it was) */
 CCTStatusType mps_set_precision(MpsSolver* s, int precision);
 
 typedef struct MpsLearnedInfo {

@@ -117,6 +117,7 @@ struct Dev {
     double* dragv;
     // neighbour rows: the FP32 list pass writes SELL-32 (nbr, nbrw, nbr16, w16); the FP64 one
     // writes each row contiguously (row i at i*K: rnbr, rw), k_rows_sell transposes the interior ones
+    // (NULL until a solver's first use of FP64)
     int* rnbr;
     void* rw;
     int* nbr;                  // SELL-32 32-bit columns: slices with sbase = -1, or every slice when rows_c32

@@ -159,6 +159,13 @@ struct Solver {
     }
 
     bool fp64() const { return opt.precision == MPS_PREC_FP64; }
+    // the rows that the FP64 list pass writes before their transpose: 12 bytes x K a particle,
+    // 4 GB at 882,080, allocated with the first use of that precision
+    cudaError_t row_major_rows() {
+        const size_t count = ((size_t)nmax + 31) / 32 * 32 * d.K;
+        cudaError_t e = d.rnbr ? cudaSuccess : mk(&d.rnbr, count);
+        return e || d.rw ? e : mk((double**)&d.rw, count);
+    }
 
     // ---- gate of the learned initial guess (MpsSolverOptions::learned_gate) ----
     // events on the solver stream: [0] rows ready (the warm start, the first refinement
@@ -293,7 +300,7 @@ struct Solver {
         e = e ? e : mk(&d.dragv, 3 * N);
         e = e ? e : mk(&d.tcs, 4 * (size_t)d.cells);   // list bounds of the 2 cells keys (walls, drag)
         const size_t N32 = (N + 31) / 32 * 32;
-        e = e ? e : mk(&d.rnbr, N32 * d.K); e = e ? e : mk((char**)&d.rw, N32 * d.K * wsz);
+        if (fp64()) e = e ? e : row_major_rows();
         e = e ? e : mk(&d.nbr, N32 * d.K); e = e ? e : mk((char**)&d.nbrw, N32 * d.K * wsz);
         e = e ? e : mk(&d.nbr16, N32 * d.K); e = e ? e : mk(&d.sbase, N32 / 32 + 1);
         e = e ? e : mk(&d.skmax, N32 / 32 + 1);
@@ -2240,6 +2247,13 @@ CCTStatusType CalcPoisson(void* Stream, MpsSolver* s, Integer ParticleNum, Scala
 
 CCTStatusType mps_set_precision(MpsSolver* s, int precision) {
     if (!s || (precision != MPS_PREC_FP64 && precision != MPS_PREC_FP32_IR)) return CCT_PARAMERR;
+    if (precision == MPS_PREC_FP64) {
+        if (const cudaError_t e = s->s.row_major_rows()) {
+            cudaGetLastError();
+            mps::note_error("mps_set_precision: rows of the FP64 solver", e);
+            return CCT_MEMERR;
+        }
+    }
     s->s.opt.precision = precision;
     return CCT_NOERR;
 }
