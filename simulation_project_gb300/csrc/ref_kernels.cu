@@ -450,7 +450,7 @@ __global__ void k_tri_reset_wall(int t, int step, const CTriangle* __restrict__ 
 // entries while most meet none, and a thread per particle ran them one after another, each
 // with three FP64 divisions: 535 us for 108,186 particles and 9,216 triangles, DRAM idle.
 // A warp for four: 184 us (drag 548 -> 179); 882,080 particles 478 -> 367 (376 -> 314).  Where
-// most particles see few triangles a lane per particle goes first (near_short_first).
+// most particles see few triangles a lane per particle goes first (near_short_most).
 constexpr int kNearT = 4;
 template <bool DRAG>
 __device__ __forceinline__ void ref_nearest(const RefBind& b, const Scalar3& p, bool live, CDistance& nd, int& nid) {
@@ -542,11 +542,11 @@ __device__ __forceinline__ void ref_nearest(const RefBind& b, const Scalar3& p, 
     if (nid != -1) nd.Magnitude = ref_tri_distance(ref_tri(b.triangles[nid]), p, nd.Direction);
 }
 
-// A lane per particle: the serial loop itself where its lists hold at most kNearShort entries in
+// A lane per particle: the serial loop itself where its lists hold at most `most` entries in
 // all (false: more, nothing done).  The 27 lengths are loaded nine at a time.
-constexpr unsigned kNearShort = 32;
 template <bool DRAG>
-__device__ __forceinline__ bool ref_nearest_short(const RefBind& b, const Scalar3& p, bool live, CDistance& nd, int& nid) {
+__device__ __forceinline__ bool ref_nearest_short(const RefBind& b, const Scalar3& p, bool live, unsigned most, CDistance& nd,
+                                                  int& nid) {
     nd.Magnitude = 1e8f;
     nd.Direction = s3(0, 0, 0);
     nid = -1;
@@ -565,14 +565,18 @@ __device__ __forceinline__ bool ref_nearest_short(const RefBind& b, const Scalar
         held += len;
         if (len) some |= 1u << c;
     }
-    if (held > kNearShort) return false;
+    if (held > most) return false;
+    int met0 = -1, met1 = -1;   // triangles met last: one met before is never the nearer one
     while (some) {
         const CCell& cell = b.cells[key(__ffs(some) - 1)];
         some &= some - 1u;
         const int len = (int)min(cell.m_TriangleNum, (unsigned)CELLMAXTRIANGLENUM);
         for (int l = 0; l < len; ++l) {
             const int t = cell.m_TriangleID[l];
-            if (t < 0 || t >= b.triangle_num || (DRAG && !b.tri_params[b.triangles[t].ModelIDNumber].isDrag)) continue;
+            if (t < 0 || t >= b.triangle_num || t == nid || t == met0 || t == met1) continue;
+            met1 = met0;
+            met0 = t;
+            if (DRAG && !b.tri_params[b.triangles[t].ModelIDNumber].isDrag) continue;
             Scalar3 dir;
             const float d = ref_tri_distance(ref_tri(b.triangles[t]), p, dir);
             if (d < nd.Magnitude) {
@@ -586,23 +590,34 @@ __device__ __forceinline__ bool ref_nearest_short(const RefBind& b, const Scalar
 }
 constexpr int kNearLeft = -2;   // mark of the particles that the lane per particle leaves
 
-// particles of a CTA of four warps, kNearT to a warp at a time
-template <bool LEFT>
-constexpr int near_particles() { return LEFT ? 32 : 4 * kNearT; }
+// The two launches of a call of which the first does the short lists: the second one may start
+// when every CTA of the first has (programmatic dependent launch) and waits for what they wrote.
+__device__ __forceinline__ void near_next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void near_wait_for_marks() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// particles of a CTA of four warps: kNearT to a warp, or LEFT marks (a multiple of 32) of which
+// the warps share those that are set
+template <int LEFT>
+constexpr int near_particles() { return LEFT ? LEFT : 4 * kNearT; }
 // work(id, mine): a warp's kNearT particles, one in each of its first lanes; LEFT: those with
 // the mark alone (mark[id] == kNearLeft)
-template <bool LEFT, class Work>
+template <int LEFT, class Work>
 __device__ __forceinline__ void near_groups(int n, const int* mark, Work&& work) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = blockIdx.x * near_particles<LEFT>();
     if constexpr (!LEFT) {
         const int id = first + warp * kNearT + lane;
         work(id, lane < kNearT && id < n);
     } else {
-        __shared__ int list[32];
-        const bool on = first + lane < n && mark[first + lane] == kNearLeft;
-        const unsigned found = __ballot_sync(~0u, on);   // the same in every warp
-        const int count = __popc(found);
-        if (on && warp == 0) list[__popc(found & ((1u << lane) - 1u))] = first + lane;
+        __shared__ int list[LEFT];
+        near_wait_for_marks();
+        int count = 0;
+#pragma unroll
+        for (int k = 0; k < LEFT / 32; ++k) {   // the same in every warp
+            const int id = first + 32 * k + lane;
+            const bool on = id < n && mark[id] == kNearLeft;
+            const unsigned found = __ballot_sync(~0u, on);
+            if (on && warp == k) list[count + __popc(found & ((1u << lane) - 1u))] = id;
+            count += __popc(found);
+        }
         if (count == 0) return;
         __syncthreads();
         for (int g = warp * kNearT; g < count; g += 4 * kNearT) {
@@ -614,7 +629,7 @@ __device__ __forceinline__ void near_groups(int n, const int* mark, Work&& work)
 
 // CalcSTLDistance_Kernel (DeviceProcess_Kernel.h:853-919): a warp for kNearT particles, those
 // that k_ref_stl_short has left, or all
-template <bool LEFT>
+template <int LEFT>
 __global__ void __launch_bounds__(128, 8) k_ref_stl_distance(int n, const __grid_constant__ RefBind b) {
     near_groups<LEFT>(n, b.stl_id, [&](int id, bool mine) {
         CDistance nd;
@@ -625,12 +640,13 @@ __global__ void __launch_bounds__(128, 8) k_ref_stl_distance(int n, const __grid
         b.stl_id[id] = nid;
     });
 }
-__global__ void __launch_bounds__(128) k_ref_stl_short(int n, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(128) k_ref_stl_short(int n, unsigned most, const __grid_constant__ RefBind b) {
+    near_next_may_start();
     const int id = blockIdx.x * 128 + threadIdx.x;
     if (id >= n) return;
     CDistance nd;
     int nid;
-    if (ref_nearest_short<false>(b, b.pos[id], true, nd, nid)) b.stl_distance[id] = nd;
+    if (ref_nearest_short<false>(b, b.pos[id], true, most, nd, nid)) b.stl_distance[id] = nd;
     else nid = kNearLeft;
     b.stl_id[id] = nid;
 }
@@ -685,7 +701,7 @@ __device__ __forceinline__ void ref_drag_finish(const RefBind& b, int id, bool g
     }
 }
 // as k_ref_stl_distance and k_ref_stl_short
-template <bool LEFT>
+template <int LEFT>
 __global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constant__ RefBind b) {
     near_groups<LEFT>(n, b.out_type, [&](int id, bool mine) {
         const bool gone = mine && b.out_id[id] < -1;
@@ -695,13 +711,14 @@ __global__ void __launch_bounds__(128, 8) k_ref_drag(int n, const __grid_constan
         if (mine) ref_drag_finish(b, id, gone, nd, nid);
     });
 }
-__global__ void __launch_bounds__(128) k_ref_drag_short(int n, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(128) k_ref_drag_short(int n, unsigned most, const __grid_constant__ RefBind b) {
+    near_next_may_start();
     const int id = blockIdx.x * 128 + threadIdx.x;
     if (id >= n) return;
     const bool gone = b.out_id[id] < -1;
     CDistance nd;
     int nid;
-    if (ref_nearest_short<true>(b, b.pos[id], !gone, nd, nid)) ref_drag_finish(b, id, gone, nd, nid);
+    if (ref_nearest_short<true>(b, b.pos[id], !gone, most, nd, nid)) ref_drag_finish(b, id, gone, nd, nid);
     else b.out_type[id] = kNearLeft;
 }
 
@@ -1169,13 +1186,35 @@ cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
 constexpr int kTriFew = 2048;
 // Wall distance and drag: most particles of a large set see few triangles or none, and a warp
 // per four of them is then most of the time.  With 64,000 particles and 100 for every
-// triangle a lane per particle does the short lists first.  us, a thread per particle (its
-// divisions in FP64) / a warp per four / both in turn: no triangles near 882,000 particles 44 / 101 /
-// 38, 110,000 15 / 17 / 12, 16,000 14 / 7 / 10; 12 triangles around 1,024,000 65 / 175 / 74, around
-// 250,000 42 / 58 / 48; 4,096 around 882,080 177 / 196 / 169 (drag, none of them: 58 / 118 / 67);
-// the line: 9,216 with drag spheres among 882,080 (96 to one) 539 / 347 / 350, 4,176 among 513,279
-// (123 to one) 211 / 136 / 135, among 318,675 (76 to one) 240 / 108 / 125.
-bool near_short_first(int n) { return n >= 64000 && n / 100 >= g_bind.triangle_num; }
+// triangle a lane per particle does the short lists first.  us, wall distance then drag, a
+// thread per particle (its divisions in FP64) / a warp per four / both in turn: no triangles near
+// 882,000 particles 44 / 101 / 29, 110,000 14 / 17 / 8, 16,000 14 / 7 / 10; the line: 9,216 with drag
+// spheres among 882,080 (96 to one) 539 / 347 / 350, 4,176 among 513,279 (123 to one) 211 / 136 / 130,
+// among 318,675 (76 to one) 240 / 108 / 125.
+// Up to how many entries, and how many of the others' marks a CTA of the second launch looks at:
+// 32 and 32, or 64 and 64 with 200 particles for every triangle, whose lists repeat the few
+// triangles around and leave fewer particles (us, thread per particle / 32 / 64): 12 triangles
+// around 65,536 38.0, 14.5 / 36.6, 16.5 / 24.7, 12.6, around 1,000,000 88.8, 50.6 / 84.7, 57.6 /
+// 63.5, 45.3; 4,096 around 882,080 (215 to one) 176.5, 57.4 / 159.9, 65.6 / 147.8, 52.5; the 123 to
+// one above 211, 158 / 130, 90 / 194, 144; 9,216 among 1,117,134 (121 to one) 613, 548 / 374, 326 /
+// 425, 376.
+int near_short_most(int n) {   // 0: no short lists first
+    if (n < 64000 || n / 100 < g_bind.triangle_num) return 0;
+    return n / 200 < g_bind.triangle_num ? 32 : 64;
+}
+template <class Left>
+cudaError_t near_left_launch(cudaStream_t st, int n, int marks, Left left) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)div_up(n, marks));
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return MPS_COUNT_LAUNCH cudaLaunchKernelEx(&cfg, left, n, (const RefBind)g_bind);
+}
 constexpr int kRefFew = 20000, kRefFewTurbulence = 100000;
 // From here on the predictor, whose radius is the cell size (250 of 1,728 candidates
 // accepted), runs a lane per target whatever the density (us, eight targets per warp / a lane
@@ -1446,11 +1485,11 @@ CCTStatusType CalcSTLDistance(cudaStream_t& Stream, Integer ComputeParticleNum) 
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (triangles_failed()) return CCT_CUDAERR;
     const int n = ComputeParticleNum;
-    if (near_short_first(n)) {
-        MPS_COUNT_LAUNCH k_ref_stl_short<<<div_up(n, 128), 128, 0, Stream>>>(n, g_bind);
-        MPS_COUNT_LAUNCH k_ref_stl_distance<true><<<div_up(n, near_particles<true>()), 128, 0, Stream>>>(n, g_bind);
+    if (const int most = near_short_most(n)) {
+        MPS_COUNT_LAUNCH k_ref_stl_short<<<div_up(n, 128), 128, 0, Stream>>>(n, (unsigned)most, g_bind);
+        MPS_CUDA_TRY(near_left_launch(Stream, n, most, most == 32 ? k_ref_stl_distance<32> : k_ref_stl_distance<64>));
     } else {
-        MPS_COUNT_LAUNCH k_ref_stl_distance<false><<<div_up(n, near_particles<false>()), 128, 0, Stream>>>(n, g_bind);
+        MPS_COUNT_LAUNCH k_ref_stl_distance<0><<<div_up(n, near_particles<0>()), 128, 0, Stream>>>(n, g_bind);
     }
     return launch_status();
 }
@@ -1459,11 +1498,11 @@ CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
     if (ComputeParticleNum <= 0) return CCT_NOERR;
     if (triangles_failed()) return CCT_CUDAERR;
     const int n = ComputeParticleNum;
-    if (near_short_first(n)) {
-        MPS_COUNT_LAUNCH k_ref_drag_short<<<div_up(n, 128), 128, 0, Stream>>>(n, g_bind);
-        MPS_COUNT_LAUNCH k_ref_drag<true><<<div_up(n, near_particles<true>()), 128, 0, Stream>>>(n, g_bind);
+    if (const int most = near_short_most(n)) {
+        MPS_COUNT_LAUNCH k_ref_drag_short<<<div_up(n, 128), 128, 0, Stream>>>(n, (unsigned)most, g_bind);
+        MPS_CUDA_TRY(near_left_launch(Stream, n, most, most == 32 ? k_ref_drag<32> : k_ref_drag<64>));
     } else {
-        MPS_COUNT_LAUNCH k_ref_drag<false><<<div_up(n, near_particles<false>()), 128, 0, Stream>>>(n, g_bind);
+        MPS_COUNT_LAUNCH k_ref_drag<0><<<div_up(n, near_particles<0>()), 128, 0, Stream>>>(n, g_bind);
     }
     return launch_status();
 }

@@ -47,6 +47,15 @@ def test_list_lengths(tris):
     assert (st.stl_id >= 0).any() and (st.stl_id < 0).any()
 
 
+# 200 particles for every triangle, and one fewer: lists of up to 64 and of up to 32 entries
+@pytest.mark.parametrize("n", [64000, 64199, 64257])
+@pytest.mark.parametrize("more", [0, 1])
+def test_the_longer_short_lists(n, more):
+    t = np.concatenate([_spheres(4, 0.05, 1, 0.1), np.asarray(_spheres(1, 0.05, 0, 0.1))])[:n // 200 + more]
+    st = _check(_state(t, n_side=41, n=n))
+    assert (st.stl_id >= 0).any() and (st.stl_id < 0).any()
+
+
 def test_no_triangles_near():
     _check(_state(np.asarray(_spheres(2, 0.02, 0, 0.1)) + 0.8, n_side=41))
 
