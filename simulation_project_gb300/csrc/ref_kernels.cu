@@ -1022,33 +1022,48 @@ struct RefOp<RpGradient> {
 __device__ __forceinline__ void ref_beside_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void ref_beside_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// one operator over targets 0 .. n-1, T per warp
+// One operator over targets 0 .. n-1, T per warp; with four, a warp takes `per` groups one after
+// another, its CTA's next to each other (rp_per)
 template <class Op, int T>
-__global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::NS > 3 ? 5 : 7) k_ref_pairs(int n, float coef, float minus_zero, int sparse, const __grid_constant__ RefBind b) {
+__global__ void __launch_bounds__(kRpWarps * 32, T == 2 ? 6 : Op::NX > 0 || Op::NS > 3 ? 5 : 7) k_ref_pairs(int n, float coef, float minus_zero, int sparse, int per,
+                                                               const __grid_constant__ RefBind b) {
     using W = RpWarp<Op, T>;
     __shared__ __align__(16) float sm[kRpWarps * W::kFloats];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = (blockIdx.x * kRpWarps + warp) * T;
     ref_beside_start();
-    if ((sparse > 0 && rp_sparse(b, n, sparse)) || first >= n) return;
-    const int id = first + lane;
-    RpTarget t{};
-    int cx = 0, cy = 0, cz = 0;
-    bool walk = false, fin = false;
-    if (lane < T && id < n) {
-        t.pos = b.pos[id];
-        fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
-    }
-    W w(b, sm + warp * W::kFloats, RefOp<Op>::radius(b.param), minus_zero, first, t);
-    w.run(b, walk && fin, cx, cy, cz);
-    float sum[Op::NS], rare[W::NXR];
+    if (sparse > 0 && rp_sparse(b, n, sparse)) return;
+    auto group = [&](int first) {
+        const int id = first + lane;
+        RpTarget t{};
+        int cx = 0, cy = 0, cz = 0;
+        bool walk = false, fin = false;
+        if (lane < T && id < n) {
+            t.pos = b.pos[id];
+            fin = RefOp<Op>::begin(b, id, t, cx, cy, cz, walk);
+        }
+        W w(b, sm + warp * W::kFloats, RefOp<Op>::radius(b.param), minus_zero, first, t);
+        w.run(b, walk && fin, cx, cy, cz);
+        float sum[Op::NS], rare[W::NXR];
 #pragma unroll
-    for (int c = 0; c < Op::NS; ++c) sum[c] = w.sum(c);
-    if constexpr (Op::NX > 0) {
+        for (int c = 0; c < Op::NS; ++c) sum[c] = w.sum(c);
+        if constexpr (Op::NX > 0) {
 #pragma unroll
-        for (int c = 0; c < Op::NX; ++c) rare[c] = w.rare_sum(c);
+            for (int c = 0; c < Op::NX; ++c) rare[c] = w.rare_sum(c);
+        }
+        if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
+    };
+    if constexpr (T == 4) {
+#pragma unroll 1
+        for (int r = 0; r < per; ++r) {
+            const int first = ((blockIdx.x * per + r) * kRpWarps + warp) * T;
+            if (first >= n) return;
+            group(first);
+            __syncwarp();
+        }
+    } else {
+        const int first = (blockIdx.x * kRpWarps + warp) * T;
+        if (first < n) group(first);
     }
-    if (fin) RefOp<Op>::finish(b, id, t, sum, rare, coef);
 }
 
 // a lane per target
@@ -1073,6 +1088,8 @@ __global__ void __launch_bounds__(128) k_ref_walk(int n, float coef, const __gri
 template <class Op>
 __global__ void __launch_bounds__(128) k_ref_walk_sparse(int n, float coef, int sparse, const __grid_constant__ RefBind b) {
     __shared__ int2 run[9][128];
+    // one share: as a condition instead of a loop the same work took 890 us instead of 792
+    // (pressure, 882,000 particles, 40 % of them in dense fluid)
     if (rp_sparse(b, n, sparse))
         for (int id = blockIdx.x * 128 + threadIdx.x; id < n; id += gridDim.x * 128)
             ref_walk<Op>(b, id, coef, &run[0][threadIdx.x]);
@@ -1120,17 +1137,17 @@ constexpr int kRefSlices = 40000;
 // From here on a call asks first whether the fluid is sparse and leaves it to k_ref_walk if so.
 // The kernels that share candidates between targets have little to share there, and a warp
 // per few targets is 8 to 32 times fewer targets at a time (us, without and with k_ref_walk,
-// 0.03 particles per cube of the particle distance): pressure 1,262 / 175 at 882,000
-// particles, 198 / 33 at 50,000, 50 / 30 at 19,000, 38 / 32 at 10,000; turbulence 2,353 / 296 at
+// 0.03 particles per cube of the particle distance): pressure 1,262 / 173 at 882,000
+// particles, 198 / 33 at 50,000, 50 / 30 at 19,000, 38 / 32 at 10,000; turbulence 2,353 / 245 at
 // 882,000, predictor 311 / 69 at 110,000.  In dense fluid the question and the second launch
 // cost 1 to 4 % (pressure 77.7 / 79.5 at 103,823, gradient 151 / 153, turbulence 2,215 / 2,269 at
 // 884,736); at 15,625 they would cost 8 % of the pressure.
 constexpr int kRefSplit = 16384;
 // Particles per cell below which k_ref_walk is the faster one.  Measured on random fluid of
 // 0.004 to 1 per cube of the distance (64 such cubes are a cell), us at the densities on both
-// sides of the line, kernel that shares / k_ref_walk: pressure (slices) 0.15: 581 / 410, 0.3:
-// 383 / 670 at 882,000; eight targets per warp 0.06: 65 / 42, 0.15: 48 / 71 at 30,000;
-// turbulence (four per warp) 0.5: 2,015 / 1,605, 1.0: 2,882 / 2,885 at 882,000; predictor 0.1:
+// sides of the line, kernel that shares / k_ref_walk: pressure (slices) 0.15: 581 / 386, 0.3:
+// 383 / 626 at 882,000; eight targets per warp 0.06: 65 / 42, 0.15: 48 / 71 at 30,000;
+// turbulence (four per warp) 0.5: 2,015 / 1,570, 1.0: 2,882 / 2,839 at 882,000; predictor 0.1:
 // 96 / 95 at 30,000 and 0.2: 257 / 210, 0.3: 280 / 282 at 110,000.
 template <class Op>
 int rp_few(int n, bool slices, bool pairs2) {
@@ -1140,11 +1157,21 @@ int rp_few(int n, bool slices, bool pairs2) {
     return std::is_same<Op, RpExplicitly>::value && n >= 64000 ? 16 : 10;
 }
 
-// beside the launch before it; one wave of CTAs, which mostly find that there is nothing to do
+// Four targets per warp are so many CTAs that starting them to find sparse fluid took a tenth of
+// the call: a CTA takes several groups while 40 CTAs per SM (eight rounds of five) are left.
+// us at 882,000 particles, one group / about twelve rounds / six / three: turbulence at 0.01 per
+// cube 201 / 158 / 153 / 151, at 1.0 2,906 / 2,896 / 2,932 / 3,012; at 300,000 76 / 67 / 62 / 60 and
+// 979 / 983 / 1,001 / 1,024.
+inline int rp_per(int groups) { return std::max(1, groups / (152 * 40)); }
+
+// Beside the launch before it.  With one wave of CTAs that take several shares each it left the
+// GPU idle at the end (us, a wave / a CTA per share at 882,000 particles: pressure at 0.15 per
+// cube 428 / 386, gradient with 40 % of the particles in dense fluid 1,411 / 1,252); in dense
+// fluid, where all it does is ask, the two are alike (558).
 template <class Op>
 cudaError_t ref_walk_beside(cudaStream_t st, int n, float coef, int sparse) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)std::min(div_up(n, 128), 152 * 16));
+    cfg.gridDim = dim3((unsigned)div_up(n, 128));
     cfg.blockDim = dim3(128);
     cfg.stream = st;
     cudaLaunchAttribute at = {};
@@ -1167,15 +1194,15 @@ cudaError_t ref_op_launch(cudaStream_t st, int n, int few, float coef = 0.0f) {
     int sparse = n < kRefSplit ? 0 : rp_few<Op>(n, kSlices && n >= kRefSlices, n < few);
     if ((long long)n >= (long long)sparse * g_bind.cell_num) sparse = 0;
     if (n < few) {
-        MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse, g_bind);
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, 2><<<div_up(n, kRpWarps * 2), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse, 1, g_bind);
     } else if (kSlices && n >= kRefSlices) {
         if constexpr (kSlices) {
             constexpr int W = rs_warps<Op>();
             MPS_COUNT_LAUNCH k_ref_slices<Op><<<div_up(n, W * 32), W * 32, 0, st>>>(n, -0.0f, sparse, g_bind);
         }
     } else {
-        MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(n, kRpWarps * kMany), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse,
-                                                                                                        g_bind);
+        const int groups = div_up(n, kRpWarps * kMany), per = kMany == 4 && sparse ? rp_per(groups) : 1;
+        MPS_COUNT_LAUNCH k_ref_pairs<Op, kMany><<<div_up(groups, per), kRpWarps * 32, 0, st>>>(n, coef, -0.0f, sparse, per, g_bind);
     }
     const cudaError_t e = cudaGetLastError();
     return e || sparse == 0 ? e : ref_walk_beside<Op>(st, n, coef, sparse);

@@ -50,6 +50,13 @@ def test_all_particles_far_outside():
     _compare(sc, setup, ops=SLICE_OPS)
 
 
+@pytest.mark.parametrize("n", [194_560, 291_853])
+@pytest.mark.parametrize("density", [0.03, 0.8])
+def test_turbulence_groups_in_turn(density, n):
+    """Two and three groups per warp, the last CTA with fewer; the walk beside it."""
+    _compare(_scene(_cloud(n, density, 6), 6), ops=[("CalcTurbulenceViscosity", ORC.calc_turbulence_viscosity)])
+
+
 @pytest.mark.parametrize("n", [215_999, 216_000, 216_001])
 def test_predictor_takeover(n):
     """Eight targets per warp, then a lane per target, in dense fluid."""
