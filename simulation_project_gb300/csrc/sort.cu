@@ -27,7 +27,11 @@
 // all (random keys 68: their scatter takes 14, 16,000 keys 21 to 26).  Two CTAs per SM took
 // 40 and 72; from 2.5 million keys on they are the faster (us, a call with one / two per SM:
 // 2,000,000 nearly sorted 92 / 97, random 226 / 223; 5,000,000 236 / 195 and 467 / 437; 30,000,000
-// 1,540 / 1,172 and 2,778 / 2,488).  It replaces three launches per 8-bit pass, 13 to 16 per sort with
+// 1,540 / 1,172 and 2,778 / 2,488).  There a tile's pairs are staged as well: a warp's 32 pairs of
+// random keys lay in as many runs, and memory saw a sector for each word, which from 5 million
+// keys on was slower than the separate launches of before (us, a call with those / without the
+// stage / with it: 3,178,892 random of 30 bits 381 / 356 / 271; 10,000,000 of 24 bits 766 / 932 / 598;
+// 30,000,000 of 30 bits 2,644 / 2,876 / 1,787, nearly sorted 1,054 / 1,172 / 1,002).  It replaces three launches per 8-bit pass, 13 to 16 per sort with
 // the range's and those of passes beyond the range, which returned at once; finding the
 // range alone took 27 us at 882,080 keys (19,456 atomics on one address).
 #include <limits.h>
@@ -44,6 +48,7 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortRounds = 12;                          // most rounds of 32 keys per warp and tile
 constexpr int kSortTile = kSortThreads * kSortRounds;    // most keys of a tile
 constexpr int kRadix = 1 << kRadixDigitBits;
+constexpr int kSortStage = kSortTile * 2 * (int)sizeof(int);
 static_assert(kRadix == kSortThreads, "a thread per digit");
 
 // Exclusive scan of len unsigned values, in place, by one CTA of 1024 threads.
@@ -177,12 +182,16 @@ struct SortScratch {
     int *keys, *vals;   // [n]
 };
 
-// bits: the keys lie in [0, 2^bits); < 0: any int range (found first)
+// bits: the keys lie in [0, 2^bits); < 0: any int range (found first).  STAGED: a tile's pairs go
+// through shared memory (kSortStage bytes) in the order of their digits, so that a warp writes
+// whole runs
+template <bool STAGED>
 __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* keys, int* vals, int bits, SortScratch s,
                                                        unsigned* err, unsigned bit) {
     __shared__ unsigned wcount[kSortWarps][kRadix];
     __shared__ unsigned off[kRadix];
     __shared__ unsigned wsum[32];
+    extern __shared__ int staged[];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const int c = blockIdx.x, ctas = gridDim.x;
@@ -303,11 +312,9 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
             else prefix(std::integral_constant<int, 2 * kHalf>());
             if (!coop_barrier(s.bar, err, bit)) return;
         }
-        // ---- first position of each digit's keys of this CTA ----
-        {
-            const unsigned total = ctas > 1 ? __ldcg(s.total + tid) : mine;
-            const unsigned before = ctas > 1 ? __ldcg(s.counts + (size_t)c * kRadix + tid) : 0u;
-            unsigned inc = total;
+        // exclusive sum of the threads' x (in the order of the digits)
+        auto below = [&](unsigned x) {
+            unsigned inc = x;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
@@ -316,17 +323,23 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
             if (lane == 31) wsum[w] = inc;
             __syncthreads();
             if (w == 0) {
-                const unsigned x = lane < kSortWarps ? wsum[lane] : 0u;
-                unsigned xi = x;
+                const unsigned y = lane < kSortWarps ? wsum[lane] : 0u;
+                unsigned yi = y;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned v = __shfl_up_sync(0xffffffffu, xi, o);
-                    if (lane >= o) xi += v;
+                    const unsigned v = __shfl_up_sync(0xffffffffu, yi, o);
+                    if (lane >= o) yi += v;
                 }
-                wsum[lane] = xi - x;
+                wsum[lane] = yi - y;
             }
             __syncthreads();
-            off[tid] = inc - total + wsum[w] + before;
+            return inc - x + wsum[w];
+        };
+        // ---- first position of each digit's keys of this CTA ----
+        {
+            const unsigned total = ctas > 1 ? __ldcg(s.total + tid) : mine;
+            const unsigned before = ctas > 1 ? __ldcg(s.counts + (size_t)c * kRadix + tid) : 0u;
+            off[tid] = below(total) + before;
         }
         // ---- scatter ----
         for (int t0 = beg; t0 < end; t0 += kSortTile) {
@@ -352,7 +365,47 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                 }
             }
             __syncthreads();
-            {
+            if constexpr (STAGED) {
+                int* const tkey = staged;
+                int* const tval = staged + kSortTile;
+                unsigned tile = 0;
+#pragma unroll
+                for (int q = 0; q < kSortWarps; ++q) tile += wcount[q][tid];
+                const unsigned first = below(tile);   // of the digit's pairs in the tile
+                unsigned run = first;
+#pragma unroll
+                for (int q = 0; q < kSortWarps; ++q) {
+                    const unsigned x = wcount[q][tid];
+                    wcount[q][tid] = run;
+                    run += x;
+                }
+                const unsigned next = off[tid] + tile;
+                off[tid] -= first;   // place in the tile -> position
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < kSortRounds; ++r) {
+                    if (r < rounds) {
+                        const unsigned d = at[r] & 1023u;
+                        if (d < (unsigned)kRadix) {
+                            const unsigned u = wcount[w][d] + (at[r] >> 10);
+                            tkey[u] = key[r];
+                            tval[u] = val[r];
+                        }
+                    }
+                }
+                __syncthreads();
+#pragma unroll 4
+                for (int u = tid; u < tend - t0; u += kSortThreads) {
+                    const int k = tkey[u];
+                    const unsigned dst = off[digit(k)] + (unsigned)u;
+                    if (dst < (unsigned)n) {   // not where another CTA gave up at a barrier
+                        kb[dst] = k;
+                        vb[dst] = tval[u];
+                    }
+                }
+                __syncthreads();
+                off[tid] = next;   // the next tile's first positions
+            } else {
                 unsigned run = off[tid];
 #pragma unroll
                 for (int q = 0; q < kSortWarps; ++q) {
@@ -361,22 +414,22 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(int n, int part, int* 
                     run += x;
                 }
                 off[tid] = run;   // the next tile's first positions
-            }
-            __syncthreads();
+                __syncthreads();
 #pragma unroll
-            for (int r = 0; r < kSortRounds; ++r) {
-                if (r < rounds) {
-                    const unsigned d = at[r] & 1023u;
-                    if (d < (unsigned)kRadix) {
-                        const unsigned dst = wcount[w][d] + (at[r] >> 10);
-                        if (dst < (unsigned)n) {   // not where another CTA gave up at a barrier
-                            kb[dst] = key[r];
-                            vb[dst] = val[r];
+                for (int r = 0; r < kSortRounds; ++r) {
+                    if (r < rounds) {
+                        const unsigned d = at[r] & 1023u;
+                        if (d < (unsigned)kRadix) {
+                            const unsigned dst = wcount[w][d] + (at[r] >> 10);
+                            if (dst < (unsigned)n) {   // not where another CTA gave up at a barrier
+                                kb[dst] = key[r];
+                                vb[dst] = val[r];
+                            }
                         }
                     }
                 }
+                __syncthreads();
             }
-            __syncthreads();
         }
         if (!coop_barrier(s.bar, err, bit)) return;
         int* t = ka; ka = kb; kb = t;
@@ -420,13 +473,16 @@ cudaError_t radix_sort_pairs(int n, int* keys, int* vals, int bits, void* scratc
         s.keys = (int*)(s.counts + (size_t)ctas * kRadix);
         s.vals = s.keys + n;
         if (ctas == 1) {
-            MPS_COUNT_LAUNCH k_sort<<<1, kSortThreads, 0, st>>>(n, part, keys, vals, bits, s, err, bit);
+            MPS_COUNT_LAUNCH k_sort<false><<<1, kSortThreads, 0, st>>>(n, part, keys, vals, bits, s, err, bit);
             return cudaGetLastError();
         }
         cudaError_t e = cudaMemsetAsync(s.bar, 0, sizeof(unsigned), st);
         if (e) return e;
         void* args[] = {(void*)&n, (void*)&part, (void*)&keys, (void*)&vals, (void*)&bits, (void*)&s, (void*)&err, (void*)&bit};
-        e = cudaLaunchCooperativeKernel((const void*)k_sort, dim3(ctas), dim3(kSortThreads), args, 0, st);
+        const bool staged = n >= kRadixTwoPerSm;
+        const void* const kernel = staged ? (const void*)k_sort<true> : (const void*)k_sort<false>;
+        if (staged && (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortStage))) return e;
+        e = cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kSortThreads), args, staged ? kSortStage : 0, st);
         if (e == cudaSuccess) MPS_COUNT_LAUNCH 0;
         if (!coop_refused(e)) return e;
         if (e == cudaErrorNotSupported) most = 2;   // one CTA next

@@ -3,6 +3,9 @@ several tiles per CTA, ragged ends, one to four passes, and keys in order, in re
 import numpy as np
 import pytest
 
+from simulation_project_gb300.lib import DeviceArray, call
+from simulation_project_gb300.types import MpsError
+from test_gpu_barrier_timeouts import no_polls
 from test_gpu_sort import _check
 
 pytestmark = pytest.mark.gpu
@@ -21,3 +24,12 @@ def test_ordered_and_equal_keys():
     _check(k[::-1].copy())
     _check(np.full(n, 5, np.int32))
     _check((k + np.random.default_rng(0).integers(-3, 4, n)).astype(np.int32))
+
+
+def test_a_sort_that_gives_up():
+    """Reported, and the next one is right."""
+    keys = np.random.default_rng(1).integers(0, 2 ** 24, 2_600_003).astype(np.int32)
+    dk, dv = DeviceArray.from_host(keys), DeviceArray.from_host(np.arange(len(keys), dtype=np.int32))
+    with no_polls(), pytest.raises(MpsError):
+        call("SortUsingThrust", len(keys), dk.ptr, dv.ptr)
+    _check(keys)
