@@ -1218,21 +1218,30 @@ constexpr int kTriFew = 2048;
 // 882,000 particles 44 / 101 / 29, 110,000 14 / 17 / 8, 16,000 14 / 7 / 10; the line: 9,216 with drag
 // spheres among 882,080 (96 to one) 539 / 347 / 350, 4,176 among 513,279 (123 to one) 211 / 136 / 130,
 // among 318,675 (76 to one) 240 / 108 / 125.
-// Up to how many entries, and how many of the others' marks a CTA of the second launch looks at:
-// 32 and 32, or 64 and 64 with 200 particles for every triangle, whose lists repeat the few
+// Up to how many entries, and how many of the others' marks a CTA of the second launch looks at
+// (near_marks): 32 and 32, or 64 and 64 with 200 particles for every triangle, whose lists repeat the few
 // triangles around and leave fewer particles (us, thread per particle / 32 / 64): 12 triangles
 // around 65,536 38.0, 14.5 / 36.6, 16.5 / 24.7, 12.6, around 1,000,000 88.8, 50.6 / 84.7, 57.6 /
 // 63.5, 45.3; 4,096 around 882,080 (215 to one) 176.5, 57.4 / 159.9, 65.6 / 147.8, 52.5; the 123 to
 // one above 211, 158 / 130, 90 / 194, 144; 9,216 among 1,117,134 (121 to one) 613, 548 / 374, 326 /
 // 425, 376.
+// From 600,000 particles on 50 for every triangle are enough: the lanes fill the GPU, so a list
+// costs what it holds and not its latency, from 2,000,000 on up to 128 entries (thread per particle /
+// warps / 32 / 128: a cylinder of 16,128 triangles around 882,080 327, 82 / 248, 123 / 231, 78 / 272,
+// 72; four cylinders and 512 spheres, 58,624, among 3,178,892 1,330, 780 / 1,425, 1,178 / 1,251, 999 /
+// 1,248, 794; 28,096 among 2,116,620 1,364, 1,293 / 1,131, 1,120 / 1,109, 1,114 / 1,190, 1,171; below
+// the line, 28,096 among 1,236,510 (44 to one), 1,335, 1,282 / 933, 928 / 985, 987 / 1,094, 1,075).
 int near_short_most(int n) {   // 0: no short lists first
-    if (n < 64000 || n / 100 < g_bind.triangle_num) return 0;
-    return n / 200 < g_bind.triangle_num ? 32 : 64;
+    const int t = g_bind.triangle_num;
+    if (n >= 600000 && n / 100 < t && n / 50 >= t) return n < 2000000 ? 32 : 128;
+    if (n < 64000 || n / 100 < t) return 0;
+    return n / 200 < t ? 32 : 64;
 }
+constexpr int near_marks(int most) { return most == 32 ? 32 : 64; }
 template <class Left>
-cudaError_t near_left_launch(cudaStream_t st, int n, int marks, Left left) {
+cudaError_t near_left_launch(cudaStream_t st, int n, int most, Left left) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)div_up(n, marks));
+    cfg.gridDim = dim3((unsigned)div_up(n, near_marks(most)));
     cfg.blockDim = dim3(128);
     cfg.stream = st;
     cudaLaunchAttribute at = {};
@@ -1514,7 +1523,7 @@ CCTStatusType CalcSTLDistance(cudaStream_t& Stream, Integer ComputeParticleNum) 
     const int n = ComputeParticleNum;
     if (const int most = near_short_most(n)) {
         MPS_COUNT_LAUNCH k_ref_stl_short<<<div_up(n, 128), 128, 0, Stream>>>(n, (unsigned)most, g_bind);
-        MPS_CUDA_TRY(near_left_launch(Stream, n, most, most == 32 ? k_ref_stl_distance<32> : k_ref_stl_distance<64>));
+        MPS_CUDA_TRY(near_left_launch(Stream, n, most, near_marks(most) == 32 ? k_ref_stl_distance<32> : k_ref_stl_distance<64>));
     } else {
         MPS_COUNT_LAUNCH k_ref_stl_distance<0><<<div_up(n, near_particles<0>()), 128, 0, Stream>>>(n, g_bind);
     }
@@ -1527,7 +1536,7 @@ CCTStatusType CalcDragEffect(cudaStream_t& Stream, Integer ComputeParticleNum) {
     const int n = ComputeParticleNum;
     if (const int most = near_short_most(n)) {
         MPS_COUNT_LAUNCH k_ref_drag_short<<<div_up(n, 128), 128, 0, Stream>>>(n, (unsigned)most, g_bind);
-        MPS_CUDA_TRY(near_left_launch(Stream, n, most, most == 32 ? k_ref_drag<32> : k_ref_drag<64>));
+        MPS_CUDA_TRY(near_left_launch(Stream, n, most, near_marks(most) == 32 ? k_ref_drag<32> : k_ref_drag<64>));
     } else {
         MPS_COUNT_LAUNCH k_ref_drag<0><<<div_up(n, near_particles<0>()), 128, 0, Stream>>>(n, g_bind);
     }

@@ -56,6 +56,13 @@ def test_the_longer_short_lists(n, more):
     assert (st.stl_id >= 0).any() and (st.stl_id < 0).any()
 
 
+# from 600,000 particles on 50 for every triangle are enough, from 2,000,000 on for longer lists
+@pytest.mark.parametrize("n,balls", [(599_999, 100), (600_000, 100), (600_033, 149), (600_033, 151), (2_000_021, 260)])
+def test_many_particles(n, balls):
+    st = _check(_state(_spheres(balls, 0.03, 1, 0.8), n_side=127 if n > 700_000 else 85, n=n))
+    assert (st.stl_id >= 0).any() and (st.stl_id < 0).any()
+
+
 def test_no_triangles_near():
     _check(_state(np.asarray(_spheres(2, 0.02, 0, 0.1)) + 0.8, n_side=41))
 
