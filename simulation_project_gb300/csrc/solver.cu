@@ -899,7 +899,10 @@ struct Solver {
     // / kTriWarps: drag 113 / 65, walls 34 / 22 at 108,186 particles, 141 / 76 and 31 / 32 at 256,000,
     // 86 / 110 and 36 / 85 at 882,080: there are warps enough and most CTAs find no triangles;
     // all wall work of a step with 64 drag bodies 205 / 186 at 255,976, 208 / 214 at 361,444, 192 / 241
-    // at 513,279; without drag 113 / 102 at 194,376, 103 / 105 at 255,976, 110 / 127 at 361,444)
+    // at 513,279; without drag 113 / 102 at 194,376, 103 / 105 at 255,976, 110 / 127 at 361,444).  For the walls with fewer than 200
+    // particles for every triangle alone: beside a few large ones lists are short (12 triangles, 44,688
+    // particles 35 / 44, 128,000 33 / 43, 250,000 31 / 54; 1,024 around 255,976 74 / 97, around
+    // 108,186 75 / 74, around 29,568 97 / 64); those of drag bodies are long wherever there are any
     static constexpr int kTriSplit = 300000;
     template <class T, int W>
     void launch_tri(bool drag) {
@@ -909,7 +912,7 @@ struct Solver {
     }
     template <class T>
     void launch_tri(bool drag) {
-        if (sizeof(T) == 4 && d.n < kTriSplit) launch_tri<T, sizeof(T) == 4 ? kTriWarps : 1>(drag);
+        if (sizeof(T) == 4 && d.n < kTriSplit && (drag || d.n / 200 < d.tri_n)) launch_tri<T, sizeof(T) == 4 ? kTriWarps : 1>(drag);
         else launch_tri<T, 1>(drag);
     }
     template <class T>

@@ -46,3 +46,9 @@ def test_wall_part_of_the_number_density(n, m):
     extent = np.abs(sc.pos).max() + L0
     tol = 2.1 / 0.16 * 16 * 2.0 ** -24 * extent / L0 + 64 * 2.0 ** -24 * b.max() + 2e-5
     assert np.abs(a - b).max() <= tol
+
+
+# 200 particles for every triangle, and fewer: a lane per particle, and eight warps for 32
+@pytest.mark.parametrize("n,m", [(3599, 3), (3600, 3), (3601, 3), (4000, 1)])
+def test_few_triangles(n, m):
+    test_wall_part_of_the_number_density(n, m)
